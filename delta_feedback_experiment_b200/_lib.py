@@ -1,8 +1,10 @@
-"""ctypes binding of ``libpkda_b200.so`` (declared in ``include/pkda_b200.h``).
+"""Loads ``libpkda_b200.so`` (declared in ``include/pkda_b200.h``) and ``_native.so``, the
+torch host layer every operator call goes through.
 
-The library is the product; this module only loads it, mirrors its argument
-structs and turns status codes into ``RuntimeError``.  There is no fallback: if
-the shared library is missing or does not load, every operator raises.
+The ctypes mirror of the C library's structs serves the calls that stay outside torch
+(the no-allocation entry point, switches, timing) and as a template for other hosts.
+Status codes become ``RuntimeError``.  There is no fallback: if a shared library is
+missing or does not load, every operator raises.
 """
 
 from __future__ import annotations
@@ -15,6 +17,7 @@ import torch
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libpkda_b200.so")
+NATIVE_PATH = os.path.join(HERE, "_native.so")
 
 PKDA_BF16, PKDA_F32 = 0, 1
 ABI_VERSION = 1
@@ -248,9 +251,31 @@ def load() -> C.CDLL:
     return lib
 
 
+_native = None
+
+
+def built() -> bool:
+    """Whether both shared libraries exist (nothing is loaded)."""
+    return os.path.exists(LIB_PATH) and os.path.exists(NATIVE_PATH)
+
+
+def native():
+    """The torch host layer (``csrc/pkda_torch.cpp``): launchers that take tensors, and the
+    ``delta_feedback`` operators, which its import registers.  ``RuntimeError`` if it is missing."""
+    global _native
+    if _native is None:
+        load()  # the C library first: the host layer resolves to this very instance
+        try:
+            from . import _native as module
+        except ImportError as exc:
+            raise RuntimeError(f"PKDA CUDA library unavailable: {exc}") from exc
+        _native = module
+    return _native
+
+
 def available() -> bool:
     try:
-        load()
+        native()
         return True
     except RuntimeError:
         return False

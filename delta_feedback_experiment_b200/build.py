@@ -1,9 +1,10 @@
-"""Builds ``libpkda_b200.so`` (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds ``libpkda_b200.so`` (the C-ABI library, nvcc for sm_100a) and ``_native.so`` (the
+torch host layer on top of it, g++) in-tree.
 
     python -m delta_feedback_experiment_b200.build [--force] [--verbose]
 
-nvcc cross-compiles without a GPU.  The library is rebuilt only when a source
-file is newer than the existing ``.so`` (or ``--force`` is given).
+nvcc cross-compiles without a GPU.  The libraries are rebuilt only when a source
+file is newer than an existing ``.so`` (or ``--force`` is given).
 """
 
 from __future__ import annotations
@@ -18,11 +19,13 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "libpkda_b200.so")
+NATIVE_PATH = os.path.join(HERE, "_native.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 SOURCES = ["pkda_abi.cu", "pkda_recurrent.cu", "pkda_chunk_fwd.cu", "pkda_chunk_bwd.cu",
            "pkda_static_scratch.cu", "pkda_intra_fwd_tc.cu", "pkda_intra_bwd_tc.cu", "pkda_out_tc.cu", "pkda_scan_tc.cu", "pkda_scan_bwd_tc.cu",
            "pkda_recurrent_bwd.cu", "pkda_qkv_conv.cu", "pkda_norm_gate.cu", "pkda_decode_step.cu", "pkda_controls.cu"]
+NATIVE_SOURCE = "pkda_torch.cpp"
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-ftz=true",
     "-Xcompiler", "-fPIC", "-Xptxas", "-v",
@@ -44,10 +47,37 @@ def _deps() -> list[str]:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not (os.path.exists(LIB_PATH) and os.path.exists(NATIVE_PATH)):
         return True
-    stamp = os.path.getmtime(LIB_PATH)
+    stamp = min(os.path.getmtime(LIB_PATH), os.path.getmtime(NATIVE_PATH))
     return any(os.path.getmtime(d) > stamp for d in _deps())
+
+
+def _compile_native() -> str:
+    """Object file of the torch host layer (headers and ABI of the running torch)."""
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    obj = os.path.join(OBJ_DIR, NATIVE_SOURCE.replace(".cpp", ".o"))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I", INCLUDE]
+    for inc in [*include_paths("cuda"), sysconfig.get_paths()["include"]]:
+        cmd += ["-isystem", inc]
+    res = subprocess.run([*cmd, "-c", os.path.join(CSRC, NATIVE_SOURCE), "-o", obj], capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on {NATIVE_SOURCE}:\n{res.stdout}\n{res.stderr}")
+    return obj
+
+
+def _link_native(obj: str) -> None:
+    from torch.utils.cpp_extension import library_paths
+    cmd = ["g++", "-shared", "-o", NATIVE_PATH, obj, LIB_PATH, "-Wl,-rpath,$ORIGIN"]
+    for path in library_paths("cuda"):
+        cmd += ["-L", path]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -64,15 +94,18 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError(f"nvcc failed on {src}:\n{res.stdout}\n{res.stderr}")
         return obj, res.stderr
 
-    with ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
+    with ThreadPoolExecutor(max_workers=len(SOURCES) + 1) as pool:
+        native = pool.submit(_compile_native)
         results = list(pool.map(compile_one, SOURCES))
     if verbose:
         for _, log in results:
             sys.stderr.write(log)
-    cmd = [nvcc, "-shared", "-o", LIB_PATH, *[o for o, _ in results], "-lcudart"]
+    native_obj = native.result()
+    cmd = [nvcc, "-shared", "-o", LIB_PATH, "-Xlinker", "-soname=libpkda_b200.so", *[o for o, _ in results], "-lcudart"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _link_native(native_obj)
     return LIB_PATH
 
 

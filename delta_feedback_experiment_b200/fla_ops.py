@@ -6,16 +6,15 @@ B200 kernels behind them instead of the Triton fork.
 * ``delta_feedback::pkda_recurrence`` (reference ``fla_ops.py:252-349``)
 * ``delta_feedback::pkda_recurrence_backward`` (``fla_ops.py:381-499``)
 
-Both have fake implementations (so ``torch.compile(fullgraph=True)`` keeps them
-in one graph) and an autograd registration.  Launches go to the current stream,
+Schema, CUDA kernel and autograd kernel of both are registered by the native host layer
+(``csrc/pkda_torch.cpp``); the fake implementations (so that ``torch.compile(fullgraph=True)``
+keeps them in one graph) stand here.  Launches go to the current stream,
 never synchronise and allocate only through torch, so they can be captured in
 CUDA graphs.  There is no fallback: without the CUDA library the operators
 raise ``RuntimeError``.
 """
 
 from __future__ import annotations
-
-from typing import Optional
 
 import torch
 from torch import Tensor
@@ -65,40 +64,36 @@ def _check_intermediates(tensors, q: Tensor, v: Tensor, lean: bool) -> None:
                                f"implementation promises {(tuple(shape), dtype, q.device, True)}")
 
 
-def _chunk_capable(q: Tensor) -> bool:
-    return q.dtype == torch.bfloat16 and q.shape[-1] == 128
+def _missing(*_args, **_kwargs):
+    raise RuntimeError("the PKDA libraries were not built when this package was imported "
+                       "(python -m delta_feedback_experiment_b200.build)")
 
 
-@torch.library.custom_op("delta_feedback::pkda_recurrence", mutates_args=(), device_types="cuda")
-def pkda_recurrence(
-    q: Tensor, k: Tensor, v: Tensor, g: Tensor, g_atk: Tensor, beta_atk: Tensor, beta: Tensor,
-    A_log: Tensor, dt_bias: Tensor, log_atk_scale: Tensor,
-    scale: float, squash_x: float, squash_eps: float, lean: bool,
-) -> tuple[Tensor, list[Tensor]]:
-    """Dense training / prefill forward without recurrent state: returns the
-    output and the intermediates its backward reuses (all eleven unless
-    ``lean``).  ``g`` is the raw decay projection; the gate and its chunk-local
-    cumulative sum are computed inside the kernels."""
-    if _chunk_capable(q):
-        o, _, _, saved = ops.chunk_forward(
-            q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-            scale, squash_x, squash_eps)
-        saved = saved[:6] if lean else saved
-        _check_intermediates(saved, q, v, lean)
-        return o, saved
-    # fp32 activations or another head width: exact token-by-token kernel.
-    o, _, _ = ops.recurrent_forward(
-        q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-        scale, squash_x, squash_eps, output_final_state=False)
-    # The exact backward needs none of the intermediates; the list only keeps the
-    # operator's output contract (names, shapes, dtypes), so it is left unwritten.
-    saved = [torch.empty(shape, device=q.device, dtype=dt)
-             for shape, dt in _intermediate_meta(q, v, lean)]
-    _check_intermediates(saved, q, v, lean)
-    return o, saved
+def _operator(name: str):
+    """The registered operator ``delta_feedback::<name>``, or a stand-in that raises if the
+    native layer does not exist or load."""
+    if not (_lib.built() and _lib.available()):
+        return _missing
+    return getattr(torch.ops.delta_feedback, name).default
 
 
-@pkda_recurrence.register_fake
+def _register_fake(name: str):
+    """``torch.library.register_fake`` for an operator of the native layer, where there is one."""
+    if not (_lib.built() and _lib.available()):
+        return lambda fn: fn
+    return torch.library.register_fake(f"delta_feedback::{name}")
+
+
+pkda_recurrence = _operator("pkda_recurrence")
+"""``(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, scale, squash_x,
+squash_eps, lean) -> (o, saved)``: dense training / prefill forward without recurrent state;
+returns the output and the intermediates its backward reuses (all eleven unless ``lean``).
+``g`` is the raw decay projection; the gate and its chunk-local cumulative sum are computed
+inside the kernels.  bf16 activations of 128-channel heads take the chunked kernels, everything
+else the exact token-by-token ones (which leave the intermediates unwritten)."""
+
+
+@_register_fake("pkda_recurrence")
 def _pkda_recurrence_fake(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
                           scale, squash_x, squash_eps, lean):
     output = torch.empty((*q.shape[:3], v.shape[-1]), device=q.device, dtype=q.dtype)
@@ -107,38 +102,7 @@ def _pkda_recurrence_fake(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log
     return output, saved
 
 
-@torch.library.custom_op("delta_feedback::pkda_recurrence_backward", mutates_args=(),
-                         device_types="cuda")
-def _pkda_recurrence_backward(
-    q: Tensor, k: Tensor, v: Tensor, g: Tensor, g_atk: Tensor, beta_atk: Tensor, beta: Tensor,
-    A_log: Tensor, dt_bias: Tensor, log_atk_scale: Tensor, saved: list[Tensor], do: Tensor,
-    scale: float, squash_x: float, squash_eps: float,
-    autocast_dtype: Optional[torch.dtype], lean: bool,
-) -> list[Tensor]:
-    """Ten input gradients, each in its input's dtype (``g_atk``, ``A_log``,
-    ``dt_bias``, ``log_atk_scale`` stay fp32).  ``autocast_dtype`` is accepted
-    for signature parity; the kernels fix their own arithmetic (bf16 operands,
-    fp32 accumulation) and do not consult autocast."""
-    del autocast_dtype
-    expected = len(PKDA_INTERMEDIATES) + (0 if lean else len(PKDA_RETAINED))
-    if len(saved) != expected:
-        raise RuntimeError(
-            f"PKDA backward received {len(saved)} intermediates, not {expected}")
-    if not _chunk_capable(q):
-        # fp32 activations or another head width: exact backward (ignores ``saved``)
-        grads, _, _ = ops.recurrent_backward(
-            q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-            scale, squash_x, squash_eps, do)
-        inputs = (q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale)
-        return [gr.reshape(t.shape).to(t.dtype) for gr, t in zip(grads, inputs)]
-    grads, _, _ = ops.chunk_backward(
-        q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-        scale, squash_x, squash_eps, saved, do, lean=lean)
-    inputs = (q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale)
-    return [gr.reshape(t.shape).to(t.dtype) for gr, t in zip(grads, inputs)]
-
-
-@_pkda_recurrence_backward.register_fake
+@_register_fake("pkda_recurrence_backward")
 def _pkda_recurrence_backward_fake(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias,
                                    log_atk_scale, saved, do, scale, squash_x, squash_eps,
                                    autocast_dtype, lean):
@@ -146,27 +110,6 @@ def _pkda_recurrence_backward_fake(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_
     return [t.new_empty(t.shape) for t in
             (q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale)]
 
-
-def _recurrence_setup_context(ctx, inputs, output) -> None:
-    *tensors, scale, squash_x, squash_eps, lean = inputs
-    _o, saved = output
-    ctx.save_for_backward(*tensors, *saved)
-    ctx.scalars = (scale, squash_x, squash_eps, lean)
-    ctx.autocast_dtype = (
-        torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else None)
-    ctx.mark_non_differentiable(*saved)
-
-
-def _recurrence_backward(ctx, do, _dsaved):
-    tensors = ctx.saved_tensors  # unpacked exactly once (checkpoint replays allow no more)
-    inputs, saved = tensors[:10], list(tensors[10:])
-    scale, squash_x, squash_eps, lean = ctx.scalars
-    grads = _pkda_recurrence_backward(
-        *inputs, saved, do, scale, squash_x, squash_eps, ctx.autocast_dtype, lean)
-    return (*grads, None, None, None, None)
-
-
-pkda_recurrence.register_autograd(_recurrence_backward, setup_context=_recurrence_setup_context)
 
 __all__ = ["CHUNK_SIZE", "PKDA_INTERMEDIATES", "PKDA_RETAINED", "fla_ops_available",
            "pkda_recurrence"]

@@ -10,10 +10,9 @@ from __future__ import annotations
 
 from typing import Optional
 
-import torch
 from torch import Tensor
 
-from . import _lib, ops
+from . import _lib
 from .fla_ops import fla_ops_available, pkda_recurrence
 
 
@@ -47,72 +46,9 @@ def fused_recurrent_precond_kda(
     _check_flags(use_gate_in_kernel, use_qk_l2norm_in_kernel)
     if log_atk_scale is None:
         raise RuntimeError("log_atk_scale is required")
-    with torch.no_grad():
-        return ops.recurrent_forward(
-            q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, scale, x, eps,
-            initial_state, initial_A_state, cu_seqlens, output_final_state, inplace_state)
-
-
-class _ChunkPKDA(torch.autograd.Function):
-    """Chunked recurrence with optional initial / final state and packing."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-                initial_state, initial_A_state, scale, x, eps, cu_seqlens, output_final_state,
-                lean):
-        o, S, A, saved = ops.chunk_forward(
-            q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, scale, x, eps,
-            initial_state, initial_A_state, cu_seqlens, output_final_state)
-        keep = saved[:6] if lean else saved
-        ctx.save_for_backward(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-                              initial_state, initial_A_state, cu_seqlens, *keep)
-        ctx.conf = (scale, x, eps, lean)
-        if S is not None:
-            ctx.mark_non_differentiable(A)
-            return o, S, A
-        return o, None, None
-
-    @staticmethod
-    def backward(ctx, do, dS, _dA):
-        t = ctx.saved_tensors
-        inputs, S0, A0, cu, saved = t[:10], t[10], t[11], t[12], list(t[13:])
-        scale, x, eps, lean = ctx.conf
-        want = S0 is not None or A0 is not None
-        grads, dS0, dA0 = ops.chunk_backward(
-            *inputs, scale, x, eps, saved, do, S0, A0, cu, dS, lean, want)
-        out = [gr.reshape(i.shape).to(i.dtype) for gr, i in zip(grads, inputs)]
-        return (*out, dS0 if S0 is not None else None, dA0 if A0 is not None else None,
-                None, None, None, None, None, None)
-
-
-class _ExactPKDA(torch.autograd.Function):
-    """Token-by-token kernels (exact fp32 arithmetic) with autograd: the path for
-    fp32 activations and for head widths other than 128."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-                initial_state, initial_A_state, scale, x, eps, cu_seqlens, output_final_state):
-        o, S, A = ops.recurrent_forward(
-            q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, scale, x, eps,
-            initial_state, initial_A_state, cu_seqlens, output_final_state)
-        ctx.save_for_backward(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-                              initial_state, initial_A_state, cu_seqlens)
-        ctx.conf = (scale, x, eps)
-        if S is not None:
-            ctx.mark_non_differentiable(A)
-            return o, S, A
-        return o, None, None
-
-    @staticmethod
-    def backward(ctx, do, dS, _dA):
-        t = ctx.saved_tensors
-        inputs, S0, A0, cu = t[:10], t[10], t[11], t[12]
-        scale, x, eps = ctx.conf
-        want = S0 is not None or A0 is not None
-        grads, dS0, dA0 = ops.recurrent_backward(*inputs, scale, x, eps, do, S0, A0, cu, dS, want)
-        out = [gr.reshape(i.shape).to(i.dtype) for gr, i in zip(grads, inputs)]
-        return (*out, dS0 if S0 is not None else None, dA0 if A0 is not None else None,
-                None, None, None, None, None)
+    return _lib.native().recurrent_forward(
+        q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, initial_state,
+        initial_A_state, cu_seqlens, scale, x, eps, output_final_state, inplace_state)
 
 
 def chunk_precond_kda(
@@ -135,13 +71,9 @@ def chunk_precond_kda(
     _check_flags(use_gate_in_kernel, use_qk_l2norm_in_kernel)
     if log_atk_scale is None:
         raise RuntimeError("log_atk_scale is required")
-    if q.dtype == torch.bfloat16 and q.shape[-1] == 128:
-        return _ChunkPKDA.apply(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-                                initial_state, initial_A_state, scale, x, eps, cu_seqlens,
-                                output_final_state, not disable_recompute)
-    return _ExactPKDA.apply(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
-                            initial_state, initial_A_state, scale, x, eps, cu_seqlens,
-                            output_final_state)
+    return _lib.native().recurrence(
+        q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, initial_state,
+        initial_A_state, cu_seqlens, scale, x, eps, output_final_state, not disable_recompute)
 
 
 def pkda_cuda_recurrence(
