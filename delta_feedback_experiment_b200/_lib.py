@@ -139,7 +139,9 @@ class PackControlArgs(C.Structure):
 
 
 EXPORTS = (
-    "pkda_recurrent_fwd", "pkda_recurrent_bwd", "pkda_recurrent_bwd_workspace_bytes", "pkda_chunk_fwd_workspace_bytes", "pkda_chunk_fwd",
+    "pkda_recurrent_fwd", "pkda_recurrent_bwd", "pkda_recurrent_bwd_workspace_bytes",
+    "pkda_recurrent_saved_bytes", "pkda_recurrent_fwd_saving", "pkda_recurrent_bwd_saved_workspace_bytes",
+    "pkda_recurrent_bwd_saved", "pkda_chunk_fwd_workspace_bytes", "pkda_chunk_fwd",
     "pkda_chunk_bwd_workspace_bytes", "pkda_chunk_bwd", "pkda_abi_version",
     "pkda_status_string", "pkda_sizeof_problem", "pkda_sizeof_recurrent_args",
     "pkda_sizeof_chunk_fwd_args", "pkda_sizeof_chunk_bwd_args", "pkda_last_launch_count",
@@ -156,7 +158,6 @@ EXPORTS = (
 )
 
 _lib: Optional[C.CDLL] = None
-_load_error: Optional[str] = None
 
 
 def _configure(lib: C.CDLL) -> None:
@@ -166,6 +167,13 @@ def _configure(lib: C.CDLL) -> None:
     lib.pkda_recurrent_bwd.restype = C.c_int
     lib.pkda_recurrent_bwd_workspace_bytes.argtypes = [C.POINTER(Problem)]
     lib.pkda_recurrent_bwd_workspace_bytes.restype = C.c_size_t
+    lib.pkda_recurrent_fwd_saving.argtypes = [C.POINTER(RecurrentArgs), C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.pkda_recurrent_fwd_saving.restype = C.c_int
+    lib.pkda_recurrent_bwd_saved.argtypes = [C.POINTER(RecurrentBwdArgs), C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.pkda_recurrent_bwd_saved.restype = C.c_int
+    for name in ("pkda_recurrent_saved_bytes", "pkda_recurrent_bwd_saved_workspace_bytes"):
+        getattr(lib, name).argtypes = [C.POINTER(Problem)]
+        getattr(lib, name).restype = C.c_size_t
     lib.pkda_chunk_fwd.argtypes = [C.POINTER(ChunkFwdArgs), C.c_void_p]
     lib.pkda_chunk_fwd.restype = C.c_int
     lib.pkda_chunk_fwd_static.argtypes = [C.POINTER(ChunkFwdArgs), C.c_void_p]
@@ -218,12 +226,11 @@ def _configure(lib: C.CDLL) -> None:
 
 
 def load() -> C.CDLL:
-    """Loads the shared library once; raises ``RuntimeError`` if that fails."""
-    global _lib, _load_error
+    """Loads the shared library once; raises ``RuntimeError`` if that fails (and tries again the
+    next time: the library may have been built in between)."""
+    global _lib
     if _lib is not None:
         return _lib
-    if _load_error is not None:
-        raise RuntimeError(_load_error)
     try:
         if not os.path.exists(LIB_PATH):
             raise OSError(f"{LIB_PATH} has not been built "
@@ -244,9 +251,8 @@ def load() -> C.CDLL:
         for size, struct in sizes:
             if size != C.sizeof(struct):
                 raise OSError(f"struct layout mismatch for {struct.__name__}")
-    except OSError as exc:
-        _load_error = f"PKDA CUDA library unavailable: {exc}"
-        raise RuntimeError(_load_error) from exc
+    except (OSError, AttributeError) as exc:  # AttributeError: an older build without some export
+        raise RuntimeError(f"PKDA CUDA library unavailable: {exc}") from exc
     _lib = lib
     return lib
 

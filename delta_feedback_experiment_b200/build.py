@@ -101,6 +101,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         for _, log in results:
             sys.stderr.write(log)
     native_obj = native.result()
+    for path in (LIB_PATH, NATIVE_PATH):  # new files, not new contents: an older build may be loaded right now
+        if os.path.exists(path):
+            os.unlink(path)
     cmd = [nvcc, "-shared", "-o", LIB_PATH, "-Xlinker", "-soname=libpkda_b200.so", *[o for o, _ in results], "-lcudart"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:

@@ -122,7 +122,15 @@ extern "C" {
 int pkda_recurrent_fwd(const pkda_recurrent_args* args, void* cuda_stream) {
   if (!args) return PKDA_ERR_NULL;
   pkda::reset_launch_count();
-  return pkda::recurrent_fwd(args, static_cast<cudaStream_t>(cuda_stream));
+  return pkda::recurrent_fwd(args, nullptr, 0, static_cast<cudaStream_t>(cuda_stream));
+}
+
+size_t pkda_recurrent_saved_bytes(const pkda_problem* p) { return p ? pkda::recurrent_saved_bytes(*p) : 0; }
+
+int pkda_recurrent_fwd_saving(const pkda_recurrent_args* args, void* saved, size_t saved_bytes, void* cuda_stream) {
+  if (!args || !saved) return PKDA_ERR_NULL;
+  pkda::reset_launch_count();
+  return pkda::recurrent_fwd(args, saved, saved_bytes, static_cast<cudaStream_t>(cuda_stream));
 }
 
 size_t pkda_recurrent_bwd_workspace_bytes(const pkda_problem* p) {
@@ -132,7 +140,18 @@ size_t pkda_recurrent_bwd_workspace_bytes(const pkda_problem* p) {
 int pkda_recurrent_bwd(const pkda_recurrent_bwd_args* args, void* cuda_stream) {
   if (!args) return PKDA_ERR_NULL;
   pkda::reset_launch_count();
-  return pkda::recurrent_bwd(args, static_cast<cudaStream_t>(cuda_stream));
+  return pkda::recurrent_bwd(args, nullptr, 0, static_cast<cudaStream_t>(cuda_stream));
+}
+
+size_t pkda_recurrent_bwd_saved_workspace_bytes(const pkda_problem* p) {
+  return p ? pkda::recurrent_bwd_saved_workspace(*p) : 0;
+}
+
+int pkda_recurrent_bwd_saved(const pkda_recurrent_bwd_args* args, const void* saved, size_t saved_bytes,
+                             void* cuda_stream) {
+  if (!args || !saved) return PKDA_ERR_NULL;
+  pkda::reset_launch_count();
+  return pkda::recurrent_bwd(args, saved, saved_bytes, static_cast<cudaStream_t>(cuda_stream));
 }
 
 size_t pkda_chunk_fwd_workspace_bytes(const pkda_problem* p) {

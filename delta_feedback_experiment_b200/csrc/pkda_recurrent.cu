@@ -1,13 +1,19 @@
-// Token-by-token PKDA recurrence: the decode step, short cached prefill, and
-// the exact fp32 forward.  One CTA owns one (sequence, head) and keeps the
-// whole D x D fp32 state in registers for all of its tokens, so a decode step
-// moves the state through HBM exactly once in each direction (128-bit loads
-// and stores, one full state row per warp request).
+// Token-by-token PKDA recurrence: short cached prefill, packed short sequences, and the exact fp32
+// forward (fp32 activations, head widths other than 128).  Single-token steps on a cached state run
+// in pkda_decode_step.cu.
 //
-// Follows delta_feedback_experiment/pkda.py:390-410 literally:
+// Follows delta_feedback_experiment/pkda.py:390-410:
 //   A  <- exp(gP) A + bP k^2 ;  kw = k * precond_factor(A)
 //   S  <- diag(exp(g)) S ;  e = v - S^T k ;  S <- S + (beta kw) e^T ;  o = S^T (scale q)
-#include "pkda_common.cuh"
+//
+// What bounds it: the chain of dependent tokens.  The value columns of S are independent of one
+// another, so each warp takes 4 or 8 columns with all D rows (ScanLay) and the step's only exchange
+// is log2(8) = 3 shuffles for e; with one CTA holding the whole state the step crossed three block
+// barriers and two shared-memory reductions.  The row vectors (exp(g), k, beta kw, q) do not depend
+// on S: producer warps make them for 8 tokens at a time, double buffered, while the consumer warps
+// run the chain; the sum for o is off the chain and is reduced for 8 tokens at once.
+// Measured: 4 x 16 units, 48 tokens, D = 128, bf16: 67 -> 25 us; 2 x 4 units, 512 tokens,
+// D = 64, fp32: 548 -> 85 us.
 #include "pkda_launch.h"
 #include "pkda_recurrent.cuh"
 
@@ -22,16 +28,219 @@ struct RecParams {
   const float *S0, *A0;
   void* o;
   float *ST, *AT;
-  float *Sb, *Ab;  // optional checkpoints at every 64-token boundary: [chunks][H][D][D], [chunks][H][D]
+  RecSaved save;     // kSave only
+  int nw, groups;    // consumer warps per CTA, CTAs per (sequence, head)
+  int inplace_A;     // AT aliases A0: written only after every CTA of the unit has read it (a cluster)
   float scale, ln_x, eps;
 };
 
-// kCkpt: also store the states entering every 64-token chunk (first pass of the exact
-// backward); a separate instantiation so that the decode kernel keeps its register budget
-// (two CTAs per SM at D = 128).
-template <int D, typename T, bool kCkpt>
-__global__ void __launch_bounds__(RecCfg<D>::kThreads, D == 128 ? 2 : 1)
+template <int D, int kCPL, typename T, bool kSave>
+__global__ void __launch_bounds__(ScanLay<D, kCPL>::kProd + 32 * ScanLay<D, kCPL>::kMaxConsumers)
 pkda_recurrent_kernel(const RecParams p) {
+  using L = ScanLay<D, kCPL>;
+  constexpr int TB = L::kTB, TPG = L::kTPG, RG = L::kRG, R = L::kR, RUNS = L::kR / L::kU, VEC = L::kVecs * D;
+  extern __shared__ __align__(16) float stage[];  // [2][TB][5][D]: exp(g) k, exp(g), beta kw, scale q, v
+  const int H = p.geo.heads;
+  const int unit = blockIdx.x / p.groups, cg = blockIdx.x - unit * p.groups;
+  const int n = unit / H, h = unit - n * H;
+  const SeqInfo sq = seq_info(p.geo, n);
+  const int nblk = (sq.len + TB - 1) / TB;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nthreads = 32 * p.nw + L::kProd;
+
+  if (warp >= p.nw) {
+    // ------------------------------------------------ producers: row vectors of TB tokens at a time
+    const int ptid = threadIdx.x - 32 * p.nw;
+    const int grp = ptid / L::kProdPerGroup, c = ptid - grp * L::kProdPerGroup;
+    const bool act = c < D;
+    const float ea = expf(p.A_log[h]), centre = p.log_atk_scale[h];
+    const float bias = act ? p.dt_bias[h * D + c] : 0.f;
+    float A = (act && p.A0) ? p.A0[(size_t)unit * D + c] : 0.f;
+    if (p.inplace_A) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    const size_t step = (size_t)H * D;
+    const size_t base = ((size_t)sq.bos * H + h) * D + (act ? c : 0);
+    const T *kp = static_cast<const T*>(p.k) + base, *qp = static_cast<const T*>(p.q) + base,
+            *gp = static_cast<const T*>(p.g) + base, *vp = static_cast<const T*>(p.v) + base;
+    typename Raw<T>::type kr[TB], qr[TPG], gr[TPG], vr[TPG], bt;
+    float sc;
+    auto fetch = [&](int t0) {
+#pragma unroll
+      for (int i = 0; i < TB; ++i) kr[i] = (act && t0 + i < sq.len) ? Raw<T>::load(kp + (size_t)(t0 + i) * step) : 0;
+#pragma unroll
+      for (int i = 0; i < TPG; ++i) {
+        const int t = t0 + TPG * grp + i;
+        const bool ok = act && t < sq.len;
+        qr[i] = ok ? Raw<T>::load(qp + (size_t)t * step) : 0;
+        gr[i] = ok ? Raw<T>::load(gp + (size_t)t * step) : 0;
+        vr[i] = ok ? Raw<T>::load(vp + (size_t)t * step) : 0;
+      }
+      // the token's three scalars: lane = 8 * kind + token
+      const int t = t0 + (lane & 7), kind = lane >> 3;
+      const size_t sidx = (size_t)(sq.bos + t) * H + h;
+      sc = 0.f;
+      bt = 0;
+      if (t < sq.len && kind == 0) sc = p.g_atk[sidx];
+      if (t < sq.len && (kind == 1 || kind == 2)) bt = Raw<T>::load(static_cast<const T*>(kind == 1 ? p.beta_atk : p.beta) + sidx);
+    };
+    if (nblk > 0) fetch(0);
+    for (int b = 0; b < nblk; ++b) {
+      const int s = b & 1, t0 = b * TB;
+      float kc[TPG], An[TPG], qc[TPG], gc[TPG], vc[TPG];
+      const float scal = lane < 8 ? expf(sc) : Raw<T>::value(bt);
+#pragma unroll
+      for (int i = 0; i < TB; ++i) {
+        const float pd = __shfl_sync(0xffffffffu, scal, i), ba = __shfl_sync(0xffffffffu, scal, 8 + i);
+        const float kf = Raw<T>::value(kr[i]);
+        A = pd * A + ba * kf * kf;
+        if (i < TPG || grp == i / TPG) { An[i % TPG] = A; kc[i % TPG] = kf; }
+      }
+#pragma unroll
+      for (int i = 0; i < TPG; ++i) { qc[i] = Raw<T>::value(qr[i]); gc[i] = Raw<T>::value(gr[i]); vc[i] = Raw<T>::value(vr[i]); }
+      if (b + 1 < nblk) fetch(t0 + TB);
+      if (b >= 2) bar_sync_n(3 + s, nthreads);
+      float* st = stage + s * L::kStage;
+#pragma unroll
+      for (int i = 0; i < TPG; ++i) {
+        const int tl = TPG * grp + i;
+        const float bw = __shfl_sync(0xffffffffu, scal, 16 + tl);
+        const bool ok = t0 + tl < sq.len;  // tokens past the end leave the state as it is
+        float al = expf(-ea * softplus_series(gc[i] + bias));  // (selects, no branches: the tokens interleave)
+        al = ok ? al : 1.f;
+        const float wk = bw * (kc[i] * precond_factor_nb(An[i], p.eps, centre, p.ln_x));
+        if (act) {
+          float* row = st + tl * VEC + c;
+          row[0] = al * kc[i];
+          row[D] = al;
+          row[2 * D] = wk;
+          row[3 * D] = qc[i] * p.scale;
+          row[4 * D] = vc[i];
+          if (kSave && cg == 0 && ok) {
+            const size_t idx = base + (size_t)(t0 + tl) * step;
+            p.save.al[idx] = al;
+            p.save.w[idx] = wk;
+            p.save.A[idx] = An[i];
+          }
+        }
+      }
+      bar_arrive_n(1 + s, nthreads);
+    }
+    if (p.inplace_A) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (p.AT && cg == 0 && grp == 0 && act) p.AT[(size_t)unit * D + c] = A;
+    return;
+  }
+
+  // ---------------------------------------------------- consumers: the chain over tokens
+  if (p.inplace_A) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  const int rg = lane & (RG - 1);
+  const int col0 = (cg * p.nw + warp) * L::kCols + (lane / RG) * kCPL;
+  const size_t sbase = (size_t)unit * D * D + col0;
+  float2 S[kCPL][R / 2];
+  // element (row, column c) of the lane's part of the state
+  auto elem = [&](int row, int c) -> float& { return (row & 1) ? S[c][row / 2].y : S[c][row / 2].x; };
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float* src = p.S0 + sbase + (size_t)(L::row(i / L::kU, rg) + i % L::kU) * D;
+    float x[kCPL];
+#pragma unroll
+    for (int c = 0; c < kCPL; ++c) x[c] = 0.f;
+    if (p.S0) {
+      if (kCPL == 4) *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(src);
+      else x[0] = *src;
+    }
+#pragma unroll
+    for (int c = 0; c < kCPL; ++c) elem(i, c) = x[c];
+  }
+  auto store_state = [&](float* base) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      float* dst = base + (size_t)(L::row(i / L::kU, rg) + i % L::kU) * D;
+      if (kCPL == 4) *reinterpret_cast<float4*>(dst) = make_float4(elem(i, 0), elem(i, 1 % kCPL), elem(i, 2 % kCPL), elem(i, 3 % kCPL));
+      else *dst = elem(i, 0);
+    }
+  };
+  T* o = static_cast<T*>(p.o);
+  const size_t tstep = (size_t)H * D;
+  const size_t tbase = ((size_t)sq.bos * H + h) * D + col0;
+  for (int b = 0; b < nblk; ++b) {
+    const int s = b & 1, t0 = b * TB;
+    if (kSave && (t0 & (kCkpt - 1)) == 0)
+      store_state(p.save.S + ((ckpt_base(p.geo, n, sq.bos) + t0 / kCkpt) * H + h) * (size_t)(D * D) + col0);
+    bar_sync_n(1 + s, nthreads);
+    const float* st = stage + s * L::kStage;
+    float oacc[L::kTO * kCPL], ekeep[L::kSums];  // [token][column]
+    float2 kx[R / 2];  // exp(g) k of the token
+    load_rows<L>(st, rg, kx);
+#pragma unroll
+    for (int t = 0; t < TB; ++t) {
+      const float* vec = st + t * VEC;
+      float e[kCPL];
+#pragma unroll
+      for (int c = 0; c < kCPL; ++c) {
+        float2 a0 = __fmul2_rn(kx[0], S[c][0]), a1 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 1; i < R / 2; ++i) {
+          if (i & 1) a1 = __ffma2_rn(kx[i], S[c][i], a1);
+          else a0 = __ffma2_rn(kx[i], S[c][i], a0);
+        }
+        e[c] = (a0.x + a0.y) + (a1.x + a1.y);
+      }
+      // every other row vector the token needs, and the next token's first one, is asked for before
+      // the shuffles below so that none of these loads sits on the chain
+      float2 al[R / 2], wk[R / 2], qs[R / 2];
+      load_rows<L>(vec + D, rg, al);
+      load_rows<L>(vec + 2 * D, rg, wk);
+      load_rows<L>(vec + 3 * D, rg, qs);
+      if (t + 1 < TB) load_rows<L>(vec + VEC, rg, kx);
+      float vt[kCPL];
+      if (kCPL == 4) *reinterpret_cast<float4*>(vt) = *reinterpret_cast<const float4*>(vec + 4 * D + col0);
+      else vt[0] = vec[4 * D + col0];
+      rg_sum<RG>(e, rg);
+#pragma unroll
+      for (int c = 0; c < kCPL; ++c) e[c] = vt[c] - e[c];
+      if (kSave && rg == t / L::kSums) ekeep[t % L::kSums] = e[0];
+#pragma unroll
+      for (int c = 0; c < kCPL; ++c)
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i)
+          S[c][i] = __ffma2_rn(wk[i], make_float2(e[c], e[c]), __fmul2_rn(al[i], S[c][i]));
+#pragma unroll
+      for (int c = 0; c < kCPL; ++c) {
+        float2 a0 = __fmul2_rn(qs[0], S[c][0]);
+#pragma unroll
+        for (int i = 1; i < R / 2; ++i) a0 = __ffma2_rn(qs[i], S[c][i], a0);
+        oacc[(t % L::kTO) * kCPL + c] = a0.x + a0.y;
+      }
+      if ((t + 1) % L::kTO == 0) {
+        rg_sum_transposed<RG, L::kTO * kCPL>(oacc, rg);
+#pragma unroll
+        for (int i = 0; i < L::kSums; ++i) {
+          const int x = rg * L::kSums + i, to = t0 + t + 1 - L::kTO + x / kCPL;
+          if (to < sq.len) o[tbase + (size_t)to * tstep + x % kCPL] = from_f<T>(oacc[i]);
+        }
+      }
+    }
+    if (b + 2 < nblk) bar_arrive_n(3 + s, nthreads);
+    if (kSave) {  // (one column per lane)
+#pragma unroll
+      for (int i = 0; i < L::kSums; ++i) {
+        const int t = t0 + rg * L::kSums + i;
+        if (t < sq.len) p.save.e[tbase + (size_t)t * tstep] = ekeep[i];
+      }
+    }
+  }
+  if (p.ST) store_state(p.ST + sbase);
+  if (p.inplace_A) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// A few tokens for more (sequence, head) units than SMs, e.g. a speculative block of a large batch:
+// reading and writing the states is most of the call.  One CTA keeps the whole state in registers
+// (thread = 16 rows x 4 columns, state rows moved in full 512-byte lines, two CTAs per SM), as the
+// decode step does, and crosses three block barriers per token.  D = 128, bf16, us at 2 / 8 / 16 tokens:
+// 256 units (one wave of this kernel, two of the sliced one) 8.2 / 18.5 / 32.5 against 21.0 / 21.0 / 30.9;
+// 1024 units 39.7 / 94.8 / 164 against 74.9 / 76.0 / 109.
+template <int D, typename T>
+__global__ void __launch_bounds__(RecCfg<D>::kThreads, D == 128 ? 2 : 1)
+pkda_recurrent_few_kernel(const RecParams p) {
   using Cfg = RecCfg<D>;
   constexpr int VQ = Cfg::kVQ, KW = Cfg::kKW, R = Cfg::kR;
   const int tid = threadIdx.x;
@@ -74,15 +283,6 @@ pkda_recurrent_kernel(const RecParams p) {
   T* o = static_cast<T*>(p.o);
 
   for (int t = 0; t < sq.len; ++t) {
-    if (kCkpt && (t & (kChunk - 1)) == 0) {  // checkpoint the state entering this chunk
-      const size_t chh = (size_t)(sq.chunk0 + t / kChunk) * H + h;
-      if (active) {
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-          *reinterpret_cast<float4*>(p.Sb + chh * D * D + (size_t)(krow0 + r) * D + 4 * vq) = S[r];
-      }
-      if (tid < D) p.Ab[chh * D + tid] = A;
-    }
     const size_t tok = (size_t)(sq.bos + t);
     const size_t sidx = tok * H + h;
     if (tid < D) {
@@ -143,68 +343,130 @@ pkda_recurrent_kernel(const RecParams p) {
   if (p.AT && tid < D) p.AT[((size_t)n * H + h) * D + tid] = A;
 }
 
-template <int D, typename T>
-static int launch_rec(const RecParams& rp, cudaStream_t st) {
-  const bool ckpt = rp.Sb != nullptr;
-  dim3 grid(rp.geo.n_seqs * rp.geo.heads), block(RecCfg<D>::kThreads);
+int sm_count() {
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+template <int D, int kCPL, typename T, bool kSave>
+static int launch_rec(RecParams rp, cudaStream_t st) {
+  using L = ScanLay<D, kCPL>;
+  auto kernel = pkda_recurrent_kernel<D, kCPL, T, kSave>;
+  const int units = rp.geo.n_seqs * rp.geo.heads;
+  rp.nw = scan_consumers(units, L::kWarps, L::kMaxConsumers, sm_count());
+  if (rp.inplace_A)  // the unit's CTAs form one cluster: at most eight of them
+    while (L::kWarps / rp.nw > 8) rp.nw *= 2;
+  rp.groups = L::kWarps / rp.nw;
+  if (rp.groups == 1) rp.inplace_A = 0;
+  if (!ensure_dynamic_smem(kernel, L::kSmem)) return PKDA_ERR_LAUNCH;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(units * rp.groups));
+  cfg.blockDim = dim3((unsigned)(32 * rp.nw + L::kProd));
+  cfg.dynamicSmemBytes = L::kSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)rp.groups;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = rp.inplace_A ? 1 : 0;
   begin_stage(kStageRecurrent, st);
-  if (ckpt) pkda_recurrent_kernel<D, T, true><<<grid, block, 0, st>>>(rp);
-  else pkda_recurrent_kernel<D, T, false><<<grid, block, 0, st>>>(rp);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, rp);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+}
+
+template <int D, typename T>
+static int launch_rec_d(const RecParams& rp, bool save, cudaStream_t st) {
+  if (save) return launch_rec<D, 1, T, true>(rp, st);
+  const long units = (long)rp.geo.n_seqs * rp.geo.heads;
+  const int few = units <= 2L * sm_count() ? 14 : 8;  // break-even in tokens, see that kernel
+  if (rp.geo.seq_len > 0 && rp.geo.seq_len < few && units > sm_count()) {
+    begin_stage(kStageRecurrent, st);
+    pkda_recurrent_few_kernel<D, T><<<(unsigned)units, RecCfg<D>::kThreads, 0, st>>>(rp);
+    end_stage(st);
+    return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  }
+  // Four columns per lane once the one-column warps number more than two per scheduler (4 per SM).
+  constexpr bool kFour = D >= 64;
+  const long warps = units * ScanLay<D, 1>::kWarps;
+  if (kFour && warps > 8L * sm_count()) return launch_rec<D, kFour ? 4 : 1, T, false>(rp, st);
+  return launch_rec<D, 1, T, false>(rp, st);
 }
 
 template <typename T>
-static int dispatch_rec(int D, const RecParams& rp, cudaStream_t st) {
+static int dispatch_rec(int D, const RecParams& rp, bool save, cudaStream_t st) {
   switch (D) {
-    case 8: return launch_rec<8, T>(rp, st);
-    case 16: return launch_rec<16, T>(rp, st);
-    case 32: return launch_rec<32, T>(rp, st);
-    case 64: return launch_rec<64, T>(rp, st);
-    case 128: return launch_rec<128, T>(rp, st);
+    case 8: return launch_rec_d<8, T>(rp, save, st);
+    case 16: return launch_rec_d<16, T>(rp, save, st);
+    case 32: return launch_rec_d<32, T>(rp, save, st);
+    case 64: return launch_rec_d<64, T>(rp, save, st);
+    case 128: return launch_rec_d<128, T>(rp, save, st);
     default: return PKDA_ERR_SHAPE;
   }
 }
 
-int recurrent_fwd(const pkda_recurrent_args* a, cudaStream_t st) {
-  const pkda_problem& p = a->p;
-  int rc = check_problem(p);
-  if (rc != PKDA_OK) return rc;
-  if (p.n_seqs == 0 || p.total_tokens == 0) return PKDA_OK;
-  if (!a->o) return PKDA_ERR_NULL;
-  // One token per sequence on a cached state: the decode-step kernel (all loads of the step issued
-  // up front), without its convolution and gate stages.
-  if (!p.cu_seqlens && p.seq_len == 1 && p.initial_state && a->final_state &&
-      (p.dtype == PKDA_BF16 || p.dtype == PKDA_F32))
-    return decode_direct(p, a->o, a->final_state, a->final_A_state, st);
+RecSaved carve_rec_saved(const pkda_problem& p, void* base, size_t* bytes) {
+  RecSaved s;
+  const size_t units = (size_t)p.total_tokens * p.heads, D = p.head_dim;
+  size_t off = 0;
+  unsigned char* b = static_cast<unsigned char*>(base);
+  auto take = [&](size_t n) { float* x = reinterpret_cast<float*>(b + off); off += align_up(n * 4); return x; };
+  s.al = take(units * D);
+  s.w = take(units * D);
+  s.A = take(units * D);
+  s.e = take(units * D);
+  s.S = take(ckpt_bound(p) * p.heads * D * D);
+  if (bytes) *bytes = off;
+  return s;
+}
+
+static int run_rec(const pkda_problem& p, void* o, float* ST, float* AT, const RecSaved* save, cudaStream_t st) {
   RecParams rp;
   rp.geo = make_geo(p, nullptr);
   rp.q = p.q; rp.k = p.k; rp.v = p.v; rp.g = p.g; rp.g_atk = p.g_atk;
   rp.beta_atk = p.beta_atk; rp.beta = p.beta;
   rp.A_log = p.A_log; rp.dt_bias = p.dt_bias; rp.log_atk_scale = p.log_atk_scale;
   rp.S0 = p.initial_state; rp.A0 = p.initial_A_state;
-  rp.o = a->o; rp.ST = a->final_state; rp.AT = a->final_A_state; rp.Sb = nullptr; rp.Ab = nullptr;
+  rp.o = o; rp.ST = ST; rp.AT = AT;
+  rp.save = save ? *save : RecSaved{};
+  rp.inplace_A = AT && AT == p.initial_A_state;
   rp.scale = p.scale; rp.ln_x = logf(p.squash_x); rp.eps = p.squash_eps;
-  if (p.dtype == PKDA_BF16) return dispatch_rec<bf16>(p.head_dim, rp, st);
-  if (p.dtype == PKDA_F32) return dispatch_rec<float>(p.head_dim, rp, st);
+  if (p.dtype == PKDA_BF16) return dispatch_rec<bf16>(p.head_dim, rp, save != nullptr, st);
+  if (p.dtype == PKDA_F32) return dispatch_rec<float>(p.head_dim, rp, save != nullptr, st);
   return PKDA_ERR_DTYPE;
 }
 
-// Forward pass that also leaves the states at every chunk boundary (first pass of
-// the exact backward).
-int recurrent_fwd_checkpointed(const pkda_problem& p, const int* chunk_offsets, void* o_scratch, float* Sb,
-                               float* Ab, cudaStream_t st) {
-  RecParams rp;
-  rp.geo = make_geo(p, chunk_offsets);
-  rp.q = p.q; rp.k = p.k; rp.v = p.v; rp.g = p.g; rp.g_atk = p.g_atk;
-  rp.beta_atk = p.beta_atk; rp.beta = p.beta;
-  rp.A_log = p.A_log; rp.dt_bias = p.dt_bias; rp.log_atk_scale = p.log_atk_scale;
-  rp.S0 = p.initial_state; rp.A0 = p.initial_A_state;
-  rp.o = o_scratch; rp.ST = nullptr; rp.AT = nullptr; rp.Sb = Sb; rp.Ab = Ab;
-  rp.scale = p.scale; rp.ln_x = logf(p.squash_x); rp.eps = p.squash_eps;
-  if (p.dtype == PKDA_BF16) return dispatch_rec<bf16>(p.head_dim, rp, st);
-  if (p.dtype == PKDA_F32) return dispatch_rec<float>(p.head_dim, rp, st);
-  return PKDA_ERR_DTYPE;
+int recurrent_fwd(const pkda_recurrent_args* a, void* saved, size_t saved_bytes, cudaStream_t st) {
+  const pkda_problem& p = a->p;
+  int rc = check_problem(p);
+  if (rc != PKDA_OK) return rc;
+  if (p.n_seqs == 0 || p.total_tokens == 0) return PKDA_OK;
+  if (!a->o) return PKDA_ERR_NULL;
+  if (saved) {
+    size_t need = 0;
+    const RecSaved s = carve_rec_saved(p, saved, &need);
+    if (saved_bytes < need) return PKDA_ERR_WORKSPACE;
+    return run_rec(p, a->o, a->final_state, a->final_A_state, &s, st);
+  }
+  // One token per sequence on a cached state: the decode-step kernel (all loads of the step issued
+  // up front), without its convolution and gate stages.
+  if (!p.cu_seqlens && p.seq_len == 1 && p.initial_state && a->final_state &&
+      (p.dtype == PKDA_BF16 || p.dtype == PKDA_F32))
+    return decode_direct(p, a->o, a->final_state, a->final_A_state, st);
+  return run_rec(p, a->o, a->final_state, a->final_A_state, nullptr, st);
+}
+
+// Forward pass that only leaves what the exact backward needs (its output goes to scratch).
+int recurrent_fwd_saving(const pkda_problem& p, void* o_scratch, const RecSaved& save, cudaStream_t st) {
+  return run_rec(p, o_scratch, nullptr, nullptr, &save, st);
+}
+
+size_t recurrent_saved_bytes(const pkda_problem& p) {
+  size_t bytes = 0;
+  carve_rec_saved(p, nullptr, &bytes);
+  return bytes;
 }
 
 }  // namespace pkda

@@ -240,7 +240,8 @@ Forward chunk_forward(const Inputs& in, bool final_state) {
   return r;
 }
 
-Forward recurrent_forward(const Inputs& in, bool final_state, bool inplace) {
+// `save`: also leave what the exact backward needs (one byte tensor in `saved`).
+Forward recurrent_forward(const Inputs& in, bool final_state, bool inplace, bool save = false) {
   Problem P(in);
   c10::cuda::CUDAGuard guard(P.dev);
   Forward r;
@@ -262,7 +263,13 @@ Forward recurrent_forward(const Inputs& in, bool final_state, bool inplace) {
     a.final_state = r.S.data_ptr<float>();
     a.final_A_state = r.A.data_ptr<float>();
   }
-  finish(pkda_recurrent_fwd(&a, stream()), "pkda_recurrent_fwd");
+  if (save) {
+    r.saved.push_back(scratch(pkda_recurrent_saved_bytes(&P.p), P.dev));
+    finish(pkda_recurrent_fwd_saving(&a, r.saved[0].data_ptr(), (size_t)r.saved[0].numel(), stream()),
+           "pkda_recurrent_fwd_saving");
+  } else {
+    finish(pkda_recurrent_fwd(&a, stream()), "pkda_recurrent_fwd");
+  }
   return r;
 }
 
@@ -335,18 +342,25 @@ std::vector<Tensor> chunk_backward(const Inputs& in, std::vector<Tensor> saved, 
   return grads;
 }
 
-// Exact backward of the recurrence: any supported head width, needs no saved intermediates.
-std::vector<Tensor> recurrent_backward(const Inputs& in, const Tensor& d_o, const OptTensor& dS, bool want_state) {
+// Exact backward of the recurrence: any supported head width.  `saved`: what a saving forward left, or
+// undefined (the forward runs again).
+std::vector<Tensor> recurrent_backward(const Inputs& in, const Tensor& d_o, const OptTensor& dS, bool want_state,
+                                       const Tensor& saved = Tensor()) {
   Problem P(in);
   c10::cuda::CUDAGuard guard(P.dev);
   pkda_recurrent_bwd_args a{};
   a.p = P.p;
   cotangents(P, a, d_o, dS);
   std::vector<Tensor> grads = alloc_grads(P, a, want_state);
-  a.workspace_bytes = pkda_recurrent_bwd_workspace_bytes(&P.p);
+  a.workspace_bytes = saved.defined() ? pkda_recurrent_bwd_saved_workspace_bytes(&P.p)
+                                      : pkda_recurrent_bwd_workspace_bytes(&P.p);
   Tensor ws = scratch(a.workspace_bytes, P.dev);
   a.workspace = ws.data_ptr();
-  finish(pkda_recurrent_bwd(&a, stream()), "pkda_recurrent_bwd");
+  if (saved.defined())
+    finish(pkda_recurrent_bwd_saved(&a, saved.const_data_ptr(), (size_t)saved.numel(), stream()),
+           "pkda_recurrent_bwd_saved");
+  else
+    finish(pkda_recurrent_bwd(&a, stream()), "pkda_recurrent_bwd");
   return grads;
 }
 
@@ -364,7 +378,7 @@ struct StatefulRecurrence : torch::autograd::Function<StatefulRecurrence> {
                                bool final_state, bool lean) {
     const Inputs in{q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, S0, A0, cu, scale, x, eps};
     const bool chunked = chunk_capable(q);
-    Forward f = chunked ? chunk_forward(in, final_state) : recurrent_forward(in, final_state, false);
+    Forward f = chunked ? chunk_forward(in, final_state) : recurrent_forward(in, final_state, false, !lean);
     if (lean && chunked) f.saved.resize(kKept);
     variable_list keep{q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale,
                        S0.value_or(Tensor()), A0.value_or(Tensor()), cu.value_or(Tensor())};
@@ -387,7 +401,7 @@ struct StatefulRecurrence : torch::autograd::Function<StatefulRecurrence> {
     std::vector<Tensor> got =
         chunk_capable(t[0])
             ? chunk_backward(in, std::vector<Tensor>(t.begin() + 13, t.end()), grads[0], dS, conf[3] != 0.0, want)
-            : recurrent_backward(in, grads[0], dS, want);
+            : recurrent_backward(in, grads[0], dS, want, t.size() > 13 ? t[13] : Tensor());
     variable_list out(18);
     for (int i = 0; i < 10; ++i) out[i] = like_input(std::move(got[i]), t[i]);
     if (S0) out[10] = std::move(got[10]);

@@ -124,6 +124,16 @@ typedef struct pkda_recurrent_bwd_args {
 size_t pkda_recurrent_bwd_workspace_bytes(const pkda_problem* p);
 int pkda_recurrent_bwd(const pkda_recurrent_bwd_args* args, void* cuda_stream);
 
+/* The same pair with the forward's by-products kept between them: pkda_recurrent_fwd_saving is
+ * pkda_recurrent_fwd that also fills `saved` (pkda_recurrent_saved_bytes), pkda_recurrent_bwd_saved the
+ * backward that reads it instead of running the forward again (and needs the smaller workspace of
+ * pkda_recurrent_bwd_saved_workspace_bytes).  Contents and layout of `saved` are the library's own. */
+size_t pkda_recurrent_saved_bytes(const pkda_problem* p);
+int pkda_recurrent_fwd_saving(const pkda_recurrent_args* args, void* saved, size_t saved_bytes, void* cuda_stream);
+size_t pkda_recurrent_bwd_saved_workspace_bytes(const pkda_problem* p);
+int pkda_recurrent_bwd_saved(const pkda_recurrent_bwd_args* args, const void* saved, size_t saved_bytes,
+                             void* cuda_stream);
+
 /*
  * Chunked forward (training / prefill), bf16 activations, D = 128, chunk 64.
  * Replaces kda_gate_chunk_cumsum + chunk_precond_kda_fwd
