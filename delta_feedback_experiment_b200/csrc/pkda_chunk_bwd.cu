@@ -1284,7 +1284,7 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
     // tcgen05 / TMEM / TMA at every size unless the mma.sync kernel is pinned (pkda_set_variant).
     const bool scan_mma = stage_variant(kStageScanBwd) == 1;
     begin_stage(kStageScanBwd, st);
-    if (!scan_mma && scan_by_columns(units))
+    if (!scan_mma && scan_columns(units))
       rc = launch_scan_bwd_cols(geo, p.total_tokens, units, kg, w, qg, sp.d_o, Aqk, ws.beta_c, gc, a->d_final_state,
                                 ws.dh, ws.dF, a->d_initial_state, ws.status, st);
     else if (!scan_mma)

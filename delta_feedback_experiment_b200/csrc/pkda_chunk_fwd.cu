@@ -761,10 +761,10 @@ int check_chunk_problem(const pkda_problem& p) {
   return PKDA_OK;
 }
 
-bool scan_by_columns(int units) {
+int scan_columns(int units) {
   int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return 4L * units <= sms;
+  return 8L * units <= sms ? 8 : 4L * units <= sms ? 4 : 0;
 }
 
 template <int VB, bool kRecompute>
@@ -848,7 +848,7 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   const bool fuse_out = o && !recompute && stage_variant(kStageOutFwd) == 0;
   if (o_done) *o_done = false;
   begin_stage(kStageScanFwd, st);
-  if (status && !scan_mma && scan_by_columns(units)) {
+  if (status && !scan_mma && scan_columns(units)) {
     rc = launch_scan_fwd_cols(geo, p.total_tokens, units, w, kg, u_ws, beta_c, gc, p.initial_state, h, v_new,
                               recompute ? nullptr : ST, status, qg, Aqk, fuse_out ? o : nullptr, st);
     if (o_done) *o_done = fuse_out;

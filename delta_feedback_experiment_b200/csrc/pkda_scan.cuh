@@ -12,7 +12,7 @@
 // Why not tensor memory here: a chunk step through TMEM is a chain of MMA -> commit -> wait -> TMEM read ->
 // shared memory -> fence -> block barrier, three times, about 4,500 cycles however few columns a CTA
 // has; here it is some 140 mma.sync at 8.2 cycles each and a few hundred cycles between them, and the eight
-// warps of a unit spread over four SMs.  Why not for many units: every warp reads whole B tiles from shared
+// warps of a unit spread over four or eight SMs.  Why not for many units: every warp reads whole B tiles from shared
 // memory (448 KB per unit and step when all eight sit on one SM), which took 330 us against the 192 us of
 // the tensor-memory kernel at 128 units, T = 4096.
 //
@@ -118,9 +118,9 @@ __device__ __forceinline__ float2 get2f(const unsigned char* s) { return *reinte
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// One poll each of two barriers in flight together (a poll takes about a hundred cycles even when its phase
-// is complete), then the bounded waits if need be.
-__device__ __forceinline__ bool mbar_wait2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
+// One poll of each of two barriers, both in flight together.  A poll takes about a hundred cycles even when
+// its phase is complete, so it is issued well before its answer is needed.
+__device__ __forceinline__ bool mbar_try2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
   uint32_t d0, d1;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
@@ -128,7 +128,13 @@ __device__ __forceinline__ bool mbar_wait2(uint32_t bar0, uint32_t parity0, uint
       "mbarrier.try_wait.parity.shared::cta.b64 q, [%4], %5;\n\t"
       "selp.u32 %0, 1, 0, p;\n\tselp.u32 %1, 1, 0, q;\n\t}"
       : "=r"(d0), "=r"(d1) : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1) : "memory");
-  return (d0 || tc::mbar_wait(bar0, parity0)) && (d1 || tc::mbar_wait(bar1, parity1));
+  return d0 & d1;
+}
+// The same with a bounded wait behind it; the answer is the warp's.
+__device__ __forceinline__ bool mbar_wait2(bool tried, uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
+  if (__all_sync(0xffffffffu, tried)) return true;
+  const bool ok = tc::mbar_wait(bar0, parity0) && tc::mbar_wait(bar1, parity1);
+  return __all_sync(0xffffffffu, ok);
 }
 // One arrival for the warp, after all its lanes are done.
 __device__ __forceinline__ void warp_arrive(uint32_t bar, int lane) {
@@ -147,21 +153,37 @@ __device__ __forceinline__ uint32_t identity_b(const Lane& L) {
   return L.g == 2 * L.t ? 0x00003F80u : L.g == 2 * L.t + 1 ? 0x3F800000u : 0u;
 }
 
-// X^T += f x tile: k steps of 16 tokens (tile rows), all 16 column tiles.
-__device__ __forceinline__ void update_state(float (&X)[16][4], const uint32_t (&f)[4][4], uint32_t tile, const Lane& L) {
+// The four fragment pairs of a k step (N form), and of half a k step of a state update (T form, eight of the
+// sixteen column tiles).
+struct Frags { uint32_t r[4][4]; };
+__device__ __forceinline__ void load_n(Frags& b, uint32_t tile, const Lane& L, int ks) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
+  for (int np = 0; np < 4; ++np) ldb_n(b.r[np], tile, L, ks, np);
+}
+__device__ __forceinline__ void load_t(Frags& b, uint32_t tile, const Lane& L, int half) {
 #pragma unroll
-    for (int nq = 0; nq < 2; ++nq) {
-      uint32_t b[4][4];
+  for (int x = 0; x < 4; ++x) ldb_t(b.r[x], tile, L, half >> 1, 4 * (half & 1) + x);
+}
+__device__ __forceinline__ void mma4(float (*acc)[4], const uint32_t (&a)[4], const Frags& b) {
 #pragma unroll
-      for (int x = 0; x < 4; ++x) ldb_t(b[x], tile, L, j, 4 * nq + x);
+  for (int np = 0; np < 4; ++np) {
+    mma_bf16(acc[2 * np], a, b.r[np][0], b.r[np][1]);
+    mma_bf16(acc[2 * np + 1], a, b.r[np][2], b.r[np][3]);
+  }
+}
+
+// X^T += f x tile: k steps of 16 tokens (tile rows), all 16 column tiles.  The fragments of the next half
+// step are asked for before the products of the current one (the assembler keeps this order; loads behind
+// the products cost their latency, about 50 cycles, every time); b: those of the first half, loaded before.
+__device__ __forceinline__ void update_state(float (&X)[16][4], const uint32_t (&f)[4][4], uint32_t tile, const Lane& L,
+                                             const Frags& first) {
+  Frags b[2];
+  b[0] = first;
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        mma_bf16(X[8 * nq + 2 * x], f[j], b[x][0], b[x][1]);
-        mma_bf16(X[8 * nq + 2 * x + 1], f[j], b[x][2], b[x][3]);
-      }
-    }
+  for (int i = 0; i < 8; ++i) {
+    if (i < 7) load_t(b[(i + 1) & 1], tile, L, i + 1);
+    mma4(&X[8 * (i & 1)], f[i >> 1], b[i & 1]);
+  }
 }
 
 // [64 tok][128] tile of an activation [tokens][H][128] in one TMA: dims {64, tokens, 2, H}.

@@ -1,5 +1,5 @@
-// Forward state scan for few units, with the output formed on the way.  Four CTAs per (sequence, head),
-// 32 value columns each.  Per 64-token chunk and group of 16 columns (transposed, see pkda_scan.cuh):
+// Forward state scan for few units, with the output formed on the way.  Eight or four CTAs per (sequence,
+// head), 16 or 32 value columns each.  Per 64-token chunk and group of 16 columns (transposed, see pkda_scan.cuh):
 //   chain warp    h    = bf16(S)                   registers, A operand as they stand
 //                 S   *= Gam_last (per k)
 //                 E^T  = U^T I - h^T W^T           64 + 8 mma.sync
@@ -8,8 +8,9 @@
 //   output warp   O^T  = h^T qg^T + E^T (P diag beta)^T   84 mma.sync, stores o
 //   store warp    stores h and E (v_new)
 //   copy warp     W, kg, U, qg, P, beta, Gam_last by TMA, up to three chunks ahead
-// The chain warp leaves h and E for the other two in shared memory, two slots deep.  Every wait is
-// bounded: on a timeout the warp sets the status word and leaves.
+// The chain warp leaves h and E for the other two in shared memory, two slots deep.  A step takes 1.05 us with
+// one column group per CTA and 1.45 us with two (the SM's shared memory then moves 1,700 of the 2,700 cycles);
+// T = 8192, 16 units: 360 -> 136 us, T = 4096, 24 units: 180 -> 93 us.  Every wait is bounded: on a timeout the warp sets the status word and leaves.
 #include "pkda_scan.cuh"
 
 namespace pkda {
@@ -23,8 +24,9 @@ struct ScanFwdParams {
   int* status;
 };
 
-template <bool kOut> struct ScanFwdLay {
-  static constexpr int NW = 2;                               // column groups per CTA
+// NW: column groups (of 16) per CTA.
+template <int NW, bool kOut> struct ScanFwdLay {
+  static constexpr int kSplit = 8 / NW;                      // CTAs per unit
   static constexpr int kReaders = kOut ? 2 : 1;              // of the h / E slots, per group
   static constexpr int kWorkers = NW * (1 + kReaders);
   static constexpr int kStageUsers = NW * (kOut ? 2 : 1);
@@ -42,17 +44,17 @@ template <bool kOut> struct ScanFwdLay {
   static_assert(kSmem <= 232448, "shared memory of one SM");
 };
 
-template <bool kOut>
-__global__ void __launch_bounds__(ScanFwdLay<kOut>::kThreads, 1)
+template <int NW, bool kOut>
+__global__ void __launch_bounds__(ScanFwdLay<NW, kOut>::kThreads, 1)
 pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_kg,
                           const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_qg,
                           const __grid_constant__ CUtensorMap tm_p, const ScanFwdParams p) {
   using namespace scanw;
-  using Y = ScanFwdLay<kOut>;
+  using Y = ScanFwdLay<NW, kOut>;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* const sm = smem_raw + (base - smem_u32(smem_raw));
-  const int unit = blockIdx.x >> 2, grp0 = (blockIdx.x & 3) * Y::NW;
+  const int unit = blockIdx.x / Y::kSplit, grp0 = (blockIdx.x % Y::kSplit) * NW;
   const int H = p.geo.heads, n = unit / H, h = unit - n * H;
   const SeqInfo sq = seq_info(p.geo, n);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -65,7 +67,7 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       tc::mbar_init(bar_full(s), 1);
       tc::mbar_init(bar_empty(s), Y::kStageUsers);
     }
-    for (int w = 0; w < Y::NW; ++w)
+    for (int w = 0; w < NW; ++w)
       for (int s = 0; s < 2; ++s) {
         tc::mbar_init(bar_ready(w, s), 1);
         tc::mbar_init(bar_free(w, s), Y::kReaders);
@@ -101,24 +103,12 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   }
 
   const Lane L(lane);
-  const int role = warp / Y::NW;                 // 0: chain, 1: output (kOut), last: store
-  const int cw = warp - role * Y::NW;            // column group inside the CTA
+  const int role = warp / NW;                 // 0: chain, 1: output (kOut), last: store
+  const int cw = warp - role * NW;            // column group inside the CTA
   const int v0 = 16 * (grp0 + cw);               // first value column of the warp
   const int piece = 2 * ((grp0 + cw) & 3);       // its 16-byte piece inside the 64-column block
   unsigned char* const slot0 = sm + Y::oSlots + cw * 2 * Y::kSlot + 16 * lane;
   const size_t gld = (size_t)H * kD;
-  // acc[tok tiles] += a (k step ks) x tile rows [tok][k], the fragments first
-  auto product = [&](float (&acc)[8][4], const uint32_t (&a)[4], uint32_t tile, int ks) {
-    uint32_t b[4][4];
-#pragma unroll
-    for (int np = 0; np < 4; ++np) ldb_n(b[np], tile, L, ks, np);
-#pragma unroll
-    for (int np = 0; np < 4; ++np) {
-      mma_bf16(acc[2 * np], a, b[np][0], b[np][1]);
-      mma_bf16(acc[2 * np + 1], a, b[np][2], b[np][3]);
-    }
-  };
-
   if (role == 0) {
     // ------------------------------------------------------------------------ the chain
     float S[16][4];  // S^T: rows v0 + g, v0 + g + 8, columns k = 8 nt + 2 t, + 1
@@ -129,26 +119,30 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       for (int e = 0; e < 4; ++e)
         S[nt][e] = p.S0 ? p.S0[sbase + (size_t)(8 * nt + 2 * L.t + (e & 1)) * kD + 8 * (e >> 1)] : 0.f;
     const uint32_t one = identity_b(L);
+    bool tried = false;
     for (int i = 0; i < sq.nchunks; ++i) {
       const int s = i % Y::kStages;
       const uint32_t st = base + s * Y::kStage;
       unsigned char *stp = sm + s * Y::kStage, *sl = slot0 + (i & 1) * Y::kSlot;
-      ok = i < 2 ? tc::mbar_wait(bar_full(s), (i / Y::kStages) & 1)
-                 : mbar_wait2(bar_full(s), (i / Y::kStages) & 1, bar_free(cw, i & 1), ((i >> 1) - 1) & 1);
-      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      // (for the first two chunks the slot is free as it stands: the parity of the phase before the first)
+      ok = mbar_wait2(tried, bar_full(s), (i / Y::kStages) & 1, bar_free(cw, i & 1), ((i >> 1) - 1) & 1);
+      if (!ok) break;
+      Frags b[2];
+      load_n(b[0], st + Y::oW, L, 0);
       uint32_t u[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) ld_cols(u[j], st + Y::oU, L, j, piece);
       float acc[8][4];
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
         uint32_t a[4], na[4];
+        if (ks < 7) load_n(b[(ks + 1) & 1], st + Y::oW, L, ks + 1);
+        else load_t(b[0], st + Y::oKg, L, 0);  // the state update's first fragments
+        if (ks >= 4) ld_cols(u[ks - 4], st + Y::oU, L, ks - 4, piece);
         pack_a(a, S, ks);
 #pragma unroll
         for (int x = 0; x < 4; ++x) na[x] = a[x] ^ 0x80008000u;
-        product(acc, na, st + Y::oW, ks);
+        mma4(acc, na, b[ks & 1]);
         put4(sl + ks * 512, a);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {  // S *= Gam_last
@@ -174,7 +168,9 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
         put4(sl + 4096 + j * 512, e[j]);
       }
       warp_arrive(bar_ready(cw, i & 1), lane);
-      update_state(S, f, st + Y::oKg, L);
+      tried = mbar_try2(bar_full((i + 1) % Y::kStages), ((i + 1) / Y::kStages) & 1, bar_free(cw, (i + 1) & 1),
+                        (((i + 1) >> 1) - 1) & 1);
+      update_state(S, f, st + Y::oKg, L, b[0]);
       warp_arrive(bar_empty(s), lane);
     }
     if (ok && p.ST) {
@@ -193,8 +189,9 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       const int tok0 = sq.bos + i * kChunk, valid = min(kChunk, sq.len - i * kChunk);
       const size_t chh = (size_t)(sq.chunk0 + i) * H + h;
       // (the chunk's tiles stood before the chain could write its h: the first wait only orders the reads)
-      ok = mbar_wait2(bar_full(s), (i / Y::kStages) & 1, bar_ready(cw, i & 1), (i >> 1) & 1);
-      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      const bool tried = mbar_try2(bar_full(s), (i / Y::kStages) & 1, bar_ready(cw, i & 1), (i >> 1) & 1);
+      ok = mbar_wait2(tried, bar_full(s), (i / Y::kStages) & 1, bar_ready(cw, i & 1), (i >> 1) & 1);
+      if (!ok) break;
       uint32_t a[8][4], e[4][4];
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) get4(sl + ks * 512, a[ks]);
@@ -214,18 +211,23 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       float acc[8][4];
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+      Frags b[2];
+      load_n(b[0], st + Y::oQg, L, 0);
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) product(acc, a[ks], st + Y::oQg, ks);
+      for (int ks = 0; ks < 8; ++ks) {
+        if (ks < 7) load_n(b[(ks + 1) & 1], st + Y::oQg, L, ks + 1);
+        else load_n(b[0], st + Y::oP, L, 0);
+        mma4(acc, a[ks], b[ks & 1]);
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 b0 = get2f(stp + Y::oBeta + (16 * j + 2 * L.t) * 4), b1 = get2f(stp + Y::oBeta + (16 * j + 8 + 2 * L.t) * 4);
+        if (j < 3) load_n(b[(j + 1) & 1], st + Y::oP, L, j + 1);
+        const Frags& pf = b[j & 1];
 #pragma unroll
-        for (int np = 0; np < 4; ++np) {
-          if (np < j) continue;  // P is lower triangular: those tokens come before the ones of this k step
-          uint32_t b[4];
-          ldb_n(b, st + Y::oP, L, j, np);
-          mma_bf16(acc[2 * np], e[j], scale_pair(b[0], b0), scale_pair(b[1], b1));
-          mma_bf16(acc[2 * np + 1], e[j], scale_pair(b[2], b0), scale_pair(b[3], b1));
+        for (int np = j; np < 4; ++np) {  // P is lower triangular: tokens before the k step's own see none of it
+          mma_bf16(acc[2 * np], e[j], scale_pair(pf.r[np][0], b0), scale_pair(pf.r[np][1], b1));
+          mma_bf16(acc[2 * np + 1], e[j], scale_pair(pf.r[np][2], b0), scale_pair(pf.r[np][3], b1));
         }
       }
       warp_arrive(bar_free(cw, i & 1), lane);
@@ -251,6 +253,15 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
     p.o[((size_t)sq.bos * H + h) * kD + v0 + lane] = __float2bfloat16(__int_as_float(0x7fc00000));
 }
 
+template <int NW, bool kOut>
+static int launch(const CUtensorMap (&tm)[5], const ScanFwdParams& sp, int units, cudaStream_t st) {
+  using Y = ScanFwdLay<NW, kOut>;
+  if (!ensure_dynamic_smem(pkda_scan_fwd_cols_kernel<NW, kOut>, Y::kSmem)) return PKDA_ERR_LAUNCH;
+  pkda_scan_fwd_cols_kernel<NW, kOut><<<units * Y::kSplit, Y::kThreads, Y::kSmem, st>>>(tm[0], tm[1], tm[2], tm[3],
+                                                                                       tm[4], sp);
+  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+}
+
 // o == NULL: h, v_new and the final state only.
 int launch_scan_fwd_cols(const Geo& geo, int total_tokens, int units, const bf16* w, const bf16* kg, const bf16* u,
                          const float* beta_c, const float* gc, const float* S0, bf16* h, bf16* v_new, float* ST,
@@ -268,16 +279,9 @@ int launch_scan_fwd_cols(const Geo& geo, int total_tokens, int units, const bf16
   ScanFwdParams sp;
   sp.geo = geo; sp.beta_c = beta_c; sp.gc = gc; sp.S0 = S0; sp.h = h; sp.v_new = v_new; sp.ST = ST; sp.o = o;
   sp.status = status;
-  if (o) {
-    if (!ensure_dynamic_smem(pkda_scan_fwd_cols_kernel<true>, ScanFwdLay<true>::kSmem)) return PKDA_ERR_LAUNCH;
-    pkda_scan_fwd_cols_kernel<true><<<units * 4, ScanFwdLay<true>::kThreads, ScanFwdLay<true>::kSmem, st>>>(
-        tm[0], tm[1], tm[2], tm[3], tm[4], sp);
-  } else {
-    if (!ensure_dynamic_smem(pkda_scan_fwd_cols_kernel<false>, ScanFwdLay<false>::kSmem)) return PKDA_ERR_LAUNCH;
-    pkda_scan_fwd_cols_kernel<false><<<units * 4, ScanFwdLay<false>::kThreads, ScanFwdLay<false>::kSmem, st>>>(
-        tm[0], tm[1], tm[2], tm[3], tm[4], sp);
-  }
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  const int split = scan_columns(units);
+  if (o) return split == 8 ? launch<1, true>(tm, sp, units, st) : launch<2, true>(tm, sp, units, st);
+  return split == 8 ? launch<1, false>(tm, sp, units, st) : launch<2, false>(tm, sp, units, st);
 }
 
 }  // namespace pkda
