@@ -160,8 +160,9 @@ __device__ __forceinline__ void for_tile(const float (&t)[2][4], int i0, int j0,
     for (int e = 0; e < 4; ++e) f(i0 + gq + 8 * (e >> 1), j0 + 8 * nt + 2 * tq + (e & 1), t[nt][e]);
 }
 
-// kRecompute: rebuild w,u,kg,qg only (backward's lean mode); the products, the
-// write keys and the decay totals already exist and are left untouched.
+// kRecompute: rebuild w,u,kg,qg only (backward's lean mode); the products, their inverse T (as it was
+// rounded for W and U), the write keys and the decay totals already exist, so the levels and the inversion
+// are left out (1,300 strongly decaying chunks: 178 us with them, 77 without).
 // One (chunk bx, head by) item; every thread of the CTA takes part.
 template <bool kRecompute>
 __device__ __forceinline__ void intra_fwd_item(const IntraParams& p, int bx, int by) {
@@ -216,7 +217,11 @@ __device__ __forceinline__ void intra_fwd_item(const IntraParams& p, int bx, int
   if (!kRecompute && tid >= kD && tid < 2 * kD) a_first = p.a_start[chh * kD + tid - kD];
   tile_load_async(sQ, kLdD, p.q + row0, gld, kChunk, kD, valid, kThreads);
   tile_load_async(sK, kLdD, p.k + row0, gld, kChunk, kD, valid, kThreads);
-  if (kRecompute) tile_load_async(sKt, kLdD, p.kt + row0, gld, kChunk, kD, valid, kThreads);
+  if (kRecompute) {
+    tile_load_async(sKt, kLdD, p.kt + row0, gld, kChunk, kD, valid, kThreads);
+    tile_load_async(sTmb, kLdC, p.Akk + ((size_t)tok0 * H + h) * kChunk, (long)H * kChunk, kChunk, kChunk, valid, kThreads);
+    tile_load_async(sXk, kLdD, p.v + row0, gld, kChunk, kD, valid, kThreads);
+  }
   cp_async_commit();
   if (tid < kChunk) {
     const bool ok = tid < valid;
@@ -226,8 +231,9 @@ __device__ __forceinline__ void intra_fwd_item(const IntraParams& p, int bx, int
   } else if (tid < kChunk + kD) {
     sBias[tid - kChunk] = s_bias;
   }
-  // zero the P staging tile (upper triangle must read as zero)
-  for (int i = tid; i < kChunk * kLdC / 8; i += kThreads) reinterpret_cast<uint4*>(sTmb)[i] = make_uint4(0, 0, 0, 0);
+  if (!kRecompute) {  // zero the P staging tile (upper triangle must read as zero)
+    for (int i = tid; i < kChunk * kLdC / 8; i += kThreads) reinterpret_cast<uint4*>(sTmb)[i] = make_uint4(0, 0, 0, 0);
+  }
   __syncthreads();
 
   // ---- 2. decay gate (elementwise, all threads; the q and k tiles are still landing), then
@@ -237,13 +243,15 @@ __device__ __forceinline__ void intra_fwd_item(const IntraParams& p, int bx, int
   __syncthreads();
   if (tid < kD) {
     gate_cumsum(sG, tid);
-    float dmax[6];
-    block_decay_max(sG, tid, dmax);
+    if (!kRecompute) {
+      float dmax[6];
+      block_decay_max(sG, tid, dmax);
 #pragma unroll
-    for (int e = 0; e < 6; ++e) {
+      for (int e = 0; e < 6; ++e) {
 #pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) dmax[e] = fmaxf(dmax[e], __shfl_xor_sync(0xffffffffu, dmax[e], o));
-      if (lane == 0) sWarpMax[warp * 6 + e] = dmax[e];
+        for (int o = 16; o >= 1; o >>= 1) dmax[e] = fmaxf(dmax[e], __shfl_xor_sync(0xffffffffu, dmax[e], o));
+        if (lane == 0) sWarpMax[warp * 6 + e] = dmax[e];
+      }
     }
   } else if (!kRecompute && tid < 2 * kD) {
     const int c = tid - kD;
@@ -277,6 +285,7 @@ __device__ __forceinline__ void intra_fwd_item(const IntraParams& p, int bx, int
     __syncthreads();
   }
 
+  if (!kRecompute) {
   // ---- 3. gated pair products, level by level.
   // warps 0-7 : (mat, I) own the diagonal 16x16 tile (I,I): levels 8,4,2,1 (and the ungated diagonal of P)
   // warps 8-15: (mat, idx) own one tile of level 32 and (idx < 2) one tile of level 16
@@ -365,7 +374,7 @@ __device__ __forceinline__ void intra_fwd_item(const IntraParams& p, int bx, int
     }
   }
   __syncthreads();
-  if (!kRecompute) {
+  {
     for (int i = tid; i < kChunk * kChunk / 8; i += kThreads) {
       const int r = i >> 3, c8 = (i & 7) << 3;
       if (r < valid)
@@ -380,16 +389,19 @@ __device__ __forceinline__ void intra_fwd_item(const IntraParams& p, int bx, int
     const int r = i >> 5, c2 = (i & 31) << 1;
     const uint32_t pk = pack_bf16(sT[r * kLdL + c2], sT[r * kLdL + c2 + 1]);
     *reinterpret_cast<uint32_t*>(sTmb + r * kLdC + c2) = pk;
-    if (!kRecompute && r < valid)
+    if (r < valid)
       *reinterpret_cast<uint32_t*>(p.Akk + ((size_t)(tok0 + r) * H + h) * kChunk + c2) = pk;
   }
   __syncthreads();
+  }  // !kRecompute
 
   // ---- 6. decayed operands: Kd -> smem; qg, kg, gc -> global; V tile -> smem
   bf16* sKd = sXq;
   bf16* sV = sXk;
-  tile_load_async(sV, kLdD, p.v + row0, gld, kChunk, kD, valid, kThreads);
-  cp_async_commit();
+  if (!kRecompute) {
+    tile_load_async(sV, kLdD, p.v + row0, gld, kChunk, kD, valid, kThreads);
+    cp_async_commit();
+  }
   for (int idx = tid; idx < kChunk * kD / 8; idx += kThreads) {
     const int r = idx >> 4, c8 = (idx & 15) << 3;
     const float4 g0 = *reinterpret_cast<const float4*>(sG + r * kLdG + c8);

@@ -35,6 +35,9 @@
 
 namespace pkda {
 
+// 2^-(kDirectLimit + 1)
+constexpr float kSurelySlow = 9.62964972e-35f;
+
 namespace intratc {
 constexpr int kThreads = 256;
 constexpr int kLdL = 68;                    // row stride of L and T: float4 rows, and conflict-free MMA fragments
@@ -160,6 +163,23 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   // compiler from computing all of them ahead of the loop and holding them in registers.
   uint32_t dbase = base;
   asm volatile("" : "+r"(dbase));
+
+  // When recomputing, the chunk's decay totals are known: one that is past the limit by more than the
+  // rounding of their base-2 exponential is handed over before anything of it is loaded (strongly decaying
+  // gates: 50 -> 18 us for the pass over 1,536 chunks); near the limit the totals are formed as the forward
+  // formed them, so that both passes decide alike.
+  if (kRecompute) {
+    const float least = tid < kD ? p.gc[chh * kD + tid] : 1.f;
+    if (__syncthreads_or(least < kSurelySlow)) {
+      if (tid == 0) {
+        p.slow_list[atomicAdd(p.counts + 1, 1)] = item;
+        s_next = atomicAdd(p.counts, 1);
+      }
+      __syncthreads();
+      draw = s_next;
+      continue;
+    }
+  }
 
   // ---- 0. V (and T when recomputing) by TMA; this thread's strips of g, k and q by cp.async
   if (tid == 0) {
