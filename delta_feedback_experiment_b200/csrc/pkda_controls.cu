@@ -28,6 +28,7 @@ struct CtrlParams {
   const float* d_g_atk;
   void* d_packed;
   float* part;  // [gridDim.x][2][heads]
+  int pairs;    // the hidden slices can be moved two elements at a time
 };
 
 constexpr int kCtrlThreads = 256;
@@ -50,56 +51,101 @@ pkda_controls_fwd_kernel(const CtrlParams p) {
 
 // One thread per (row, column of the packed gradient).  Columns of the three logit
 // slices recompute their activation from the saved packed row.
+// Backward: the packed gradient row and the per-head parameter gradients.  A CTA owns a contiguous range of
+// rows and takes ctrl_rows(H) of them at a time: the two hidden slices are copied and the three activations
+// differentiated with one element (or pair) per thread, the contributions to the per-head sums go through
+// shared memory and are added rows ascending, so that the sums have a fixed order.  (Row after row with one
+// thread per column took a memory round trip per row: 45 us for 2,000 rows of 280, now 5.)
+__host__ __device__ inline int ctrl_rows(int heads) { return heads >= 512 ? 1 : heads >= 256 ? 4 : 8; }
+
 template <typename T>
 __global__ void __launch_bounds__(kCtrlThreads)
 pkda_controls_bwd_kernel(const CtrlParams p) {
-  extern __shared__ float sAcc[];  // [2][heads] per-CTA partial sums, then the block reduction scratch
-  const int H = p.heads, D = p.hidden, total = p.total;
-  for (int i = threadIdx.x; i < 2 * H; i += blockDim.x) sAcc[i] = 0.f;
+  extern __shared__ float sAcc[];  // [2][H] sums of the CTA, then [2][rows][H] contributions
+  const int H = p.heads, D = p.hidden, total = p.total, tid = threadIdx.x;
+  const int R = ctrl_rows(H);
+  float* sPart = sAcc + 2 * H;
+  for (int i = tid; i < 2 * H; i += kCtrlThreads) sAcc[i] = 0.f;
   __syncthreads();
   const T* packed = static_cast<const T*>(p.packed);
   T* out = static_cast<T*>(p.d_packed);
-  // a CTA owns a contiguous range of rows, so that its per-head sums are added in a fixed order
+  const T *h0 = static_cast<const T*>(p.d_hidden0), *h1 = static_cast<const T*>(p.d_hidden1);
   const long long rows_per = (p.rows + gridDim.x - 1) / gridDim.x;
   const long long r_begin = (long long)blockIdx.x * rows_per;
   const long long r_end = r_begin + rows_per < p.rows ? r_begin + rows_per : p.rows;
-  for (long long r = r_begin; r < r_end; ++r) {
-    for (int c = threadIdx.x; c < total; c += blockDim.x) {
-      float v;
-      if (c < D) {
-        v = p.d_hidden0 ? to_f(static_cast<const T*>(p.d_hidden0)[r * D + c]) : 0.f;
-      } else if (c >= D + 3 * H) {
-        v = p.d_hidden1 ? to_f(static_cast<const T*>(p.d_hidden1)[r * D + (c - D - 3 * H)]) : 0.f;
-      } else {
-        const int s = (c - D) / H, h = (c - D) - s * H;
-        const float logit = to_f(packed[r * total + c]);
-        if (s == 1) {
-          const float dg = p.d_g_atk ? p.d_g_atk[r * H + h] : 0.f;
-          const float z = logit + p.dt_bias[h], ea = expf(p.A_log[h]);
-          v = dg * (-ea) / (1.f + expf(-z));            // d softplus = sigmoid
-          // fixed order: thread c alone accumulates head h of this CTA, rows ascending
-          sAcc[h] += dg * (-ea) * softplus_acc(z);       // d/dA_log = g_atk
-          sAcc[H + h] += v;                              // d/ddt_bias
-        } else {
-          const T* dsrc = static_cast<const T*>(s == 0 ? p.d_beta : p.d_beta_atk);
-          const float dv = dsrc ? to_f(dsrc[r * H + h]) : 0.f;
-          const float sg = 1.f / (1.f + expf(-logit));
-          v = dv * sg * (1.f - sg);
-        }
+  struct alignas(2 * sizeof(T)) Pair { T a, b; };
+  for (long long r0 = r_begin; r0 < r_end; r0 += R) {
+    const int nr = (int)(r_end - r0 < R ? r_end - r0 : R);
+    if (p.pairs) {
+      const int w = D >> 1;
+      const Pair zero = {from_f<T>(0.f), from_f<T>(0.f)};
+      for (int i = tid; i < nr * w; i += kCtrlThreads) {
+        const int r = i / w, c = 2 * (i - r * w);
+        const Pair x = h0 ? *reinterpret_cast<const Pair*>(h0 + (r0 + r) * D + c) : zero;
+        const Pair y = h1 ? *reinterpret_cast<const Pair*>(h1 + (r0 + r) * D + c) : zero;
+        T* row = out + (r0 + r) * total + c;
+        *reinterpret_cast<Pair*>(row) = x;
+        *reinterpret_cast<Pair*>(row + D + 3 * H) = y;
       }
-      out[r * total + c] = from_f<T>(v);
+    } else {
+      for (int i = tid; i < nr * D; i += kCtrlThreads) {
+        const int r = i / D, c = i - r * D;
+        T* row = out + (r0 + r) * total + c;
+        row[0] = h0 ? h0[(r0 + r) * D + c] : from_f<T>(0.f);
+        row[D + 3 * H] = h1 ? h1[(r0 + r) * D + c] : from_f<T>(0.f);
+      }
     }
+    for (int i = tid; i < nr * H; i += kCtrlThreads) {
+      const int r = i / H, h = i - r * H;
+      const long long at = (r0 + r) * H + h;
+      const T* in = packed + (r0 + r) * total + D + h;
+      T* row = out + (r0 + r) * total + D + h;
+      const float l0 = to_f(in[0]), l2 = to_f(in[2 * H]), z = to_f(in[H]) + p.dt_bias[h], ea = expf(p.A_log[h]);
+      const float d0 = p.d_beta ? to_f(static_cast<const T*>(p.d_beta)[at]) : 0.f;
+      const float d1 = p.d_g_atk ? p.d_g_atk[at] : 0.f;
+      const float d2 = p.d_beta_atk ? to_f(static_cast<const T*>(p.d_beta_atk)[at]) : 0.f;
+      const float s0 = 1.f / (1.f + expf(-l0)), s2 = 1.f / (1.f + expf(-l2));
+      const float v = d1 * (-ea) / (1.f + expf(-z));   // d softplus = sigmoid
+      row[0] = from_f<T>(d0 * s0 * (1.f - s0));
+      row[H] = from_f<T>(v);
+      row[2 * H] = from_f<T>(d2 * s2 * (1.f - s2));
+      const float da = d1 * (-ea) * softplus_acc(z);   // d/dA_log = g_atk;  v = d/ddt_bias
+      if (R == 1) {
+        sAcc[i] += da;
+        sAcc[H + i] += v;
+      } else {
+        sPart[i] = da;
+        sPart[R * H + i] = v;
+      }
+    }
+    if (R == 1) continue;  // (a head belongs to one thread)
+    __syncthreads();
+    for (int i = tid; i < 2 * H; i += kCtrlThreads) {
+      const float* col = i < H ? sPart + i : sPart + R * H + (i - H);
+      float acc = sAcc[i];
+      for (int r = 0; r < nr; ++r) acc += col[r * H];
+      sAcc[i] = acc;
+    }
+    __syncthreads();
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * H; i += blockDim.x) p.part[(size_t)blockIdx.x * 2 * H + i] = sAcc[i];
+  for (int i = tid; i < 2 * H; i += kCtrlThreads) p.part[(size_t)blockIdx.x * 2 * H + i] = sAcc[i];
 }
 
-__global__ void pkda_controls_reduce_kernel(const float* part, float* dA_log, float* ddt_bias, int heads, int groups) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 2 * heads) return;
+// One CTA per sum: strided partial sums, then a tree (fixed order).
+__global__ void __launch_bounds__(128)
+pkda_controls_reduce_kernel(const float* part, float* dA_log, float* ddt_bias, int heads, int groups) {
+  __shared__ float s[128];
+  const int i = blockIdx.x, tid = threadIdx.x;
   float a = 0.f;
-  for (int g = 0; g < groups; ++g) a += part[(size_t)g * 2 * heads + i];
-  if (i < heads) dA_log[i] = a; else ddt_bias[i - heads] = a;
+  for (int g = tid; g < groups; g += 128) a += part[(size_t)g * 2 * heads + i];
+  s[tid] = a;
+  __syncthreads();
+  for (int o = 64; o >= 1; o >>= 1) {
+    if (tid < o) s[tid] += s[tid + o];
+    __syncthreads();
+  }
+  if (tid == 0) (i < heads ? dA_log[i] : ddt_bias[i - heads]) = s[0];
 }
 
 // out[r][:] = concat of five slices
@@ -130,13 +176,14 @@ static int ctrl_check(const pkda_controls_args& a, CtrlParams& p) {
   p.packed = a.packed; p.A_log = a.A_log_precond; p.dt_bias = a.dt_bias_precond;
   p.beta = a.beta; p.beta_atk = a.beta_atk; p.g_atk = a.g_atk;
   p.d_hidden0 = a.d_decay_hidden; p.d_beta = a.d_beta; p.d_beta_atk = a.d_beta_atk; p.d_hidden1 = a.d_gate_hidden;
-  p.d_g_atk = a.d_g_atk; p.d_packed = a.d_packed; p.part = nullptr;
+  p.d_g_atk = a.d_g_atk; p.d_packed = a.d_packed; p.part = nullptr; p.pairs = 0;
   return PKDA_OK;
 }
 
 static int ctrl_bwd_grid(const pkda_controls_args& a) {
-  const long long want = (a.rows + 31) / 32;  // at least 32 rows per CTA
-  return (int)(want < 1 ? 1 : (want < 1184 ? want : 1184));
+  const int r = ctrl_rows(a.heads);
+  const long long want = (a.rows + r - 1) / r;  // one turn per CTA until the chip is full several times over
+  return (int)(want < 1 ? 1 : (want < 2368 ? want : 2368));
 }
 
 int controls_fwd(const pkda_controls_args* a, cudaStream_t st) {
@@ -172,13 +219,18 @@ int controls_bwd(const pkda_controls_args* a, cudaStream_t st) {
   if (!a->workspace || a->workspace_bytes < controls_bwd_workspace(*a)) return PKDA_ERR_WORKSPACE;
   p.part = static_cast<float*>(a->workspace);
   const int grid = ctrl_bwd_grid(*a);
-  const size_t smem = (size_t)2 * a->heads * sizeof(float);
+  const int turn = ctrl_rows(a->heads);
+  const size_t smem = (size_t)2 * a->heads * (turn == 1 ? 1 : 1 + turn) * sizeof(float);
+  // pairs: every slice starts at an even column of an even row, and every tensor at a pair
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(a->d_decay_hidden) | reinterpret_cast<uintptr_t>(a->d_gate_hidden) |
+                         reinterpret_cast<uintptr_t>(a->d_packed);
+  p.pairs = !(a->heads & 1) && !(a->hidden & 1) && ptrs % (a->dtype == PKDA_BF16 ? 4 : 8) == 0;
   begin_stage(kStageControlsBwd, st);
   if (a->dtype == PKDA_BF16) pkda_controls_bwd_kernel<bf16><<<grid, kCtrlThreads, smem, st>>>(p);
   else pkda_controls_bwd_kernel<float><<<grid, kCtrlThreads, smem, st>>>(p);
   end_stage(st);
   begin_stage(kStageControlsBwd, st);
-  pkda_controls_reduce_kernel<<<(2 * a->heads + 127) / 128, 128, 0, st>>>(p.part, a->dA_log_precond, a->ddt_bias_precond,
+  pkda_controls_reduce_kernel<<<2 * a->heads, 128, 0, st>>>(p.part, a->dA_log_precond, a->ddt_bias_precond,
                                                                          a->heads, grid);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
