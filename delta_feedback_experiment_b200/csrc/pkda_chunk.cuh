@@ -236,37 +236,8 @@ __device__ __forceinline__ void warp_gemm_lvl(float (&acc)[1][kNT][4], const bf1
 }
 
 // One doubling step of the triangular inverse: for every pair of inverted diagonal
-// blocks T11, T22 of size N and their coupling block L21, T21 = -T22 (L21 T11).
-// Loops run over full N (the blocks' upper triangles are zero) so they unroll.
-template <int N>
-__device__ __forceinline__ void inverse_merge(const float* sL, float* sT, float* sY2, int ldl, int ldt, int tid,
-                                              int nthreads) {
-  constexpr int SH = N == 4 ? 2 : (N == 8 ? 3 : (N == 16 ? 4 : 5));
-  for (int o = tid; o < 32 * N; o += nthreads) {
-    const int pr = o >> (2 * SH), r = (o >> SH) & (N - 1), c = o & (N - 1);
-    const int base = pr * 2 * N;
-    const float* Lrow = sL + (base + N + r) * ldl + base;
-    const float* Tcol = sT + base * ldt + base + c;
-    float s = 0.f;
-#pragma unroll
-    for (int m = 0; m < N; ++m) s += Lrow[m] * Tcol[m * ldt];
-    sY2[o] = s;
-  }
-  __syncthreads();
-  for (int o = tid; o < 32 * N; o += nthreads) {
-    const int pr = o >> (2 * SH), r = (o >> SH) & (N - 1), c = o & (N - 1);
-    const int base = pr * 2 * N;
-    const float* Trow = sT + (base + N + r) * ldt + base + N;
-    const float* Ycol = sY2 + (pr << (2 * SH)) + c;
-    float t = 0.f;
-#pragma unroll
-    for (int m = 0; m < N; ++m) t -= Trow[m] * Ycol[m << SH];
-    sT[(base + N + r) * ldt + base + c] = t;
-  }
-  __syncthreads();
-}
-
-// The same merge on the tensor cores for N = 16 and 32: both products as
+// blocks T11, T22 of size N (16 or 32) and their coupling block L21,
+// T21 = -T22 (L21 T11), on the tensor cores: both products as
 // mma.sync m16n8k8 TF32 with every fp32 operand split into a high and a low TF32
 // part (three MMAs per step: lo*hi + hi*lo + hi*hi), which keeps fp32-level
 // accuracy (the dropped lo*lo term is 2^-22 relative).  One warp per 16 x 8
@@ -348,33 +319,45 @@ __device__ __forceinline__ void inverse_merge_tc(const float* sL, float* sT, flo
   __syncthreads();
 }
 
-// T = (I + L)^-1 for a 64 x 64 strictly lower triangular L (fp32; row strides ldl of L
-// and ldt of T), all nthreads threads of the CTA (at least 256): 4 x 4 diagonal blocks by
-// forward substitution, then four doubling steps, the last two on the tensor cores.  sY2 is
-// a scratch of 1024 floats (kYPad = 0) or 1280 (kYPad = 8).  The result does not depend on
+// T = (I + L)^-1 for a 64 x 64 strictly lower triangular L (fp32; row strides ldl of L, a
+// multiple of 4, and ldt of T), all nthreads threads of the CTA (at least 256): the 16 x 16
+// diagonal blocks by forward substitution, one column per thread of two warps with the column in
+// registers, while the other warps zero the blocks above them; then two doubling steps on the
+// tensor cores.  (Substitution only up to 4 x 4 and two fp32 doubling steps more are six block
+// barriers and about 1,500 cycles of dependent shared-memory round trips instead of 500.)
+// sY2 is a scratch of 1024 floats (kYPad = 0) or 1280 (kYPad = 8).  The result does not depend on
 // the strides or on kYPad.  L must be visible to every thread on entry (a barrier after its
 // last write); ends with a __syncthreads().
 template <int kYPad = 0>
 __device__ __forceinline__ void unit_lower_inverse_64(const float* sL, float* sT, float* sY2, int ldl, int ldt, int tid,
                                                       int nthreads) {
-  for (int i = tid; i < kChunk * kChunk; i += nthreads) sT[(i >> 6) * ldt + (i & 63)] = 0.f;
-  __syncthreads();
   if (tid < 64) {
-    const int base = (tid >> 2) << 2, col = tid & 3;
-    float x[4];
+    const int base = tid & 48, col = tid & 15;
+    const float* L = sL + base * ldl + base;
+    float* T = sT + base * ldt + base + col;
+    float x[16];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float s = (i == col) ? 1.f : 0.f;
+    for (int i = 0; i < 16; ++i) {
+      float s = (i == col) ? 1.f : 0.f, s2 = 0.f;
 #pragma unroll
-      for (int m = 0; m < i; ++m) s -= sL[(base + i) * ldl + base + m] * x[m];
-      x[i] = s;
+      for (int m = 0; m < i; m += 4) {
+        const float4 l = *reinterpret_cast<const float4*>(L + i * ldl + m);
+        s -= l.x * x[m];
+        if (m + 1 < i) s2 -= l.y * x[m + 1];
+        if (m + 2 < i) s -= l.z * x[m + 2];
+        if (m + 3 < i) s2 -= l.w * x[m + 3];
+      }
+      x[i] = s + s2;
+      T[i * ldt] = x[i];
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) sT[(base + i) * ldt + base + col] = x[i];
+  } else {
+    // the 16 x 16 blocks above the diagonal: block rows 0..2, four columns per thread and step
+    for (int i = tid - 64; i < 48 * 16; i += nthreads - 64) {
+      const int r = i >> 4, c4 = (i & 15) << 2;
+      if ((c4 >> 4) > (r >> 4)) *reinterpret_cast<float4*>(sT + r * ldt + c4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
   __syncthreads();
-  inverse_merge<4>(sL, sT, sY2, ldl, ldt, tid, nthreads);
-  inverse_merge<8>(sL, sT, sY2, ldl, ldt, tid, nthreads);
   inverse_merge_tc<16, kYPad, true>(sL, sT, sY2, ldl, ldt, tid);
   inverse_merge_tc<32, kYPad, true>(sL, sT, sY2, ldl, ldt, tid);
 }
