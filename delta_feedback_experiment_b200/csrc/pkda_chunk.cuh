@@ -384,23 +384,28 @@ __device__ __forceinline__ void row_sums8(float (&v)[8], int lane) {
   v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-// Tail of the classifier kernels: a CTA of 256 threads has put the kind of its 64 items into sKind
-// (-1: none, 0: tensor-memory kernel, 1: mma.sync kernel) and appends them to the two work lists with
-// one atomic per list, keeping their order.
-__device__ __forceinline__ void append_work_items(const int* sKind, int* sBase, int* fast_list, int* slow_list,
+// Tail of the classifier kernel: a CTA has put the kind of its 64 items into sKind (-1: none, 0:
+// tensor-memory kernel, 1: mma.sync kernel) and their first tokens into sTok, and appends them to the two
+// work lists with one atomic per list, keeping their order.  One warp per list, two items per lane.
+__device__ __forceinline__ void append_work_items(const int* sKind, const int* sTok, int2* fast_list, int* slow_list,
                                                   int* counts, int first_item, int tid) {
   __syncthreads();
-  if (tid < 2) {
-    int cnt = 0;
-    for (int i = 0; i < 64; ++i) cnt += sKind[i] == tid;
-    sBase[tid] = cnt ? atomicAdd(counts + tid, cnt) : 0;
-  }
-  __syncthreads();
-  if (tid < 2) {
-    int* list = tid ? slow_list : fast_list;
-    int pos = sBase[tid];
-    for (int i = 0; i < 64; ++i)
-      if (sKind[i] == tid) list[pos++] = first_item + i;
+  const int list = tid >> 5, lane = tid & 31;
+  if (list >= 2) return;
+  const bool in0 = sKind[lane] == list, in1 = sKind[lane + 32] == list;
+  const uint32_t m0 = __ballot_sync(0xffffffffu, in0), m1 = __ballot_sync(0xffffffffu, in1);
+  const int n0 = __popc(m0), n1 = __popc(m1);
+  int at = 0;
+  if (lane == 0 && n0 + n1) at = atomicAdd(counts + list, n0 + n1);
+  at = __shfl_sync(0xffffffffu, at, 0);
+  const uint32_t below = (1u << lane) - 1;
+  const int p0 = at + __popc(m0 & below), p1 = at + n0 + __popc(m1 & below);
+  if (list) {
+    if (in0) slow_list[p0] = first_item + lane;
+    if (in1) slow_list[p1] = first_item + lane + 32;
+  } else {
+    if (in0) fast_list[p0] = make_int2(first_item + lane, sTok[lane]);
+    if (in1) fast_list[p1] = make_int2(first_item + lane + 32, sTok[lane + 32]);
   }
 }
 
@@ -466,17 +471,19 @@ struct IntraBwdParams {
   float *c_loc, *partC;
   float ln_x, eps;
   // Work lists of (chunk * heads + head) items written by pkda_bwd_classify_kernel: fast_list for the
-  // tensor-memory kernel, slow_list for the mma.sync kernel; fast_count[0] / fast_count[1] are their
+  // tensor-memory kernel (each with its chunk's first token: a full chunk is all that this kernel takes),
+  // slow_list for the mma.sync kernel; fast_count[0] / fast_count[1] are their
   // lengths and fast_count[2] the cursor the mma.sync CTAs draw items with (all zeroed before every
   // call).  slow_list == NULL: the mma.sync kernel takes every chunk, one CTA per (chunk, head).
-  int *fast_list, *slow_list, *fast_count;
+  int2* fast_list;
+  int *slow_list, *fast_count;
 };
 
 // tcgen05 / tensor-memory chunk-parallel backward stage (pkda_intra_bwd_tc.cu).
 int launch_intra_bwd_tc(const IntraBwdParams& ip, cudaStream_t st);
 // The backward's first kernel on the default path: sorts the items into the two work lists (counts zeroed
 // before) and packs beta chunk-major.
-int launch_bwd_classify(const Geo& geo, const float* gc, int direct_cap, int* fast_list, int* slow_list, int* counts,
+int launch_bwd_classify(const Geo& geo, const float* gc, int direct_cap, int2* fast_list, int* slow_list, int* counts,
                         const bf16* beta, float* beta_c, cudaStream_t st);
 
 // tcgen05 / TMA output stage (pkda_out_tc.cu).

@@ -1173,7 +1173,8 @@ struct BwdWorkspace {
   float* beta_c;
   bf16 *u, *dF, *dh;
   float *dk_read, *dkt, *partA, *partB, *partC, *c_loc, *lam_in;
-  int *fast_list, *slow_list, *counts;
+  int2* fast_list;
+  int *slow_list, *counts;
   int *fwd_lists, *fwd_counts;  // work lists of the recompute pass (lean backward)
   int* status;
   size_t bytes;
@@ -1201,7 +1202,7 @@ static BwdWorkspace carve_bwd(const pkda_problem& p, void* base) {
   w.partC = static_cast<float*>(take(chunks * H * 4));
   w.c_loc = static_cast<float*>(take(chunks * H * kD * 4));
   w.lam_in = static_cast<float*>(take(chunks * H * kD * 4));
-  w.fast_list = static_cast<int*>(take(chunks * H * sizeof(int)));
+  w.fast_list = static_cast<int2*>(take(chunks * H * sizeof(int2)));
   w.slow_list = static_cast<int*>(take(chunks * H * sizeof(int)));
   w.fwd_lists = static_cast<int*>(take(chunks * H * sizeof(int)));
   w.status = static_cast<int*>(take(16 * sizeof(int)));  // status word, then lengths and cursors of the work lists
@@ -1336,7 +1337,8 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   // Full chunks that are one direct block run on tcgen05 / tensor memory; a classifier in front sorts
   // the chunks into two work lists and the mma.sync kernel works off the second one (every chunk, one
   // CTA each, when it is pinned).
-  ip.fast_list = ip.slow_list = ip.fast_count = nullptr;
+  ip.fast_list = nullptr;
+  ip.slow_list = ip.fast_count = nullptr;
   int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (tc_intra) {
