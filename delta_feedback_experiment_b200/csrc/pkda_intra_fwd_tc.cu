@@ -16,9 +16,11 @@
 //    The two sequential passes over the rows (cumulative log-decay, the preconditioner
 //    recurrence A_t) are blocked scans: eight rows in registers, one exchange of (block total,
 //    block decay) through shared memory, then each block continues from the prefix it is owed.
-//  * q, k and the raw gate arrive by cp.async straight into the places of the operand tiles
-//    their gated values will take (128-byte-swizzled canonical layout); the gating happens in
-//    place, each thread touching only its own 8-byte pieces.  The rows of k and q are stacked
+//  * q, k and the raw gate arrive by TMA straight in the places of the operand tiles their
+//    gated values will take (128-byte-swizzled canonical layout); the gating happens in
+//    place, each thread touching only its own 8-byte pieces.  (24 eight-byte cp.async a thread
+//    instead cost 100 instructions of address arithmetic: 475 -> 467 us for 8 x 4,096 tokens of
+//    16 heads, 1,865 -> 1,795 us for 65,536 packed tokens of 32.)  The rows of k and q are stacked
 //    to one 128-row A operand, the write keys are the B operand: eight tcgen05.mma (M = 128,
 //    N = 64, K = 16) give M = k kt^T in accumulator rows 0..63 and P = q kt^T in rows 64..127.
 //    All eight warps read the accumulator back (one tensor-memory lane = one row per thread)
@@ -89,7 +91,9 @@ template <bool kRecompute>
 __global__ void __launch_bounds__(intratc::kThreads, 2)
 pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_akk,
                          const __grid_constant__ CUtensorMap tm_aqk, const __grid_constant__ CUtensorMap tm_w,
-                         const __grid_constant__ CUtensorMap tm_u, const IntraParams p) {
+                         const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_g,
+                         const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_q,
+                         const IntraParams p) {
   using namespace intratc;
   extern __shared__ unsigned char smem_raw[];
   const int H = p.geo.heads;
@@ -99,7 +103,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* tiles = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t bar_tma = base + oBar, bar_mma = base + oBar + 8, tmem_slot = base + oBar + 16;
+  const uint32_t bar_tma = base + oBar, bar_mma = base + oBar + 8, tmem_slot = base + oBar + 16, bar_in = base + oBar + 24;
   float* sL = reinterpret_cast<float*>(tiles + oL);
   float* sBeta = reinterpret_cast<float*>(tiles + oBeta);
   float* sDiag = reinterpret_cast<float*>(tiles + oDiag);
@@ -129,6 +133,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   if (tid == 0) {
     tc::mbar_init(bar_tma, 1);
     tc::mbar_init(bar_mma, 1);
+    tc::mbar_init(bar_in, 1);
     tc::fence_barrier_init();
   }
   if (warp == 1) tc::tmem_alloc(tmem_slot, kCols);
@@ -137,25 +142,38 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   tc::tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tiles + oBar + 16);
   bool ok = true;
-  uint32_t mma_phase = 0, tma_phase = 0;
+  uint32_t mma_phase = 0, tma_phase = 0, in_phase = 0;
   const int R = 32 * (warp & 3) + lane;     // this thread's accumulator row in the pair products
   const int ei = R & 63, j0 = 32 * (warp >> 2);
   const bool isP = (warp & 3) >= 2;
 
   // Items differ in cost (a chunk that is handed over costs a fraction of one that is finished), so
-  // the CTAs draw them one at a time from a cursor instead of striding through them.
-  __shared__ int s_next;
-  if (tid == 0) s_next = atomicAdd(p.counts, 1);
+  // the CTAs draw them one at a time from a cursor instead of striding through them.  One thread draws the
+  // next item and looks its chunk up while the current one waits for its products, and the item's rows are
+  // asked into L2 from then on: drawn at the end of an item, the cursor, the lookup and the rows were four
+  // dependent memory round trips of every item.  (An item only ever waits for items drawn before it, also
+  // for ones that are still next on their CTA, so the chained mode cannot lock up.)
+  __shared__ int4 s_item[2];  // {item or -1, first token, valid tokens, sequence}: this item, the next one
+  auto describe = [&](int draw) {
+    int4 it = make_int4(-1, 0, 0, 0);
+    if (draw < n_items) {
+      // in chained mode chunk level draw / units of unit draw % units (a dense batch)
+      const int level = chain ? draw / units : 0;
+      it.x = chain ? ((draw % units) / H * p.geo.chunks_per_seq + level) * H + (draw % units) % H : draw;
+      if (!chunk_lookup(p.geo, it.x / H, it.w, it.y, it.z)) it.x = -1;  // past the last real chunk of a packed batch (items ascend)
+    }
+    return it;
+  };
+  if (tid == kThreads - 1) s_item[0] = describe(atomicAdd(p.counts, 1));
   __syncthreads();
-  int draw = s_next;
+  int slot = 0;
 #pragma unroll 1
-  while (draw < n_items) {
-  // the draw-th item: in chained mode chunk level draw / units of unit draw % units (a dense batch)
-  const int level = chain ? draw / units : 0;
-  const int item = chain ? ((draw % units) / H * p.geo.chunks_per_seq + level) * H + (draw % units) % H : draw;
+  for (;; slot ^= 1) {
+  const int4 cur = s_item[slot];
+  const int item = cur.x, tok0 = cur.y, valid = cur.z, n = cur.w;
+  if (item < 0) break;
   const int h = item % H;
-  int n, tok0, valid;
-  if (!chunk_lookup(p.geo, item / H, n, tok0, valid)) break;  // past the last real chunk of a packed batch (items ascend)
+  const int level = chain ? (tok0 - n * p.geo.seq_len) / kChunk : 0;
   const size_t chh = (size_t)item;
   const size_t row0 = ((size_t)tok0 * H + h) * kD;
   const bool full = valid == kChunk;
@@ -171,33 +189,27 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   if (kRecompute) {
     const float least = tid < kD ? p.gc[chh * kD + tid] : 1.f;
     if (__syncthreads_or(least < kSurelySlow)) {
-      if (tid == 0) {
-        p.slow_list[atomicAdd(p.counts + 1, 1)] = item;
-        s_next = atomicAdd(p.counts, 1);
-      }
+      if (tid == 0) p.slow_list[atomicAdd(p.counts + 1, 1)] = item;
+      if (tid == kThreads - 1) s_item[slot ^ 1] = describe(atomicAdd(p.counts, 1));
       __syncthreads();
-      draw = s_next;
       continue;
     }
   }
 
-  // ---- 0. V (and T when recomputing) by TMA; this thread's strips of g, k and q by cp.async
+  // ---- 0. V (and T when recomputing) by TMA, and the strips of g, k and q, right into their operand slots
   if (tid == 0) {
     tc::mbar_expect_tx(bar_tma, kRecompute ? 16384 + 8192 : 16384);
     tc::tma_load_3d(base + oV, &tm_v, bar_tma, 0, h, tok0);
     tc::tma_load_3d(base + oV + 8192, &tm_v, bar_tma, 64, h, tok0);
     if (kRecompute) tc::tma_load_3d(base + oTm, &tm_akk, bar_tma, 0, h, tok0);
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const bool okr = r0 + i < valid;
-    const size_t off = row0 + (size_t)(okr ? r0 + i : 0) * gld + c4;
-    const int nb = okr ? 8 : 0;  // rows past the sequence end read as zero
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(yBase + slot_off(i))), "l"(p.g + off), "r"(nb));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(aBase + slot_off(i))), "l"(p.k + off), "r"(nb));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(aBase + 8192 + slot_off(i))), "l"(p.q + off), "r"(nb));
+  if (lane == 0) {  // two 64-channel blocks each, issued by six warps
+    const int b = warp & 1;
+    if (warp == 0) tc::mbar_expect_tx(bar_in, 6 * 8192);
+    if (warp < 2) tc::tma_load_3d(base + oY + b * 8192, &tm_g, bar_in, 64 * b, h, tok0);
+    else if (warp < 4) tc::tma_load_3d(base + oA + b * 16384, &tm_k, bar_in, 64 * b, h, tok0);
+    else if (warp < 6) tc::tma_load_3d(base + oA + 8192 + b * 16384, &tm_q, bar_in, 64 * b, h, tok0);
   }
-  cp_async_commit();
   uint2 ktraw[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -242,7 +254,17 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     }
     centre = p.log_atk_scale[h];
   }
-  cp_async_wait<0>();
+  ok = tc::mbar_wait(bar_in, in_phase) && ok;
+  in_phase ^= 1;
+  if (!full) {  // rows past the sequence end read as zero, whatever lies there
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (r0 + i >= valid) {
+        *reinterpret_cast<uint2*>(yBase + slot_off(i)) = make_uint2(0, 0);
+        *reinterpret_cast<uint2*>(aBase + slot_off(i)) = make_uint2(0, 0);
+        *reinterpret_cast<uint2*>(aBase + 8192 + slot_off(i)) = make_uint2(0, 0);
+      }
+  }
 
   // ---- 1. decay gate, strip-local cumulative sum; strip-local preconditioner scan from zero
   float G[8][4];
@@ -343,9 +365,9 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       if (tid == 0) p.slow_list[atomicAdd(p.counts + 1, 1)] = item;
       ok = tc::mbar_wait(bar_tma, tma_phase) && ok;  // the V tile in flight must land before the tile is reused
       tma_phase ^= 1;
-      if (tid == 0) s_next = atomicAdd(p.counts, 1);
+      if (tid == kThreads - 1) s_item[slot ^ 1] = describe(atomicAdd(p.counts, 1));
+      tc::fence_proxy_async();  // the strips have been read: the next item's copies may overwrite them
       __syncthreads();
-      draw = s_next;
       continue;
     }
   }
@@ -414,6 +436,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
         *reinterpret_cast<float4*>(p.gc + chh * kD + c4) = make_float4(glE[0], glE[1], glE[2], glE[3]);
     }
   }
+  int drawn = 0;
+  if (tid == kThreads - 1) drawn = atomicAdd(p.counts, 1);  // (not used before the products are back)
   tc::fence_proxy_async();
   tc::tc_fence_before();
   __syncthreads();  // (the strip exchange arrays are dead from here on: L takes their place)
@@ -473,8 +497,22 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
         *reinterpret_cast<uint4*>(tiles + oV + (pc >> 3) * 8192 + r * 128 + ((pc & 7) << 4)) = make_uint4(0, 0, 0, 0);
     }
   }
+  if (tid == kThreads - 1) s_item[slot ^ 1] = describe(drawn);
   tc::fence_proxy_async();
   __syncthreads();
+  {  // the next item's rows of g, k, q and v: one 256-byte request per thread
+    const int4 nx = s_item[slot ^ 1];
+    const int r = tid & 63;
+    if (nx.x >= 0 && r < nx.z) {
+      const bf16* const src[4] = {p.g, p.k, p.q, p.v};
+      const bf16* a = src[0];
+      if (tid >= 64) a = src[1];
+      if (tid >= 128) a = src[2];
+      if (tid >= 192) a = src[3];
+      a += ((size_t)(nx.y + r) * H + nx.x % H) * kD;
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], 256;" ::"l"(a) : "memory");
+    }
+  }
 
   if (!kRecompute) {
     // ---- 5. scaled P -> Aqk;  T = (I + L)^-1 -> bf16 operand tile and Akk
@@ -561,10 +599,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       tc::bulk_commit();
     }
     tc::bulk_wait_read();  // the tiles stay in place until every store of this item has read them
-    s_next = atomicAdd(p.counts, 1);
   }
   __syncthreads();  // the next item's copies overwrite the tiles
-  draw = s_next;
   }  // item loop
   if (__syncthreads_or(!ok) && tid == 0) atomicExch(p.status, 1);
   tc::tc_fence_before();
@@ -575,12 +611,13 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 // ------------------------------------------------------------------ host side
 int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) {
   const uint64_t H = ip.geo.heads, tok = ip.geo.total_tokens;
-  CUtensorMap tm_v, tm_akk, tm_aqk, tm_w, tm_u;
+  CUtensorMap tm_v, tm_akk, tm_aqk, tm_w, tm_u, tm_g, tm_k, tm_q;
   {
     const uint64_t dims[3] = {kD, H, tok}, str[2] = {kD * 2, H * kD * 2};
     const uint32_t box[3] = {64, 1, 64};
     if (!encode_bf16_map(&tm_v, ip.v, 3, dims, str, box) || !encode_bf16_map(&tm_w, ip.w, 3, dims, str, box) ||
-        !encode_bf16_map(&tm_u, ip.u, 3, dims, str, box))
+        !encode_bf16_map(&tm_u, ip.u, 3, dims, str, box) || !encode_bf16_map(&tm_g, ip.g, 3, dims, str, box) ||
+        !encode_bf16_map(&tm_k, ip.k, 3, dims, str, box) || !encode_bf16_map(&tm_q, ip.q, 3, dims, str, box))
       return PKDA_ERR_LAUNCH;
   }
   {
@@ -597,11 +634,13 @@ int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) 
   if (recompute) {
     if (!ensure_dynamic_smem(pkda_intra_fwd_tc_kernel<true>, intratc::kSmem, 100))
       return PKDA_ERR_LAUNCH;
-    pkda_intra_fwd_tc_kernel<true><<<grid, intratc::kThreads, intratc::kSmem, st>>>(tm_v, tm_akk, tm_aqk, tm_w, tm_u, ip);
+    pkda_intra_fwd_tc_kernel<true><<<grid, intratc::kThreads, intratc::kSmem, st>>>(tm_v, tm_akk, tm_aqk, tm_w, tm_u, tm_g,
+                                                                                  tm_k, tm_q, ip);
   } else {
     if (!ensure_dynamic_smem(pkda_intra_fwd_tc_kernel<false>, intratc::kSmem, 100))
       return PKDA_ERR_LAUNCH;
-    pkda_intra_fwd_tc_kernel<false><<<grid, intratc::kThreads, intratc::kSmem, st>>>(tm_v, tm_akk, tm_aqk, tm_w, tm_u, ip);
+    pkda_intra_fwd_tc_kernel<false><<<grid, intratc::kThreads, intratc::kSmem, st>>>(tm_v, tm_akk, tm_aqk, tm_w, tm_u, tm_g,
+                                                                                  tm_k, tm_q, ip);
   }
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
