@@ -47,7 +47,8 @@ __global__ void pkda_pack_beta_kernel(Geo geo, const bf16* beta, float* beta_c) 
 
 // Chunk-local preconditioner scan from A = 0: loc[c] = sum_j (prod_{m>j} d_m) bP_j k_j[c]^2
 // and the chunk's summed log-decay; also the chunk-major fp32 copy of beta (when beta_c is
-// given), which saves a launch.  grid (chunks, H), 256 threads: warp w scans rows 8w..8w+7 with
+// given), which saves a launch.  grid chunks * H, the heads of a chunk next to each other (they share the
+// sectors of the per-token scalars and lie side by side in k), 256 threads: warp w scans rows 8w..8w+7 with
 // lane l holding channels 4l..4l+3 (64-bit loads, one token row per warp request), then the
 // eight row blocks are chained in order through shared memory.
 __global__ void __launch_bounds__(256)
@@ -56,34 +57,51 @@ pkda_atk_local_kernel(Geo geo, const bf16* k, const float* g_atk, const bf16* be
   __shared__ __align__(16) float sEnd[8][kD];
   __shared__ float sDec[8], sSum[8];
   int n, tok0, valid;
-  if (!chunk_lookup(geo, blockIdx.x, n, tok0, valid)) return;
-  const int h = blockIdx.y, H = geo.heads, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const size_t chh = (size_t)blockIdx.x * H + h;
+  const int H = geo.heads, chunk = blockIdx.x / H, h = blockIdx.x % H;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (geo.cu_seqlens) {
+    // the whole CTA looks its chunk up at once (the sequences that start at or before it), one round trip
+    // instead of one per step of a binary search
+    n = -1;
+    for (int i0 = 0; i0 < geo.n_seqs; i0 += 256)
+      n += __syncthreads_count(i0 + tid < geo.n_seqs && geo.chunk_offsets[i0 + tid] <= chunk);
+    const int total = geo.chunk_offsets[geo.n_seqs], first = geo.chunk_offsets[n];
+    const int bos = geo.cu_seqlens[n], eos = geo.cu_seqlens[n + 1];
+    if (chunk >= total) return;
+    tok0 = bos + (chunk - first) * kChunk;
+    valid = min(kChunk, eos - tok0);
+  } else if (!chunk_lookup(geo, chunk, n, tok0, valid)) {
+    return;
+  }
+  const size_t chh = blockIdx.x;
   const int c4 = lane << 2, r0 = warp * 8;
   uint2 kraw[8];
-  float lg[8], bp[8];
+  float lg_l = 0.f, bp_l = 0.f;  // lane i < 8: the scalars of row r0 + i
+  if (lane < 8 && r0 + lane < valid) {  // all loads first
+    const size_t s = (size_t)(tok0 + r0 + lane) * H + h;
+    lg_l = g_atk[s];
+    bp_l = to_f(beta_atk[s]);
+  }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {  // all loads first
-    const int r = r0 + i;
-    const bool ok = r < valid;
-    const size_t s = (size_t)(tok0 + (ok ? r : 0)) * H + h;
+  for (int i = 0; i < 8; ++i) {
+    const bool ok = r0 + i < valid;
+    const size_t s = (size_t)(tok0 + (ok ? r0 + i : 0)) * H + h;
     kraw[i] = ok ? *reinterpret_cast<const uint2*>(k + s * kD + c4) : make_uint2(0, 0);
-    lg[i] = ok ? g_atk[s] : 0.f;
-    bp[i] = ok ? to_f(beta_atk[s]) : 0.f;
   }
   if (beta_c && tid < kChunk)
     beta_c[chh * kChunk + tid] = tid < valid ? to_f(beta[(size_t)(tok0 + tid) * H + h]) : 0.f;
   float a[4] = {0.f, 0.f, 0.f, 0.f}, dblk = 1.f, gsum = 0.f;
+  const float pd_l = __expf(lg_l);  // rows past the end: decay 1, beta 0
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float2 x = unpack_bf16(kraw[i].x), y = unpack_bf16(kraw[i].y);
-    const float pd = __expf(lg[i]);  // rows past the end: decay 1, beta 0
-    a[0] = pd * a[0] + bp[i] * x.x * x.x;
-    a[1] = pd * a[1] + bp[i] * x.y * x.y;
-    a[2] = pd * a[2] + bp[i] * y.x * y.x;
-    a[3] = pd * a[3] + bp[i] * y.y * y.y;
+    const float pd = __shfl_sync(0xffffffffu, pd_l, i), bp = __shfl_sync(0xffffffffu, bp_l, i);
+    a[0] = pd * a[0] + bp * x.x * x.x;
+    a[1] = pd * a[1] + bp * x.y * x.y;
+    a[2] = pd * a[2] + bp * y.x * y.x;
+    a[3] = pd * a[3] + bp * y.y * y.y;
     dblk *= pd;
-    gsum += lg[i];
+    gsum += __shfl_sync(0xffffffffu, lg_l, i);
   }
   *reinterpret_cast<float4*>(&sEnd[warp][c4]) = make_float4(a[0], a[1], a[2], a[3]);
   if (lane == 0) { sDec[warp] = dblk; sSum[warp] = gsum; }
@@ -911,9 +929,8 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
   // chunks itself (and packs beta).  Otherwise two small kernels in front do.
   const bool chained = forward_chain_possible(p);
   if (!chained) {
-    dim3 gridc(geo.total_chunks, p.heads);
     begin_stage(kStageAtkLocal, st);
-    pkda_atk_local_kernel<<<gridc, 256, 0, st>>>(geo, static_cast<const bf16*>(p.k), p.g_atk,
+    pkda_atk_local_kernel<<<geo.total_chunks * p.heads, 256, 0, st>>>(geo, static_cast<const bf16*>(p.k), p.g_atk,
                                                  static_cast<const bf16*>(p.beta_atk), static_cast<const bf16*>(p.beta),
                                                  a->ac_atk, a->sa_atk, ws.beta_c);
     PKDA_CHECK_LAUNCH();
