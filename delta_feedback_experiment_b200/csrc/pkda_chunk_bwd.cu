@@ -867,7 +867,7 @@ pkda_atk_bwd_kernel(const AtkBwdParams p, int n_tiles) {
     if (pos < n_tiles) {
       tile = (!kFinal && p.tile_list) ? p.tile_list[pos] : pos;
       int n;
-      live_n = chunk_lookup(p.geo, tile / H, n, tok0_n, valid_n);
+      live_n = chunk_lookup_warp(p.geo, tile / H, n, tok0_n, valid_n);
     }
     tile_n = tile;
     if (live_n) {

@@ -85,6 +85,29 @@ __device__ __forceinline__ bool chunk_lookup(const Geo& g, int c, int& n, int& t
   return true;
 }
 
+// The same, by all lanes of a warp together (one and the same c): the last 32 candidates are compared at
+// once, so that a packed batch of few sequences costs two dependent loads instead of six.
+__device__ __forceinline__ bool chunk_lookup_warp(const Geo& g, int c, int& n, int& tok0, int& valid) {
+  if (!g.cu_seqlens) return chunk_lookup(g, c, n, tok0, valid);
+  const int lane = threadIdx.x & 31, total = g.chunk_offsets[g.n_seqs];
+  int lo = 0, len = g.n_seqs;  // the sequence is one of [lo, lo + len)
+  while (len > 32) {
+    const int half = len >> 1;
+    if (g.chunk_offsets[lo + half] <= c) {
+      lo += half;
+      len -= half;
+    } else {
+      len = half;
+    }
+  }
+  n = lo + __popc(__ballot_sync(0xffffffffu, lane < len && g.chunk_offsets[lo + lane] <= c)) - 1;
+  const int first = g.chunk_offsets[n], bos = g.cu_seqlens[n], eos = g.cu_seqlens[n + 1];
+  if (c >= total) return false;
+  tok0 = bos + (c - first) * kChunk;
+  valid = min(kChunk, eos - tok0);
+  return true;
+}
+
 // ---------------------------------------------------------------- scalar math
 __device__ __forceinline__ float to_f(float x) { return x; }
 __device__ __forceinline__ float to_f(bf16 x) { return __bfloat162float(x); }

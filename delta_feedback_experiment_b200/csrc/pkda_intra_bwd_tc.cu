@@ -130,7 +130,7 @@ pkda_bwd_classify_kernel(Geo geo, const float* gc, int direct_cap, int2* fast_li
   for (int k = 0; k < 8; ++k) {
     const int chh = blockIdx.x * 64 + warp * 8 + k;
     int n;
-    live[k] = chh < items && chunk_lookup(geo, chh / H, n, tok0s[k], valids[k]);
+    live[k] = chh < items && chunk_lookup_warp(geo, chh / H, n, tok0s[k], valids[k]);  // (chh is the warp's)
     x[k] = make_float4(1.f, 1.f, 1.f, 1.f);
     bv[k][0] = bv[k][1] = 0.f;
     if (live[k]) {
