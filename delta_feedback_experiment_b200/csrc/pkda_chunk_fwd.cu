@@ -53,9 +53,10 @@ __global__ void pkda_pack_beta_kernel(Geo geo, const bf16* beta, float* beta_c) 
 // eight row blocks are chained in order through shared memory.
 __global__ void __launch_bounds__(256)
 pkda_atk_local_kernel(Geo geo, const bf16* k, const float* g_atk, const bf16* beta_atk, const bf16* beta,
-                      float* ac_local, float* sa, float* beta_c) {
+                      float* ac_local, float* sa, float* beta_c, int* zero) {
   __shared__ __align__(16) float sEnd[8][kD];
   __shared__ float sDec[8], sSum[8];
+  if (blockIdx.x == 0 && threadIdx.x < 8) zero[threadIdx.x] = 0;  // status word and cursors of the kernels behind
   int n, tok0, valid;
   const int H = geo.heads, chunk = blockIdx.x / H, h = blockIdx.x % H;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -932,7 +933,7 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
     begin_stage(kStageAtkLocal, st);
     pkda_atk_local_kernel<<<geo.total_chunks * p.heads, 256, 0, st>>>(geo, static_cast<const bf16*>(p.k), p.g_atk,
                                                  static_cast<const bf16*>(p.beta_atk), static_cast<const bf16*>(p.beta),
-                                                 a->ac_atk, a->sa_atk, ws.beta_c);
+                                                 a->ac_atk, a->sa_atk, ws.beta_c, ws.status);
     PKDA_CHECK_LAUNCH();
     begin_stage(kStageAtkCarry, st);
     pkda_atk_carry_kernel<<<dim3(p.n_seqs, p.heads), kD, 0, st>>>(geo, a->ac_atk, a->sa_atk, p.initial_A_state,
@@ -940,8 +941,10 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
     PKDA_CHECK_LAUNCH();
   }
 
-  const size_t zero_ints = 8 + (chained ? (size_t)geo.total_chunks * p.heads : 0);  // status, cursors, chain counters
-  if (cudaMemsetAsync(ws.status, 0, zero_ints * sizeof(int), st) != cudaSuccess) return PKDA_ERR_LAUNCH;
+  // status, cursors and chain counters; the local scan zeroes the first two when it runs (one launch fewer:
+  // 2 us of a small call's host time)
+  if (chained && cudaMemsetAsync(ws.status, 0, (8 + (size_t)geo.total_chunks * p.heads) * sizeof(int), st) != cudaSuccess)
+    return PKDA_ERR_LAUNCH;
   ChainArgs chain_args;
   chain_args.beta_c_w = ws.beta_c; chain_args.a_chain = a->a_atk; chain_args.sa = a->sa_atk;
   chain_args.AT = a->final_A_state; chain_args.flags = ws.chain_flags;
