@@ -73,6 +73,7 @@ pkda_scan_bwd_cols_kernel(const __grid_constant__ CUtensorMap tm_kg, const __gri
   const int last = sq.nchunks - 1;  // j counts processed chunks, chunk index = last - j
 
   if (warp == 2 * NW) {
+    // ---------------------------------------------------------------- the copies
     if (lane == 0) {
       for (int j = 0; j < sq.nchunks; ++j) {
         const int s = j % Y::kStages, i = last - j;
@@ -107,6 +108,7 @@ pkda_scan_bwd_cols_kernel(const __grid_constant__ CUtensorMap tm_kg, const __gri
   };
 
   if (warp >= NW) {
+    // ----------------------------------------------------------------------- the stores
     for (int j = 0; j < sq.nchunks; ++j) {
       const int i = last - j;
       const unsigned char* sl = slot0 + (j & 1) * Y::kSlot;
@@ -129,6 +131,7 @@ pkda_scan_bwd_cols_kernel(const __grid_constant__ CUtensorMap tm_kg, const __gri
                  e[jj + 1], L.t);
     }
   } else {
+    // ------------------------------------------------------------------------ the chain
     float S[16][4];  // dS^T: rows v0 + g, v0 + g + 8, columns k = 8 nt + 2 t, + 1
     const size_t sbase = (size_t)unit * kD * kD + v0 + L.g;
 #pragma unroll
