@@ -29,6 +29,7 @@
 #include <torch/library.h>
 
 #include <atomic>
+#include <functional>
 #include <mutex>
 
 #include "pkda_b200.h"
@@ -452,6 +453,29 @@ auto typed_op(const char* name) {
   return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<F>();
 }
 
+// The backward operators have no derivative of their own.  Where one could be asked for (a graph is being
+// recorded, create_graph = True), their results hang on a node that raises: without it they would come out as
+// constants and a second derivative would silently be missing.
+struct NotTwice : torch::autograd::Function<NotTwice> {
+  static variable_list forward(AutogradContext* ctx, at::TensorList, const std::function<variable_list()>& run,
+                               const char* name) {
+    ctx->saved_data["name"] = std::string(name);
+    return run();
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list) {
+    TORCH_CHECK(false, ctx->saved_data["name"].toStringRef(), " has no derivative: the PKDA operators are differentiable once");
+  }
+};
+
+// `run` calls the operator again, below autograd; `inputs` are its tensor arguments.
+variable_list once_differentiable(const char* name, at::TensorList inputs, const std::function<variable_list()>& run) {
+  at::AutoDispatchBelowADInplaceOrView below;
+  if (at::GradMode::is_enabled())
+    for (const Tensor& t : inputs)
+      if (t.requires_grad()) return NotTwice::apply(inputs, run, name);
+  return run();
+}
+
 using RecurrenceSig = std::tuple<Tensor, std::vector<Tensor>>(
     const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&,
     const Tensor&, const Tensor&, const Tensor&, double, double, double, bool);
@@ -509,6 +533,21 @@ std::tuple<Tensor, std::vector<Tensor>> recurrence_autograd(
   Tensor o = std::move(r[0]);
   r.erase(r.begin());
   return {std::move(o), std::move(r)};
+}
+
+std::vector<Tensor> recurrence_backward_autograd(
+    const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& g_atk, const Tensor& beta_atk,
+    const Tensor& beta, const Tensor& A_log, const Tensor& dt_bias, const Tensor& log_atk_scale,
+    at::TensorList saved, const Tensor& d_o, double scale, double squash_x, double squash_eps,
+    std::optional<at::ScalarType> autocast_dtype, bool lean) {
+  constexpr const char* name = "delta_feedback::pkda_recurrence_backward";
+  static const auto op = typed_op<RecurrenceBackwardSig>(name);
+  variable_list in{q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, d_o};
+  in.insert(in.end(), saved.begin(), saved.end());
+  return once_differentiable(name, in, [&]() -> variable_list {
+    return op.call(q, k, v, g, g_atk, beta_atk, beta, A_log, dt_bias, log_atk_scale, saved, d_o, scale, squash_x,
+                   squash_eps, autocast_dtype, lean);
+  });
 }
 
 // ---------------------------------------------- operator delta_feedback::pkda_qkv_conv
@@ -595,6 +634,18 @@ std::tuple<Tensor, Tensor, Tensor> conv_autograd(const Tensor& x, const Tensor& 
   return {r[0], r[1], r[2]};
 }
 
+std::tuple<Tensor, Tensor> conv_backward_autograd(const Tensor& x, const Tensor& weight, const Tensor& dq,
+                                                  const Tensor& dk, const Tensor& dv, SymInt head_dim,
+                                                  SymInt norm_channels, double eps) {
+  constexpr const char* name = "delta_feedback::pkda_qkv_conv_backward";
+  static const auto op = typed_op<ConvBackwardSig>(name);
+  variable_list r = once_differentiable(name, {x, weight, dq, dk, dv}, [&]() -> variable_list {
+    auto [dx, dw] = op.call(x, weight, dq, dk, dv, head_dim, norm_channels, eps);
+    return {dx, dw};
+  });
+  return {r[0], r[1]};
+}
+
 // --------------------------------------------- operator delta_feedback::pkda_norm_gate
 pkda_norm_gate_args norm_gate_args(const Tensor& x, const Tensor& gate, const Tensor& weight, double eps) {
   TORCH_CHECK(gate.sizes() == x.sizes() && weight.dim() == 1 && weight.size(0) == x.size(-1) && weight.size(0) > 0,
@@ -673,6 +724,18 @@ struct NormGate : torch::autograd::Function<NormGate> {
 std::tuple<Tensor, Tensor> norm_gate_autograd(const Tensor& x, const Tensor& gate, const Tensor& weight, double eps) {
   variable_list r = NormGate::apply(x, gate, weight, eps);
   return {r[0], r[1]};
+}
+
+std::tuple<Tensor, Tensor, Tensor> norm_gate_backward_autograd(const Tensor& x, const Tensor& gate,
+                                                               const Tensor& weight, const Tensor& rstd,
+                                                               const Tensor& dy, double eps) {
+  constexpr const char* name = "delta_feedback::pkda_norm_gate_backward";
+  static const auto op = typed_op<NormGateBackwardSig>(name);
+  variable_list r = once_differentiable(name, {x, gate, weight, rstd, dy}, [&]() -> variable_list {
+    auto [dx, dg, dw] = op.call(x, gate, weight, rstd, dy, eps);
+    return {dx, dg, dw};
+  });
+  return {r[0], r[1], r[2]};
 }
 
 // ------------------------------------------------------------------ control epilogue
@@ -829,8 +892,11 @@ TORCH_LIBRARY_IMPL(delta_feedback, CUDA, m) {
 
 TORCH_LIBRARY_IMPL(delta_feedback, Autograd, m) {
   m.impl("pkda_recurrence", recurrence_autograd);
+  m.impl("pkda_recurrence_backward", recurrence_backward_autograd);
   m.impl("pkda_qkv_conv", conv_autograd);
+  m.impl("pkda_qkv_conv_backward", conv_backward_autograd);
   m.impl("pkda_norm_gate", norm_gate_autograd);
+  m.impl("pkda_norm_gate_backward", norm_gate_backward_autograd);
 }
 
 // ----------------------------------------------------------------- Python entry points
