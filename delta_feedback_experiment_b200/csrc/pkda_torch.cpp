@@ -963,12 +963,15 @@ struct ParsedInputs {
   }
 };
 
-bool any_requires_grad(const ParsedInputs& p) {
-  if (!at::GradMode::is_enabled()) return false;
+// Whether the call has to go through its autograd function: some input takes part in a recorded graph, or carries
+// a forward-mode tangent (which that function refuses; past it the tangent would silently be dropped).
+bool takes_autograd(const ParsedInputs& p) {
+  const bool graph = at::GradMode::is_enabled();
+  auto takes = [&](const Tensor& t) { return (graph && t.requires_grad()) || t._fw_grad(0).defined(); };
   for (const Tensor* t : {&p.in.q, &p.in.k, &p.in.v, &p.in.g, &p.in.g_atk, &p.in.beta_atk, &p.in.beta, &p.in.A_log,
                           &p.in.dt_bias, &p.in.log_atk_scale})
-    if (t->requires_grad()) return true;
-  return (p.S0 && p.S0->requires_grad()) || (p.A0 && p.A0->requires_grad());
+    if (takes(*t)) return true;
+  return (p.S0 && takes(*p.S0)) || (p.A0 && takes(*p.A0));
 }
 
 // recurrence(<inputs>, output_final_state, lean) -> (o, S | None, A | None), differentiable
@@ -980,7 +983,7 @@ PyObject* py_recurrence(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Tensor o, S, AT;
   {
     pybind11::gil_scoped_release no_gil;
-    if (any_requires_grad(P)) {
+    if (takes_autograd(P)) {
       variable_list r = StatefulRecurrence::apply(P.in.q, P.in.k, P.in.v, P.in.g, P.in.g_atk, P.in.beta_atk, P.in.beta,
                                                   P.in.A_log, P.in.dt_bias, P.in.log_atk_scale, P.S0, P.A0, P.cu,
                                                   P.in.scale, P.in.squash_x, P.in.squash_eps, final_state, lean);
