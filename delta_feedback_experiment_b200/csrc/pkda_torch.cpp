@@ -208,6 +208,32 @@ void alloc_saved(const Problem& P, std::vector<Tensor>& saved, int from, int to)
   }
 }
 
+// The list that the operator hands back must be exactly what its fake implementation promises to a compiler
+// (count, and per entry shape, dtype, device, contiguity): a mismatch would surface far away, as a stride or
+// shape error inside a compiled graph.  Derived from the inputs, not from alloc_saved, and run on every call
+// of the operator (under a microsecond).
+void check_intermediates(at::TensorList got, const Tensor& q, const Tensor& v, bool lean) {
+  static const char* const names[kSaved] = {"Aqk", "Akk", "k_precond", "ac_atk", "a_atk", "sa_atk",
+                                            "w", "kg", "v_new", "h", "qg"};
+  const size_t count = lean ? kKept : kSaved;
+  TORCH_CHECK(got.size() == count, "the PKDA forward produced ", got.size(), " intermediates where ", count,
+              " are promised");
+  const int64_t B = q.size(0), T = q.size(1), H = q.size(2), K = q.size(3), V = v.size(3), N = (T + 63) / 64;
+  const int64_t pairs[] = {B, T, H, 64}, keys[] = {B, T, H, K}, values[] = {B, T, H, V}, chunk_keys[] = {B, N, H, K},
+                chunk_heads[] = {B, N, H}, states[] = {B, N, H, K, V};
+  const at::IntArrayRef shapes[kSaved] = {pairs, pairs, keys, chunk_keys, chunk_keys, chunk_heads,
+                                          keys, keys, values, states, keys};
+  for (size_t i = 0; i < count; ++i) {
+    const Tensor& t = got[i];
+    const at::ScalarType dtype = i >= 3 && i <= 5 ? at::kFloat : q.scalar_type();
+    TORCH_CHECK(t.defined(), "PKDA intermediate ", names[i], ": missing from the forward's list");
+    TORCH_CHECK(t.sizes() == shapes[i] && t.scalar_type() == dtype && t.device() == q.device() && t.is_contiguous(),
+                "PKDA intermediate ", names[i], ": forward produced ", t.sizes(), " ", t.scalar_type(), " on ",
+                t.device(), t.is_contiguous() ? "" : ", not contiguous", "; the fake implementation promises ",
+                shapes[i], " ", dtype, " on ", q.device(), ", contiguous");
+  }
+}
+
 struct Forward {
   Tensor o, S, A;
   std::vector<Tensor> saved;
@@ -429,6 +455,7 @@ std::tuple<Tensor, std::vector<Tensor>> recurrence_cuda(
     Problem P(in);
     alloc_saved(P, f.saved, 0, lean ? kKept : kSaved);
   }
+  check_intermediates(f.saved, q, v, lean);
   return {std::move(f.o), std::move(f.saved)};
 }
 
@@ -912,6 +939,18 @@ struct Args {
     if (!THPVariable_Check(a[i])) throw torch::TypeError(c10::str("argument ", i, " must be a Tensor, not ", Py_TYPE(a[i])->tp_name));
     return THPVariable_Unpack(a[i]);
   }
+  // A sequence of tensors; None becomes an undefined one.
+  std::vector<Tensor> tensors(int i) const {
+    THPObjectPtr seq(PySequence_Fast(a[i], "expected a sequence of tensors"));
+    if (!seq) throw python_error();
+    std::vector<Tensor> list;
+    for (Py_ssize_t k = 0; k < PySequence_Fast_GET_SIZE(seq.get()); ++k) {
+      PyObject* t = PySequence_Fast_GET_ITEM(seq.get(), k);
+      if (t != Py_None && !THPVariable_Check(t)) throw torch::TypeError("expected a sequence of tensors");
+      list.push_back(t == Py_None ? Tensor() : THPVariable_Unpack(t));
+    }
+    return list;
+  }
   OptTensor opt(int i) const { return a[i] == Py_None ? std::nullopt : OptTensor(tensor(i)); }
   double num(int i) const {
     const double v = PyFloat_AsDouble(a[i]);
@@ -1044,15 +1083,9 @@ PyObject* py_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const ParsedInputs P(A);
   const bool exact = A.a[16] == Py_None;
   std::vector<Tensor> saved;
-  if (!exact) {
-    THPObjectPtr seq(PySequence_Fast(A.a[16], "saved must be a sequence of tensors"));
-    if (!seq) throw python_error();
-    for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq.get()); ++i) {
-      PyObject* t = PySequence_Fast_GET_ITEM(seq.get(), i);
-      if (!THPVariable_Check(t)) throw torch::TypeError("saved must hold tensors");
-      saved.push_back(THPVariable_Unpack(t));
-    }
-  }
+  if (!exact) saved = A.tensors(16);
+  for (const Tensor& t : saved)
+    if (!t.defined()) throw torch::TypeError("saved must hold tensors");
   const Tensor& d_o = A.tensor(17);
   const OptTensor dS = A.opt(18);
   const bool lean = A.flag(19), want = A.flag(20);
@@ -1132,6 +1165,16 @@ PyObject* py_norm_gate(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// check_intermediates([tensors | None], q, v, lean): the check of the operator's intermediates alone.
+PyObject* py_check_intermediates(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Args A(args, n, 4, "check_intermediates");
+  const std::vector<Tensor> list = A.tensors(0);
+  check_intermediates(list, A.tensor(1), A.tensor(2), A.flag(3));
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
 
 PyObject* py_track_status(PyObject*, PyObject* enable) {
@@ -1172,6 +1215,7 @@ PyMethodDef kMethods[] = {
     PKDA_FAST("controls", py_controls),
     PKDA_FAST("conv", py_conv),
     PKDA_FAST("norm_gate", py_norm_gate),
+    PKDA_FAST("check_intermediates", py_check_intermediates),
     {"launches", py_launches, METH_NOARGS, nullptr},
     {"track_status", py_track_status, METH_O, nullptr},
     {"tracking", py_tracking, METH_NOARGS, nullptr},

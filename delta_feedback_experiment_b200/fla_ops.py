@@ -48,20 +48,10 @@ def _intermediate_meta(q: Tensor, v: Tensor, lean: bool):
 
 
 def _check_intermediates(tensors, q: Tensor, v: Tensor, lean: bool) -> None:
-    """The list the forward hands back must be exactly what the fake implementation
-    promises to the compiler (count, and per entry shape, dtype, device, contiguity):
-    a mismatch would surface far away, as a stride or shape error inside a compiled
-    graph.  Same contract as the reference's check (``fla_ops.py:100-128``)."""
-    names = PKDA_INTERMEDIATES + (() if lean else PKDA_RETAINED)
-    promised = _intermediate_meta(q, v, lean)
-    if len(tensors) != len(promised):
-        raise RuntimeError(f"the PKDA forward produced {len(tensors)} intermediates where "
-                           f"{len(promised)} are promised")
-    for name, t, (shape, dtype) in zip(names, tensors, promised):
-        found = None if t is None else (tuple(t.shape), t.dtype, t.device, t.is_contiguous())
-        if found != (tuple(shape), dtype, q.device, True):
-            raise RuntimeError(f"PKDA intermediate {name}: forward produced {found}, the fake "
-                               f"implementation promises {(tuple(shape), dtype, q.device, True)}")
+    """The check that the operator's CUDA kernel runs on the list it hands back: count, and per
+    entry shape, dtype, device and contiguity as the fake implementation promises them (same
+    contract as the reference's check, ``fla_ops.py:100-128``)."""
+    _lib.native().check_intermediates(tensors, q, v, lean)
 
 
 def _missing(*_args, **_kwargs):

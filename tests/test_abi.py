@@ -133,3 +133,19 @@ def test_intermediate_contract_check_names_the_offender():
             fla_ops._check_intermediates(bad, q, v, lean)
     assert len(fla_ops._intermediate_meta(q, v, True)) == len(fla_ops.PKDA_INTERMEDIATES)
     assert fla_ops._intermediate_meta(q, v, False)[9][0] == (2, 3, 3, 128, 128)   # h: three chunks of 64
+
+
+def test_intermediate_contract_check_agrees_with_the_fake_implementation():
+    """The check on the operator's path and the list promised to a compiler are written in two
+    languages: they must agree over batches, ragged lengths, head widths and both dtypes."""
+    import torch
+    from delta_feedback_experiment_b200 import _lib, fla_ops
+
+    for B, T, H, D in ((1, 1, 1, 128), (3, 64, 2, 128), (2, 65, 5, 128), (1, 200, 4, 8), (2, 129, 1, 64)):
+        for dtype in (torch.bfloat16, torch.float32):
+            q = torch.empty(B, T, H, D, dtype=dtype, device="meta")
+            for lean in (True, False):
+                promised = [torch.empty(s, dtype=d, device="meta") for s, d in fla_ops._intermediate_meta(q, q, lean)]
+                _lib.native().check_intermediates(promised, q, q, lean)
+                with pytest.raises(RuntimeError, match="missing"):
+                    _lib.native().check_intermediates([*promised[:-1], None], q, q, lean)
