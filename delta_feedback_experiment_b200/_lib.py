@@ -258,23 +258,50 @@ def load() -> C.CDLL:
 
 
 _native = None
+_when_loaded: list = []   # registrations that wait for the native layer
 
 
-def built() -> bool:
-    """Whether both shared libraries exist (nothing is loaded)."""
-    return os.path.exists(LIB_PATH) and os.path.exists(NATIVE_PATH)
+def native_marker() -> bytes:
+    """The string a ``_native.so`` for the running torch carries (its ABI is that of one torch)."""
+    return f"pkda host layer built for torch {torch.__version__}".encode() + b"\0"
+
+
+def native_is_current() -> bool:
+    """Whether ``_native.so`` exists and was built for the running torch (nothing is loaded)."""
+    if not os.path.exists(NATIVE_PATH):
+        return False
+    with open(NATIVE_PATH, "rb") as f:
+        return native_marker() in f.read()
+
+
+def when_loaded(action) -> None:
+    """Runs ``action`` once the native layer is loaded: now, or when a later call loads it."""
+    if _native is not None:
+        action()
+    else:
+        _when_loaded.append(action)
 
 
 def native():
     """The torch host layer (``csrc/pkda_torch.cpp``): launchers that take tensors, and the
-    ``delta_feedback`` operators, which its import registers.  ``RuntimeError`` if it is missing."""
+    ``delta_feedback`` operators, which its import registers.  ``RuntimeError`` with the reason if
+    it does not load (the next call tries again: it may have been built in between)."""
     global _native
     if _native is None:
         load()  # the C library first: the host layer resolves to this very instance
         try:
+            if not os.path.exists(NATIVE_PATH):
+                raise ImportError(f"{NATIVE_PATH} has not been built "
+                                  "(python -m delta_feedback_experiment_b200.build)")
+            if not native_is_current():
+                raise ImportError(f"{NATIVE_PATH} was not built for torch {torch.__version__} "
+                                  "(python -m delta_feedback_experiment_b200.build)")
             from . import _native as module
         except ImportError as exc:
             raise RuntimeError(f"PKDA CUDA library unavailable: {exc}") from exc
+        while _when_loaded:
+            _when_loaded[0]()
+            _when_loaded.pop(0)
         _native = module
     return _native
 

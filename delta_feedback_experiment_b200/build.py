@@ -4,7 +4,8 @@ torch host layer on top of it, g++) in-tree.
     python -m delta_feedback_experiment_b200.build [--force] [--verbose]
 
 nvcc cross-compiles without a GPU.  The libraries are rebuilt only when a source
-file is newer than an existing ``.so`` (or ``--force`` is given).
+file is newer than an existing ``.so``, when ``_native.so`` was built for another
+torch, or with ``--force``.
 """
 
 from __future__ import annotations
@@ -15,11 +16,12 @@ import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
 
+from . import _lib
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
-LIB_PATH = os.path.join(HERE, "libpkda_b200.so")
-NATIVE_PATH = os.path.join(HERE, "_native.so")
+LIB_PATH, NATIVE_PATH = _lib.LIB_PATH, _lib.NATIVE_PATH
 OBJ_DIR = os.path.join(HERE, "build")
 
 SOURCES = ["pkda_abi.cu", "pkda_recurrent.cu", "pkda_chunk_fwd.cu", "pkda_chunk_bwd.cu",
@@ -47,7 +49,7 @@ def _deps() -> list[str]:
 
 
 def needs_build() -> bool:
-    if not (os.path.exists(LIB_PATH) and os.path.exists(NATIVE_PATH)):
+    if not (os.path.exists(LIB_PATH) and _lib.native_is_current()):
         return True
     stamp = min(os.path.getmtime(LIB_PATH), os.path.getmtime(NATIVE_PATH))
     return any(os.path.getmtime(d) > stamp for d in _deps())
@@ -60,7 +62,8 @@ def _compile_native() -> str:
     from torch.utils.cpp_extension import include_paths
     obj = os.path.join(OBJ_DIR, NATIVE_SOURCE.replace(".cpp", ".o"))
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I", INCLUDE]
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f'-DPKDA_NATIVE_MARKER="{_lib.native_marker()[:-1].decode()}"', "-I", INCLUDE]
     for inc in [*include_paths("cuda"), sysconfig.get_paths()["include"]]:
         cmd += ["-isystem", inc]
     res = subprocess.run([*cmd, "-c", os.path.join(CSRC, NATIVE_SOURCE), "-o", obj], capture_output=True, text=True)

@@ -1227,4 +1227,9 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&kModule); }
+// (The marker is what tells a library built for another torch from a current one without loading it.)
+PyMODINIT_FUNC PyInit__native() {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m && PyModule_AddStringConstant(m, "built_for", PKDA_NATIVE_MARKER) < 0) Py_CLEAR(m);
+  return m;
+}

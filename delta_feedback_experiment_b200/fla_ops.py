@@ -54,24 +54,26 @@ def _check_intermediates(tensors, q: Tensor, v: Tensor, lean: bool) -> None:
     _lib.native().check_intermediates(tensors, q, v, lean)
 
 
-def _missing(*_args, **_kwargs):
-    raise RuntimeError("the PKDA libraries were not built when this package was imported "
-                       "(python -m delta_feedback_experiment_b200.build)")
-
-
 def _operator(name: str):
-    """The registered operator ``delta_feedback::<name>``, or a stand-in that raises if the
-    native layer does not exist or load."""
-    if not (_lib.built() and _lib.available()):
-        return _missing
-    return getattr(torch.ops.delta_feedback, name).default
+    """The registered operator ``delta_feedback::<name>``.  While the native layer does not load, a
+    stand-in: each call tries to load it again and raises the reason if that fails."""
+    if _lib.available():
+        return getattr(torch.ops.delta_feedback, name).default
+
+    def stand_in(*args, **kwargs):
+        _lib.native()
+        return getattr(torch.ops.delta_feedback, name).default(*args, **kwargs)
+
+    stand_in.__name__ = name
+    return stand_in
 
 
 def _register_fake(name: str):
-    """``torch.library.register_fake`` for an operator of the native layer, where there is one."""
-    if not (_lib.built() and _lib.available()):
-        return lambda fn: fn
-    return torch.library.register_fake(f"delta_feedback::{name}")
+    """``torch.library.register_fake`` for an operator of the native layer, as soon as there is one."""
+    def register(fn):
+        _lib.when_loaded(lambda: torch.library.register_fake(f"delta_feedback::{name}", fn))
+        return fn
+    return register
 
 
 pkda_recurrence = _operator("pkda_recurrence")

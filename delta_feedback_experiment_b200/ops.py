@@ -23,7 +23,7 @@ _STATIC_LAUNCHES = 0     # kernels enqueued by the ctypes calls of this module
 def __getattr__(name: str):
     """``ops.LAUNCHES``: kernels enqueued by the operators since import (launch accounting)."""
     if name == "LAUNCHES":
-        return _STATIC_LAUNCHES + (_lib.native().launches() if _lib.built() else 0)
+        return _STATIC_LAUNCHES + (_lib.native().launches() if _lib.available() else 0)
     raise AttributeError(name)
 
 
