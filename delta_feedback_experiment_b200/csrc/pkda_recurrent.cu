@@ -104,9 +104,12 @@ pkda_recurrent_kernel(const RecParams p) {
         const int tl = TPG * grp + i;
         const float bw = __shfl_sync(0xffffffffu, scal, 16 + tl);
         const bool ok = t0 + tl < sq.len;  // tokens past the end leave the state as it is
-        float al = expf(-ea * softplus_series(gc[i] + bias));  // (selects, no branches: the tokens interleave)
+        // The same two functions as in the few-token and decoding kernels, so that a token's factors do not depend
+        // on the kernel.  (A branch-free log1p series and approximate quotients here saved 2% of a call, 193.6
+        // against 197.8 us at 2 x 512 tokens of 4 heads x 64, and cost 4% in the error against 64 bits.)
+        float al = expf(-ea * softplus_acc(gc[i] + bias));
         al = ok ? al : 1.f;
-        const float wk = bw * (kc[i] * precond_factor_nb(An[i], p.eps, centre, p.ln_x));
+        const float wk = bw * (kc[i] * precond_factor(An[i], p.eps, centre, p.ln_x));
         if (act) {
           float* row = st + tl * VEC + c;
           row[0] = al * kc[i];

@@ -80,28 +80,6 @@ template <> struct Raw<bf16> {
   static __device__ __forceinline__ float value(uint32_t r) { return __uint_as_float(r << 16); }
 };
 
-// softplus without branches, for the producers' unrolled token loops: log1p(y) = 2 atanh(y / (2 + y)) with
-// the atanh series in s = y / (2 + y) <= 1/3 (the first term left out is below 2e-9 of the sum).
-__device__ __forceinline__ float softplus_series(float x) {
-  const float y = expf(-fabsf(x));
-  const float s = __fdividef(y, 2.f + y), z = s * s;
-  float c = 1.f / 17.f;
-  c = fmaf(c, z, 1.f / 15.f);
-  c = fmaf(c, z, 1.f / 13.f);
-  c = fmaf(c, z, 1.f / 11.f);
-  c = fmaf(c, z, 1.f / 9.f);
-  c = fmaf(c, z, 1.f / 7.f);
-  c = fmaf(c, z, 1.f / 5.f);
-  c = fmaf(c, z, 1.f / 3.f);
-  c = fmaf(c, z, 1.f);
-  return fmaxf(x, 0.f) + 2.f * s * c;
-}
-// precond_factor with the quotient rounded to two ulps instead of one.
-__device__ __forceinline__ float precond_factor_nb(float A, float eps, float centre, float ln_x) {
-  const float dev = logf(A + eps) - centre;
-  return expf(__fdividef(-ln_x * dev, 1.f + fabsf(dev)));
-}
-
 // Named barriers between the producer and the consumer warps of a scan CTA.
 __device__ __forceinline__ void bar_sync_n(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
