@@ -16,6 +16,12 @@ int direct_block_cap() { return g_direct_cap; }
 
 static int g_variant[kStageCount] = {};
 
+int sm_count() {
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 bool dynamic_smem_once(const void* kernel, int bytes, int carveout) {
   static std::mutex mu;
   static std::unordered_map<const void*, unsigned long long> seen;  // kernel -> one bit per device

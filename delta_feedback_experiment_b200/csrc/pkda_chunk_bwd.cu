@@ -1339,8 +1339,7 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   // CTA each, when it is pinned).
   ip.fast_list = nullptr;
   ip.slow_list = ip.fast_count = nullptr;
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   if (tc_intra) {
     ip.fast_list = ws.fast_list; ip.slow_list = ws.slow_list; ip.fast_count = ws.counts;
     rc = launch_intra_bwd_tc(ip, st);

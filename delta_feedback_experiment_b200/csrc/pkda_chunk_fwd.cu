@@ -802,8 +802,7 @@ int check_chunk_problem(const pkda_problem& p) {
 }
 
 int scan_columns(int units) {
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   return 8L * units <= sms ? 8 : 4L * units <= sms ? 4 : 0;
 }
 
@@ -855,8 +854,7 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
     const int rc_tc = launch_intra_fwd_tc(ip, recompute, st);
     end_stage(st);
     if (rc_tc != PKDA_OK) return rc_tc;
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     gridc = dim3(items < sms ? items : sms, 1);
   }
   const int rest_stage = ip.slow_list ? kStageIntraFwdRest : kStageIntraFwd;

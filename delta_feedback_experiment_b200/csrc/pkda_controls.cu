@@ -182,8 +182,8 @@ static int ctrl_check(const pkda_controls_args& a, CtrlParams& p) {
 
 static int ctrl_bwd_grid(const pkda_controls_args& a) {
   const int r = ctrl_rows(a.heads);
-  const long long want = (a.rows + r - 1) / r;  // one turn per CTA until the chip is full several times over
-  return (int)(want < 1 ? 1 : (want < 2368 ? want : 2368));
+  const long long want = (a.rows + r - 1) / r, most = 16LL * sm_count();  // one turn per CTA until the chip is full several times over
+  return (int)(want < 1 ? 1 : (want < most ? want : most));
 }
 
 int controls_fwd(const pkda_controls_args* a, cudaStream_t st) {
@@ -193,7 +193,8 @@ int controls_fwd(const pkda_controls_args* a, cudaStream_t st) {
   if (!a->packed || !a->A_log_precond || !a->dt_bias_precond || !a->beta || !a->g_atk || !a->beta_atk)
     return PKDA_ERR_NULL;
   const long long n = a->rows * a->heads;
-  const int grid = (int)((n + kCtrlThreads - 1) / kCtrlThreads < 2368 ? (n + kCtrlThreads - 1) / kCtrlThreads : 2368);
+  const long long blocks = (n + kCtrlThreads - 1) / kCtrlThreads, most = 16LL * sm_count();
+  const int grid = (int)(blocks < most ? blocks : most);
   begin_stage(kStageControlsFwd, st);
   if (a->dtype == PKDA_BF16) pkda_controls_fwd_kernel<bf16><<<grid, kCtrlThreads, 0, st>>>(p);
   else pkda_controls_fwd_kernel<float><<<grid, kCtrlThreads, 0, st>>>(p);
@@ -247,8 +248,8 @@ int pack_control_gradients(const pkda_pack_control_args* a, cudaStream_t st) {
   if (!a->out) return PKDA_ERR_NULL;
   for (int i = 0; i < 5; ++i)
     if (a->sizes[i] > 0 && !a->grads[i]) return PKDA_ERR_NULL;
-  const long long blocks = (n + kCtrlThreads - 1) / kCtrlThreads;
-  const int grid = (int)(blocks < 4736 ? blocks : 4736);
+  const long long blocks = (n + kCtrlThreads - 1) / kCtrlThreads, most = 32LL * sm_count();
+  const int grid = (int)(blocks < most ? blocks : most);
   begin_stage(kStagePackControl, st);
   if (a->dtype == PKDA_BF16)
     pkda_pack_control_kernel<bf16><<<grid, kCtrlThreads, 0, st>>>(

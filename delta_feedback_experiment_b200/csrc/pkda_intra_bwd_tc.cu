@@ -694,8 +694,7 @@ int launch_intra_bwd_tc(const IntraBwdParams& ip, cudaStream_t st) {
     return PKDA_ERR_LAUNCH;
   const int items = ip.geo.total_chunks * ip.geo.heads;
   begin_stage(kStageIntraBwd, st);
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   pkda_intra_bwd_tc_kernel<<<items < sms ? items : sms, ibtc::kThreads, ibtc::kSmem, st>>>(ip, maps);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;

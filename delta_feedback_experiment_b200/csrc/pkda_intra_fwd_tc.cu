@@ -626,8 +626,7 @@ int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) 
     if (!encode_bf16_map(&tm_akk, ip.Akk, 3, dims, str, box) || !encode_bf16_map(&tm_aqk, ip.Aqk, 3, dims, str, box))
       return PKDA_ERR_LAUNCH;
   }
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const int items = ip.geo.total_chunks * ip.geo.heads;
   const int grid = items < 2 * sms ? items : 2 * sms;  // persistent: two CTAs per SM
   // two CTAs per SM need the largest shared-memory carve-out

@@ -40,6 +40,9 @@ inline bool ensure_dynamic_smem(K kernel, int bytes, int carveout = -1) {
   return dynamic_smem_once(reinterpret_cast<const void*>(kernel), bytes, carveout);
 }
 
+// SMs of the current device (148, the B200's, where there is none).
+int sm_count();
+
 // Upper limit for the kernels' direct block size (64 unless lowered through
 // pkda_set_direct_block_cap, a testing aid).
 int direct_block_cap();

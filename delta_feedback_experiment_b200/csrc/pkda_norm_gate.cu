@@ -267,12 +267,6 @@ __global__ void __launch_bounds__(1024) pkda_norm_gate_dw_kernel(const float* pa
 }
 
 // ------------------------------------------------------------------ host side
-static int sm_count() {
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 // Persistent grid: as many CTAs as are resident at once (never more than 8 per SM,
 // the bound the backward's partial buffer is sized for), fewer for small inputs.
 template <typename K> static int ng_grid(const pkda_norm_gate_args& a, K kernel, int smem) {

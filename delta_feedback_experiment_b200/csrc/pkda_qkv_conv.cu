@@ -570,12 +570,13 @@ static int conv_check(const pkda_qkv_conv_args& a, ConvParams& p) {
 // four CTAs (two waves of the backward's two), so that short inputs spread over the chip instead.
 static dim3 conv_grid(ConvParams& p) {
   const unsigned cols = (unsigned)((p.channels + conv::kTileCh - 1) / conv::kTileCh);
+  const long wanted = 4L * sm_count();
   p.span = conv::kMaxSpan;
   for (;; p.span /= 2) {
     const int tokens = p.span * conv::kGroups;
     p.spans_per_row = (p.seq_len + tokens - 1) / tokens;
     const dim3 grid(cols, (unsigned)(p.batch * p.spans_per_row));
-    if (p.span == conv::kMinSpan || (long)grid.x * grid.y >= 4 * 148) return grid;
+    if (p.span == conv::kMinSpan || (long)grid.x * grid.y >= wanted) return grid;
   }
 }
 

@@ -346,12 +346,6 @@ pkda_recurrent_few_kernel(const RecParams p) {
   if (p.AT && tid < D) p.AT[((size_t)n * H + h) * D + tid] = A;
 }
 
-int sm_count() {
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 template <int D, int kCPL, typename T, bool kSave>
 static int launch_rec(RecParams rp, cudaStream_t st) {
   using L = ScanLay<D, kCPL>;

@@ -160,6 +160,4 @@ inline int scan_consumers(int units, int warps_per_unit, int max_consumers, int 
   return nw;
 }
 
-int sm_count();
-
 }  // namespace pkda
