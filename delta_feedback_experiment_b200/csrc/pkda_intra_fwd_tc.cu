@@ -37,8 +37,14 @@
 
 namespace pkda {
 
-// 2^-(kDirectLimit + 1)
-constexpr float kSurelySlow = 9.62964972e-35f;
+constexpr float half_power(int n) {
+  float x = 1.f;
+  for (int i = 0; i < n; ++i) x *= 0.5f;
+  return x;
+}
+// Decay totals below this are past kDirectLimit however their base-2 exponential was rounded.
+constexpr float kSurelySlow = half_power((int)kDirectLimit + 1);
+static_assert((float)(int)kDirectLimit == kDirectLimit && kSurelySlow >= 1.17549435e-38f, "a whole, normal power of two");
 
 namespace intratc {
 constexpr int kThreads = 256;
