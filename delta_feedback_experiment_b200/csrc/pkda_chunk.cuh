@@ -184,14 +184,6 @@ __device__ __forceinline__ void gate_apply(const GateRaw<kNThreads>& gr, float* 
   }
 }
 
-template <int kNThreads>
-__device__ __forceinline__ void gate_elementwise(float* sG, const bf16* g_row0, long gld, int valid,
-                                                 const float* bias_h, float ea2, int tid) {
-  GateRaw<kNThreads> gr;
-  gate_load(gr, g_row0, gld, valid, tid);
-  gate_apply(gr, sG, valid, bias_h, ea2, tid);
-}
-
 // In-place cumulative sum over the 64 rows of sG, one channel per thread (tid < 128).
 __device__ __forceinline__ void gate_cumsum(float* sG, int c) {
   float run = 0.f;
@@ -266,7 +258,7 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
 // odd stride (65) every one of them is a 4-way conflict, and the merge is bound by them.
 template <int K>
 __device__ __forceinline__ void tile_mma_3xtf32(float (&d)[4], const float* Ap, int lda, const float* Bp, int ldb,
-                                                int lane, int kbeg = 0, int kend = K) {
+                                                int lane, int kbeg, int kend) {
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int k0 = 0; k0 < K; k0 += 8) {
@@ -287,10 +279,10 @@ __device__ __forceinline__ void tile_mma_3xtf32(float (&d)[4], const float* Ap, 
 
 // kYPad widens the rows of the scratch Y to N + kYPad floats (8 makes the second
 // product's B loads conflict-free; the scratch then holds 2 * 16 * 24 or 32 * 40 floats).
-// kSkip leaves out the k-steps in which a triangular factor is all zero (the rows of
-// T11 above the output tile's columns, the columns of T22 right of the output tile's
-// rows): the sums lose only exact zeros.
-template <int N, int kYPad, bool kSkip>
+// The k-steps in which a triangular factor is all zero (the rows of T11 above the output
+// tile's columns, the columns of T22 right of the output tile's rows) are left out: the
+// sums lose only exact zeros.
+template <int N, int kYPad>
 __device__ __forceinline__ void inverse_merge_tc(const float* sL, float* sT, float* sY2, int ldl, int ldt, int tid) {
   constexpr int kMT = N / 16, kNT = N / 8, kTiles = (32 / N) * kMT * kNT;  // N = 32: 8 tiles, N = 16: 4 tiles
   constexpr int ldy = N + kYPad;
@@ -300,7 +292,7 @@ __device__ __forceinline__ void inverse_merge_tc(const float* sL, float* sT, flo
   if (warp < kTiles) {  // Y = L21 T11
     float d[4] = {0.f, 0.f, 0.f, 0.f};
     tile_mma_3xtf32<N>(d, sL + (base + N + 16 * mt) * ldl + base, ldl, sT + base * ldt + base + 8 * nt, ldt, lane,
-                       kSkip ? 8 * nt : 0, N);
+                       8 * nt, N);
     float* y = sY2 + pr * N * ldy + (16 * mt + g) * ldy + 8 * nt + 2 * t;
     *reinterpret_cast<float2*>(y) = make_float2(d[0], d[1]);
     *reinterpret_cast<float2*>(y + 8 * ldy) = make_float2(d[2], d[3]);
@@ -309,7 +301,7 @@ __device__ __forceinline__ void inverse_merge_tc(const float* sL, float* sT, flo
   if (warp < kTiles) {  // T21 = -T22 Y
     float d[4] = {0.f, 0.f, 0.f, 0.f};
     tile_mma_3xtf32<N>(d, sT + (base + N + 16 * mt) * ldt + base + N, ldt, sY2 + pr * N * ldy + 8 * nt, ldy, lane, 0,
-                       kSkip ? 16 * mt + 16 : N);
+                       16 * mt + 16);
     float* o = sT + (base + N + 16 * mt + g) * ldt + base + 8 * nt + 2 * t;
     o[0] = -d[0];
     o[1] = -d[1];
@@ -358,8 +350,8 @@ __device__ __forceinline__ void unit_lower_inverse_64(const float* sL, float* sT
     }
   }
   __syncthreads();
-  inverse_merge_tc<16, kYPad, true>(sL, sT, sY2, ldl, ldt, tid);
-  inverse_merge_tc<32, kYPad, true>(sL, sT, sY2, ldl, ldt, tid);
+  inverse_merge_tc<16, kYPad>(sL, sT, sY2, ldl, ldt, tid);
+  inverse_merge_tc<32, kYPad>(sL, sT, sY2, ldl, ldt, tid);
 }
 
 // Sums each of v[0..7] over the 32 lanes.  On return lane l holds in v[0] the

@@ -122,7 +122,6 @@ __device__ __forceinline__ float softplus_acc(float x) {
 __device__ __forceinline__ float softplus_fast(float x) {
   return fmaxf(x, 0.f) + __logf(1.f + __expf(-fabsf(x)));
 }
-__device__ __forceinline__ float sigmoid_fast(float x) { return 1.f / (1.f + __expf(-x)); }
 
 // Write-key factor of the diagonal preconditioner:
 //   dev = log(A + eps) - centre;  B = exp(-ln(x) * dev / (1 + |dev|)).
@@ -240,11 +239,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pr
   uint32_t s = smem_u32(smem);
   int bytes = pred ? 16 : 0;  // src-size 0 => zero fill
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" :: "r"(s), "l"(gmem), "r"(bytes));
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem, bool pred) {
-  uint32_t s = smem_u32(smem);
-  int bytes = pred ? 4 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" :: "r"(s), "l"(gmem), "r"(bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N> __device__ __forceinline__ void cp_async_wait() {

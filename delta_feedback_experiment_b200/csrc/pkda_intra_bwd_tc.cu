@@ -71,32 +71,6 @@ constexpr uint32_t kCols = 512;
 constexpr uint32_t cR = 0, cStk = 64, cQs = 128, cKs = 192, cKts = 256, cKtM = 320, cKtP = 384;  // cR / cStk later Qp / Kp
 }  // namespace ibtc
 
-// Sums each of v[0..15] over the 32 lanes.  On return lane l holds in v[0] the total of entry
-// ((l >> 4) & 1) * 8 + ((l >> 3) & 1) * 4 + ((l >> 2) & 1) * 2 + ((l >> 1) & 1).
-__device__ __forceinline__ void row_sums16(float (&v)[16], int lane) {
-  const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4, b2 = lane & 2;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float keep = b16 ? v[j + 8] : v[j], send = b16 ? v[j] : v[j + 8];
-    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float keep = b8 ? v[j + 4] : v[j], send = b8 ? v[j] : v[j + 4];
-    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-  }
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const float keep = b4 ? v[j + 2] : v[j], send = b4 ? v[j] : v[j + 2];
-    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-  }
-  {
-    const float keep = b2 ? v[1] : v[0], send = b2 ? v[0] : v[1];
-    v[0] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-  }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
 // One bf16 element of shared memory by its 32-bit shared address (register + immediate addressing).
 __device__ __forceinline__ float lds_bf16(uint32_t addr) {
   unsigned short u;

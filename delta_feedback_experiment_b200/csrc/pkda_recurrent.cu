@@ -38,7 +38,7 @@ template <int D, int kCPL, typename T, bool kSave>
 __global__ void __launch_bounds__(ScanLay<D, kCPL>::kProd + 32 * ScanLay<D, kCPL>::kMaxConsumers)
 pkda_recurrent_kernel(const RecParams p) {
   using L = ScanLay<D, kCPL>;
-  constexpr int TB = L::kTB, TPG = L::kTPG, RG = L::kRG, R = L::kR, RUNS = L::kR / L::kU, VEC = L::kVecs * D;
+  constexpr int TB = L::kTB, TPG = L::kTPG, RG = L::kRG, R = L::kR, VEC = L::kVecs * D;
   extern __shared__ __align__(16) float stage[];  // [2][TB][5][D]: exp(g) k, exp(g), beta kw, scale q, v
   const int H = p.geo.heads;
   const int unit = blockIdx.x / p.groups, cg = blockIdx.x - unit * p.groups;
