@@ -442,6 +442,7 @@ int recurrent_fwd(const pkda_recurrent_args* a, void* saved, size_t saved_bytes,
   if (p.n_seqs == 0 || p.total_tokens == 0) return PKDA_OK;
   if (!a->o) return PKDA_ERR_NULL;
   if (saved) {
+    if (reinterpret_cast<uintptr_t>(saved) & 15) return PKDA_ERR_ALIGN;  // (states move four values at a time)
     size_t need = 0;
     const RecSaved s = carve_rec_saved(p, saved, &need);
     if (saved_bytes < need) return PKDA_ERR_WORKSPACE;

@@ -582,6 +582,7 @@ int recurrent_bwd(const pkda_recurrent_bwd_args* a, const void* saved, size_t sa
     return PKDA_ERR_NULL;
   const RecBwdWorkspace ws = carve_rec_bwd(p, a->workspace, saved == nullptr);
   if (!a->workspace || a->workspace_bytes < ws.bytes) return PKDA_ERR_WORKSPACE;
+  if ((reinterpret_cast<uintptr_t>(a->workspace) | reinterpret_cast<uintptr_t>(saved)) & 15) return PKDA_ERR_ALIGN;
   if (saved && saved_bytes < recurrent_saved_bytes(p)) return PKDA_ERR_WORKSPACE;
   RecBwdParams bp;
   bp.geo = make_geo(p, nullptr);

@@ -127,7 +127,8 @@ int pkda_recurrent_bwd(const pkda_recurrent_bwd_args* args, void* cuda_stream);
 /* The same pair with the forward's by-products kept between them: pkda_recurrent_fwd_saving is
  * pkda_recurrent_fwd that also fills `saved` (pkda_recurrent_saved_bytes), pkda_recurrent_bwd_saved the
  * backward that reads it instead of running the forward again (and needs the smaller workspace of
- * pkda_recurrent_bwd_saved_workspace_bytes).  Contents and layout of `saved` are the library's own. */
+ * pkda_recurrent_bwd_saved_workspace_bytes).  Contents and layout of `saved` are the library's own; it starts on
+ * a 16-byte boundary, as the workspace does (PKDA_ERR_ALIGN otherwise). */
 size_t pkda_recurrent_saved_bytes(const pkda_problem* p);
 int pkda_recurrent_fwd_saving(const pkda_recurrent_args* args, void* saved, size_t saved_bytes, void* cuda_stream);
 size_t pkda_recurrent_bwd_saved_workspace_bytes(const pkda_problem* p);

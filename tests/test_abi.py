@@ -149,3 +149,28 @@ def test_intermediate_contract_check_agrees_with_the_fake_implementation():
                 _lib.native().check_intermediates(promised, q, q, lean)
                 with pytest.raises(RuntimeError, match="missing"):
                     _lib.native().check_intermediates([*promised[:-1], None], q, q, lean)
+
+
+def test_exact_pair_refuses_misaligned_buffers_without_launch(lib):
+    """Their kernels move states four floats at a time: a misaligned buffer is an error code, not a fault."""
+    def problem(args):
+        p = args.p
+        p.n_seqs, p.seq_len, p.total_tokens, p.heads, p.head_dim, p.dtype = 1, 8, 8, 1, 32, _lib.PKDA_F32
+        for f in ("q", "k", "v", "g", "g_atk", "beta_atk", "beta", "A_log", "dt_bias", "log_atk_scale"):
+            setattr(p, f, 256)
+        return p
+
+    fwd = _lib.RecurrentArgs()
+    p = problem(fwd)
+    fwd.o = 256
+    need = lib.pkda_recurrent_saved_bytes(C.byref(p))
+    assert lib.pkda_recurrent_fwd_saving(C.byref(fwd), 264, need, None) == 6
+    bwd = _lib.RecurrentBwdArgs()
+    p = problem(bwd)
+    for f in ("d_o", "dq", "dk", "dv", "dg", "dg_atk", "dbeta_atk", "dbeta", "dA_log", "ddt_bias", "dlog_atk_scale"):
+        setattr(bwd, f, 256)
+    bwd.workspace, bwd.workspace_bytes = 256, lib.pkda_recurrent_bwd_workspace_bytes(C.byref(p))
+    assert lib.pkda_recurrent_bwd_saved(C.byref(bwd), 264, need, None) == 6
+    bwd.workspace = 260
+    assert lib.pkda_recurrent_bwd(C.byref(bwd), None) == 6
+    assert lib.pkda_last_launch_count() == 0
