@@ -58,8 +58,10 @@ void finish(int status, const char* what) {
 void track_status(Tensor& slot, const Tensor& workspace, size_t offset) {
   if (!g_track.load(std::memory_order_relaxed)) return;
   Tensor word = workspace.narrow(0, (int64_t)offset, 4).clone();
+  // The word before goes after the lock: Python may own it, and letting go of it then takes the interpreter lock,
+  // which a reader of the status holds while it waits for this one.
   std::lock_guard<std::mutex> lock(g_status_mutex);
-  slot = std::move(word);
+  std::swap(slot, word);
 }
 
 // ---------------------------------------------------------------------- tensors
