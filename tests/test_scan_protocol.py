@@ -16,32 +16,57 @@ CSRC = os.path.join(ROOT, "delta_feedback_experiment_b200", "csrc")
 STAGES, SLOTS = 3, 2
 OPS = re.compile(r"\b(?:tc::)?(mbar_wait2|mbar_wait|warp_arrive|mbar_arrive|mbar_expect_tx)\(")
 LOOP = re.compile(r"for \(int [ij] = 0; [ij] < sq\.nchunks; \+\+[ij]\) \{")
+SHARED = "const bool out = kOut && role == 1;"   # one loop for the output warps (out) and the store warps
 
 
-def _call(text, at):
-    depth, i = 1, at
+def _closing(text, at, pair):
+    """Index behind the bracket that closes the one opened just before ``at``."""
+    depth = 1
     while depth:
-        depth += {"(": 1, ")": -1}.get(text[i], 0)
-        i += 1
-    return text[at:i - 1]
+        depth += {pair[0]: 1, pair[1]: -1}.get(text[at], 0)
+        at += 1
+    return at
+
+
+def _as_role(text, out):
+    """The loop body as one role runs it: the branches on ``out`` resolved."""
+    while m := re.search(r"if \((!?)out\) \{", text):
+        end = _closing(text, m.end(), "{}")
+        body, rest = text[m.end():end - 1], text[end:]
+        other = ""
+        if e := re.match(r" else \{", rest):
+            stop = _closing(rest, e.end(), "{}")
+            other, rest = rest[e.end():stop - 1], rest[stop:]
+        taken = body if out != bool(m.group(1)) else other
+        text = text[:m.start()] + taken + ("" if "continue;" in taken else rest)
+    return text
+
+
+def _ops(text):
+    ops = []
+    for m in OPS.finditer(text):
+        bars = re.findall(r"\bbar_(full|empty|ready|free)\b", text[m.end():_closing(text, m.end(), "()")])
+        if m.group(1) == "mbar_expect_tx":
+            bars = ["full"]
+        ops += [("wait" if "wait" in m.group(1) else "signal", b) for b in bars]
+    return ops
 
 
 def roles_of(source):
     """``{role: [("wait" | "signal", barrier), ...]}`` of one chunk, in the order of the source."""
     text = open(os.path.join(CSRC, source)).read()
-    marks = [(m.group(1), m.end()) for m in re.finditer(r"// -{8,} the (copies|chain|output|stores)\b", text)]
+    marks = [(m.group(1), m.end()) for m in re.finditer(r"// -{8,} the (copies|chain|stores)\b", text)]
+    if SHARED in text:
+        marks.append(("shared", text.index(SHARED)))
     ends = [at for _, at in marks[1:]] + [text.index("template <int NW", marks[-1][1])]
     roles = {}
     for (name, at), end in zip(marks, ends):
-        block = text[at:end]
-        block = block[LOOP.search(block).end():].replace("tma_load", "").replace(", bar,", "")
-        ops = []
-        for m in OPS.finditer(block):
-            bars = re.findall(r"\bbar_(full|empty|ready|free)\b", _call(block, m.end()))
-            if m.group(1) == "mbar_expect_tx":
-                bars = ["full"]
-            ops += [("wait" if "wait" in m.group(1) else "signal", b) for b in bars]
-        roles[name] = ops
+        loop = LOOP.search(text, at)
+        block = text[loop.end():min(end, _closing(text, loop.end(), "{}"))]
+        if name == "shared":
+            roles.update(output=_ops(_as_role(block, True)), stores=_ops(_as_role(block, False)))
+        else:
+            roles[name] = _ops(block)
     return roles
 
 
