@@ -1282,7 +1282,8 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   {
     const int units = p.n_seqs * p.heads;
     const int vb = units >= 120 ? 128 : (units >= 60 ? 64 : 32);  // value columns per CTA of the mma.sync kernel
-    // tcgen05 / TMEM / TMA at every size unless the mma.sync kernel is pinned (pkda_set_variant).
+    // Columns over four or eight SMs for few units, else tcgen05 / TMEM / TMA, as in the forward; the older
+    // mma.sync kernel runs only when it is pinned (pkda_set_variant).
     const bool scan_mma = stage_variant(kStageScanBwd) == 1;
     begin_stage(kStageScanBwd, st);
     if (!scan_mma && scan_columns(units))

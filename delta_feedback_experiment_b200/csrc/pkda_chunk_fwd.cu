@@ -872,11 +872,10 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   ScanParams sp;
   sp.geo = geo; sp.w = w; sp.u = u_ws; sp.kg = kg; sp.beta_c = beta_c; sp.gc = gc;
   sp.S0 = p.initial_state; sp.h = h; sp.v_new = v_new; sp.ST = ST;
-  // The scan runs on tcgen05 / TMEM / TMA, one CTA per (sequence, head), unless the mma.sync kernel is
-  // pinned (pkda_set_variant).  That holds for few units too: a chunk step is a latency chain whose
-  // length does not depend on how many CTAs run (2 rows x 16 heads, T = 4096: 0.82 ms per
-  // forward+backward against 0.87 ms with the value-sliced mma.sync scans).  The mma.sync kernel
-  // slices the value columns when there are fewer units than SMs.
+  // Few units (scan_columns: while four or eight CTAs per unit run in one wave): the value columns of a unit
+  // spread over that many SMs, with the state in mma.sync accumulators.  More units: tcgen05 / TMEM / TMA,
+  // one CTA per (sequence, head).  The older mma.sync kernel, which slices the value columns when there are
+  // fewer units than SMs, runs only when it is pinned (pkda_set_variant).  Same bits from the first two.
   const int units = p.n_seqs * p.heads;
   const int vb = units >= 120 ? 128 : (units >= 60 ? 64 : 32);
   int rc = PKDA_ERR_LAUNCH;

@@ -49,11 +49,9 @@ pkda_controls_fwd_kernel(const CtrlParams p) {
   }
 }
 
-// One thread per (row, column of the packed gradient).  Columns of the three logit
-// slices recompute their activation from the saved packed row.
 // Backward: the packed gradient row and the per-head parameter gradients.  A CTA owns a contiguous range of
-// rows and takes ctrl_rows(H) of them at a time: the two hidden slices are copied and the three activations
-// differentiated with one element (or pair) per thread, the contributions to the per-head sums go through
+// rows and takes ctrl_rows(H) of them at a time: the two hidden slices are copied and the three activations,
+// formed again from the packed row, differentiated with one element (or pair) per thread; the contributions to the per-head sums go through
 // shared memory and are added rows ascending, so that the sums have a fixed order.  (Row after row with one
 // thread per column took a memory round trip per row: 45 us for 2,000 rows of 280, now 5.)
 __host__ __device__ inline int ctrl_rows(int heads) { return heads >= 512 ? 1 : heads >= 256 ? 4 : 8; }

@@ -7,13 +7,13 @@
 //   S  <- diag(exp(g)) S ;  e = v - S^T k ;  S <- S + (beta kw) e^T ;  o = S^T (scale q)
 //
 // What bounds it: the chain of dependent tokens.  The value columns of S are independent of one
-// another, so each warp takes 4 or 8 columns with all D rows (ScanLay) and the step's only exchange
-// is log2(8) = 3 shuffles for e; with one CTA holding the whole state the step crossed three block
-// barriers and two shared-memory reductions.  The row vectors (exp(g), k, beta kw, q) do not depend
+// another, so each warp takes 4 columns (16 once the one-column warps fill the chip, 8 at D = 8) with all D
+// rows (ScanLay) and the step's only exchange is log2(8) = 3 shuffles for e (7 for four columns per lane);
+// with one CTA holding the whole state the step crossed three block barriers and two shared-memory reductions.  The row vectors (exp(g), k, beta kw, q) do not depend
 // on S: producer warps make them for 8 tokens at a time, double buffered, while the consumer warps
 // run the chain; the sum for o is off the chain and is reduced for 8 tokens at once.
-// Measured: 4 x 16 units, 48 tokens, D = 128, bf16: 67 -> 25 us; 2 x 4 units, 512 tokens,
-// D = 64, fp32: 548 -> 85 us.
+// Measured: 4 x 16 units, 48 tokens, D = 128, bf16: 67 -> 27 us; 2 x 4 units, 512 tokens,
+// D = 64, fp32: 548 -> 86 us (90 when it leaves what the backward needs).
 #include "pkda_launch.h"
 #include "pkda_recurrent.cuh"
 
@@ -238,9 +238,9 @@ pkda_recurrent_kernel(const RecParams p) {
 // A few tokens for more (sequence, head) units than SMs, e.g. a speculative block of a large batch:
 // reading and writing the states is most of the call.  One CTA keeps the whole state in registers
 // (thread = 16 rows x 4 columns, state rows moved in full 512-byte lines, two CTAs per SM), as the
-// decode step does, and crosses three block barriers per token.  D = 128, bf16, us at 2 / 8 / 16 tokens:
-// 256 units (one wave of this kernel, two of the sliced one) 8.2 / 18.5 / 32.5 against 21.0 / 21.0 / 30.9;
-// 1024 units 39.7 / 94.8 / 164 against 74.9 / 76.0 / 109.
+// decode step does, and crosses three block barriers per token.  D = 128, bf16, us a call at 2 / 7 / 13 / 16 tokens:
+// 256 units (one wave of this kernel, two of the sliced one) 10.3 / 18.4 / 28.7 / 33.8 against 22.6 / 22.6 / 32.8 /
+// 32.8; 512 units 16 / 35 / 57 / 70 against 41 / 43 / 62 / 62; 1024 units 41 / 86 / 142 / 166 against 78 / 78 / 113 / 113.
 template <int D, typename T>
 __global__ void __launch_bounds__(RecCfg<D>::kThreads, D == 128 ? 2 : 1)
 pkda_recurrent_few_kernel(const RecParams p) {

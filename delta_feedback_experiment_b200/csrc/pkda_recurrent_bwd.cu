@@ -15,7 +15,7 @@
 // digits that S - w e^T loses under strong decay).  The preconditioner's cotangent, a diagonal scan
 // backwards over the tokens, and the terms that depend on it close the pass.
 // (One CTA per (sequence, head) that replayed and walked back every token with the whole state took
-// 1655 us for 2 x 4 units of 512 tokens at D = 64, fp32, behind a 551 us forward; these take 104 us, behind 85.)
+// 1655 us for 2 x 4 units of 512 tokens at D = 64, fp32, behind a 551 us forward; these take 110 us, behind 90.)
 #include "pkda_launch.h"
 #include "pkda_recurrent.cuh"
 

@@ -989,7 +989,7 @@ PyObject* wrap_list(const std::vector<Tensor>& v) {
   return r;
 }
 
-// The fifteen leading arguments of every recurrence call: ten inputs, S0, A0, cu_seqlens, then
+// The sixteen leading arguments of every recurrence call: ten inputs, S0, A0, cu_seqlens, then
 // scale (None: 1 / sqrt(D)), squash_x and squash_eps.
 constexpr int kInputArgs = 16;
 struct ParsedInputs {

@@ -5,9 +5,9 @@
  * stream it is given, never synchronises, never allocates and returns an int
  * status (0 = ok).  Scratch memory is supplied by the caller, sized by the
  * *_workspace_bytes functions (the one exception is pkda_chunk_fwd_static, whose
- * scratch is an array inside the library).  The Python host code in
- * delta_feedback_experiment_b200/ binds these through ctypes; any other host
- * language binds them the same way.  Kernels run on the device that is current
+ * scratch is an array inside the library).  The torch host layer
+ * (delta_feedback_experiment_b200/csrc/pkda_torch.cpp) is one caller, the ctypes
+ * mirror in _lib.py another; any host language binds them the same way.  Kernels run on the device that is current
  * when an entry point is called: the caller makes the tensors' device current.
  *
  * Device-side failures.  The tensor-core kernels wait on hardware barriers with
