@@ -184,9 +184,10 @@ def test_direct_block_variants(cap, dist):
 
 @pytest.mark.parametrize("B", [4, 8])
 def test_wide_state_slices_match_narrow_ones(B):
-    """The state scans have two implementations: tcgen05 / tensor-memory kernels (one CTA per
-    (row, head), all 128 value columns; the default at every size) and mma.sync kernels that
-    cut the value columns into 32- or 64-wide slices when there are fewer than 120 (row, head)
+    """The state scans have three implementations: tcgen05 / tensor-memory kernels (one CTA per
+    (row, head), all 128 value columns), column scans over four or eight SMs per (row, head)
+    where there are few of them (a row alone here), and the older mma.sync kernels that cut the
+    value columns into 32- or 64-wide slices when there are fewer than 120 (row, head)
     units (`set_variant("scan_fwd" / "scan_bwd", 1)`).  Rows are independent, so a row of the
     big batch must agree with the same row run alone through the other implementation.
     Both feed the same bf16 operands to the tensor cores in the same order; on this short input

@@ -26,7 +26,7 @@ def _grads(d, S0, A0, do, dS, lean, cu=None):
 
 
 @pytest.mark.parametrize("D,T,B,H", [(8, 9, 2, 3), (16, 33, 1, 2), (32, 65, 2, 1), (64, 7, 1, 4), (64, 96, 3, 5),
-                                     (128, 40, 1, 2), (128, 31, 5, 32)])
+                                     (64, 33, 20, 4), (128, 40, 1, 2), (128, 31, 5, 32)])
 def test_exact_forward_and_backward(D, T, B, H):
     d = make_inputs(B, T, H, D, seed=D + T, dist="production", dtype=torch.float32, with_state=True)
     dS = torch.randn(B, H, D, D, generator=torch.Generator().manual_seed(1)) * 0.1

@@ -1,7 +1,7 @@
 """The sharding helpers through the CUDA operator on one GPU: the shards of a plan are run
 one after the other, merged, and compared with the unsharded call.  Row tensors must be
-equal bit for bit (rows and heads are independent, and no kernel is chosen from the size of
-the problem); the per-head parameter gradients are sums over rows and are compared within
+equal bit for bit (rows and heads are independent, and the state scans that the number of
+(row, head) units chooses between give the same bits); the per-head parameter gradients are sums over rows and are compared within
 rounding."""
 
 import pytest
@@ -44,8 +44,8 @@ def _merge(parts, plan, H, packed=False):
 @pytest.mark.parametrize("B,H,world", [(16, 16, 2), (8, 32, 2), (8, 32, 16), (4, 8, 4)])
 def test_sharded_equals_unsharded(B, H, world):
     # (8, 32, 16): fewer rows than ranks, so pairs of ranks split a row's heads; (4, 8, 4): shards of
-    # 8 (row, head) units.  No kernel is chosen from the size of the problem, so shards of any
-    # size reproduce the whole problem's bits.
+    # 8 (row, head) units, whose scans spread over eight SMs each, of 32, which spread over four.  Every
+    # scan takes its products in the same order, so shards of any size reproduce the whole problem's bits.
     T = 192
     d = make_inputs(B, T, H, D, seed=61, dtype=torch.bfloat16, with_state=True)
     whole = _run(d)
