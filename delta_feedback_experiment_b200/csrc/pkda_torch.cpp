@@ -482,6 +482,16 @@ auto typed_op(const char* name) {
   return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<F>();
 }
 
+// A backward's call of its operator.  Where no graph is recorded (an ordinary backward) the operator's autograd
+// kernel has nothing to do and is passed by.  (Called behind get_saved_variables: unpacking may run the forward
+// again, which must not be below autograd.)
+template <typename Op, typename... A>
+auto call_backward(const Op& op, A&&... args) {
+  if (at::GradMode::is_enabled()) return op.call(std::forward<A>(args)...);
+  at::AutoDispatchBelowADInplaceOrView below;
+  return op.call(std::forward<A>(args)...);
+}
+
 // The backward operators have no derivative of their own.  Where one could be asked for (a graph is being
 // recorded, create_graph = True), their results hang on a node that raises: without it they would come out as
 // constants and a second derivative would silently be missing.
@@ -544,9 +554,9 @@ struct Recurrence : torch::autograd::Function<Recurrence> {
     const auto it = ctx->saved_data.find("autocast");
     if (it != ctx->saved_data.end()) autocast = (at::ScalarType)it->second.toInt();
     const Tensor d_o = grads[0].defined() ? grads[0] : at::zeros_like(t[0], at::MemoryFormat::Contiguous);
-    std::vector<Tensor> got = op.call(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9],
-                                      at::TensorList(t).slice(10), d_o, conf[0], conf[1], conf[2], autocast,
-                                      conf[3] != 0.0);
+    std::vector<Tensor> got = call_backward(op, t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9],
+                                            at::TensorList(t).slice(10), d_o, conf[0], conf[1], conf[2], autocast,
+                                            conf[3] != 0.0);
     variable_list out(14);
     std::move(got.begin(), got.end(), out.begin());
     return out;
@@ -651,8 +661,8 @@ struct Conv : torch::autograd::Function<Conv> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     static const auto op = typed_op<ConvBackwardSig>("delta_feedback::pkda_qkv_conv_backward");
     variable_list t = ctx->get_saved_variables();
-    auto [dx, dw] = op.call(t[0], t[1], grads[0], grads[1], grads[2], ctx->saved_data["head_dim"].toSymInt(),
-                            ctx->saved_data["norm_channels"].toSymInt(), ctx->saved_data["eps"].toDouble());
+    auto [dx, dw] = call_backward(op, t[0], t[1], grads[0], grads[1], grads[2], ctx->saved_data["head_dim"].toSymInt(),
+                                  ctx->saved_data["norm_channels"].toSymInt(), ctx->saved_data["eps"].toDouble());
     return {dx, dw, Tensor(), Tensor(), Tensor()};
   }
 };
@@ -744,8 +754,8 @@ struct NormGate : torch::autograd::Function<NormGate> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     static const auto op = typed_op<NormGateBackwardSig>("delta_feedback::pkda_norm_gate_backward");
     variable_list t = ctx->get_saved_variables();
-    auto [dx, dg, dw] = op.call(t[0], t[1], t[2], t[3], zeros_if_undefined(grads[0], t[0]),
-                                ctx->saved_data["eps"].toDouble());
+    auto [dx, dg, dw] = call_backward(op, t[0], t[1], t[2], t[3], zeros_if_undefined(grads[0], t[0]),
+                                      ctx->saved_data["eps"].toDouble());
     return {dx, dg, dw, Tensor()};
   }
 };
