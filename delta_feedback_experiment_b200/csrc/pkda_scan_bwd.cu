@@ -7,7 +7,7 @@
 //   store warp    stores d (the saved dh) and dF
 //   copy warp     kg, W, qg, dO, P, beta, Gam_last by TMA, up to three chunks ahead
 // The chain warp leaves d and dF for the store warp in shared memory, two slots deep.  T = 4096, 24 units:
-// 163 -> 104 us.  Every wait is bounded.
+// 163 -> 109 us.  Every wait is bounded.
 // Rows of a ragged last chunk past its end hold the next sequence's tokens (or zero fill past the end of
 // the tensor): dO is masked there, beta is zero there, nothing else of those rows reaches a kept result.
 #include "pkda_scan.cuh"

@@ -10,7 +10,8 @@
 //   copy warp     W, kg, U, qg, P, beta, Gam_last by TMA, up to three chunks ahead
 // The chain warp leaves h and E for the other two in shared memory, two slots deep.  A step takes 1.05 us with
 // one column group per CTA and 1.45 us with two (the SM's shared memory then moves 1,700 of the 2,700 cycles);
-// T = 8192, 16 units: 360 -> 136 us, T = 4096, 24 units: 180 -> 93 us.  Every wait is bounded: on a timeout the warp sets the status word and leaves.
+// T = 8192, 16 units: 360 -> 141 us, T = 4096, 24 units: 180 -> 100 us.  Every wait is bounded: on a timeout the
+// warp sets the status word and leaves.
 #include "pkda_scan.cuh"
 
 namespace pkda {

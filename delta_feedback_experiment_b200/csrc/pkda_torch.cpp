@@ -5,7 +5,7 @@
 // kernels are shorter than the interpreter work that used to surround them: filling
 // one struct through ctypes, entering the device guard and allocating tensors from
 // Python cost 33 us per decoding step and 0.8 ms per small training step, against
-// 4 us and 0.15 ms of kernels.
+// 4 us and 0.13 ms of kernels.
 //
 // Three kinds of entry:
 //  * dispatcher operators (delta_feedback::pkda_recurrence, pkda_qkv_conv, pkda_norm_gate
