@@ -416,10 +416,8 @@ struct IntraParams {
   float scale, ln_x, eps;
   int direct_cap;  // upper limit for the direct block size (64 = no limit, 1 = hierarchy only)
   int* status;     // device status word (tcgen05 kernel): set to 1 when a bounded wait gives up
-  // Work list of (chunk * heads + head) items the tensor-memory kernel leaves to the mma.sync kernel;
-  // counts[1] is its length, counts[0] and counts[2] the cursors the CTAs of the two kernels draw their
-  // items with (all zeroed before every call).  slow_list == NULL: the mma.sync kernel takes every chunk, one CTA per item.
-  int *slow_list, *counts;
+  int* cursor;     // the CTAs draw their items with it (zeroed before every call)
+  int by_strip;    // nonzero: every chunk is paired strip by strip, whatever it decays by
   // Preconditioner state across chunks inside the tensor-memory kernel (dense batches; chain != 0):
   // every item computes its chunk's local scan anyway, so it takes its chunk-entry state from the item
   // of the chunk before (a_chain, which is the saved "state at chunk starts" tensor; chain_flags counts
@@ -505,7 +503,7 @@ int scan_columns(int units);
 // Host-side pieces defined in pkda_chunk_fwd.cu and reused by the backward.
 int check_chunk_problem(const pkda_problem& p);
 int run_prologue(const pkda_problem& p, int* chunk_offsets, float* beta_c, Geo* geo, cudaStream_t st);
-// lists: room for chunks * heads ints (the forward's work list); counts: three zeroed ints.
+// cursor: a zeroed int.
 // o / o_done: the forward's output tensor; *o_done says whether the state scan has already written it.
 // What the tensor-memory intra kernel needs to carry the preconditioner state across chunks itself
 // (dense batches): see IntraParams::chain.
@@ -517,7 +515,7 @@ struct ChainArgs {
 bool forward_chain_possible(const pkda_problem& p);
 int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_c, bf16* u_ws, bf16* Aqk,
                        bf16* Akk, bf16* kt, float* gc, const float* a_start, bf16* w, bf16* kg, bf16* v_new,
-                       bf16* h, bf16* qg, float* ST, bool recompute, int* status, int* lists, int* counts,
+                       bf16* h, bf16* qg, float* ST, bool recompute, int* status, int* cursor,
                        cudaStream_t st, bf16* o = nullptr, bool* o_done = nullptr, const ChainArgs* chain = nullptr);
 
 }  // namespace pkda

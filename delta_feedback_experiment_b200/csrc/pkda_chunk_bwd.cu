@@ -1175,7 +1175,7 @@ struct BwdWorkspace {
   float *dk_read, *dkt, *partA, *partB, *partC, *c_loc, *lam_in;
   int2* fast_list;
   int *slow_list, *counts;
-  int *fwd_lists, *fwd_counts;  // work lists of the recompute pass (lean backward)
+  int* fwd_cursor;  // item cursor of the recompute pass (lean backward)
   int* status;
   size_t bytes;
 };
@@ -1204,10 +1204,9 @@ static BwdWorkspace carve_bwd(const pkda_problem& p, void* base) {
   w.lam_in = static_cast<float*>(take(chunks * H * kD * 4));
   w.fast_list = static_cast<int2*>(take(chunks * H * sizeof(int2)));
   w.slow_list = static_cast<int*>(take(chunks * H * sizeof(int)));
-  w.fwd_lists = static_cast<int*>(take(chunks * H * sizeof(int)));
   w.status = static_cast<int*>(take(16 * sizeof(int)));  // status word, then lengths and cursors of the work lists
   w.counts = w.status + 1;       // [0] fast, [1] slow, [2] cursor
-  w.fwd_counts = w.status + 5;   // [1] slow, [2] cursor
+  w.fwd_cursor = w.status + 5;
   w.bytes = off;
   return w;
 }
@@ -1271,7 +1270,7 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
     // The recompute kernels only read the products, write keys and decay totals.
     rc = run_forward_stages(p, geo, ws.beta_c, ws.u, const_cast<bf16*>(Aqk), const_cast<bf16*>(Akk),
                             const_cast<bf16*>(kt), const_cast<float*>(gc), a->a_atk, w, kg, v_new, h, qg,
-                            nullptr, true, ws.status, ws.fwd_lists, ws.fwd_counts, st);
+                            nullptr, true, ws.status, ws.fwd_cursor, st);
     if (rc != PKDA_OK) return rc;
   }
 

@@ -6,16 +6,14 @@
 //   atk_local chunk-local preconditioner accumulation (from A = 0) and decay sums
 //   atk_carry sequential over a sequence's chunks: A at every chunk start
 //   intra     per chunk: log-decay cumsum, write keys, gated pair products
-//             M (k x kt) and P (q x kt) by a binary hierarchy of reference rows,
+//             M (k x kt) and P (q x kt), relative to one reference row or strip by strip,
 //             Tm = (I + tril(M) diag(beta))^-1, W = Tm (k*Gam), U = Tm v,
 //             kg = kt * exp(G_last - G), qg = scale q * Gam
 //   scan      sequential over chunks, V split across CTAs: h_n, E = U - W h_n,
 //             S <- Gam_last * S + kg^T (beta E)
 //   out       per chunk: o = qg h_n + P (beta E)
 // With per-channel decay exp(G_i - G_j) cannot be factored as exp(G_i)exp(-G_j)
-// (overflow after a few tokens); level L of the hierarchy pairs rows whose index
-// has bit L set with rows of the same 2L-block whose bit L is clear, both
-// expressed relative to the first row of the upper half, so every factor is <= 1.
+// (overflow after a few tokens), hence the reference rows (pkda_intra_fwd_tc.cu).
 #include <algorithm>
 
 #include "pkda_chunk.cuh"
@@ -156,354 +154,6 @@ pkda_atk_carry_kernel(Geo geo, const float* ac_local, const float* sa, const flo
     }
   }
   if (AT) AT[((size_t)n * H + h) * kD + c] = A;
-}
-
-// ------------------------------------------------------------------ intra-chunk kernel
-namespace intra {
-constexpr int kThreads = 512;
-constexpr int oQ = 0;
-constexpr int oK = oQ + kTileBytes;
-constexpr int oKt = oK + kTileBytes;
-constexpr int oG = oKt + kTileBytes;              // fp32 [64][kLdG]
-constexpr int oStage = oG + kChunk * kLdG * 4;    // 3 bf16 tiles; aliased (see below)
-constexpr int oTmb = oStage + 3 * kTileBytes;     // bf16 [64][72]: P staging, then Tm
-constexpr int oSmall = oTmb + kChunk * kLdC * 2;  // beta[64] pd[64] bp[64] bias[128]
-constexpr int kSmem = oSmall + (3 * kChunk + kD + 24) * 4;  // + per-warp block-decay maxima
-// aliases inside the staging area
-constexpr int oAt = oStage;                       // fp32 [64][kLdG] preconditioner states (before the levels)
-constexpr int kLdL = 68;                          // = 4 (mod 8): the inverse's MMA fragments load without bank conflicts
-constexpr int oL = oStage;                        // after the levels: L, T, Y2
-constexpr int oT = oL + kChunk * kLdL * 4;
-constexpr int oY2 = oT + kChunk * kLdL * 4;       // fp32 [1280]
-static_assert(oY2 + 1280 * 4 <= oTmb, "inverse scratch must fit in the staging area");
-static_assert(kChunk * kLdG * 4 <= 3 * kTileBytes, "A_t array must fit in the staging area");
-}  // namespace intra
-
-// Writes one 16x16 accumulator tile pair (two n8 tiles) through a functor f(i, j, value).
-template <typename F>
-__device__ __forceinline__ void for_tile(const float (&t)[2][4], int i0, int j0, int gq, int tq, F f) {
-#pragma unroll
-  for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) f(i0 + gq + 8 * (e >> 1), j0 + 8 * nt + 2 * tq + (e & 1), t[nt][e]);
-}
-
-// kRecompute: rebuild w,u,kg,qg only (backward's lean mode); the products, their inverse T (as it was
-// rounded for W and U), the write keys and the decay totals already exist, so the levels and the inversion
-// are left out (1,300 strongly decaying chunks: 178 us with them, 77 without).
-// One (chunk bx, head by) item; every thread of the CTA takes part.
-template <bool kRecompute>
-__device__ __forceinline__ void intra_fwd_item(const IntraParams& p, int bx, int by) {
-  using namespace intra;
-  extern __shared__ __align__(128) unsigned char smem[];
-  bf16* sQ = reinterpret_cast<bf16*>(smem + oQ);
-  bf16* sK = reinterpret_cast<bf16*>(smem + oK);
-  bf16* sKt = reinterpret_cast<bf16*>(smem + oKt);
-  float* sG = reinterpret_cast<float*>(smem + oG);
-  bf16* sXq = reinterpret_cast<bf16*>(smem + oStage);
-  bf16* sXk = sXq + kChunk * kLdD;
-  bf16* sY = sXk + kChunk * kLdD;
-  bf16* sTmb = reinterpret_cast<bf16*>(smem + oTmb);
-  float* sBeta = reinterpret_cast<float*>(smem + oSmall);
-  float* sPd = sBeta + kChunk;
-  float* sBp = sPd + kChunk;
-  float* sBias = sBp + kChunk;
-  float* sWarpMax = sBias + kD;  // [4][6]
-  float* sAt = reinterpret_cast<float*>(smem + oAt);
-  float* sL = reinterpret_cast<float*>(smem + oL);
-  float* sT = reinterpret_cast<float*>(smem + oT);
-  float* sY2 = reinterpret_cast<float*>(smem + oY2);
-
-  int n, tok0, valid;
-  if (!chunk_lookup(p.geo, bx, n, tok0, valid)) return;
-  const int h = by, H = p.geo.heads;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int gq = lane >> 2, tq = lane & 3;
-  const size_t chh = (size_t)bx * H + h;
-  const size_t row0 = ((size_t)tok0 * H + h) * kD;  // element offset of (tok0, h, 0)
-  const long gld = (long)H * kD;
-
-  // ---- 1. tiles and per-row scalars.  The per-row scalars are requested first (the first barrier
-  // waits for them and they would otherwise queue behind the 48 KB of tile traffic), then the raw
-  // gate (needed next), then the q and k tiles.
-  float s_beta = 0.f, s_pd = 0.f, s_bp = 0.f, s_bias = 0.f;
-  if (tid < kChunk) {
-    const size_t s = (size_t)(tok0 + min(tid, valid - 1)) * H + h;
-    s_beta = p.beta_c[chh * kChunk + tid];
-    s_pd = p.g_atk[s];
-    s_bp = to_f(p.beta_atk[s]);
-  } else if (tid < kChunk + kD) {
-    s_bias = p.dt_bias[h * kD + tid - kChunk];
-  }
-  GateRaw<kThreads> graw;
-  gate_load(graw, p.g + row0, gld, valid, tid);
-  // Scalars of later phases are fetched here: a global load issued where it is used costs
-  // that phase a full memory round trip with nothing to overlap it.
-  const float a_log = p.A_log[h];
-  const float centre = kRecompute ? 0.f : p.log_atk_scale[h];
-  float a_first = 0.f;
-  if (!kRecompute && tid >= kD && tid < 2 * kD) a_first = p.a_start[chh * kD + tid - kD];
-  tile_load_async(sQ, kLdD, p.q + row0, gld, kChunk, kD, valid, kThreads);
-  tile_load_async(sK, kLdD, p.k + row0, gld, kChunk, kD, valid, kThreads);
-  if (kRecompute) {
-    tile_load_async(sKt, kLdD, p.kt + row0, gld, kChunk, kD, valid, kThreads);
-    tile_load_async(sTmb, kLdC, p.Akk + ((size_t)tok0 * H + h) * kChunk, (long)H * kChunk, kChunk, kChunk, valid, kThreads);
-    tile_load_async(sXk, kLdD, p.v + row0, gld, kChunk, kD, valid, kThreads);
-  }
-  cp_async_commit();
-  if (tid < kChunk) {
-    const bool ok = tid < valid;
-    sBeta[tid] = s_beta;
-    sPd[tid] = ok ? __expf(s_pd) : 1.f;
-    sBp[tid] = ok ? s_bp : 0.f;
-  } else if (tid < kChunk + kD) {
-    sBias[tid - kChunk] = s_bias;
-  }
-  if (!kRecompute) {  // zero the P staging tile (upper triangle must read as zero)
-    for (int i = tid; i < kChunk * kLdC / 8; i += kThreads) reinterpret_cast<uint4*>(sTmb)[i] = make_uint4(0, 0, 0, 0);
-  }
-  __syncthreads();
-
-  // ---- 2. decay gate (elementwise, all threads; the q and k tiles are still landing), then
-  // the two per-channel sequential passes side by side: cumulative sum | preconditioner recurrence A_t
-  gate_apply(graw, sG, valid, sBias, __expf(a_log) * kLog2e, tid);
-  cp_async_wait<0>();
-  __syncthreads();
-  if (tid < kD) {
-    gate_cumsum(sG, tid);
-    if (!kRecompute) {
-      float dmax[6];
-      block_decay_max(sG, tid, dmax);
-#pragma unroll
-      for (int e = 0; e < 6; ++e) {
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) dmax[e] = fmaxf(dmax[e], __shfl_xor_sync(0xffffffffu, dmax[e], o));
-        if (lane == 0) sWarpMax[warp * 6 + e] = dmax[e];
-      }
-    }
-  } else if (!kRecompute && tid < 2 * kD) {
-    const int c = tid - kD;
-    float A = a_first;
-#pragma unroll 8
-    for (int r = 0; r < kChunk; ++r) {
-      const float kc = to_f(sK[r * kLdD + c]);
-      A = sPd[r] * A + sBp[r] * kc * kc;
-      sAt[r * kLdG + c] = A;
-    }
-  }
-  __syncthreads();
-  if (!kRecompute) {
-    // write keys kt = k * exp(-ln(x) * dev / (1 + |dev|)), dev = log(A + eps) - centre
-    for (int idx = tid; idx < kChunk * kD / 8; idx += kThreads) {
-      const int r = idx >> 4, c8 = (idx & 15) << 3;
-      const float4 A0 = *reinterpret_cast<const float4*>(sAt + r * kLdG + c8);
-      const float4 A1 = *reinterpret_cast<const float4*>(sAt + r * kLdG + c8 + 4);
-      const float Av[8] = {A0.x, A0.y, A0.z, A0.w, A1.x, A1.y, A1.z, A1.w};
-      float f[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float dev = __logf(Av[j] + p.eps) - centre;
-        f[j] = __expf(-p.ln_x * __fdividef(dev, 1.f + fabsf(dev)));
-      }
-      uint4 x = *reinterpret_cast<const uint4*>(sK + r * kLdD + c8);
-      scale8(x, f);
-      *reinterpret_cast<uint4*>(sKt + r * kLdD + c8) = x;
-      if (r < valid) *reinterpret_cast<uint4*>(p.kt + row0 + (size_t)r * gld + c8) = x;
-    }
-    __syncthreads();
-  }
-
-  if (!kRecompute) {
-  // ---- 3. gated pair products, level by level.
-  // warps 0-7 : (mat, I) own the diagonal 16x16 tile (I,I): levels 8,4,2,1 (and the ungated diagonal of P)
-  // warps 8-15: (mat, idx) own one tile of level 32 and (idx < 2) one tile of level 16
-  // mat 0 = M (rows k), mat 1 = P (rows q).
-  const bool diagw = warp < 8;
-  const int mat = (warp >> 2) & 1, I = warp & 3;
-  float accA[2][4], accB[2][4];  // diag warps: accA; off warps: accA = level-32 tile, accB = level-16 tile
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) accA[a][e] = accB[a][e] = 0.f;
-  const int I32 = 2 + (I >> 1), J32 = I & 1;   // level-32 tile of an off warp
-  const int I16 = 1 + 2 * I, J16 = 2 * I;      // level-16 tile (I < 2)
-
-  // Pairs inside a b-block go through the direct level (lvl = 0), the rest through
-  // hierarchy levels >= b.  Each off-diagonal tile is produced exactly once.
-  const int bdir = pick_direct_block(sWarpMax, 4, p.direct_cap);
-#pragma unroll 1
-  for (int it = (bdir > 1 ? 0 : 1); it <= 6; ++it) {
-    const int lvl = it ? (64 >> it) : 0;  // 0 (direct), 32, 16, 8, 4, 2, 1
-    if (lvl && lvl < bdir) break;
-    stage_level(sXq, sXk, sY, sQ, sK, sKt, sG, lvl, bdir, tid, kThreads);
-    __syncthreads();
-    const bf16* X = mat ? sXq : sXk;
-    float tmp[1][2][4];
-    if (!diagw) {
-      // level-32 region tile: by hierarchy level 32 unless the direct block covers it (b = 64)
-      if ((lvl == 32) || (lvl == 0 && bdir > 32)) {
-        zero_acc(tmp);
-        warp_gemm<1, 2, false, false>(tmp, X, kLdD, 16 * I32, sY, kLdD, 16 * J32, 0, kD);
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) accA[a][e] = tmp[0][a][e];
-      }
-      // level-16 region tile: by hierarchy level 16 unless the direct block covers it (b >= 32)
-      if (I < 2 && ((lvl == 16 && bdir <= 16) || (lvl == 0 && bdir > 16))) {
-        zero_acc(tmp);
-        warp_gemm<1, 2, false, false>(tmp, X, kLdD, 16 * I16, sY, kLdD, 16 * J16, 0, kD);
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) accB[a][e] = tmp[0][a][e];
-      }
-    } else if (lvl <= 8) {
-      zero_acc(tmp);
-      warp_gemm<1, 2, false, false>(tmp, X, kLdD, 16 * I, sY, kLdD, 16 * I, 0, kD);
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = 16 * I + gq + ((e >> 1) << 3);
-          const int j = 16 * I + 8 * nt + 2 * tq + (e & 1);
-          if (pair_ok(i, j, lvl, bdir)) accA[nt][e] += tmp[0][nt][e];
-        }
-    }
-    __syncthreads();
-  }
-  if (diagw && mat == 1) {  // diagonal of P: ungated q_i . kt_i
-    float tmp[1][2][4];
-    zero_acc(tmp);
-    warp_gemm<1, 2, false, false>(tmp, sQ, kLdD, 16 * I, sKt, kLdD, 16 * I, 0, kD);
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = 16 * I + gq + ((e >> 1) << 3);
-        const int j = 16 * I + 8 * nt + 2 * tq + (e & 1);
-        if (i == j) accA[nt][e] += tmp[0][nt][e];
-      }
-  }
-
-  // ---- 4. P -> bf16 staging tile (scaled) ; L = tril(M,-1) diag(beta) -> smem fp32
-  for (int i = tid; i < kChunk * kLdL; i += kThreads) sL[i] = 0.f;
-  __syncthreads();
-  {
-    auto putP = [&](int i, int j, float v) { if (j <= i) sTmb[i * kLdC + j] = __float2bfloat16(v * p.scale); };
-    auto putL = [&](int i, int j, float v) { if (j < i) sL[i * kLdL + j] = v * sBeta[j]; };
-    if (diagw) {
-      if (mat) for_tile(accA, 16 * I, 16 * I, gq, tq, putP); else for_tile(accA, 16 * I, 16 * I, gq, tq, putL);
-    } else {
-      if (mat) for_tile(accA, 16 * I32, 16 * J32, gq, tq, putP); else for_tile(accA, 16 * I32, 16 * J32, gq, tq, putL);
-      if (I < 2) {
-        if (mat) for_tile(accB, 16 * I16, 16 * J16, gq, tq, putP); else for_tile(accB, 16 * I16, 16 * J16, gq, tq, putL);
-      }
-    }
-  }
-  __syncthreads();
-  {
-    for (int i = tid; i < kChunk * kChunk / 8; i += kThreads) {
-      const int r = i >> 3, c8 = (i & 7) << 3;
-      if (r < valid)
-        *reinterpret_cast<uint4*>(p.Aqk + ((size_t)(tok0 + r) * H + h) * kChunk + c8) =
-            *reinterpret_cast<const uint4*>(sTmb + r * kLdC + c8);
-    }
-  }
-
-  // ---- 5. T = (I + L)^-1 in fp32
-  unit_lower_inverse_64<8>(sL, sT, sY2, kLdL, kLdL, tid, kThreads);  // ends with a __syncthreads()
-  for (int i = tid; i < kChunk * kChunk / 2; i += kThreads) {
-    const int r = i >> 5, c2 = (i & 31) << 1;
-    const uint32_t pk = pack_bf16(sT[r * kLdL + c2], sT[r * kLdL + c2 + 1]);
-    *reinterpret_cast<uint32_t*>(sTmb + r * kLdC + c2) = pk;
-    if (r < valid)
-      *reinterpret_cast<uint32_t*>(p.Akk + ((size_t)(tok0 + r) * H + h) * kChunk + c2) = pk;
-  }
-  __syncthreads();
-  }  // !kRecompute
-
-  // ---- 6. decayed operands: Kd -> smem; qg, kg, gc -> global; V tile -> smem
-  bf16* sKd = sXq;
-  bf16* sV = sXk;
-  if (!kRecompute) {
-    tile_load_async(sV, kLdD, p.v + row0, gld, kChunk, kD, valid, kThreads);
-    cp_async_commit();
-  }
-  for (int idx = tid; idx < kChunk * kD / 8; idx += kThreads) {
-    const int r = idx >> 4, c8 = (idx & 15) << 3;
-    const float4 g0 = *reinterpret_cast<const float4*>(sG + r * kLdG + c8);
-    const float4 g1 = *reinterpret_cast<const float4*>(sG + r * kLdG + c8 + 4);
-    const float4 l0 = *reinterpret_cast<const float4*>(sG + (kChunk - 1) * kLdG + c8);
-    const float4 l1 = *reinterpret_cast<const float4*>(sG + (kChunk - 1) * kLdG + c8 + 4);
-    const float G[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-    const float Gl[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-    float e[8], es[8], tl[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      e[j] = ex2(G[j]);
-      es[j] = e[j] * p.scale;
-      tl[j] = ex2(Gl[j] - G[j]);
-    }
-    uint4 kk = *reinterpret_cast<const uint4*>(sK + r * kLdD + c8);
-    scale8(kk, e);
-    *reinterpret_cast<uint4*>(sKd + r * kLdD + c8) = kk;
-    if (r < valid) {
-      uint4 qq = *reinterpret_cast<const uint4*>(sQ + r * kLdD + c8);
-      uint4 kt = *reinterpret_cast<const uint4*>(sKt + r * kLdD + c8);
-      scale8(qq, es);
-      scale8(kt, tl);
-      const size_t off = row0 + (size_t)r * gld + c8;
-      *reinterpret_cast<uint4*>(p.qg + off) = qq;
-      *reinterpret_cast<uint4*>(p.kg + off) = kt;
-    }
-    if (!kRecompute && r == kChunk - 1) {
-      *reinterpret_cast<float4*>(p.gc + chh * kD + c8) = make_float4(e[0], e[1], e[2], e[3]);
-      *reinterpret_cast<float4*>(p.gc + chh * kD + c8 + 4) = make_float4(e[4], e[5], e[6], e[7]);
-    }
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-
-  // ---- 7. W = Tm Kd, U = Tm V   (warp: matrix = warp>>3, rows 16*((warp>>1)&3), column half warp&1)
-  {
-    const int m7 = warp >> 3, I7 = (warp >> 1) & 3, n0 = 64 * (warp & 1);
-    float acc2[1][8][4];
-    zero_acc(acc2);
-    warp_gemm<1, 8, false, true>(acc2, sTmb, kLdC, 16 * I7, m7 ? sV : sKd, kLdD, n0, 0, 16 * (I7 + 1));
-    bf16* dst = m7 ? p.u : p.w;
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = 16 * I7 + gq + 8 * half;
-        if (i < valid)
-          *reinterpret_cast<uint32_t*>(dst + row0 + (size_t)i * gld + n0 + 8 * nt + 2 * tq) =
-              pack_bf16(acc2[0][nt][2 * half], acc2[0][nt][2 * half + 1]);
-      }
-  }
-}
-
-// grid (chunks, heads): one item per CTA; or, with a work list, a few persistent CTAs that walk it.
-template <bool kRecompute>
-__global__ void __launch_bounds__(intra::kThreads, 1)
-pkda_intra_fwd_kernel(const IntraParams p) {
-  if (!p.slow_list) {
-    intra_fwd_item<kRecompute>(p, blockIdx.x, blockIdx.y);
-    return;
-  }
-  // items differ in cost (the number of pairing levels follows the decay): CTAs draw them one at a time
-  __shared__ int s_item;
-  const int n_items = p.counts[1], H = p.geo.heads;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(p.counts + 2, 1);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= n_items) break;
-    const int chh = p.slow_list[item];
-    intra_fwd_item<kRecompute>(p, chh / H, chh % H);
-    __syncthreads();  // the next item reuses every shared-memory region (and s_item)
-  }
 }
 
 // ------------------------------------------------------------------ forward state scan
@@ -743,8 +393,7 @@ struct FwdWorkspace {
   int* chunk_offsets;
   float* beta_c;
   bf16* u;
-  int* lists;   // work list of the intra-chunk stage (chunks * heads ints)
-  int* status;  // device status word: 0 = ok, 1 = a bounded wait in a kernel gave up; then the list lengths
+  int* status;  // device status word: 0 = ok, 1 = a bounded wait in a kernel gave up; then the item cursor
   size_t bytes;
 };
 
@@ -759,8 +408,6 @@ static FwdWorkspace carve_fwd(const pkda_problem& p, void* base) {
   off += align_up(chunks * p.heads * kChunk * sizeof(float));
   w.u = reinterpret_cast<bf16*>(b + off);
   off += align_up((size_t)p.total_tokens * p.heads * kD * sizeof(bf16));
-  w.lists = reinterpret_cast<int*>(b + off);
-  off += align_up(chunks * p.heads * sizeof(int));
   w.status = reinterpret_cast<int*>(b + off);
   off += 8 * sizeof(int);
   w.chain_flags = reinterpret_cast<int*>(b + off);
@@ -817,9 +464,8 @@ static int launch_scan_fwd(const ScanParams& sp, int units, cudaStream_t st) {
 int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_c, bf16* u_ws,
                        bf16* Aqk, bf16* Akk, bf16* kt, float* gc, const float* a_start,
                        bf16* w, bf16* kg, bf16* v_new, bf16* h, bf16* qg, float* ST,
-                       bool recompute, int* status, int* lists, int* counts, cudaStream_t st, bf16* o,
+                       bool recompute, int* status, int* cursor, cudaStream_t st, bf16* o,
                        bool* o_done, const ChainArgs* chain) {
-  const int chunks = geo.total_chunks;
   IntraParams ip;
   ip.geo = geo;
   ip.q = static_cast<const bf16*>(p.q); ip.k = static_cast<const bf16*>(p.k);
@@ -831,43 +477,21 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   ip.w = w; ip.u = u_ws; ip.kg = kg; ip.qg = qg;
   ip.scale = p.scale; ip.ln_x = logf(p.squash_x); ip.eps = p.squash_eps;
   ip.direct_cap = direct_block_cap();
-  ip.status = status;
-  ip.slow_list = ip.counts = nullptr;
+  ip.by_strip = stage_variant(kStageIntraFwd) != 0 || ip.direct_cap < 64;
+  ip.status = status; ip.cursor = cursor;
   ip.chain = 0;
   ip.beta = static_cast<const bf16*>(p.beta); ip.A0 = p.initial_A_state;
   ip.beta_c_w = ip.a_chain = ip.sa = ip.AT = nullptr;
   ip.chain_flags = nullptr;
-  if (chain && !recompute && status && lists && forward_chain_possible(p)) {
+  if (chain && !recompute && forward_chain_possible(p)) {
     ip.chain = 1;
     ip.beta_c_w = chain->beta_c_w; ip.a_chain = chain->a_chain; ip.sa = chain->sa; ip.AT = chain->AT;
     ip.chain_flags = chain->flags;
   }
-  dim3 gridc(chunks, p.heads);
-  // Chunks that are one direct block run on tcgen05 / tensor memory; that kernel lists the others and
-  // the mma.sync kernel works the list off (it takes every chunk, one CTA each, when it is pinned or the
-  // direct block is capped).  The recompute pass of a lean backward decides the same way, from the same
-  // inputs, so that every chunk is rebuilt by the kernel that built it.
-  if (status && lists && stage_variant(kStageIntraFwd) == 0 && ip.direct_cap >= 64) {
-    const int items = chunks * p.heads;
-    ip.slow_list = lists; ip.counts = counts;
-    begin_stage(kStageIntraFwd, st);
-    const int rc_tc = launch_intra_fwd_tc(ip, recompute, st);
-    end_stage(st);
-    if (rc_tc != PKDA_OK) return rc_tc;
-    const int sms = sm_count();
-    gridc = dim3(items < sms ? items : sms, 1);
-  }
-  const int rest_stage = ip.slow_list ? kStageIntraFwdRest : kStageIntraFwd;
-  if (recompute) {
-    if (!set_smem(pkda_intra_fwd_kernel<true>, intra::kSmem)) return PKDA_ERR_LAUNCH;
-    begin_stage(rest_stage, st);
-    pkda_intra_fwd_kernel<true><<<gridc, intra::kThreads, intra::kSmem, st>>>(ip);
-  } else {
-    if (!set_smem(pkda_intra_fwd_kernel<false>, intra::kSmem)) return PKDA_ERR_LAUNCH;
-    begin_stage(rest_stage, st);
-    pkda_intra_fwd_kernel<false><<<gridc, intra::kThreads, intra::kSmem, st>>>(ip);
-  }
-  PKDA_CHECK_LAUNCH();
+  begin_stage(kStageIntraFwd, st);
+  int rc = launch_intra_fwd_tc(ip, recompute, st);
+  end_stage(st);
+  if (rc != PKDA_OK) return rc;
 
   ScanParams sp;
   sp.geo = geo; sp.w = w; sp.u = u_ws; sp.kg = kg; sp.beta_c = beta_c; sp.gc = gc;
@@ -878,7 +502,6 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   // fewer units than SMs, runs only when it is pinned (pkda_set_variant).  Same bits from the first two.
   const int units = p.n_seqs * p.heads;
   const int vb = units >= 120 ? 128 : (units >= 60 ? 64 : 32);
-  int rc = PKDA_ERR_LAUNCH;
   const bool scan_mma = stage_variant(kStageScanFwd) == 1;
   // The tcgen05 scan also produces the output (it holds h and E of every chunk) unless a separate
   // output kernel is asked for (pkda_set_variant("out_fwd", 1: mma.sync, 2: tcgen05)).
@@ -958,7 +581,7 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
   rc = run_forward_stages(p, geo, ws.beta_c, ws.u, static_cast<bf16*>(a->Aqk), static_cast<bf16*>(a->Akk),
                           static_cast<bf16*>(a->k_precond), a->ac_atk, a->a_atk, static_cast<bf16*>(a->w),
                           static_cast<bf16*>(a->kg), static_cast<bf16*>(a->v_new), static_cast<bf16*>(a->h),
-                          static_cast<bf16*>(a->qg), a->final_state, false, ws.status, ws.lists, ws.status + 1, st,
+                          static_cast<bf16*>(a->qg), a->final_state, false, ws.status, ws.status + 1, st,
                           static_cast<bf16*>(a->o), &o_done, chained ? &chain_args : nullptr);
   if (rc != PKDA_OK) return rc;
 

@@ -1,15 +1,14 @@
 // Intra-chunk stage of the chunked forward on tcgen05 / tensor memory (D = 128, chunk 64).
 //
 // Persistent CTAs of 256 threads, two per SM (about 105 KB of shared memory and 256 tensor-memory
-// columns each), walk the (chunk, head) items.  The kernel finishes the chunks whose decay lets
-// the whole chunk be ONE direct block (pkda_chunk.cuh): the gated operands are then k 2^G, q 2^G
-// and kt 2^-G with G the cumulative log2-decay from the chunk start, one set for all pairs, and
-// k 2^G is at the same time the operand Kd of W.  A chunk that turns out (once its cumulative
-// decay is known) to decay by more than kDirectLimit is put on a work list and left to the
-// mma.sync kernel of pkda_chunk_fwd.cu, which runs right after this one and pairs such chunks
-// level by level.  The decision depends on the inputs only, so the recompute pass of a lean
-// backward sends every chunk to the kernel that built it.  What the stage computes is described
-// at the top of pkda_chunk_fwd.cu; this file differs from the kernel there in how:
+// columns each), walk the (chunk, head) items.  What the stage computes is described at the top of
+// pkda_chunk_fwd.cu.  A chunk whose decay lets it be ONE direct block (pkda_chunk.cuh) has one set of gated
+// operands for all its pairs, k 2^G, q 2^G and kt 2^-G with G the cumulative log2-decay from the chunk
+// start, and its pair products are tcgen05.mma.  A chunk that turns out (once its cumulative decay is known)
+// to decay by more than kDirectLimit takes its pair products strip by strip on mma.sync (pairs_of_strip
+// below) and rejoins the others at the inverse.  The decision depends on the inputs only, so the
+// recompute pass of a lean backward decides the same way.  (Such chunks used to go on a list for a kernel of
+// their own, 198 KB of staged operands and one CTA per SM: 2,048 of them 303 us with the pass that listed them, 164 here.)
 //
 //  * Elementwise work runs on registers in a "strip" layout: warp w owns rows 8w..8w+7 of the
 //    chunk, lane l owns channels 4l..4l+3, so a warp reads or writes whole 256-byte token rows.
@@ -37,15 +36,6 @@
 
 namespace pkda {
 
-constexpr float half_power(int n) {
-  float x = 1.f;
-  for (int i = 0; i < n; ++i) x *= 0.5f;
-  return x;
-}
-// Decay totals below this are past kDirectLimit however their base-2 exponential was rounded.
-constexpr float kSurelySlow = half_power((int)kDirectLimit + 1);
-static_assert((float)(int)kDirectLimit == kDirectLimit && kSurelySlow >= 1.17549435e-38f, "a whole, normal power of two");
-
 namespace intratc {
 constexpr int kThreads = 256;
 constexpr int kLdL = 68;                    // row stride of L and T: float4 rows, and conflict-free MMA fragments
@@ -54,7 +44,11 @@ constexpr int oA = 0;                       // 2 blocks [128 rows][64 ch]: rows 
 constexpr int oY = oA + 32768;              // 2 blocks [64 rows][64 ch]: kt 2^-G (K-major B); + 1 KB so that T fits
 constexpr int oV = oY + 16384 + 1024;       // 2 blocks [64 tok][64 ch]: V (MN-major A of U^T)
 constexpr int oTm = oV + 16384;             // [64 i][64 j] bf16 T (K-major B)
-constexpr int oP = oTm + 8192;              // [64 i][64 j] bf16 scale * P
+constexpr int oX = oTm + 8192;              // the last quarter of oG
+constexpr int oG = oV;                      // f32 [64][128], while a chunk is paired by strips: kt 2^(z - G), or G; V, T and 8 KB more
+constexpr int oZ6 = oY, oD0 = oZ6 + 4096, oD1 = oD0 + 4096, oStep = oD1 + 4096;  // f32 [8][128] each, also then: G of row 6 of
+                                            // every strip, and the factors between the strips (pairs_of_strip)
+constexpr int oP = oX + 8192;               // [64 i][64 j] bf16 scale * P
 constexpr int oL = oP + 8192;               // f32 [64][68] L; before the products: the scan exchange arrays
 constexpr int oBeta = oL + 64 * kLdL * 4;   // f32 [64]
 constexpr int oDiag = oBeta + 256;          // f32 [64] q_i . kt_i
@@ -69,7 +63,9 @@ constexpr int oA0 = oSum + 32;              // f32 [128] the chunk-entry precond
 // while the inverse runs: T in the (dead) write-key operand, its scratch in the (dead) q rows of block 0
 constexpr int oT = oY;                      // f32 [64][68]
 constexpr int oY2 = oA + 8192;              // f32 [1280]
+static_assert(oG + 32768 == oP && oBar % 8 == 0, "the decays fill what lies between the write keys and P");
 static_assert(oA0 + 512 <= oBeta && oT + 64 * kLdL * 4 <= oV && oY2 + 5120 <= oA + 16384, "aliases must fit");
+static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs per SM");
 constexpr uint32_t kCols = 256;             // pair accumulator 0..63, W^T 64..127, U^T 128..191
 }  // namespace intratc
 
@@ -91,6 +87,144 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 }
 __device__ __forceinline__ void red_release_add(int* p, int v) {
   asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// ---- Pair products of a chunk that decays too much for one reference row.
+//
+// The unit is a strip of 8 rows, one per warp.  Its k rows and its q rows together are the 16-row A operand of
+// mma.sync m16n8k16, the 8 write keys of strip J <= I the B operand, so one product gives both M and P of
+// a strip pair.  With a reference row x(I) for the rows of strip I and z(J) for the columns of strip J,
+//   2^(G_i - G_j) = 2^(G_i - x(I)) 2^(x(I) - z(J)) 2^(z(J) - G_j):
+// the first factor is in the A operand, staged once per strip; kt times the third is kept in fp32, and a warp
+// multiplies it with the second, one number per channel and strip pair, and rounds the product to the B operand.
+// x(I) is the strip's first row and z(J) its last, so every factor of two strips is <= 1; inside a strip the second one is
+// 2^(decay of 7 tokens), which kDirectLimit bounds.  Strips that decay by more take their second and their last but one row (5
+// tokens; the outer tokens' factors are then > 1, at most 2^kOuter, and what rounds to zero is below 2^(2 kOuter - 126)).  Chunks
+// beyond that go through pair_exact.  A strip pair costs 11 instructions per 16 channels and no exponential;
+// gating both fragments from G by exponentials took 66, and with them the pairs were 10,000 of the 34,000 cycles of an
+// item alone on its SM instead of 4,500 (2,048 chunks: 182 us instead of 164).
+constexpr float kOuter = 32.f;
+struct PairLane {
+  uint32_t a_row, a_x, b_row, b_x, g_x;
+  int g, t;
+  __device__ __forceinline__ explicit PairLane(int lane) {
+    const uint32_t m = lane >> 3, r = lane & 7;
+    a_row = (m & 1) * 8192 + r * 128;         // matrices: k rows, q rows (channels 0..7 of the step), k rows, q rows (8..15)
+    a_x = ((m >> 1) ^ r) << 4;
+    b_row = r * 128;                          // matrices: write keys (channels 0..7, 8..15), twice
+    b_x = ((m & 1) ^ r) << 4;
+    g = lane >> 2;
+    t = lane & 3;
+    g_x = row_x(g);
+  }
+  // Byte offset of this lane's channel pair 2 t inside an fp32 row whose index is r (mod 4): the 16-byte pieces of a
+  // row are permuted by 2 (r mod 4), so that the 4 rows x 2 pieces of half a warp lie in different banks.  A step
+  // of 16 channels flips bits from 64 up, the pair 8 channels on is 32 bytes away (both by exclusive or).
+  __device__ __forceinline__ uint32_t row_x(int r) const { return (((t >> 1) ^ ((r & 3) << 1)) << 4) + ((t & 1) << 3); }
+};
+__device__ __forceinline__ float2 ld_f2(const unsigned char* s) { return *reinterpret_cast<const float2*>(s); }
+// L = tril(M, -1) diag(beta) and scale * tril(P) (its diagonal is ungated) of strip pair (I, J).
+__device__ __forceinline__ void put_pair(unsigned char* tiles, const PairLane& L, int I, int J, const float (&acc)[4], float scale) {
+  using namespace intratc;
+  const int i = 8 * I + L.g, j = 8 * J + 2 * L.t;
+  const float2 be = ld_f2(tiles + oBeta + 4 * j);
+  const float dv = *reinterpret_cast<const float*>(tiles + oDiag + 4 * i);
+  *reinterpret_cast<float2*>(tiles + oL + (i * kLdL + j) * 4) =
+      make_float2(j < i ? acc[0] * be.x : 0.f, j + 1 < i ? acc[1] * be.y : 0.f);
+  const float p0 = j < i ? acc[2] : j == i ? dv : 0.f, p1 = j + 1 < i ? acc[3] : j + 1 == i ? dv : 0.f;
+  *reinterpret_cast<uint32_t*>(tiles + oP + i * 128 + ((J ^ L.g) << 4) + 4 * L.t) = pack_bf16(p0 * scale, p1 * scale);
+}
+// All pairs of strip I (the warp's).  sD0, sD1, sStep: f32 [8][128], 2^(x(I) - z(I)), 2^(x(I) - z(I - 1)), 2^(z(J) - z(J - 1)).
+__device__ __forceinline__ void pairs_of_strip(unsigned char* tiles, uint32_t base, int I, int lane, float scale) {
+  using namespace intratc;
+  const PairLane L(lane);
+  // Strips whose factor is zero (below the smallest normal number) in all channels are left out.
+  int n = 1;
+  {
+    float4 d = *reinterpret_cast<const float4*>(tiles + oD1 + I * 512 + (lane << 4));
+    while (n <= I && __any_sync(0xffffffffu, fmaxf(fmaxf(d.x, d.y), fmaxf(d.z, d.w)) > 0.f)) {
+      ++n;
+      const float4 f = *reinterpret_cast<const float4*>(tiles + oStep + (I - n + 1) * 512 + (lane << 4));
+      d.x *= f.x; d.y *= f.y; d.z *= f.z; d.w *= f.w;
+    }
+  }
+  float acc[8][4];  // [d]: strip I - d
+#pragma unroll
+  for (int d = 0; d < 8; ++d) acc[d][0] = acc[d][1] = acc[d][2] = acc[d][3] = 0.f;
+  const uint32_t ra = base + oA + L.a_row + I * 1024, tx = L.row_x(0);
+  const unsigned char *y = tiles + oG + (8 * I + L.g) * 512, *d0 = tiles + oD0 + I * 512, *d1 = tiles + oD1 + I * 512,
+                      *step = tiles + oStep + I * 512;
+  uint32_t a[4];
+  ldsm_x4(a, ra + L.a_x);
+#pragma unroll 1
+  for (int ks = 0; ks < 8; ++ks) {
+    const uint32_t yo = L.g_x ^ (ks << 6), to = tx + (ks << 6);
+    uint32_t an[4] = {0u, 0u, 0u, 0u};
+    if (ks < 7) ldsm_x4(an, ra + ((ks + 1) >> 2) * 16384 + (L.a_x ^ (((ks + 1) & 3) << 5)));
+    float2 f0 = ld_f2(d0 + to), f1 = ld_f2(d0 + to + 32);
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+      // in twos: a strip too many (before the chunk's first, or one that has vanished) is computed and dropped
+      if (!(d & 1) && d >= n) break;
+      if (d == 1) {
+        f0 = ld_f2(d1 + to);
+        f1 = ld_f2(d1 + to + 32);
+      } else if (d > 1) {
+        const float2 s0 = ld_f2(step + to - (d - 1) * 512), s1 = ld_f2(step + to + 32 - (d - 1) * 512);
+        f0.x *= s0.x; f0.y *= s0.y; f1.x *= s1.x; f1.y *= s1.y;
+      }
+      const float2 y0 = ld_f2(y + yo - d * 4096), y1 = ld_f2(y + (yo ^ 32) - d * 4096);
+      mma_bf16(acc[d], a, pack_bf16(y0.x * f0.x, y0.y * f0.y), pack_bf16(y1.x * f1.x, y1.y * f1.y));
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) a[e] = an[e];
+  }
+#pragma unroll
+  for (int d = 0; d < 8; ++d) {
+    if (d >= n) acc[d][0] = acc[d][1] = acc[d][2] = acc[d][3] = 0.f;
+    if (d <= I) put_pair(tiles, L, I, I - d, acc[d], scale);
+  }
+}
+// Strip pair (I, J) at any decay, from the raw rows and G.  J < I: relative to the first row of I.  J = I: the pairs of
+// level lvl = 4, 2, 1 (rows with that bit set against rows without, relative to the first row of the upper half; every row
+// has its own reference); acc keeps the others.
+__device__ __forceinline__ void pair_exact(float (&acc)[4], const unsigned char* tiles, uint32_t base, const PairLane& L, int I,
+                                           int J, int lvl) {
+  using namespace intratc;
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  const int rr = J < I ? 0 : (L.g & ~(2 * lvl - 1)) + lvl;
+  const unsigned char *gi = tiles + oG + (8 * I + L.g) * 512, *gj = tiles + oG + (8 * J + L.g) * 512, *gr = tiles + oG + (8 * I + rr) * 512;
+  const uint32_t r_x = L.row_x(rr);
+#pragma unroll 1
+  for (int ks = 0; ks < 8; ++ks) {
+    const uint32_t go = L.g_x ^ (ks << 6), ro = r_x ^ (ks << 6), blk = ks >> 2, kx = (ks & 3) << 5;
+    uint32_t a[4], y[4];
+    ldsm_x4(a, base + oA + L.a_row + I * 1024 + blk * 16384 + (L.a_x ^ kx));
+    ldsm_x4(y, base + oY + L.b_row + J * 1024 + blk * 8192 + (L.b_x ^ kx));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float2 r = ld_f2(gr + (ro ^ (32 * u))), x = ld_f2(gi + (go ^ (32 * u))), z = ld_f2(gj + (go ^ (32 * u)));
+      const float fx = ex2(-fabsf(x.x - r.x)), fy = ex2(-fabsf(x.y - r.y));
+      const float2 k2 = unpack_bf16(a[2 * u]), q2 = unpack_bf16(a[2 * u + 1]), y2 = unpack_bf16(y[u]);
+      a[2 * u] = pack_bf16(k2.x * fx, k2.y * fy);
+      a[2 * u + 1] = pack_bf16(q2.x * fx, q2.y * fy);
+      y[u] = pack_bf16(y2.x * ex2(-fabsf(z.x - r.x)), y2.y * ex2(-fabsf(z.y - r.y)));
+    }
+    mma_bf16(d, a, y[0], y[1]);
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (J < I || level_pair_ok(L.g, 2 * L.t + (e & 1), lvl)) acc[e] = d[e];
+}
+__device__ __forceinline__ void pairs_of_strip_exact(unsigned char* tiles, uint32_t base, int I, int lane, float scale) {
+  const PairLane L(lane);
+#pragma unroll 1
+  for (int J = 0; J <= I; ++J) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int lvl = 4; lvl; lvl = J < I ? 0 : lvl >> 1) pair_exact(acc, tiles, base, L, I, J, lvl);
+    put_pair(tiles, L, I, J, acc, scale);
+  }
 }
 
 template <bool kRecompute>
@@ -153,7 +287,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   const int ei = R & 63, j0 = 32 * (warp >> 2);
   const bool isP = (warp & 3) >= 2;
 
-  // Items differ in cost (a chunk that is handed over costs a fraction of one that is finished), so
+  // Items differ in cost (one that is paired by level takes longer), so
   // the CTAs draw them one at a time from a cursor instead of striding through them.  One thread draws the
   // next item and looks its chunk up while the current one waits for its products, and the item's rows are
   // asked into L2 from then on: drawn at the end of an item, the cursor, the lookup and the rows were four
@@ -170,7 +304,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     }
     return it;
   };
-  if (tid == kThreads - 1) s_item[0] = describe(atomicAdd(p.counts, 1));
+  if (tid == kThreads - 1) s_item[0] = describe(atomicAdd(p.cursor, 1));
   __syncthreads();
   int slot = 0;
 #pragma unroll 1
@@ -188,27 +322,14 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   uint32_t dbase = base;
   asm volatile("" : "+r"(dbase));
 
-  // When recomputing, the chunk's decay totals are known: one that is past the limit by more than the
-  // rounding of their base-2 exponential is handed over before anything of it is loaded (strongly decaying
-  // gates: 50 -> 18 us for the pass over 1,536 chunks); near the limit the totals are formed as the forward
-  // formed them, so that both passes decide alike.
-  if (kRecompute) {
-    const float least = tid < kD ? p.gc[chh * kD + tid] : 1.f;
-    if (__syncthreads_or(least < kSurelySlow)) {
-      if (tid == 0) p.slow_list[atomicAdd(p.counts + 1, 1)] = item;
-      if (tid == kThreads - 1) s_item[slot ^ 1] = describe(atomicAdd(p.counts, 1));
-      __syncthreads();
-      continue;
-    }
-  }
-
-  // ---- 0. V (and T when recomputing) by TMA, and the strips of g, k and q, right into their operand slots
-  if (tid == 0) {
+  // ---- 0. the strips of g, k and q by TMA, right into their operand slots; V (and T when recomputing)
+  auto request_v = [&]() {  // one thread
     tc::mbar_expect_tx(bar_tma, kRecompute ? 16384 + 8192 : 16384);
     tc::tma_load_3d(base + oV, &tm_v, bar_tma, 0, h, tok0);
     tc::tma_load_3d(base + oV + 8192, &tm_v, bar_tma, 64, h, tok0);
     if (kRecompute) tc::tma_load_3d(base + oTm, &tm_akk, bar_tma, 0, h, tok0);
-  }
+  };
+  if (kRecompute && tid == 0) request_v();  // (the forward asks for V once it knows whether the decays need its place first)
   if (lane == 0) {  // two 64-channel blocks each, issued by six warps
     const int b = warp & 1;
     if (warp == 0) tc::mbar_expect_tx(bar_in, 6 * 8192);
@@ -363,26 +484,35 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     }
     if (tid == 0) p.sa[chh] = gs;
   }
-  // A chunk that decays too much for one direct block goes to the mma.sync kernel (the decision is
-  // the same for all threads: every thread holds the totals of its four channels, the CTA all 128).
-  {
-    const float worst = -fminf(fminf(Glast[0], Glast[1]), fminf(Glast[2], Glast[3]));
-    if (__syncthreads_or(worst > kDirectLimit)) {
-      if (tid == 0) p.slow_list[atomicAdd(p.counts + 1, 1)] = item;
-      ok = tc::mbar_wait(bar_tma, tma_phase) && ok;  // the V tile in flight must land before the tile is reused
-      tma_phase ^= 1;
-      if (tid == kThreads - 1) s_item[slot ^ 1] = describe(atomicAdd(p.counts, 1));
-      tc::fence_proxy_async();  // the strips have been read: the next item's copies may overwrite them
-      __syncthreads();
-      continue;
+  // Does the chunk decay too much for one direct block?  (The same answer for all threads: every thread holds the
+  // totals of its four channels, the CTA all 128.)  If so, which reference rows do its strips take?
+  const bool by_strip =
+      __syncthreads_or(-fminf(fminf(Glast[0], Glast[1]), fminf(Glast[2], Glast[3])) > kDirectLimit) || p.by_strip;
+  int refs = 0;  // 0: first and last row, 1: second and last but one, 2: pair_exact
+  if (!kRecompute) {
+    if (!by_strip) {
+      if (tid == 0) request_v();
+    } else {
+      float all = 0.f, mid = 0.f, outer = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        all = fmaxf(all, G[0][e] - G[7][e]);
+        mid = fmaxf(mid, G[1][e] - G[6][e]);
+        outer = fmaxf(outer, fmaxf(G[0][e] - G[1][e], G[6][e] - G[7][e]));
+      }
+      *reinterpret_cast<float4*>(tiles + oZ6 + warp * 512 + (lane << 4)) = make_float4(G[6][0], G[6][1], G[6][2], G[6][3]);
+      if (__syncthreads_or(all > kDirectLimit)) refs = 1 + (__syncthreads_or(mid > kDirectLimit || outer > kOuter) != 0);
+      if (p.direct_cap < 8) refs = 2;
     }
   }
 
+  uint2 kd[8];  // Kd of a chunk that is paired by strips
   // ---- 3. one pass over the strip: preconditioner states of its rows -> write keys kt = k * B(A_t)
   // (to global memory), kg = kt * decay to the chunk end, the diagonal q_i . kt_i, and the gated operands
   // in place: Kd = k 2^G (rows 0..63 of the stacked operand, later the operand of W^T), q 2^G (rows
   // 64..127), kt 2^-G (into the slots g has left); qg goes to global memory.  The decay to the chunk
   // end is 2^G_last times the 2^-G the operand needs anyway.  Nothing of the strip is needed afterwards.
+  // A chunk that is paired by strips leaves its operands as pairs_of_strip or pair_exact reads them, and Kd in registers.
   {
     if (chain) a_first = *reinterpret_cast<const float4*>(sA0 + c4);  // (written before the barrier of the decision)
     float A[4] = {a_first.x, a_first.y, a_first.z, a_first.w};
@@ -394,6 +524,29 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       }
     }
     const float glE[4] = {ex2(Glast[0]), ex2(Glast[1]), ex2(Glast[2]), ex2(Glast[3])};
+    if (!kRecompute && warp == 0)
+      *reinterpret_cast<float4*>(p.gc + chh * kD + c4) = make_float4(glE[0], glE[1], glE[2], glE[3]);
+    float zr[4], xr[4];  // the strip's reference rows
+    if (!kRecompute && by_strip && refs < 2) {
+      float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);  // z of the strip before
+      if (refs) {
+        if (warp) prev = *reinterpret_cast<const float4*>(tiles + oZ6 + (warp - 1) * 512 + (lane << 4));
+      } else {
+        for (int wp = 0; wp < warp; ++wp) {
+          const float4 to = *reinterpret_cast<const float4*>(sTot + wp * kD + c4);
+          prev.x += to.x; prev.y += to.y; prev.z += to.z; prev.w += to.w;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        zr[c] = refs ? G[6][c] : G[7][c];
+        xr[c] = refs ? G[1][c] : G[0][c];
+      }
+      unsigned char* at = tiles + warp * 512 + (lane << 4);
+      *reinterpret_cast<float4*>(at + oD0) = make_float4(ex2(xr[0] - zr[0]), ex2(xr[1] - zr[1]), ex2(xr[2] - zr[2]), ex2(xr[3] - zr[3]));
+      *reinterpret_cast<float4*>(at + oD1) = make_float4(ex2(xr[0] - prev.x), ex2(xr[1] - prev.y), ex2(xr[2] - prev.z), ex2(xr[3] - prev.w));
+      *reinterpret_cast<float4*>(at + oStep) = make_float4(ex2(zr[0] - prev.x), ex2(zr[1] - prev.y), ex2(zr[2] - prev.z), ex2(zr[3] - prev.w));
+    }
     float dg[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -417,18 +570,49 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
         unpack4(qr, qc);
         dg[i] = qc[0] * kc2[0] + qc[1] * kc2[1] + qc[2] * kc2[2] + qc[3] * kc2[3];
       }
-      float e[4], es[4], fi[4], tl[4];
+      float e[4], es[4], tl[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         e[c] = ex2(G[i][c]);
         es[c] = e[c] * p.scale;
-        fi[c] = __fdividef(1.f, e[c]);
-        tl[c] = glE[c] * fi[c];
       }
-      *reinterpret_cast<uint2*>(aBase + off) = scale4(kr, e);
-      if (!kRecompute) {
-        *reinterpret_cast<uint2*>(aBase + 8192 + off) = scale4(qr, e);
-        *reinterpret_cast<uint2*>(yBase + off) = scale4(kt, fi);
+      if (!by_strip) {
+        float fi[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          fi[c] = __fdividef(1.f, e[c]);
+          tl[c] = glE[c] * fi[c];
+        }
+        *reinterpret_cast<uint2*>(aBase + off) = scale4(kr, e);
+        if (!kRecompute) {
+          *reinterpret_cast<uint2*>(aBase + 8192 + off) = scale4(qr, e);
+          *reinterpret_cast<uint2*>(yBase + off) = scale4(kt, fi);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tl[c] = ex2(Glast[c] - G[i][c]);
+        if (kRecompute) {
+          *reinterpret_cast<uint2*>(aBase + off) = scale4(kr, e);
+        } else {
+          kd[i] = scale4(kr, e);
+          float y[4];
+          if (refs < 2) {
+            float x[4];
+            unpack4(kt, y);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              x[c] = ex2(G[i][c] - xr[c]);
+              y[c] *= ex2(zr[c] - G[i][c]);
+            }
+            *reinterpret_cast<uint2*>(aBase + off) = scale4(kr, x);
+            *reinterpret_cast<uint2*>(aBase + 8192 + off) = scale4(qr, x);
+          } else {
+            *reinterpret_cast<uint2*>(yBase + off) = kt;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) y[c] = G[i][c];
+          }
+          *reinterpret_cast<float4*>(tiles + oG + (r0 + i) * 512 + ((lane ^ ((i & 3) << 1)) << 4)) = make_float4(y[0], y[1], y[2], y[3]);
+        }
       }
       if (r0 + i < valid) {
         *reinterpret_cast<uint2*>(p.kg + row0 + (size_t)(r0 + i) * gld + c4) = scale4(kt, tl);
@@ -438,16 +622,26 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     if (!kRecompute) {
       row_sums8(dg, lane);
       if ((lane & 3) == 0) sDiag[r0 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = dg[0];
-      if (warp == 0)
-        *reinterpret_cast<float4*>(p.gc + chh * kD + c4) = make_float4(glE[0], glE[1], glE[2], glE[3]);
     }
   }
   int drawn = 0;
-  if (tid == kThreads - 1) drawn = atomicAdd(p.counts, 1);  // (not used before the products are back)
+  if (tid == kThreads - 1) drawn = atomicAdd(p.cursor, 1);  // (not used before the products are back)
   tc::fence_proxy_async();
   tc::tc_fence_before();
   __syncthreads();  // (the strip exchange arrays are dead from here on: L takes their place)
-  if (!kRecompute) {
+  if (!kRecompute && by_strip) {
+    // what lies above the strip diagonal of P reads as zero
+    for (int J = warp + 1 + (lane >> 3); J < 8; J += 4)
+      *reinterpret_cast<uint4*>(tiles + oP + (r0 + (lane & 7)) * 128 + ((J ^ (lane & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+    if (refs < 2) {
+      pairs_of_strip(tiles, base, warp, lane, p.scale);
+    } else {
+      pairs_of_strip_exact(tiles, base, warp, lane, p.scale);
+    }
+    __syncwarp();  // (only this warp reads the k rows of its strip)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) *reinterpret_cast<uint2*>(aBase + slot_off(i)) = kd[i];
+  } else if (!kRecompute) {
     if (tid == 0) {
       tc::tc_fence_after();
       constexpr uint32_t idesc_pair = tc::idesc_bf16(128, 64, false, false);
@@ -494,29 +688,27 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     }
     tc::tc_fence_before();
   }
-  ok = tc::mbar_wait(bar_tma, tma_phase) && ok;  // V (and T) landed long ago
-  tma_phase ^= 1;
-  if (!full) {  // rows past the sequence end hold another sequence's data: they must not reach the product
-    for (int idx = tid; idx < kChunk * 16; idx += kThreads) {
-      const int r = idx >> 4, pc = idx & 15;
-      if (r >= valid)
-        *reinterpret_cast<uint4*>(tiles + oV + (pc >> 3) * 8192 + r * 128 + ((pc & 7) << 4)) = make_uint4(0, 0, 0, 0);
+  auto await_v = [&]() {
+    ok = tc::mbar_wait(bar_tma, tma_phase) && ok;  // V (and T) landed long ago
+    tma_phase ^= 1;
+    if (!full) {  // rows past the sequence end hold another sequence's data: they must not reach the product
+      for (int idx = tid; idx < kChunk * 16; idx += kThreads) {
+        const int r = idx >> 4, pc = idx & 15;
+        if (r >= valid)
+          *reinterpret_cast<uint4*>(tiles + oV + (pc >> 3) * 8192 + r * 128 + ((pc & 7) << 4)) = make_uint4(0, 0, 0, 0);
+      }
     }
-  }
+  };
+  if (kRecompute) await_v();
   if (tid == kThreads - 1) s_item[slot ^ 1] = describe(drawn);
   tc::fence_proxy_async();
   __syncthreads();
-  {  // the next item's rows of g, k, q and v: one 256-byte request per thread
+  if (!kRecompute && by_strip && tid == 0) request_v();  // (the decays have been read)
+  if (lane == 0) {  // the next item's tiles of g, k, q and v
     const int4 nx = s_item[slot ^ 1];
-    const int r = tid & 63;
-    if (nx.x >= 0 && r < nx.z) {
-      const bf16* const src[4] = {p.g, p.k, p.q, p.v};
-      const bf16* a = src[0];
-      if (tid >= 64) a = src[1];
-      if (tid >= 128) a = src[2];
-      if (tid >= 192) a = src[3];
-      a += ((size_t)(nx.y + r) * H + nx.x % H) * kD;
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], 256;" ::"l"(a) : "memory");
+    if (nx.x >= 0) {
+      const CUtensorMap* m = warp < 2 ? &tm_g : warp < 4 ? &tm_k : warp < 6 ? &tm_q : &tm_v;
+      tc::tma_prefetch_3d(m, 64 * (warp & 1), nx.x % H, nx.y);
     }
   }
 
@@ -547,6 +739,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       if (!full && r < valid)
         *reinterpret_cast<uint4*>(p.Akk + ((size_t)(tok0 + r) * H + h) * kChunk + 8 * pc) = pk;
     }
+    await_v();
     tc::fence_proxy_async();
     tc::tc_fence_before();
     __syncthreads();

@@ -247,9 +247,10 @@ int pkda_last_launch_count(void);
 /*
  * Testing aid.  The chunked kernels pair tokens inside blocks of b rows through a
  * single reference row whenever the decay across the block is small enough, and
- * through a binary hierarchy of reference rows otherwise; b is chosen per
+ * through several reference rows otherwise; b is chosen per
  * (chunk, head) from the data.  This caps b (a power of two in 1..64; 64 = no cap,
- * 1 = hierarchy only) so that tests can exercise every variant on the same input.
+ * 1 = a reference for every level of pairs) so that tests can exercise every variant on
+ * the same input.  (The forward knows b = 64, strips of 8 rows, and less than 8.)
  */
 int pkda_set_direct_block_cap(int cap);
 
@@ -260,6 +261,8 @@ int pkda_set_direct_block_cap(int cap);
  * pkda_set_variant(stage name as pkda_stage_name reports it, 1) pins the older
  * kernel for that stage, (.., 0) restores the default.  Stages with two
  * implementations: "intra_fwd", "scan_fwd", "out_fwd", "scan_bwd", "intra_bwd".
+ * (The forward's intra stage is one kernel: "intra_fwd" makes it take the pair
+ * products of every chunk on mma.sync, as it does for strongly decaying ones.)
  * "out_fwd" has three: by default the tcgen05 state scan produces the output
  * itself (no output launch), 2 runs the stand-alone tcgen05 output kernel, 1 the
  * mma.sync one.
