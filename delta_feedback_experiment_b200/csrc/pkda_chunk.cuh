@@ -420,8 +420,8 @@ struct IntraParams {
   int by_strip;    // nonzero: every chunk is paired strip by strip, whatever it decays by
   // Preconditioner state across chunks inside the tensor-memory kernel (dense batches; chain != 0):
   // every item computes its chunk's local scan anyway, so it takes its chunk-entry state from the item
-  // of the chunk before (a_chain, which is the saved "state at chunk starts" tensor; chain_flags counts
-  // the four warps that have published an entry), and publishes the next chunk's.  The items are
+  // of the chunk before (a_chain, which is the saved "state at chunk starts" tensor; launch_chain_init
+  // has marked all of it as not there yet), and publishes the next chunk's.  The items are
   // then drawn chunk level by chunk level across all (row, head) units, so that an item's predecessor
   // started long before it.  beta (raw) is packed to beta_c_w on the way; sa takes the chunk's summed
   // preconditioner log-decay, A0 / AT are the initial / final preconditioner states (may be NULL).
@@ -429,11 +429,12 @@ struct IntraParams {
   const bf16* beta;
   float *beta_c_w, *a_chain, *sa, *AT;
   const float* A0;
-  int* chain_flags;
 };
 
 // tcgen05 / tensor-memory intra-chunk forward stage (pkda_intra_fwd_tc.cu).
 int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st);
+// What a chained launch finds: no entry of a_chain there yet, the status word and the cursors zero.
+int launch_chain_init(float* a_chain, size_t items, int* zero, cudaStream_t st);
 
 // Arguments of the chunk-parallel backward stage (both implementations).
 struct IntraBwdParams {
@@ -509,7 +510,6 @@ int run_prologue(const pkda_problem& p, int* chunk_offsets, float* beta_c, Geo* 
 // (dense batches): see IntraParams::chain.
 struct ChainArgs {
   float *beta_c_w, *a_chain, *sa, *AT;
-  int* flags;
 };
 // True when the forward can run in chained mode (no preconditioner kernels in front of the intra stage).
 bool forward_chain_possible(const pkda_problem& p);

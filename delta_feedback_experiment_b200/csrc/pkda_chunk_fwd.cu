@@ -389,7 +389,6 @@ pkda_out_fwd_kernel(const OutParams p) {
 
 // ------------------------------------------------------------------ host side
 struct FwdWorkspace {
-  int* chain_flags;  // one counter per (chunk, head) item, right behind the status slot (zeroed with it)
   int* chunk_offsets;
   float* beta_c;
   bf16* u;
@@ -409,9 +408,7 @@ static FwdWorkspace carve_fwd(const pkda_problem& p, void* base) {
   w.u = reinterpret_cast<bf16*>(b + off);
   off += align_up((size_t)p.total_tokens * p.heads * kD * sizeof(bf16));
   w.status = reinterpret_cast<int*>(b + off);
-  off += 8 * sizeof(int);
-  w.chain_flags = reinterpret_cast<int*>(b + off);
-  off += align_up(chunks * p.heads * sizeof(int));
+  off += align_up(8 * sizeof(int));
   w.bytes = off;
   return w;
 }
@@ -482,11 +479,9 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   ip.chain = 0;
   ip.beta = static_cast<const bf16*>(p.beta); ip.A0 = p.initial_A_state;
   ip.beta_c_w = ip.a_chain = ip.sa = ip.AT = nullptr;
-  ip.chain_flags = nullptr;
   if (chain && !recompute && forward_chain_possible(p)) {
     ip.chain = 1;
     ip.beta_c_w = chain->beta_c_w; ip.a_chain = chain->a_chain; ip.sa = chain->sa; ip.AT = chain->AT;
-    ip.chain_flags = chain->flags;
   }
   begin_stage(kStageIntraFwd, st);
   int rc = launch_intra_fwd_tc(ip, recompute, st);
@@ -570,13 +565,11 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
     PKDA_CHECK_LAUNCH();
   }
 
-  // status, cursors and chain counters; the local scan zeroes the first two when it runs (one launch fewer:
-  // 2 us of a small call's host time)
-  if (chained && cudaMemsetAsync(ws.status, 0, (8 + (size_t)geo.total_chunks * p.heads) * sizeof(int), st) != cudaSuccess)
-    return PKDA_ERR_LAUNCH;
+  // (The local scan also zeroes the status word and the cursor when it runs.)
+  if (chained && (rc = launch_chain_init(a->a_atk, (size_t)geo.total_chunks * p.heads, ws.status, st)) != PKDA_OK) return rc;
   ChainArgs chain_args;
   chain_args.beta_c_w = ws.beta_c; chain_args.a_chain = a->a_atk; chain_args.sa = a->sa_atk;
-  chain_args.AT = a->final_A_state; chain_args.flags = ws.chain_flags;
+  chain_args.AT = a->final_A_state;
   bool o_done = false;
   rc = run_forward_stages(p, geo, ws.beta_c, ws.u, static_cast<bf16*>(a->Aqk), static_cast<bf16*>(a->Akk),
                           static_cast<bf16*>(a->k_precond), a->ac_atk, a->a_atk, static_cast<bf16*>(a->w),

@@ -44,15 +44,14 @@ constexpr int oA = 0;                       // 2 blocks [128 rows][64 ch]: rows 
 constexpr int oY = oA + 32768;              // 2 blocks [64 rows][64 ch]: kt 2^-G (K-major B); + 1 KB so that T fits
 constexpr int oV = oY + 16384 + 1024;       // 2 blocks [64 tok][64 ch]: V (MN-major A of U^T)
 constexpr int oTm = oV + 16384;             // [64 i][64 j] bf16 T (K-major B)
-constexpr int oX = oTm + 8192;              // the last quarter of oG
+constexpr int oX = oTm + 8192;              // the last quarter of oG; with oP the place U leaves from (W: from oV)
 constexpr int oG = oV;                      // f32 [64][128], while a chunk is paired by strips: kt 2^(z - G), or G; V, T and 8 KB more
-constexpr int oZ6 = oY, oD0 = oZ6 + 4096, oD1 = oD0 + 4096, oStep = oD1 + 4096;  // f32 [8][128] each, also then: G of row 6 of
-                                            // every strip, and the factors between the strips (pairs_of_strip)
 constexpr int oP = oX + 8192;               // [64 i][64 j] bf16 scale * P
 constexpr int oL = oP + 8192;               // f32 [64][68] L; before the products: the scan exchange arrays
 constexpr int oBeta = oL + 64 * kLdL * 4;   // f32 [64]
 constexpr int oDiag = oBeta + 256;          // f32 [64] q_i . kt_i
-constexpr int oBar = oDiag + 256;           // TMA barrier, MMA barrier, tensor-memory base address
+constexpr int oStep = oDiag + 256;          // f32 [8][128] factors between the strips (pairs_of_strip)
+constexpr int oBar = oStep + 4096;          // TMA barrier, MMA barrier, tensor-memory base address
 constexpr int kSmem = oBar + 64 + 1024;     // + slack to align the tiles to 1024 bytes
 // inside the L region before the products
 constexpr int oTot = oL;                    // f32 [8][128] per-strip decay totals
@@ -60,11 +59,14 @@ constexpr int oEnd = oL + 4096;             // f32 [8][128] per-strip end value 
 constexpr int oDec = oL + 8192;             // f32 [8] per-strip product of preconditioner decays
 constexpr int oSum = oDec + 32;             // f32 [8] per-strip sum of the preconditioner's log-decays
 constexpr int oA0 = oSum + 32;              // f32 [128] the chunk-entry preconditioner state (chained mode)
+constexpr int oZ6 = oL + 9216;              // f32 [8][128] G of row 6 of every strip
+// between those and the products, the strip's own factors where its rows of P come later: strip w, 2 x f32 [128]
+constexpr int oD0 = oP, oD1 = oP + 512;     // + 1024 w
 // while the inverse runs: T in the (dead) write-key operand, its scratch in the (dead) q rows of block 0
 constexpr int oT = oY;                      // f32 [64][68]
 constexpr int oY2 = oA + 8192;              // f32 [1280]
 static_assert(oG + 32768 == oP && oBar % 8 == 0, "the decays fill what lies between the write keys and P");
-static_assert(oA0 + 512 <= oBeta && oT + 64 * kLdL * 4 <= oV && oY2 + 5120 <= oA + 16384, "aliases must fit");
+static_assert(oA0 + 512 <= oZ6 && oZ6 + 4096 <= oBeta && oT + 64 * kLdL * 4 <= oV && oY2 + 5120 <= oA + 16384, "aliases must fit");
 static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs per SM");
 constexpr uint32_t kCols = 256;             // pair accumulator 0..63, W^T 64..127, U^T 128..191
 }  // namespace intratc
@@ -79,14 +81,27 @@ __device__ __forceinline__ uint2 scale4(uint2 r, const float (&f)[4]) {
   return make_uint2(pack_bf16(x[0] * f[0], x[1] * f[1]), pack_bf16(x[2] * f[2], x[3] * f[3]));
 }
 
-// Acquire load / release add at device scope: the hand-over of the preconditioner state between items.
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// The hand-over of the preconditioner state between items: one 32-bit word per channel that is either kNotYet or the
+// value, so that nothing has to be ordered (no arithmetic result has this bit pattern: a NaN comes out as 0x7fffffff).
+constexpr uint32_t kNotYet = 0xffffffffu;
+__device__ __forceinline__ uint32_t ld_relaxed(const float* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void red_release_add(int* p, int v) {
-  asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_relaxed(float* p, float v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(__float_as_uint(v)) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_u16(const bf16* p) {
+  uint32_t v;
+  asm volatile("ld.global.nc.u16 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+// Before a chained launch: every word of the hand-over to kNotYet, the status word and the cursors to zero.
+__global__ void __launch_bounds__(256) pkda_chain_init_kernel(uint4* a_chain, size_t n, int* zero) {
+  if (blockIdx.x == 0 && threadIdx.x < 8) zero[threadIdx.x] = 0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    a_chain[i] = make_uint4(kNotYet, kNotYet, kNotYet, kNotYet);
 }
 
 // ---- Pair products of a chunk that decays too much for one reference row.
@@ -105,11 +120,14 @@ __device__ __forceinline__ void red_release_add(int* p, int v) {
 // item alone on its SM instead of 4,500 (2,048 chunks: 182 us instead of 164).
 constexpr float kOuter = 32.f;
 struct PairLane {
-  uint32_t a_row, a_x, b_row, b_x, g_x;
+  uint32_t a_row, s_row, s_blk, a_x, b_row, b_x, g_x;
   int g, t;
   __device__ __forceinline__ explicit PairLane(int lane) {
+    using namespace intratc;
     const uint32_t m = lane >> 3, r = lane & 7;
-    a_row = (m & 1) * 8192 + r * 128;         // matrices: k rows, q rows (channels 0..7 of the step), k rows, q rows (8..15)
+    a_row = oA + (m & 1) * 8192 + r * 128;    // matrices: k rows, q rows (channels 0..7 of the step), k rows, q rows (8..15)
+    s_row = ((m & 1) ? oA + 8192 : oY) + r * 128;  // the same of the staged operand: its k rows are where the write keys
+    s_blk = (m & 1) ? 16384 : 8192;                // of other chunks are (Kd has the place of k)
     a_x = ((m >> 1) ^ r) << 4;
     b_row = r * 128;                          // matrices: write keys (channels 0..7, 8..15), twice
     b_x = ((m & 1) ^ r) << 4;
@@ -134,14 +152,15 @@ __device__ __forceinline__ void put_pair(unsigned char* tiles, const PairLane& L
   const float p0 = j < i ? acc[2] : j == i ? dv : 0.f, p1 = j + 1 < i ? acc[3] : j + 1 == i ? dv : 0.f;
   *reinterpret_cast<uint32_t*>(tiles + oP + i * 128 + ((J ^ L.g) << 4) + 4 * L.t) = pack_bf16(p0 * scale, p1 * scale);
 }
-// All pairs of strip I (the warp's).  sD0, sD1, sStep: f32 [8][128], 2^(x(I) - z(I)), 2^(x(I) - z(I - 1)), 2^(z(J) - z(J - 1)).
+// All pairs of strip I (the warp's), with the factors 2^(x(I) - z(I)) at oD0, 2^(x(I) - z(I - 1)) at oD1 and
+// 2^(z(J) - z(J - 1)) at oStep.
 __device__ __forceinline__ void pairs_of_strip(unsigned char* tiles, uint32_t base, int I, int lane, float scale) {
   using namespace intratc;
   const PairLane L(lane);
   // Strips whose factor is zero (below the smallest normal number) in all channels are left out.
   int n = 1;
   {
-    float4 d = *reinterpret_cast<const float4*>(tiles + oD1 + I * 512 + (lane << 4));
+    float4 d = *reinterpret_cast<const float4*>(tiles + oD1 + I * 1024 + (lane << 4));
     while (n <= I && __any_sync(0xffffffffu, fmaxf(fmaxf(d.x, d.y), fmaxf(d.z, d.w)) > 0.f)) {
       ++n;
       const float4 f = *reinterpret_cast<const float4*>(tiles + oStep + (I - n + 1) * 512 + (lane << 4));
@@ -151,8 +170,8 @@ __device__ __forceinline__ void pairs_of_strip(unsigned char* tiles, uint32_t ba
   float acc[8][4];  // [d]: strip I - d
 #pragma unroll
   for (int d = 0; d < 8; ++d) acc[d][0] = acc[d][1] = acc[d][2] = acc[d][3] = 0.f;
-  const uint32_t ra = base + oA + L.a_row + I * 1024, tx = L.row_x(0);
-  const unsigned char *y = tiles + oG + (8 * I + L.g) * 512, *d0 = tiles + oD0 + I * 512, *d1 = tiles + oD1 + I * 512,
+  const uint32_t ra = base + L.s_row + I * 1024, tx = L.row_x(0);
+  const unsigned char *y = tiles + oG + (8 * I + L.g) * 512, *d0 = tiles + oD0 + I * 1024, *d1 = tiles + oD1 + I * 1024,
                       *step = tiles + oStep + I * 512;
   uint32_t a[4];
   ldsm_x4(a, ra + L.a_x);
@@ -160,7 +179,7 @@ __device__ __forceinline__ void pairs_of_strip(unsigned char* tiles, uint32_t ba
   for (int ks = 0; ks < 8; ++ks) {
     const uint32_t yo = L.g_x ^ (ks << 6), to = tx + (ks << 6);
     uint32_t an[4] = {0u, 0u, 0u, 0u};
-    if (ks < 7) ldsm_x4(an, ra + ((ks + 1) >> 2) * 16384 + (L.a_x ^ (((ks + 1) & 3) << 5)));
+    if (ks < 7) ldsm_x4(an, ra + ((ks + 1) >> 2) * L.s_blk + (L.a_x ^ (((ks + 1) & 3) << 5)));
     float2 f0 = ld_f2(d0 + to), f1 = ld_f2(d0 + to + 32);
 #pragma unroll
     for (int d = 0; d < 8; ++d) {
@@ -179,6 +198,7 @@ __device__ __forceinline__ void pairs_of_strip(unsigned char* tiles, uint32_t ba
 #pragma unroll
     for (int e = 0; e < 4; ++e) a[e] = an[e];
   }
+  __syncwarp();  // (P takes the place of the strip's factors)
 #pragma unroll
   for (int d = 0; d < 8; ++d) {
     if (d >= n) acc[d][0] = acc[d][1] = acc[d][2] = acc[d][3] = 0.f;
@@ -199,7 +219,7 @@ __device__ __forceinline__ void pair_exact(float (&acc)[4], const unsigned char*
   for (int ks = 0; ks < 8; ++ks) {
     const uint32_t go = L.g_x ^ (ks << 6), ro = r_x ^ (ks << 6), blk = ks >> 2, kx = (ks & 3) << 5;
     uint32_t a[4], y[4];
-    ldsm_x4(a, base + oA + L.a_row + I * 1024 + blk * 16384 + (L.a_x ^ kx));
+    ldsm_x4(a, base + L.a_row + I * 1024 + blk * 16384 + (L.a_x ^ kx));
     ldsm_x4(y, base + oY + L.b_row + J * 1024 + blk * 8192 + (L.b_x ^ kx));
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
@@ -282,10 +302,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   tc::tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tiles + oBar + 16);
   bool ok = true;
-  uint32_t mma_phase = 0, tma_phase = 0, in_phase = 0;
-  const int R = 32 * (warp & 3) + lane;     // this thread's accumulator row in the pair products
-  const int ei = R & 63, j0 = 32 * (warp >> 2);
-  const bool isP = (warp & 3) >= 2;
+  uint32_t ph = 0;  // bit 0: bar_mma, 1: bar_tma, 2: bar_in
 
   // Items differ in cost (one that is paired by level takes longer), so
   // the CTAs draw them one at a time from a cursor instead of striding through them.  One thread draws the
@@ -304,8 +321,51 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     }
     return it;
   };
-  if (tid == kThreads - 1) s_item[0] = describe(atomicAdd(p.cursor, 1));
+  // The strips of an item by TMA: g as soon as the item before it no longer needs the write-key operand (the inverse is
+  // over), k and q once its last products have read the stacked operand; their epilogue and stores go on meanwhile.
+  // With the scalars below, the hand-over in one word and the rows of pass 3 read ahead: 8 x 4,096 tokens of 16 heads
+  // 466 -> 436 us; asked for at the top of an item, strips and scalars were 4,000 of its 30,000 cycles, and the stores 1,400.
+  auto request_g = [&](const int4& it) {  // one thread; also arms the barrier for k and q
+    tc::mbar_expect_tx(bar_in, 6 * 8192);
+    tc::tma_load_3d(base + oY, &tm_g, bar_in, 0, it.x % H, it.y);
+    tc::tma_load_3d(base + oY + 8192, &tm_g, bar_in, 64, it.x % H, it.y);
+  };
+  auto request_kq = [&](const int4& it) {  // all warps
+    if (lane != 0 || warp < 2 || warp >= 6) return;
+    const int b = warp & 1;
+    if (warp < 4) tc::tma_load_3d(base + oA + b * 16384, &tm_k, bar_in, 64 * b, it.x % H, it.y);
+    else tc::tma_load_3d(base + oA + 8192 + b * 16384, &tm_q, bar_in, 64 * b, it.x % H, it.y);
+  };
+  // The scalars of an item, asked for with its strips, and not used, not even converted, before they are needed.
+  uint32_t n_beta = 0, n_bp = 0, n_chain = 0;  // lane i < 8: of row r0 + i; thread < 128: the entry state of its channel
+  float n_pd = 0.f, n_alog = 0.f, n_centre = 0.f;
+  float4 n_bias = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto request_scalars = [&](const int4& it) {
+    const int h = it.x % H, r = r0 + (lane & 7);
+    const size_t chh = it.x, s = (size_t)(it.y + min(r, it.z - 1)) * H + h;  // (rows past the end are masked where they are used)
+    n_beta = chain ? ld_u16(p.beta + s) : __float_as_uint(p.beta_c[chh * kChunk + r]);
+    if (!kRecompute) {
+      n_pd = p.g_atk[s];
+      n_bp = ld_u16(p.beta_atk + s);
+      n_centre = p.log_atk_scale[h];
+      if (tid < kD) {  // (chained: normally published long ago by the item of the chunk before)
+        if (!chain) n_chain = __float_as_uint(p.a_start[chh * kD + tid]);
+        else if (it.y > it.w * p.geo.seq_len) n_chain = ld_relaxed(p.a_chain + chh * kD + tid);
+        else n_chain = p.A0 ? __float_as_uint(p.A0[((size_t)it.w * H + h) * kD + tid]) : 0u;
+      }
+    }
+    n_bias = *reinterpret_cast<const float4*>(p.dt_bias + h * kD + c4);
+    n_alog = p.A_log[h];
+  };
+  if (tid == 32) {
+    s_item[0] = describe(atomicAdd(p.cursor, 1));
+    if (s_item[0].x >= 0) request_g(s_item[0]);
+  }
   __syncthreads();
+  if (s_item[0].x >= 0) {
+    request_kq(s_item[0]);
+    request_scalars(s_item[0]);
+  }
   int slot = 0;
 #pragma unroll 1
   for (;; slot ^= 1) {
@@ -313,7 +373,6 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   const int item = cur.x, tok0 = cur.y, valid = cur.z, n = cur.w;
   if (item < 0) break;
   const int h = item % H;
-  const int level = chain ? (tok0 - n * p.geo.seq_len) / kChunk : 0;
   const size_t chh = (size_t)item;
   const size_t row0 = ((size_t)tok0 * H + h) * kD;
   const bool full = valid == kChunk;
@@ -322,21 +381,17 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   uint32_t dbase = base;
   asm volatile("" : "+r"(dbase));
 
-  // ---- 0. the strips of g, k and q by TMA, right into their operand slots; V (and T when recomputing)
-  auto request_v = [&]() {  // one thread
+  // ---- 0. V (and T when recomputing) by TMA; the strips of g, k and q are on their way into their operand slots
+  auto request_v = [&]() {  // thread 0, when its stores from there are done
     tc::mbar_expect_tx(bar_tma, kRecompute ? 16384 + 8192 : 16384);
     tc::tma_load_3d(base + oV, &tm_v, bar_tma, 0, h, tok0);
     tc::tma_load_3d(base + oV + 8192, &tm_v, bar_tma, 64, h, tok0);
     if (kRecompute) tc::tma_load_3d(base + oTm, &tm_akk, bar_tma, 0, h, tok0);
   };
-  if (kRecompute && tid == 0) request_v();  // (the forward asks for V once it knows whether the decays need its place first)
-  if (lane == 0) {  // two 64-channel blocks each, issued by six warps
-    const int b = warp & 1;
-    if (warp == 0) tc::mbar_expect_tx(bar_in, 6 * 8192);
-    if (warp < 2) tc::tma_load_3d(base + oY + b * 8192, &tm_g, bar_in, 64 * b, h, tok0);
-    else if (warp < 4) tc::tma_load_3d(base + oA + b * 16384, &tm_k, bar_in, 64 * b, h, tok0);
-    else if (warp < 6) tc::tma_load_3d(base + oA + 8192 + b * 16384, &tm_q, bar_in, 64 * b, h, tok0);
-  }
+  if (kRecompute && tid == 0) {
+    tc::bulk_wait_read();
+    request_v();
+  }  // (the forward asks for V once it knows whether the decays need its place first)
   uint2 ktraw[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -344,45 +399,19 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     if (kRecompute && r0 + i < valid)
       ktraw[i] = *reinterpret_cast<const uint2*>(p.kt + row0 + (size_t)(r0 + i) * gld + c4);
   }
-  float sc_beta = 0.f, sc_pd = 0.f, sc_bp = 0.f;  // lane i < 8: scalars of row r0 + i
-  if (lane < 8) {
-    const int r = r0 + lane;
-    if (chain) {  // beta is packed chunk-major on the way (the later stages read that copy)
-      sc_beta = r < valid ? to_f(p.beta[(size_t)(tok0 + r) * H + h]) : 0.f;
-      p.beta_c_w[chh * kChunk + r] = sc_beta;
-    } else {
-      sc_beta = p.beta_c[chh * kChunk + r];
-    }
-    if (!kRecompute && r < valid) {
-      const size_t s = (size_t)(tok0 + r) * H + h;
-      sc_pd = p.g_atk[s];
-      sc_bp = to_f(p.beta_atk[s]);
-    }
-  }
-  const float4 bias4 = *reinterpret_cast<const float4*>(p.dt_bias + h * kD + c4);
-  const float ea2 = __expf(p.A_log[h]) * kLog2e;
-  float4 a_first = make_float4(0.f, 0.f, 0.f, 0.f);
-  float centre = 0.f;
-  // Chained mode: the chunk-entry state of the preconditioner was normally published long ago by the
-  // item of the chunk before; it is asked for now, so that the two dependent loads (counter, then
-  // value) are back when the strips are.
-  int chain_seen = 4;
-  float chain_a0 = 0.f;
-  if (!kRecompute) {
-    if (!chain) {
-      a_first = *reinterpret_cast<const float4*>(p.a_start + chh * kD + c4);
-    } else if (tid < kD) {
-      if (level == 0) {
-        if (p.A0) chain_a0 = p.A0[((size_t)n * H + h) * kD + tid];
-      } else {
-        chain_seen = ld_acquire(p.chain_flags + item);
-        if (chain_seen >= 4) chain_a0 = __ldcg(p.a_chain + chh * kD + tid);
-      }
-    }
-    centre = p.log_atk_scale[h];
-  }
-  ok = tc::mbar_wait(bar_in, in_phase) && ok;
-  in_phase ^= 1;
+  // (opaque, so that nothing is computed from them, and waits for them, where they were asked for)
+  asm volatile("" : "+r"(n_beta), "+r"(n_bp), "+r"(n_chain), "+f"(n_pd), "+f"(n_alog), "+f"(n_centre), "+f"(n_bias.x), "+f"(n_bias.y),
+               "+f"(n_bias.z), "+f"(n_bias.w));
+  const bool row_in = lane < 8 && r0 + lane < valid;  // lane i < 8: scalars of row r0 + i
+  const float sc_beta = !chain || row_in ? __uint_as_float(chain ? n_beta << 16 : n_beta) : 0.f;
+  const float sc_bp = row_in ? __uint_as_float(n_bp << 16) : 0.f;
+  float sc_pd = row_in ? n_pd : 0.f;
+  if (chain && lane < 8) p.beta_c_w[chh * kChunk + r0 + lane] = sc_beta;  // packed chunk-major on the way, for the later stages
+  const float4 bias4 = n_bias;
+  const float ea2 = __expf(n_alog) * kLog2e, centre = n_centre;
+  uint32_t chain_a0 = n_chain;
+  ok = tc::mbar_wait(bar_in, ph >> 2) && ok;
+  ph ^= 4;
   if (!full) {  // rows past the sequence end read as zero, whatever lies there
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -453,37 +482,32 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 #pragma unroll
       for (int e = 0; e < 4; ++e) G[i][e] += pre[e];
   }
+  if (!kRecompute && !chain && tid < kD) sA0[tid] = __uint_as_float(chain_a0);
   // Chained mode: this chunk's entry state of the preconditioner comes from the item of the chunk
-  // before it (or the initial state), the next chunk's goes out.  Four warps, one channel per thread;
-  // a warp publishes with a fence and one count on the successor's flag, which the successor's four
-  // warps poll (bounded) until all four counts are in.
+  // before it (or the initial state), the next chunk's goes out.  Four warps, one channel per thread.
   if (chain && tid < kD) {
+    const int level = (tok0 - n * p.geo.seq_len) / kChunk;
     float loc = 0.f, gs = 0.f;
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
       loc = sDec[b] * loc + sEnd[b * kD + tid];
       gs += sSum[b];
     }
-    float a0 = chain_a0;
     if (level == 0) {
-      p.a_chain[chh * kD + tid] = a0;
-    } else if (chain_seen < 4) {  // not there yet when the item began: poll (bounded)
-      uint32_t it = 0;
-      while ((chain_seen = ld_acquire(p.chain_flags + item)) < 4 && ++it < tc::kSpinLimit) {}
-      ok = ok && chain_seen >= 4;
-      a0 = __ldcg(p.a_chain + chh * kD + tid);
+      p.a_chain[chh * kD + tid] = __uint_as_float(chain_a0);
+    } else {
+      uint32_t it = 0;  // not there yet when it was asked for: poll (bounded)
+      while (chain_a0 == kNotYet && ++it < tc::kSpinLimit) chain_a0 = ld_relaxed(p.a_chain + chh * kD + tid);
+      ok = ok && chain_a0 != kNotYet;
     }
+    const float a0 = __uint_as_float(chain_a0);
     sA0[tid] = a0;
     const float an = __expf(gs) * a0 + loc;
-    if (level + 1 < p.geo.chunks_per_seq) {
-      p.a_chain[(chh + H) * kD + tid] = an;
-      __syncwarp();
-      if (lane == 0) red_release_add(p.chain_flags + item + H, 1);  // (orders the warp's stores before the count)
-    } else if (p.AT) {
-      p.AT[((size_t)n * H + h) * kD + tid] = an;
-    }
+    if (level + 1 < p.geo.chunks_per_seq) st_relaxed(p.a_chain + (chh + H) * kD + tid, an);
+    else if (p.AT) p.AT[((size_t)n * H + h) * kD + tid] = an;
     if (tid == 0) p.sa[chh] = gs;
   }
+  if (!kRecompute && tid == 0) tc::bulk_wait_read();  // the stores of the item before from the tiles that are written next
   // Does the chunk decay too much for one direct block?  (The same answer for all threads: every thread holds the
   // totals of its four channels, the CTA all 128.)  If so, which reference rows do its strips take?
   const bool by_strip =
@@ -506,26 +530,32 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     }
   }
 
-  uint2 kd[8];  // Kd of a chunk that is paired by strips
   // ---- 3. one pass over the strip: preconditioner states of its rows -> write keys kt = k * B(A_t)
   // (to global memory), kg = kt * decay to the chunk end, the diagonal q_i . kt_i, and the gated operands
   // in place: Kd = k 2^G (rows 0..63 of the stacked operand, later the operand of W^T), q 2^G (rows
   // 64..127), kt 2^-G (into the slots g has left); qg goes to global memory.  The decay to the chunk
   // end is 2^G_last times the 2^-G the operand needs anyway.  Nothing of the strip is needed afterwards.
-  // A chunk that is paired by strips leaves its operands as pairs_of_strip or pair_exact reads them, and Kd in registers.
+  // A chunk that is paired by strips leaves its operands as pairs_of_strip or pair_exact reads them.
   {
-    if (chain) a_first = *reinterpret_cast<const float4*>(sA0 + c4);  // (written before the barrier of the decision)
-    float A[4] = {a_first.x, a_first.y, a_first.z, a_first.w};
+    float A[4] = {0.f, 0.f, 0.f, 0.f};
     if (!kRecompute) {
+      const float4 a0 = *reinterpret_cast<const float4*>(sA0 + c4);  // (written before the barrier of the decision)
+      A[0] = a0.x; A[1] = a0.y; A[2] = a0.z; A[3] = a0.w;
       for (int b = 0; b < warp; ++b) {
         const float d = sDec[b];
         const float4 e4 = *reinterpret_cast<const float4*>(sEnd + b * kD + c4);
         A[0] = d * A[0] + e4.x; A[1] = d * A[1] + e4.y; A[2] = d * A[2] + e4.z; A[3] = d * A[3] + e4.w;
       }
     }
-    const float glE[4] = {ex2(Glast[0]), ex2(Glast[1]), ex2(Glast[2]), ex2(Glast[3])};
-    if (!kRecompute && warp == 0)
-      *reinterpret_cast<float4*>(p.gc + chh * kD + c4) = make_float4(glE[0], glE[1], glE[2], glE[3]);
+    if (!by_strip || (!kRecompute && warp == 0)) {
+      const float glE[4] = {ex2(Glast[0]), ex2(Glast[1]), ex2(Glast[2]), ex2(Glast[3])};
+      if (!kRecompute && warp == 0)
+        *reinterpret_cast<float4*>(p.gc + chh * kD + c4) = make_float4(glE[0], glE[1], glE[2], glE[3]);
+      if (!by_strip) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) Glast[c] = glE[c];  // from here on the decay itself (one set of registers for both kinds)
+      }
+    }
     float zr[4], xr[4];  // the strip's reference rows
     if (!kRecompute && by_strip && refs < 2) {
       float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);  // z of the strip before
@@ -542,16 +572,22 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
         zr[c] = refs ? G[6][c] : G[7][c];
         xr[c] = refs ? G[1][c] : G[0][c];
       }
-      unsigned char* at = tiles + warp * 512 + (lane << 4);
+      unsigned char* at = tiles + warp * 1024 + (lane << 4);
       *reinterpret_cast<float4*>(at + oD0) = make_float4(ex2(xr[0] - zr[0]), ex2(xr[1] - zr[1]), ex2(xr[2] - zr[2]), ex2(xr[3] - zr[3]));
       *reinterpret_cast<float4*>(at + oD1) = make_float4(ex2(xr[0] - prev.x), ex2(xr[1] - prev.y), ex2(xr[2] - prev.z), ex2(xr[3] - prev.w));
-      *reinterpret_cast<float4*>(at + oStep) = make_float4(ex2(zr[0] - prev.x), ex2(zr[1] - prev.y), ex2(zr[2] - prev.z), ex2(zr[3] - prev.w));
+      *reinterpret_cast<float4*>(tiles + oStep + warp * 512 + (lane << 4)) = make_float4(ex2(zr[0] - prev.x), ex2(zr[1] - prev.y), ex2(zr[2] - prev.z), ex2(zr[3] - prev.w));
     }
     float dg[8];
+    // (the next row is read before this one is written: the compiler cannot tell their places apart and would start it after)
+    uint2 k_next = ld_k(0), q_next = ld_q(0);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int off = slot_off(i);
-      const uint2 kr = ld_k(i), qr = ld_q(i);
+      const uint2 kr = k_next, qr = q_next;
+      if (i < 7) {
+        k_next = ld_k(i + 1);
+        q_next = ld_q(i + 1);
+      }
       uint2 kt = ktraw[i];
       if (!kRecompute) {
         const float pd = __shfl_sync(0xffffffffu, sc_pd, i), bp = __shfl_sync(0xffffffffu, sc_bp, i);
@@ -581,7 +617,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           fi[c] = __fdividef(1.f, e[c]);
-          tl[c] = glE[c] * fi[c];
+          tl[c] = Glast[c] * fi[c];
         }
         *reinterpret_cast<uint2*>(aBase + off) = scale4(kr, e);
         if (!kRecompute) {
@@ -594,7 +630,6 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
         if (kRecompute) {
           *reinterpret_cast<uint2*>(aBase + off) = scale4(kr, e);
         } else {
-          kd[i] = scale4(kr, e);
           float y[4];
           if (refs < 2) {
             float x[4];
@@ -604,7 +639,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
               x[c] = ex2(G[i][c] - xr[c]);
               y[c] *= ex2(zr[c] - G[i][c]);
             }
-            *reinterpret_cast<uint2*>(aBase + off) = scale4(kr, x);
+            *reinterpret_cast<uint2*>(aBase + off) = scale4(kr, e);
+            *reinterpret_cast<uint2*>(yBase + off) = scale4(kr, x);
             *reinterpret_cast<uint2*>(aBase + 8192 + off) = scale4(qr, x);
           } else {
             *reinterpret_cast<uint2*>(yBase + off) = kt;
@@ -625,22 +661,28 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     }
   }
   int drawn = 0;
-  if (tid == kThreads - 1) drawn = atomicAdd(p.cursor, 1);  // (not used before the products are back)
+  if (tid == 32) drawn = atomicAdd(p.cursor, 1);  // (looked up while the pair products run)
   tc::fence_proxy_async();
   tc::tc_fence_before();
   __syncthreads();  // (the strip exchange arrays are dead from here on: L takes their place)
+  if (kRecompute && tid == 32) s_item[slot ^ 1] = describe(drawn);
   if (!kRecompute && by_strip) {
-    // what lies above the strip diagonal of P reads as zero
-    for (int J = warp + 1 + (lane >> 3); J < 8; J += 4)
-      *reinterpret_cast<uint4*>(tiles + oP + (r0 + (lane & 7)) * 128 + ((J ^ (lane & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+    if (tid == 32) s_item[slot ^ 1] = describe(drawn);
     if (refs < 2) {
       pairs_of_strip(tiles, base, warp, lane, p.scale);
     } else {
       pairs_of_strip_exact(tiles, base, warp, lane, p.scale);
-    }
-    __syncwarp();  // (only this warp reads the k rows of its strip)
+      __syncwarp();  // (only this warp reads the k rows of its strip; they become Kd)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) *reinterpret_cast<uint2*>(aBase + slot_off(i)) = kd[i];
+      for (int i = 0; i < 8; ++i) {
+        const float4 g4 = *reinterpret_cast<const float4*>(tiles + oG + (r0 + i) * 512 + ((lane ^ ((i & 3) << 1)) << 4));
+        const float e[4] = {ex2(g4.x), ex2(g4.y), ex2(g4.z), ex2(g4.w)};
+        *reinterpret_cast<uint2*>(aBase + slot_off(i)) = scale4(ld_k(i), e);
+      }
+    }
+    // what lies above the strip diagonal of P reads as zero
+    for (int J = warp + 1 + (lane >> 3); J < 8; J += 4)
+      *reinterpret_cast<uint4*>(tiles + oP + (r0 + (lane & 7)) * 128 + ((J ^ (lane & 7)) << 4)) = make_uint4(0, 0, 0, 0);
   } else if (!kRecompute) {
     if (tid == 0) {
       tc::tc_fence_after();
@@ -653,12 +695,17 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       }
       tc::umma_commit(bar_mma);
     }
-    ok = tc::mbar_wait(bar_mma, mma_phase) && ok;
-    mma_phase ^= 1;
+    if (tid == 32) s_item[slot ^ 1] = describe(drawn);
+    ok = tc::mbar_wait(bar_mma, ph & 1) && ok;
+    ph ^= 1;
     tc::tc_fence_after();
     {
+      int wl = tid;  // (opaque: what follows from it is formed here and not kept all along)
+      asm volatile("" : "+r"(wl));
+      const int wp = wl >> 5, ei = (32 * (wp & 3) + (wl & 31)) & 63, j0 = 32 * (wp >> 2);  // this thread's accumulator row and columns
+      const bool isP = (wp & 3) >= 2;
       float acc[32];
-      tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + j0, acc);
+      tc::tmem_ld32(tmem + ((uint32_t)(32 * (wp & 3)) << 16) + j0, acc);
       tc::tmem_ld_wait();
       if (!isP) {  // L = tril(M, -1) diag(beta)
 #pragma unroll
@@ -689,8 +736,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     tc::tc_fence_before();
   }
   auto await_v = [&]() {
-    ok = tc::mbar_wait(bar_tma, tma_phase) && ok;  // V (and T) landed long ago
-    tma_phase ^= 1;
+    ok = tc::mbar_wait(bar_tma, (ph >> 1) & 1) && ok;  // V (and T) landed long ago
+    ph ^= 2;
     if (!full) {  // rows past the sequence end hold another sequence's data: they must not reach the product
       for (int idx = tid; idx < kChunk * 16; idx += kThreads) {
         const int r = idx >> 4, pc = idx & 15;
@@ -700,12 +747,11 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     }
   };
   if (kRecompute) await_v();
-  if (tid == kThreads - 1) s_item[slot ^ 1] = describe(drawn);
   tc::fence_proxy_async();
   __syncthreads();
   if (!kRecompute && by_strip && tid == 0) request_v();  // (the decays have been read)
-  if (lane == 0) {  // the next item's tiles of g, k, q and v
-    const int4 nx = s_item[slot ^ 1];
+  const int4 nx = s_item[slot ^ 1];
+  if (lane == 0) {  // the next item's tiles of g, k, q and v into L2
     if (nx.x >= 0) {
       const CUtensorMap* m = warp < 2 ? &tm_g : warp < 4 ? &tm_k : warp < 6 ? &tm_q : &tm_v;
       tc::tma_prefetch_3d(m, 64 * (warp & 1), nx.x % H, nx.y);
@@ -740,12 +786,16 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
         *reinterpret_cast<uint4*>(p.Akk + ((size_t)(tok0 + r) * H + h) * kChunk + 8 * pc) = pk;
     }
     await_v();
+    if (tid == 0) tc::bulk_wait_read();  // (scale P has left: U takes its place)
     tc::fence_proxy_async();
     tc::tc_fence_before();
     __syncthreads();
   }
 
   // ---- 6. W^T = Kd^T T^T, U^T = V^T T^T
+  if (nx.x >= 0) {
+    if (tid == 32) request_g(nx);
+  }
   if (tid == 0) {
     tc::tc_fence_after();
     if (!kRecompute && full) {
@@ -763,9 +813,13 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
                     idesc, kk > 0);
     tc::umma_commit(bar_mma);
   }
-  ok = tc::mbar_wait(bar_mma, mma_phase) && ok;
-  mma_phase ^= 1;
+  ok = tc::mbar_wait(bar_mma, ph & 1) && ok;
+  ph ^= 1;
   tc::tc_fence_after();
+  if (nx.x >= 0) {
+    request_kq(nx);
+    request_scalars(nx);
+  }
   {
     const int ch = 32 * (warp & 3) + lane, t0 = 32 * (warp >> 2);  // accumulator row = channel; this warp's tokens
 #pragma unroll
@@ -774,7 +828,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 + 64 * m + t0, acc);
       tc::tmem_ld_wait();
       if (full) {  // transposed into a swizzled [token][channel] tile for the TMA store
-        unsigned char* out = tiles + oA + m * 16384;
+        unsigned char* out = tiles + (m ? oX : oV);
 #pragma unroll
         for (int t = 0; t < 32; ++t)
           *reinterpret_cast<bf16*>(out + sw128_offset(t0 + t, ch, 8192)) = __float2bfloat16(acc[t]);
@@ -791,16 +845,15 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   __syncthreads();
   if (tid == 0) {
     if (full) {
-      tc::tma_store_3d(&tm_w, base + oA, 0, h, tok0);
-      tc::tma_store_3d(&tm_w, base + oA + 8192, 64, h, tok0);
-      tc::tma_store_3d(&tm_u, base + oA + 16384, 0, h, tok0);
-      tc::tma_store_3d(&tm_u, base + oA + 16384 + 8192, 64, h, tok0);
+      tc::tma_store_3d(&tm_w, base + oV, 0, h, tok0);
+      tc::tma_store_3d(&tm_w, base + oV + 8192, 64, h, tok0);
+      tc::tma_store_3d(&tm_u, base + oX, 0, h, tok0);
+      tc::tma_store_3d(&tm_u, base + oX + 8192, 64, h, tok0);
       tc::bulk_commit();
     }
-    tc::bulk_wait_read();  // the tiles stay in place until every store of this item has read them
   }
-  __syncthreads();  // the next item's copies overwrite the tiles
   }  // item loop
+  if (tid == 0) tc::bulk_wait_read();
   if (__syncthreads_or(!ok) && tid == 0) atomicExch(p.status, 1);
   tc::tc_fence_before();
   __syncthreads();
@@ -808,6 +861,12 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 }
 
 // ------------------------------------------------------------------ host side
+int launch_chain_init(float* a_chain, size_t items, int* zero, cudaStream_t st) {
+  const size_t n = items * (kD / 4), most = 8 * (size_t)sm_count(), blocks = (n + 255) / 256;
+  pkda_chain_init_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, st>>>(reinterpret_cast<uint4*>(a_chain), n, zero);
+  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+}
+
 int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) {
   const uint64_t H = ip.geo.heads, tok = ip.geo.total_tokens;
   CUtensorMap tm_v, tm_akk, tm_aqk, tm_w, tm_u, tm_g, tm_k, tm_q;
