@@ -376,6 +376,20 @@ __device__ __forceinline__ void row_sums8(float (&v)[8], int lane) {
   v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// The same for v[0..3], in the same order; lane l holds the total of entry ((l >> 4) & 1) * 2 + ((l >> 3) & 1).
+__device__ __forceinline__ void row_sums4(float (&v)[4], int lane) {
+  const bool hi16 = lane & 16, hi8 = lane & 8;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const float keep = hi16 ? v[j + 2] : v[j], send = hi16 ? v[j] : v[j + 2];
+    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+  const float keep = hi8 ? v[1] : v[0], send = hi8 ? v[0] : v[1];
+  v[0] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+#pragma unroll
+  for (int o = 4; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+}
+
 // Tail of the classifier kernel: a CTA has put the kind of its 64 items into sKind (-1: none, 0:
 // tensor-memory kernel, 1: mma.sync kernel) and their first tokens into sTok, and appends them to the two
 // work lists with one atomic per list, keeping their order.  One warp per list, two items per lane.

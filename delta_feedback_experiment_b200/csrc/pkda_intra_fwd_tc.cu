@@ -423,40 +423,47 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   }
 
   // ---- 1. decay gate, strip-local cumulative sum; strip-local preconditioner scan from zero
+  // (The row loops of passes 1 and 3 take four rows a turn, their rows of G moved down in between: unrolled by eight, the
+  // passes were some 40 KB of instructions that two CTAs in different phases kept evicting, and the first stall was
+  // the fetch.  2,048 items: 131 -> 125 us, strongly decaying ones 161 -> 154; issue slots in use 48 -> 55 %.)
   float G[8][4];
   {
     const float bias[4] = {bias4.x, bias4.y, bias4.z, bias4.w};
+    float run[4] = {0.f, 0.f, 0.f, 0.f}, a[4] = {0.f, 0.f, 0.f, 0.f}, dblk = 1.f, gsum = 0.f;
+    const float lg = sc_pd;
+    sc_pd = __expf(sc_pd);  // rows past the end: exp(0) = 1, beta 0
+#pragma unroll 1
+    for (int i0 = 0; i0 < 8; i0 += 4) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float x[4];
-      unpack4(ld_y(i), x);
+      for (int i = 0; i < 4; ++i) {
+        float x[4];
+        unpack4(ld_y(i0 + i), x);
+        const bool in = r0 + i0 + i < valid;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float gv = (r0 + i < valid) ? -ea2 * softplus_fast(x[e] + bias[e]) : 0.f;
-        G[i][e] = i ? G[i - 1][e] + gv : gv;
+        for (int e = 0; e < 4; ++e) {
+          const float gv = in ? -ea2 * softplus_fast(x[e] + bias[e]) : 0.f;
+          run[e] += gv;
+          G[i][e] = G[i + 4][e];
+          G[i + 4][e] = run[e];
+        }
+        if (!kRecompute) {
+          if (chain) gsum += __shfl_sync(0xffffffffu, lg, i0 + i);  // the strip's summed log-decay, added in row order
+          const float pd = __shfl_sync(0xffffffffu, sc_pd, i0 + i), bp = __shfl_sync(0xffffffffu, sc_bp, i0 + i);
+          float kc[4];
+          unpack4(ld_k(i0 + i), kc);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] = pd * a[e] + bp * kc[e] * kc[e];
+          dblk *= pd;
+        }
       }
     }
-  }
-  if (!kRecompute) {
-    if (chain) {  // the strip's summed log-decay, added in row order
-      float gsum = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) gsum += __shfl_sync(0xffffffffu, sc_pd, i);
-      if (lane == 0) sSum[warp] = gsum;
+    if (!kRecompute) {
+      *reinterpret_cast<float4*>(sEnd + warp * kD + c4) = make_float4(a[0], a[1], a[2], a[3]);
+      if (lane == 0) {
+        sDec[warp] = dblk;
+        if (chain) sSum[warp] = gsum;
+      }
     }
-    sc_pd = __expf(sc_pd);  // rows past the end: exp(0) = 1, beta 0
-    float a[4] = {0.f, 0.f, 0.f, 0.f}, dblk = 1.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float pd = __shfl_sync(0xffffffffu, sc_pd, i), bp = __shfl_sync(0xffffffffu, sc_bp, i);
-      float kc[4];
-      unpack4(ld_k(i), kc);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) a[e] = pd * a[e] + bp * kc[e] * kc[e];
-      dblk *= pd;
-    }
-    *reinterpret_cast<float4*>(sEnd + warp * kD + c4) = make_float4(a[0], a[1], a[2], a[3]);
-    if (lane == 0) sDec[warp] = dblk;
   }
   *reinterpret_cast<float4*>(sTot + warp * kD + c4) = make_float4(G[7][0], G[7][1], G[7][2], G[7][3]);
   if (lane < 8) sBeta[r0 + lane] = sc_beta;
@@ -577,20 +584,20 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       *reinterpret_cast<float4*>(at + oD1) = make_float4(ex2(xr[0] - prev.x), ex2(xr[1] - prev.y), ex2(xr[2] - prev.z), ex2(xr[3] - prev.w));
       *reinterpret_cast<float4*>(tiles + oStep + warp * 512 + (lane << 4)) = make_float4(ex2(zr[0] - prev.x), ex2(zr[1] - prev.y), ex2(zr[2] - prev.z), ex2(zr[3] - prev.w));
     }
-    float dg[8];
+    float dg[4];
     // (the next row is read before this one is written: the compiler cannot tell their places apart and would start it after)
     uint2 k_next = ld_k(0), q_next = ld_q(0);
+#pragma unroll 1
+    for (int i0 = 0; i0 < 8; i0 += 4) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int off = slot_off(i);
+    for (int i = 0; i < 4; ++i) {
+      const int row = i0 + i, off = slot_off(row);
       const uint2 kr = k_next, qr = q_next;
-      if (i < 7) {
-        k_next = ld_k(i + 1);
-        q_next = ld_q(i + 1);
-      }
+      k_next = ld_k((row + 1) & 7);
+      q_next = ld_q((row + 1) & 7);
       uint2 kt = ktraw[i];
       if (!kRecompute) {
-        const float pd = __shfl_sync(0xffffffffu, sc_pd, i), bp = __shfl_sync(0xffffffffu, sc_bp, i);
+        const float pd = __shfl_sync(0xffffffffu, sc_pd, row), bp = __shfl_sync(0xffffffffu, sc_bp, row);
         float kc[4], f[4];
         unpack4(kr, kc);
 #pragma unroll
@@ -600,7 +607,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
           f[e] = __expf(-p.ln_x * __fdividef(dev, 1.f + fabsf(dev)));
         }
         kt = scale4(kr, f);
-        if (r0 + i < valid) *reinterpret_cast<uint2*>(p.kt + row0 + (size_t)(r0 + i) * gld + c4) = kt;
+        if (r0 + row < valid) *reinterpret_cast<uint2*>(p.kt + row0 + (size_t)(r0 + row) * gld + c4) = kt;
         float kc2[4], qc[4];
         unpack4(kt, kc2);
         unpack4(qr, qc);
@@ -647,17 +654,24 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 #pragma unroll
             for (int c = 0; c < 4; ++c) y[c] = G[i][c];
           }
-          *reinterpret_cast<float4*>(tiles + oG + (r0 + i) * 512 + ((lane ^ ((i & 3) << 1)) << 4)) = make_float4(y[0], y[1], y[2], y[3]);
+          *reinterpret_cast<float4*>(tiles + oG + (r0 + row) * 512 + ((lane ^ ((i & 3) << 1)) << 4)) = make_float4(y[0], y[1], y[2], y[3]);
         }
       }
-      if (r0 + i < valid) {
-        *reinterpret_cast<uint2*>(p.kg + row0 + (size_t)(r0 + i) * gld + c4) = scale4(kt, tl);
-        *reinterpret_cast<uint2*>(p.qg + row0 + (size_t)(r0 + i) * gld + c4) = scale4(qr, es);
+      if (r0 + row < valid) {
+        *reinterpret_cast<uint2*>(p.kg + row0 + (size_t)(r0 + row) * gld + c4) = scale4(kt, tl);
+        *reinterpret_cast<uint2*>(p.qg + row0 + (size_t)(r0 + row) * gld + c4) = scale4(qr, es);
       }
     }
     if (!kRecompute) {
-      row_sums8(dg, lane);
-      if ((lane & 3) == 0) sDiag[r0 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = dg[0];
+      row_sums4(dg, lane);
+      if ((lane & 7) == 0) sDiag[r0 + i0 + ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1)] = dg[0];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) G[i][c] = G[i + 4][c];
+      ktraw[i] = ktraw[i + 4];
+    }
     }
   }
   int drawn = 0;
@@ -822,7 +836,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   }
   {
     const int ch = 32 * (warp & 3) + lane, t0 = 32 * (warp >> 2);  // accumulator row = channel; this warp's tokens
-#pragma unroll
+#pragma unroll 1
     for (int m = 0; m < 2; ++m) {
       float acc[32];
       tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 + 64 * m + t0, acc);
