@@ -11,57 +11,28 @@ constexpr int kLdD = kD + kPad;               // smem row stride of a [*][128] b
 constexpr int kLdC = kChunk + kPad;           // smem row stride of a [*][64] bf16 tile
 constexpr int kTileBytes = kChunk * kLdD * 2; // one [64][128] bf16 tile
 
-// Level `lvl` (a power of two < 64) pairs row i (bit lvl set) with row j (bit
-// lvl clear) of the same 2*lvl block.
+// Level `lvl` (4, 2 or 1, inside a strip of 8 rows) pairs row i (bit lvl set) with row j (bit
+// lvl clear) of the same 2*lvl block, relative to the first row of the upper half.
 __device__ __forceinline__ bool level_pair_ok(int i, int j, int lvl) {
   return (((i ^ j) & ~(2 * lvl - 1)) == 0) && (i & lvl) && !(j & lvl);
 }
 
 constexpr int kLdG = kD + 8;                  // smem row stride of a [64][128] fp32 array
 
-// "Direct" pairing: inside a block of b rows (b a power of two) all pairs j < i
-// use ONE reference row, the block's first: row factor 2^(G_i - G_ref) <= 1,
-// column factor 2^(G_ref - G_j) >= 1.  That is only safe while the decay across a
-// b-block stays far inside the fp32 / bf16 exponent range, so each (chunk, head)
-// picks the largest b whose worst block decay is below kDirectLimit (log2 units)
-// and covers the remaining pairs with hierarchy levels >= b.  lvl == 0 denotes the
-// direct level everywhere below.
+// "Direct" pairing: all pairs j < i of a block of rows use ONE reference row: row factor
+// 2^(G_i - G_ref) <= 1, column factor 2^(G_ref - G_j) >= 1.  That is only safe while the decay across
+// the block stays far inside the fp32 / bf16 exponent range: the whole chunk is one block where it decays by
+// at most kDirectLimit (log2 units), else strips of 8 rows have reference rows of their own.
 // With the limit at 112 the column operand kt 2^112 (|kt| <= 1.5 |k|) and the fp32 sums of up to 128
 // masked products of that size stay below 2^127, and the row operand k 2^-112 only loses (to the
 // flush of denormals) channels with |k| < 2^-14, whose products are below the bf16 rounding of the
 // others; chunks of the benchmark's gate distribution (about 75 +- 6 log2 units of decay per 64
 // tokens) then practically always form one block.
 constexpr float kDirectLimit = 112.f;
-
-__device__ __forceinline__ bool pair_ok(int i, int j, int lvl, int b) {
-  if (lvl) return level_pair_ok(i, j, lvl);
-  return (((i ^ j) & ~(b - 1)) == 0) && (j < i);
-}
-
-// Per-channel worst block decay for b = 2,4,...,64 (dmax[0..5]) from the cumulative
-// log2-decay column c of sG.
-__device__ __forceinline__ void block_decay_max(const float* sG, int c, float (&dmax)[6]) {
-#pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    const int b = 2 << e;
-    float m = 0.f;
-    for (int bs = 0; bs < kChunk; bs += b) m = fmaxf(m, sG[bs * kLdG + c] - sG[(bs + b - 1) * kLdG + c]);
-    dmax[e] = m;
-  }
-}
-
-// Largest admissible direct block size given the per-warp maxima (nw warps x 6).
-__device__ __forceinline__ int pick_direct_block(const float* sWarpMax, int nw, int cap) {
-  int b = 1;
-#pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    float m = 0.f;
-    for (int w = 0; w < nw; ++w) m = fmaxf(m, sWarpMax[w * 6 + e]);
-    if (m <= kDirectLimit && (2 << e) <= cap) b = 2 << e;
-    else break;
-  }
-  return b;
-}
+// Where a strip decays by more than that, its rows are taken relative to its third row and its columns relative to the third
+// from the end, as long as 5 tokens decay by at most kDirectLimit and the 2 outer ones by at most this (log2 units).
+constexpr float kOuterLimit = 45.f;
+constexpr int kInnerRow = 2;
 
 // 2^x by the hardware approximation (flushes denormal results to zero, which is
 // what the gating factors want: every argument here is <= 0).
@@ -77,61 +48,6 @@ __device__ __forceinline__ void scale8(uint4& x, const float (&f)[8]) {
   for (int j = 0; j < 4; ++j) {
     const float2 v = unpack_bf16(w[j]);
     w[j] = pack_bf16(v.x * f[2 * j], v.y * f[2 * j + 1]);
-  }
-}
-
-// Builds the gated operands of one level from the log2-domain cumulative decay
-// sG [64][kLdG]: rows with bit lvl set get X * 2^(G_r - G_ref) (into sXq from sQ
-// and sXk from sK), the others get Y * 2^(G_ref - G_r) (into sY from sKt), where
-// ref is the first row of the upper half of the row's 2*lvl block.  Rows of the
-// other kind are left untouched (their products are masked out).  Null
-// destinations are skipped.  sFac (optional, fp32 [64][kLdG]) receives the factor
-// each row used.  Eight channels per thread and step (128-bit accesses).
-__device__ __forceinline__ void stage_level(bf16* sXq, bf16* sXk, bf16* sY, const bf16* sQ, const bf16* sK,
-                                            const bf16* sKt, const float* sG, int lvl, int b, int tid,
-                                            int nthreads, float* sFac = nullptr) {
-  for (int idx = tid; idx < kChunk * kD / 8; idx += nthreads) {
-    const int r = idx >> 4, c8 = (idx & 15) << 3;
-    const int ref = lvl ? (r & ~(2 * lvl - 1)) + lvl : (r & ~(b - 1));
-    const bool upper = lvl ? (r & lvl) != 0 : true;
-    const float4 a0 = *reinterpret_cast<const float4*>(sG + r * kLdG + c8);
-    const float4 a1 = *reinterpret_cast<const float4*>(sG + r * kLdG + c8 + 4);
-    const float4 b0 = *reinterpret_cast<const float4*>(sG + ref * kLdG + c8);
-    const float4 b1 = *reinterpret_cast<const float4*>(sG + ref * kLdG + c8 + 4);
-    const float sgn = upper ? 1.f : -1.f;
-    float f[8];
-    f[0] = ex2(sgn * (a0.x - b0.x)); f[1] = ex2(sgn * (a0.y - b0.y));
-    f[2] = ex2(sgn * (a0.z - b0.z)); f[3] = ex2(sgn * (a0.w - b0.w));
-    f[4] = ex2(sgn * (a1.x - b1.x)); f[5] = ex2(sgn * (a1.y - b1.y));
-    f[6] = ex2(sgn * (a1.z - b1.z)); f[7] = ex2(sgn * (a1.w - b1.w));
-    if (sFac) {
-      *reinterpret_cast<float4*>(sFac + r * kLdG + c8) = make_float4(f[0], f[1], f[2], f[3]);
-      *reinterpret_cast<float4*>(sFac + r * kLdG + c8 + 4) = make_float4(f[4], f[5], f[6], f[7]);
-    }
-    if (upper) {
-      if (sXq) {
-        uint4 x = *reinterpret_cast<const uint4*>(sQ + r * kLdD + c8);
-        scale8(x, f);
-        *reinterpret_cast<uint4*>(sXq + r * kLdD + c8) = x;
-      }
-      if (sXk) {
-        uint4 x = *reinterpret_cast<const uint4*>(sK + r * kLdD + c8);
-        scale8(x, f);
-        *reinterpret_cast<uint4*>(sXk + r * kLdD + c8) = x;
-      }
-      if (!lvl && sY) {  // direct level: the same row is also a column operand, factor 1/f
-        float fi[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) fi[j] = __fdividef(1.f, f[j]);
-        uint4 x = *reinterpret_cast<const uint4*>(sKt + r * kLdD + c8);
-        scale8(x, fi);
-        *reinterpret_cast<uint4*>(sY + r * kLdD + c8) = x;
-      }
-    } else if (sY) {
-      uint4 x = *reinterpret_cast<const uint4*>(sKt + r * kLdD + c8);
-      scale8(x, f);
-      *reinterpret_cast<uint4*>(sY + r * kLdD + c8) = x;
-    }
   }
 }
 
@@ -191,39 +107,6 @@ __device__ __forceinline__ void gate_cumsum(float* sG, int c) {
   for (int r = 0; r < kChunk; ++r) {
     run += sG[r * kLdG + c];
     sG[r * kLdG + c] = run;
-  }
-}
-
-// warp_gemm for one m-tile whose A operand is a [64][64] pair-weight matrix
-// restricted to the pairs of one level.  With mask = true every A element
-// (i, j) that is not a valid pair of `lvl` is zeroed in registers after the
-// load; kATrans means the logical A is the transpose (A[m=j][k=i]).
-template <int kNT, bool kATrans, bool kBKN>
-__device__ __forceinline__ void warp_gemm_lvl(float (&acc)[1][kNT][4], const bf16* A, int lda, int m0,
-                                              const bf16* B, int ldb, int n0, int kbeg, int kend, int lvl,
-                                              int b, bool mask) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll 1
-  for (int k0 = kbeg; k0 < kend; k0 += 16) {
-    uint32_t a[4];
-    load_a_frag<kATrans>(a, A, lda, m0, k0);
-    if (mask) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int m = m0 + g + 8 * (r & 1);
-        const int kk = k0 + 2 * t + 8 * (r >> 1);
-        const bool ok0 = kATrans ? pair_ok(kk, m, lvl, b) : pair_ok(m, kk, lvl, b);
-        const bool ok1 = kATrans ? pair_ok(kk + 1, m, lvl, b) : pair_ok(m, kk + 1, lvl, b);
-        a[r] &= (ok0 ? 0x0000ffffu : 0u) | (ok1 ? 0xffff0000u : 0u);
-      }
-    }
-#pragma unroll
-    for (int np = 0; np < kNT / 2; ++np) {
-      uint32_t bf[4];
-      load_b_frag2<kBKN>(bf, B, ldb, k0, n0 + 16 * np);
-      mma_bf16(acc[0][2 * np], a, bf[0], bf[1]);
-      mma_bf16(acc[0][2 * np + 1], a, bf[2], bf[3]);
-    }
   }
 }
 

@@ -6,7 +6,7 @@
 //   dF = kg dS1 + P^T dO,  dE = beta dF,  dS0 = Gam_last dS1 + qg^T dO - W^T dE
 //   dR = Tm^T dE (= dV),  dKd = -dR S0^T,  d(tril M) = -tril(dR E^T) diag(beta)
 //   dP = scale tril(dO F^T),  dkg = F dS1^T,  dqg = dO S0^T
-// and the gated pair products are differentiated level by level with the same
+// and the gated pair products are differentiated strip by strip with the same
 // rounded operands on both sides, so that each pair's +/- contributions to the
 // log-decay gradient cancel exactly under the reverse cumulative sum.
 //
@@ -220,13 +220,15 @@ constexpr int oG = oA1 + 2 * kTileBytes;      // f32 [64][kLdG] log2-domain cumu
 constexpr int oTm = oG + kChunk * kLdG * 4;   // bf16 [64][72]
 constexpr int oDE = oTm + kChunk * kLdC * 2;  // dE | later F = beta E
 constexpr int oDR = oDE + kTileBytes;
-constexpr int oStage = oTm;                   // three gated operand tiles | later dG f32 [64][128]
-constexpr int oDP = oStage + 3 * kTileBytes;  // bf16 [64][72]
+constexpr int oStage = oTm;                   // the gated q and k tiles, then the strip factors | later dG f32 [64][128]
+constexpr int oStrip = oStage + 2 * kTileBytes;  // f32 [36][128]
+constexpr int oDP = oStrip + 36 * kD * 4;     // bf16 [64][72]
 constexpr int oDM = oDP + kChunk * kLdC * 2;
-constexpr int oFac = oDM + kChunk * kLdC * 2; // f32 [64][kLdG]
+constexpr int oFac = oDM + kChunk * kLdC * 2; // f32 [64][kLdY]: kt 2^(z - G)
+constexpr int kLdY = kD + 4;                  // = 4 (mod 32): rows 2 t and channels g of a fragment lie in different banks
 constexpr int oSmall = oFac + kChunk * kLdG * 4;
-// small: beta[64] db[64] hdh[128] gcv[128] col[4][128] rb[4][64] red[16] bias[128] warpmax[4][6]
-constexpr int kSmallFloats = 64 + 64 + 128 + 128 + 512 + 256 + 16 + 128 + 24;
+// small: beta[64] db[64] hdh[128] gcv[128] col[4][128] rb[4][64] red[16] bias[128] worst[4][3] diag[64] there[36]
+constexpr int kSmallFloats = 64 + 64 + 128 + 128 + 512 + 256 + 16 + 128 + 12 + 64 + 36;
 constexpr int oBar = oSmall + kSmallFloats * 4;  // one mbarrier
 constexpr int kSmem = oBar + 16;
 constexpr uint32_t kTmaBytes = (3 * kChunk + 2 * kD) * kLdD * 2 + kChunk * kLdC * 2;  // dO, dF, E, S0, dS1 and Tm tiles
@@ -236,29 +238,6 @@ static_assert(oBar % 8 == 0 && oA1 % 128 == 0 && oTm % 128 == 0 && oDE % 128 == 
 static_assert(oDR + kTileBytes <= oDP, "phase-A tiles must not reach the pair-gradient tiles");
 static_assert(oDE + kD * kLdD * 2 <= oDP, "dS1 tile must fit");
 }  // namespace ib
-
-// acc += fac * t and dG += sign * x * t on one warp's [16 x 32] fragment
-// (i0 = first row + lane/4, c0 = first column + 2*(lane%4)); fac is the fp32
-// level factor of each row (kInverse: its reciprocal, the column factor of the
-// direct level), x the staged bf16 operand the product was formed with.
-template <bool kInverse>
-__device__ __forceinline__ void epi_add(float (&acc)[1][4][4], float (&dG)[1][4][4], const float (&t)[1][4][4],
-                                        const float* sFac, const bf16* sX, float sign, int i0, int c0) {
-#pragma unroll
-  for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int i = i0 + 8 * half, c = c0 + 8 * nt;
-      float2 f = *reinterpret_cast<const float2*>(sFac + i * kLdG + c);
-      if (kInverse) { f.x = __fdividef(1.f, f.x); f.y = __fdividef(1.f, f.y); }
-      const float2 x = unpack_bf16(*reinterpret_cast<const uint32_t*>(sX + i * kLdD + c));
-      const float t0 = t[0][nt][2 * half], t1 = t[0][nt][2 * half + 1];
-      acc[0][nt][2 * half] += f.x * t0;
-      acc[0][nt][2 * half + 1] += f.y * t1;
-      dG[0][nt][2 * half] += sign * x.x * t0;
-      dG[0][nt][2 * half + 1] += sign * x.y * t1;
-    }
-}
 
 // One (chunk bx, head by) item; every thread of the CTA takes part.
 __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const IntraBwdMaps& maps, int bx, int by) {
@@ -274,7 +253,8 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   bf16* sdR = reinterpret_cast<bf16*>(smem + oDR);
   bf16* sdP = reinterpret_cast<bf16*>(smem + oDP);
   bf16* sdM = reinterpret_cast<bf16*>(smem + oDM);
-  float* sFac = reinterpret_cast<float*>(smem + oFac);
+  float* sY = reinterpret_cast<float*>(smem + oFac);
+  float* sStrip = reinterpret_cast<float*>(smem + oStrip);
   float* sBeta = reinterpret_cast<float*>(smem + oSmall);
   float* sDb = sBeta + 64;
   float* sHdh = sDb + 64;
@@ -283,7 +263,9 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   float* sRb = sCol + 512;   // [4][64]
   float* sRed = sRb + 256;   // [16]
   float* sBias = sRed + 16;  // [128]
-  float* sWarpMax = sBias + 128;  // [4][6]
+  float* sWorst = sBias + 128;    // [4][3]
+  float* sDiag = sWorst + 12;     // [64] diagonal of dP
+  int* sThere = reinterpret_cast<int*>(sDiag + 64);  // [36]
 
   int n, tok0, valid;
   if (!chunk_lookup(p.geo, bx, n, tok0, valid)) return;
@@ -345,13 +327,20 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   __syncthreads();
   if (tid < kD) {
     gate_cumsum(sG, tid);
-    float dmax[6];
-    block_decay_max(sG, tid, dmax);
+    // worst decays of a strip of 8 rows: all of it, all but its first or its last two tokens, these two alone
+    float worst[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int e = 0; e < 6; ++e) {
+    for (int r = 0; r < kChunk; r += 8) {
+      const float g0 = sG[r * kLdG + tid], g7 = sG[(r + 7) * kLdG + tid];
+      const float gx = sG[(r + kInnerRow) * kLdG + tid], gz = sG[(r + 7 - kInnerRow) * kLdG + tid];
+      worst[0] = fmaxf(worst[0], g0 - g7);
+      worst[1] = fmaxf(worst[1], fmaxf(g0 - gz, gx - g7));
+      worst[2] = fmaxf(worst[2], fmaxf(g0 - gx, gz - g7));
+    }
 #pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) dmax[e] = fmaxf(dmax[e], __shfl_xor_sync(0xffffffffu, dmax[e], o));
-      if (lane == 0) sWarpMax[warp * 6 + e] = dmax[e];
+    for (int e = 0; e < 3; ++e) {  // (not negative, so their bit patterns have their order)
+      const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(worst[e]));
+      if (lane == 0) sWorst[warp * 3 + e] = __uint_as_float(m);
     }
   }
   if (by_tma) {
@@ -413,9 +402,10 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = 16 * I + gq + 8 * (e >> 1), c = 32 * cq + 8 * nt + 2 * tq + (e & 1);
-      dQ[0][nt][e] = t[0][nt][e] * p.scale * ex2(sG[i * kLdG + c]);
+    for (int half = 0; half < 2; ++half) {
+      const float2 g = *reinterpret_cast<const float2*>(sG + (16 * I + gq + 8 * half) * kLdG + 32 * cq + 8 * nt + 2 * tq);
+      dQ[0][nt][2 * half] = t[0][nt][2 * half] * p.scale * ex2(g.x);
+      dQ[0][nt][2 * half + 1] = t[0][nt][2 * half + 1] * p.scale * ex2(g.y);
     }
   // dR = Tm^T dE  (= dV)
   zero_acc(t);
@@ -441,9 +431,10 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = 16 * I + gq + 8 * (e >> 1), c = 32 * cq + 8 * nt + 2 * tq + (e & 1);
-      dK[0][nt][e] = -t[0][nt][e] * ex2(sG[i * kLdG + c]);
+    for (int half = 0; half < 2; ++half) {
+      const float2 g = *reinterpret_cast<const float2*>(sG + (16 * I + gq + 8 * half) * kLdG + 32 * cq + 8 * nt + 2 * tq);
+      dK[0][nt][2 * half] = -t[0][nt][2 * half] * ex2(g.x);
+      dK[0][nt][2 * half + 1] = -t[0][nt][2 * half + 1] * ex2(g.y);
     }
   __syncthreads();  // S0 no longer needed
   // E moves into its operand tile (S0 has left it) and F = beta E into the dead dE tile
@@ -485,9 +476,12 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int i = 16 * I + gq + 8 * half, j = 16 * J + 8 * nt + 2 * tq;
+        // (the diagonal is ungated and stays out of the products)
         const float p0 = (j <= i) ? t2[0][nt][2 * half] * p.scale : 0.f;
         const float p1 = (j + 1 <= i) ? t2[0][nt][2 * half + 1] * p.scale : 0.f;
-        *reinterpret_cast<uint32_t*>(sdP + i * kLdC + j) = pack_bf16(p0, p1);
+        if (j == i) sDiag[i] = to_f(__float2bfloat16(p0));
+        if (j + 1 == i) sDiag[i] = to_f(__float2bfloat16(p1));
+        *reinterpret_cast<uint32_t*>(sdP + i * kLdC + j) = pack_bf16(j < i ? p0 : 0.f, j + 1 < i ? p1 : 0.f);
       }
   }
   if (out_tma && tid == 0) tc::bulk_wait_read();  // the dv store has read the dR tile
@@ -501,12 +495,16 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   zero_acc(t);
   warp_gemm<1, 4, false, false>(t, sF, kLdD, 16 * I, sdSC, kLdD, 32 * cq, 0, kD);
 #pragma unroll
-  for (int nt = 0; nt < 4; ++nt)
+  for (int nt = 0; nt < 4; ++nt) {
+    const int c = 32 * cq + 8 * nt + 2 * tq;
+    const float2 gl = *reinterpret_cast<const float2*>(sG + (kChunk - 1) * kLdG + c);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = 16 * I + gq + 8 * (e >> 1), c = 32 * cq + 8 * nt + 2 * tq + (e & 1);
-      dKt[0][nt][e] = t[0][nt][e] * ex2(sG[(kChunk - 1) * kLdG + c] - sG[i * kLdG + c]);
+    for (int half = 0; half < 2; ++half) {
+      const float2 g = *reinterpret_cast<const float2*>(sG + (16 * I + gq + 8 * half) * kLdG + c);
+      dKt[0][nt][2 * half] = t[0][nt][2 * half] * ex2(gl.x - g.x);
+      dKt[0][nt][2 * half + 1] = t[0][nt][2 * half + 1] * ex2(gl.y - g.y);
     }
+  }
   __syncthreads();
 
   // ================= phase B: gated pair products =================
@@ -515,7 +513,6 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   bf16* sKt = reinterpret_cast<bf16*>(smem + oA1 + kTileBytes);
   bf16* sXq = reinterpret_cast<bf16*>(smem + oStage);
   bf16* sXk = sXq + kChunk * kLdD;
-  bf16* sY = sXk + kChunk * kLdD;
   cp_async_wait<0>();
   __syncthreads();
   {
@@ -526,12 +523,16 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
     for (int nt = 0; nt < 4; ++nt) {
       cs[nt][0] = cs[nt][1] = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = 16 * I + gq + 8 * (e >> 1), c = 32 * cq + 8 * nt + 2 * tq + (e & 1);
-        const float qv = to_f(sQ[i * kLdD + c]), kv = to_f(sK[i * kLdD + c]), ktv = to_f(sKt[i * kLdD + c]);
-        const float kd = ktv * dKt[0][nt][e];
-        dG[0][nt][e] = qv * dQ[0][nt][e] + kv * dK[0][nt][e] - kd;
-        cs[nt][e & 1] += kd;
+      for (int half = 0; half < 2; ++half) {
+        const int at = (16 * I + gq + 8 * half) * kLdD + 32 * cq + 8 * nt + 2 * tq;
+        const float2 qv = unpack_bf16(*reinterpret_cast<const uint32_t*>(sQ + at));
+        const float2 kv = unpack_bf16(*reinterpret_cast<const uint32_t*>(sK + at));
+        const float2 ktv = unpack_bf16(*reinterpret_cast<const uint32_t*>(sKt + at));
+        const float kd0 = ktv.x * dKt[0][nt][2 * half], kd1 = ktv.y * dKt[0][nt][2 * half + 1];
+        dG[0][nt][2 * half] = qv.x * dQ[0][nt][2 * half] + kv.x * dK[0][nt][2 * half] - kd0;
+        dG[0][nt][2 * half + 1] = qv.y * dQ[0][nt][2 * half + 1] + kv.y * dK[0][nt][2 * half + 1] - kd1;
+        cs[nt][0] += kd0;
+        cs[nt][1] += kd1;
       }
     }
 #pragma unroll
@@ -545,65 +546,192 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
         if (gq == 0) sCol[I * kD + 32 * cq + 8 * nt + 2 * tq + b] = v;
       }
   }
-  // Rows a level does not write keep older contents; their products are removed
-  // by zeroed pair weights, which only works on finite data (0 * NaN = NaN), so
-  // the staging tiles start from zeros rather than from whatever phase A left.
-  for (int i = tid; i < 3 * kTileBytes / 16; i += kThreads)
-    reinterpret_cast<uint4*>(smem + oStage)[i] = make_uint4(0, 0, 0, 0);
-  __syncthreads();
+  // ---- The pairs, strip by strip (8 rows; the factors 2^(G_i - x(I)), 2^(x(I) - z(J)), 2^(z(J) - G_j) and their reference rows
+  // are those of pairs_of_strip in pkda_intra_fwd_tc.cu).  Staged: Xq = bf16(q 2^(G - x)), Xk likewise, y = kt 2^(z - G) in fp32;
+  // the operand of a strip pair is Y = bf16(y 2^(x(I) - z(J))), and both sides of a pair see the same X and Y.
+  //   rows of strip I     t  = [dP_I; dM_I] Y     (8 + 8 rows, K = the tokens)   dq, dk_read += 2^(G - x) t,  dG += Xq t, Xk t
+  //   columns of strip J  u_I = dP_I^T Xq + dM_I^T Xk  (K = 8 + 8 rows of I)     dkt += 2^(z - G) sum_I 2^(x(I) - z(J)) u_I,  dG -= Y u_I
+  // Chunks whose strips decay too much for that take their pairs inside a strip level by level (lvl = 4, 2, 1, every row with a
+  // reference of its own, one staging each) after those between strips.
+  // Against staged pairing levels (operands, factors and masked weights of up to seven levels a chunk): 304 -> 247 us for
+  // 1,460 strongly decaying chunks, 35 -> 29 for 40.
   float rb[2] = {0.f, 0.f};
-  // Direct level (lvl = 0) for pairs inside a b-block, hierarchy levels >= b for the rest.
-  const int bdir = pick_direct_block(sWarpMax, 4, p.direct_cap);
-#pragma unroll 1
-  for (int it = (bdir > 1 ? 0 : 1); it <= 6; ++it) {
-    const int lvl = it ? (64 >> it) : 0;
-    if (lvl && lvl < bdir) break;
-    stage_level(sXq, sXk, sY, sQ, sK, sKt, sG, lvl, bdir, tid, kThreads, sFac);
-    __syncthreads();
-    const bool big = lvl >= 16;               // whole 16-row tiles are upper or lower: no masking
-    const bool wide = !lvl && bdir >= 16;     // direct block made of whole tiles
-    const int blk = lvl ? ((16 * I) & ~(2 * lvl - 1)) : ((16 * I) & ~(bdir - 1));
-    if (!big || ((16 * I) & lvl)) {  // rows act as the upper ("i") side
-      int kb = 16 * I, ke = 16 * I + 16;
-      if (big) { kb = blk; ke = blk + lvl; }
-      else if (wide) { kb = blk; }
-      zero_acc(t);
-      warp_gemm_lvl<4, false, true>(t, sdP, kLdC, 16 * I, sY, kLdD, 32 * cq, kb, ke, lvl, bdir, !big);
-      epi_add<false>(dQ, dG, t, sFac, sXq, 1.f, 16 * I + gq, 32 * cq + 2 * tq);
-      zero_acc(t);
-      warp_gemm_lvl<4, false, true>(t, sdM, kLdC, 16 * I, sY, kLdD, 32 * cq, kb, ke, lvl, bdir, !big);
-      epi_add<false>(dK, dG, t, sFac, sXk, 1.f, 16 * I + gq, 32 * cq + 2 * tq);
-    }
-    if (!big || !((16 * I) & lvl)) {  // rows act as the lower ("j") side
-      int kb = 16 * I, ke = 16 * I + 16;
-      if (big) { kb = blk + lvl; ke = kb + lvl; }
-      else if (wide) { ke = blk + bdir; }
-      zero_acc(t);
-      warp_gemm_lvl<4, true, true>(t, sdM, kLdC, 16 * I, sXk, kLdD, 32 * cq, kb, ke, lvl, bdir, !big);
+  float worst[3];
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+  for (int e = 0; e < 3; ++e) worst[e] = fmaxf(fmaxf(sWorst[e], sWorst[3 + e]), fmaxf(sWorst[6 + e], sWorst[9 + e]));
+  const bool first_last = worst[0] <= kDirectLimit, inner = worst[1] <= kDirectLimit && worst[2] <= kOuterLimit;
+  const bool by_level = p.direct_cap < 8 || !(first_last || inner);
+  const int xo = first_last || by_level ? 0 : kInnerRow, zo = 7 - xo;  // reference rows of a strip
+#pragma unroll 1
+  for (int lvl = 0;;) {
+    // (a warp takes a row, four channels a lane: fp32 rows then move without bank conflicts)
+#pragma unroll 2
+    for (int r = warp; r < kChunk; r += kThreads / 32) {
+      const int c4 = lane << 2, own = lvl ? (r & ~(2 * lvl - 1)) + lvl : r & ~7;
+      const float4 g = *reinterpret_cast<const float4*>(sG + r * kLdG + c4);
+      const float4 gx = *reinterpret_cast<const float4*>(sG + (lvl ? own : own + xo) * kLdG + c4);
+      const float4 gz = *reinterpret_cast<const float4*>(sG + (lvl ? own : own + zo) * kLdG + c4);
+      float4 x = make_float4(ex2(g.x - gx.x), ex2(g.y - gx.y), ex2(g.z - gx.z), ex2(g.w - gx.w));
+      float4 z = make_float4(ex2(gz.x - g.x), ex2(gz.y - g.y), ex2(gz.z - g.z), ex2(gz.w - g.w));
+      if (lvl) {  // the row is on one side of its pairs only
+        if (r & lvl) z = make_float4(0.f, 0.f, 0.f, 0.f);
+        else x = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      const uint2 qr = *reinterpret_cast<const uint2*>(sQ + r * kLdD + c4), kr = *reinterpret_cast<const uint2*>(sK + r * kLdD + c4);
+      const uint2 ktr = *reinterpret_cast<const uint2*>(sKt + r * kLdD + c4);
+      const float2 q0 = unpack_bf16(qr.x), q1 = unpack_bf16(qr.y), k0 = unpack_bf16(kr.x), k1 = unpack_bf16(kr.y);
+      const float2 t0 = unpack_bf16(ktr.x), t1 = unpack_bf16(ktr.y);
+      *reinterpret_cast<uint2*>(sXq + r * kLdD + c4) = make_uint2(pack_bf16(q0.x * x.x, q0.y * x.y), pack_bf16(q1.x * x.z, q1.y * x.w));
+      *reinterpret_cast<uint2*>(sXk + r * kLdD + c4) = make_uint2(pack_bf16(k0.x * x.x, k0.y * x.y), pack_bf16(k1.x * x.z, k1.y * x.w));
+      *reinterpret_cast<float4*>(sY + r * kLdY + c4) = make_float4(t0.x * z.x, t0.y * z.y, t1.x * z.z, t1.y * z.w);
+    }
+    // The factor of every strip pair, and whether it is there at all (nonzero in some channel).
+    for (int pr = warp; pr < 36; pr += kThreads / 32) {
+      const int Is = (pr >= 1) + (pr >= 3) + (pr >= 6) + (pr >= 10) + (pr >= 15) + (pr >= 21) + (pr >= 28);
+      const int Js = pr - Is * (Is + 1) / 2;
+      float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (lvl) {
+        if (Is == Js) d = make_float4(1.f, 1.f, 1.f, 1.f);
+      } else if (!by_level || Js < Is) {
+        const float4 a = *reinterpret_cast<const float4*>(sG + (8 * Is + xo) * kLdG + 4 * lane);
+        const float4 b = *reinterpret_cast<const float4*>(sG + (8 * Js + zo) * kLdG + 4 * lane);
+        d = make_float4(ex2(a.x - b.x), ex2(a.y - b.y), ex2(a.z - b.z), ex2(a.w - b.w));
+      }
+      *reinterpret_cast<float4*>(sStrip + pr * kD + 4 * lane) = d;
+      const bool there = __any_sync(0xffffffffu, fmaxf(fmaxf(d.x, d.y), fmaxf(d.z, d.w)) > 0.f);
+      if (lane == 0) sThere[pr] = there;
+    }
+    __syncthreads();
+    const int m8 = lane >> 3, r7 = lane & 7;
+    // rows of the strips 2 I and 2 I + 1
+#pragma unroll
+    for (int sub = 0; sub < 2; ++sub) {
+      const int Is = 2 * I + sub, tri = Is * (Is + 1) / 2;
+      zero_acc(t);
+#pragma unroll 1
+      for (int K = 0; K <= I; ++K) {
+        const bool two = 2 * K + 1 <= Is;  // (the second strip of the step may be the one behind)
+        if (!sThere[tri + 2 * K] && !(two && sThere[tri + 2 * K + 1])) continue;
+        uint32_t a[4];
+        ldsm_x4(a, smem_u32(((m8 & 1) ? sdM : sdP) + (8 * Is + r7) * kLdC + 16 * K + 8 * (m8 >> 1)));
+        if (lvl) {
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            const int i = 8 * Is + gq, j = 16 * K + 2 * tq + 8 * (x >> 1);
+            a[x] &= (level_pair_ok(i, j, lvl) ? 0x0000ffffu : 0u) | (level_pair_ok(i, j + 1, lvl) ? 0xffff0000u : 0u);
+          }
+        }
+        const float* y = sY + (16 * K + 2 * tq) * kLdY + 32 * cq + gq;
+        const float* d = sStrip + (tri + 2 * K) * kD + 32 * cq + gq;
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          const float d0 = d[8 * nt], d1 = two ? d[kD + 8 * nt] : 0.f;
+          mma_bf16(t[0][nt], a, pack_bf16(y[8 * nt] * d0, y[kLdY + 8 * nt] * d0),
+                   pack_bf16(y[8 * kLdY + 8 * nt] * d1, y[9 * kLdY + 8 * nt] * d1));
+        }
+      }
+      const int i = 8 * Is + gq, ref = lvl ? (i & ~(2 * lvl - 1)) + lvl : 8 * Is + xo;
+      if (!lvl || (i & lvl)) {
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          const int c = 32 * cq + 8 * nt + 2 * tq;
+          const float2 g = *reinterpret_cast<const float2*>(sG + i * kLdG + c), gr = *reinterpret_cast<const float2*>(sG + ref * kLdG + c);
+          const float2 xq = unpack_bf16(*reinterpret_cast<const uint32_t*>(sXq + i * kLdD + c));
+          const float2 xk = unpack_bf16(*reinterpret_cast<const uint32_t*>(sXk + i * kLdD + c));
+          const float f0 = ex2(g.x - gr.x), f1 = ex2(g.y - gr.y);
+          dQ[0][nt][2 * sub] += f0 * t[0][nt][0];
+          dQ[0][nt][2 * sub + 1] += f1 * t[0][nt][1];
+          dK[0][nt][2 * sub] += f0 * t[0][nt][2];
+          dK[0][nt][2 * sub + 1] += f1 * t[0][nt][3];
+          dG[0][nt][2 * sub] += xq.x * t[0][nt][0] + xk.x * t[0][nt][2];
+          dG[0][nt][2 * sub + 1] += xq.y * t[0][nt][1] + xk.y * t[0][nt][3];
+        }
+      }
+    }
+    // columns of the strips 2 I and 2 I + 1, two tiles of 8 channels at a time
+#pragma unroll
+    for (int np = 0; np < 2; ++np) {
+      float2 y[2][2];
+      float w[2][4];
+      const int c = 32 * cq + 16 * np + 2 * tq;
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const float2 y = unpack_bf16(*reinterpret_cast<const uint32_t*>(
-              sY + (16 * I + gq + 8 * half) * kLdD + 32 * cq + 8 * nt + 2 * tq));
-          rb[half] += y.x * t[0][nt][2 * half] + y.y * t[0][nt][2 * half + 1];
+          y[x][half] = *reinterpret_cast<const float2*>(sY + (16 * I + gq + 8 * half) * kLdY + c + 8 * x);
+          w[x][2 * half] = w[x][2 * half + 1] = 0.f;
         }
-      warp_gemm_lvl<4, true, true>(t, sdP, kLdC, 16 * I, sXq, kLdD, 32 * cq, kb, ke, lvl, bdir, !big);
-      if (lvl) epi_add<false>(dKt, dG, t, sFac, sY, -1.f, 16 * I + gq, 32 * cq + 2 * tq);
-      else epi_add<true>(dKt, dG, t, sFac, sY, -1.f, 16 * I + gq, 32 * cq + 2 * tq);
+#pragma unroll 1
+      for (int Is = 2 * I; Is < 8; ++Is) {
+        const int tri = Is * (Is + 1) / 2 + 2 * I;
+        const bool two = Is > 2 * I;  // (the second strip of the columns is the one behind)
+        if (!sThere[tri] && !(two && sThere[tri + 1])) {
+          if (two && !by_level) break;  // strips further behind decay by more
+          continue;
+        }
+        uint32_t a[4], b[4];
+        ldsm_x4_t(a, smem_u32(((m8 >> 1) ? sdM : sdP) + (8 * Is + r7) * kLdC + 16 * I + 8 * (m8 & 1)));
+        ldsm_x4_t(b, smem_u32(((m8 & 1) ? sXk : sXq) + (8 * Is + r7) * kLdD + 32 * cq + 16 * np + 8 * (m8 >> 1)));
+        if (lvl) {
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            const int j = 16 * I + gq + 8 * (x & 1), i = 8 * Is + 2 * tq;
+            a[x] &= (level_pair_ok(i, j, lvl) ? 0x0000ffffu : 0u) | (level_pair_ok(i + 1, j, lvl) ? 0xffff0000u : 0u);
+          }
+        }
+        const uint32_t am[4] = {0u, 0u, a[2], a[3]};
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          float u[4] = {0.f, 0.f, 0.f, 0.f}, um[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_bf16(u, a, b[2 * x], b[2 * x + 1]);
+          mma_bf16(um, am, b[2 * x], b[2 * x + 1]);  // the part through M: its product with Y is dbeta's
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            float2 d = make_float2(0.f, 0.f);
+            if (!half || two) d = *reinterpret_cast<const float2*>(sStrip + (tri + half) * kD + c + 8 * x);
+            const float2 Y = unpack_bf16(pack_bf16(y[x][half].x * d.x, y[x][half].y * d.y));
+            const float u0 = u[2 * half], u1 = u[2 * half + 1];
+            w[x][2 * half] += d.x * u0;
+            w[x][2 * half + 1] += d.y * u1;
+            dG[0][2 * np + x][2 * half] -= Y.x * u0;
+            dG[0][2 * np + x][2 * half + 1] -= Y.y * u1;
+            rb[half] += Y.x * um[2 * half] + Y.y * um[2 * half + 1];
+          }
+        }
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int j = 16 * I + gq + 8 * half, ref = lvl ? (j & ~(2 * lvl - 1)) + lvl : (j & ~7) + zo;
+        if (lvl && (j & lvl)) continue;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float2 g = *reinterpret_cast<const float2*>(sG + j * kLdG + c + 8 * x);
+          const float2 gr = *reinterpret_cast<const float2*>(sG + ref * kLdG + c + 8 * x);
+          dKt[0][2 * np + x][2 * half] += ex2(gr.x - g.x) * w[x][2 * half];
+          dKt[0][2 * np + x][2 * half + 1] += ex2(gr.y - g.y) * w[x][2 * half + 1];
+        }
+      }
     }
     __syncthreads();
+    if (!by_level || lvl == 1) break;
+    lvl = lvl ? lvl >> 1 : 4;
   }
   // ungated diagonal of P
 #pragma unroll
-  for (int nt = 0; nt < 4; ++nt)
+  for (int half = 0; half < 2; ++half) {
+    const int i = 16 * I + gq + 8 * half;
+    const float d = sDiag[i];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = 16 * I + gq + 8 * (e >> 1), c = 32 * cq + 8 * nt + 2 * tq + (e & 1);
-      const float d = to_f(sdP[i * kLdC + i]);
-      dQ[0][nt][e] += d * to_f(sKt[i * kLdD + c]);
-      dKt[0][nt][e] += d * to_f(sQ[i * kLdD + c]);
+    for (int nt = 0; nt < 4; ++nt) {
+      const int at = i * kLdD + 32 * cq + 8 * nt + 2 * tq;
+      const float2 qv = unpack_bf16(*reinterpret_cast<const uint32_t*>(sQ + at));
+      const float2 ktv = unpack_bf16(*reinterpret_cast<const uint32_t*>(sKt + at));
+      dQ[0][nt][2 * half] += d * ktv.x;
+      dQ[0][nt][2 * half + 1] += d * ktv.y;
+      dKt[0][nt][2 * half] += d * qv.x;
+      dKt[0][nt][2 * half + 1] += d * qv.y;
     }
+  }
   // dbeta: direct part + <kt_j, dkt_j(M path)> / beta_j
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
@@ -697,7 +825,7 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   // ... then the gate's own backward, elementwise over the tile with all threads:
   //   g = -exp(A_log) softplus(raw + bias);  draw = dg * (-exp(A_log)) sigmoid(raw + bias)
   // Per-thread partial sums (dA_log: scalar; ddt_bias: per channel) are reduced in a fixed order.
-  float* sPart = sFac;  // [32][kLdG] per-(row group, channel) partials of ddt_bias (the factors are dead)
+  float* sPart = sY;  // [32][kLdG] per-(row group, channel) partials of ddt_bias (y is dead)
   {
     const float ea = __expf(p.A_log[h]);
     float pa = 0.f;

@@ -59,14 +59,14 @@ constexpr int oEnd = oL + 4096;             // f32 [8][128] per-strip end value 
 constexpr int oDec = oL + 8192;             // f32 [8] per-strip product of preconditioner decays
 constexpr int oSum = oDec + 32;             // f32 [8] per-strip sum of the preconditioner's log-decays
 constexpr int oA0 = oSum + 32;              // f32 [128] the chunk-entry preconditioner state (chained mode)
-constexpr int oZ6 = oL + 9216;              // f32 [8][128] G of row 6 of every strip
+constexpr int oZin = oL + 9216;             // f32 [8][128] G of the inner column reference of every strip
 // between those and the products, the strip's own factors where its rows of P come later: strip w, 2 x f32 [128]
 constexpr int oD0 = oP, oD1 = oP + 512;     // + 1024 w
 // while the inverse runs: T in the (dead) write-key operand, its scratch in the (dead) q rows of block 0
 constexpr int oT = oY;                      // f32 [64][68]
 constexpr int oY2 = oA + 8192;              // f32 [1280]
 static_assert(oG + 32768 == oP && oBar % 8 == 0, "the decays fill what lies between the write keys and P");
-static_assert(oA0 + 512 <= oZ6 && oZ6 + 4096 <= oBeta && oT + 64 * kLdL * 4 <= oV && oY2 + 5120 <= oA + 16384, "aliases must fit");
+static_assert(oA0 + 512 <= oZin && oZin + 4096 <= oBeta && oT + 64 * kLdL * 4 <= oV && oY2 + 5120 <= oA + 16384, "aliases must fit");
 static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs per SM");
 constexpr uint32_t kCols = 256;             // pair accumulator 0..63, W^T 64..127, U^T 128..191
 }  // namespace intratc
@@ -113,12 +113,11 @@ __global__ void __launch_bounds__(256) pkda_chain_init_kernel(uint4* a_chain, si
 // the first factor is in the A operand, staged once per strip; kt times the third is kept in fp32, and a warp
 // multiplies it with the second, one number per channel and strip pair, and rounds the product to the B operand.
 // x(I) is the strip's first row and z(J) its last, so every factor of two strips is <= 1; inside a strip the second one is
-// 2^(decay of 7 tokens), which kDirectLimit bounds.  Strips that decay by more take their second and their last but one row (5
-// tokens; the outer tokens' factors are then > 1, at most 2^kOuter, and what rounds to zero is below 2^(2 kOuter - 126)).  Chunks
-// beyond that go through pair_exact.  A strip pair costs 11 instructions per 16 channels and no exponential;
+// 2^(decay of 7 tokens), which kDirectLimit bounds.  Strips that decay by more take their third row and the third from the
+// end (kDirectLimit then bounds the decay of 5 tokens, kOuterLimit that of the outer two, whose factors are > 1: nothing inside a
+// strip is lost, and of two strips nothing above 2^(2 kOuterLimit - 126)).  Chunks beyond that go through pair_exact.  A strip pair costs 11 instructions per 16 channels and no exponential;
 // gating both fragments from G by exponentials took 66, and with them the pairs were 10,000 of the 34,000 cycles of an
 // item alone on its SM instead of 4,500 (2,048 chunks: 182 us instead of 164).
-constexpr float kOuter = 32.f;
 struct PairLane {
   uint32_t a_row, s_row, s_blk, a_x, b_row, b_x, g_x;
   int g, t;
@@ -519,7 +518,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   // totals of its four channels, the CTA all 128.)  If so, which reference rows do its strips take?
   const bool by_strip =
       __syncthreads_or(-fminf(fminf(Glast[0], Glast[1]), fminf(Glast[2], Glast[3])) > kDirectLimit) || p.by_strip;
-  int refs = 0;  // 0: first and last row, 1: second and last but one, 2: pair_exact
+  int refs = 0;  // 0: first and last row, 1: kInnerRow from either end, 2: pair_exact
   if (!kRecompute) {
     if (!by_strip) {
       if (tid == 0) request_v();
@@ -528,11 +527,12 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         all = fmaxf(all, G[0][e] - G[7][e]);
-        mid = fmaxf(mid, G[1][e] - G[6][e]);
-        outer = fmaxf(outer, fmaxf(G[0][e] - G[1][e], G[6][e] - G[7][e]));
+        mid = fmaxf(mid, fmaxf(G[0][e] - G[7 - kInnerRow][e], G[kInnerRow][e] - G[7][e]));
+        outer = fmaxf(outer, fmaxf(G[0][e] - G[kInnerRow][e], G[7 - kInnerRow][e] - G[7][e]));
       }
-      *reinterpret_cast<float4*>(tiles + oZ6 + warp * 512 + (lane << 4)) = make_float4(G[6][0], G[6][1], G[6][2], G[6][3]);
-      if (__syncthreads_or(all > kDirectLimit)) refs = 1 + (__syncthreads_or(mid > kDirectLimit || outer > kOuter) != 0);
+      constexpr int kz = 7 - kInnerRow;
+      *reinterpret_cast<float4*>(tiles + oZin + warp * 512 + (lane << 4)) = make_float4(G[kz][0], G[kz][1], G[kz][2], G[kz][3]);
+      if (__syncthreads_or(all > kDirectLimit)) refs = 1 + (__syncthreads_or(mid > kDirectLimit || outer > kOuterLimit) != 0);
       if (p.direct_cap < 8) refs = 2;
     }
   }
@@ -567,7 +567,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     if (!kRecompute && by_strip && refs < 2) {
       float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);  // z of the strip before
       if (refs) {
-        if (warp) prev = *reinterpret_cast<const float4*>(tiles + oZ6 + (warp - 1) * 512 + (lane << 4));
+        if (warp) prev = *reinterpret_cast<const float4*>(tiles + oZin + (warp - 1) * 512 + (lane << 4));
       } else {
         for (int wp = 0; wp < warp; ++wp) {
           const float4 to = *reinterpret_cast<const float4*>(sTot + wp * kD + c4);
@@ -576,8 +576,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        zr[c] = refs ? G[6][c] : G[7][c];
-        xr[c] = refs ? G[1][c] : G[0][c];
+        zr[c] = refs ? G[7 - kInnerRow][c] : G[7][c];
+        xr[c] = refs ? G[kInnerRow][c] : G[0][c];
       }
       unsigned char* at = tiles + warp * 1024 + (lane << 4);
       *reinterpret_cast<float4*>(at + oD0) = make_float4(ex2(xr[0] - zr[0]), ex2(xr[1] - zr[1]), ex2(xr[2] - zr[2]), ex2(xr[3] - zr[3]));
