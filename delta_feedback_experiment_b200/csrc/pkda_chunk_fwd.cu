@@ -416,11 +416,13 @@ static FwdWorkspace carve_fwd(const pkda_problem& p, void* base) {
 size_t chunk_fwd_workspace(const pkda_problem& p) { return carve_fwd(p, nullptr).bytes; }
 
 bool forward_chain_possible(const pkda_problem& p) {
-  // With few (row, head) units the chains are few and long compared with the number of items in
-  // flight, and an item waits for many hand-overs: measured break-even near 32 units (the state it
-  // yields is the same bit for bit either way).
-  return !p.cu_seqlens && stage_variant(kStageIntraFwd) == 0 && direct_block_cap() >= 64 &&
-         (long)p.n_seqs * p.heads >= 32;
+  if (p.cu_seqlens || stage_variant(kStageIntraFwd) != 0 || direct_block_cap() < 64) return false;
+  // A hand-over from one chunk of a chain to the next takes about 0.6 us, an item 0.05 us of the chip: with a dozen
+  // (row, head) units side by side the hand-overs hide, and the two kernels in front of the intra stage, which it
+  // spares, make up for it down to 8 (16 units of 8,191 tokens 176 -> 164 us, 8 of 8,192 110 -> 94, 8 of 16,384 156 -> 147);
+  // of fewer units, short rows only.  The state is the same bit for bit either way.  (A packed batch goes sequence after
+  // sequence, a chain per head side by side: 65,536 tokens of 32 heads 1,740 -> 1,731 us, of 12 heads 682 -> 768.)
+  return (long)p.n_seqs * p.heads >= 8 || p.seq_len <= 24 * kChunk;
 }
 size_t chunk_fwd_status_offset(const pkda_problem& p) {
   return (size_t)(reinterpret_cast<unsigned char*>(carve_fwd(p, nullptr).status) - static_cast<unsigned char*>(nullptr));
