@@ -139,6 +139,12 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
   return __bfloat1622float2(v);
 }
 
+// Packed fp32x2 arithmetic (two values per instruction).
+__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+
 // ---------------------------------------------------------------- warp MMA (bf16, fp32 accumulate)
 // Row stride padding (in bf16 elements) that makes 8 consecutive rows of an
 // ldmatrix land on distinct 16-byte bank groups.

@@ -22,11 +22,11 @@
 //   (1) dR^T  = dF^T (diag(beta) T)                      K = 64    -> dv, and rows 0..63 of the stack
 //   (2) [dR; dO] E^T                                     K = 128   -> dM = -tril(.,-1) diag(beta),
 //                                                                     dP = scale tril(.) diag(beta)
-//       Qs = S0 dO^T, Ks = -S0 dR^T, Kts = dS1 E^T       K = 128   (state-coupled parts)
+//       [Ks; Qs] = S0 [dR; dO]^T, Kts = dS1 E^T           K = 128   (state-coupled parts)
 //   (3) Qp = Y^T dP^T, Kp = Y^T dM^T, KtM = Xk^T dM, KtP = Xq^T dP   K = 64 (pair parts)
-//   dq  = 2^G (scale Qs + Qp)      dk_read = 2^G (Ks + Kp)
+//   dq  = 2^G (scale Qs + Qp)      dk_read = 2^G (Kp - Ks)
 //   dkt = 2^-G (2^G_last beta Kts + KtM + KtP)
-//   dG  = Xq (scale Qs + Qp) + Xk (Ks + Kp) - Y (2^G_last beta Kts + KtM + KtP)
+//   dG  = Xq (scale Qs + Qp) + Xk (Kp - Ks) - Y (2^G_last beta Kts + KtM + KtP)
 // with Xq = bf16(q 2^G), Xk = bf16(k 2^G), Y = bf16(kt 2^-G) the very operands of the products, so
 // that the two sides of every pair cancel under the reverse cumulative sum.
 //
@@ -68,7 +68,11 @@ constexpr int oX5 = oDM + 4096;         // f32 [4][128] slice sums of the raw-ga
 constexpr int oDb = oDM + 6144;         // f32 [4][64] per lane-quarter partial sums of dbeta
 constexpr int oX6 = oDP;                // f32 [4][128] slice sums of the preconditioner's outgoing carry
 constexpr uint32_t kCols = 512;
-constexpr uint32_t cR = 0, cStk = 64, cQs = 128, cKs = 192, cKts = 256, cKtM = 320, cKtP = 384;  // cR / cStk later Qp / Kp
+constexpr uint32_t cR = 0, cStk = 64, cKs = 128, cQs = 192, cKts = 256, cKtM = 320, cKtP = 384;
+constexpr uint32_t cKp = 0, cQp = 64;   // later, in the place of cR and cStk
+// Pairs of products with the same A operand are one product with both B operands, 128 rows one after the other (a product
+// holds up the warp that issues it while the unit is busy; 40 of them an item instead of 52: 678 -> 670 us for 8,192 items):
+static_assert(cQs == cKs + 64 && cQp == cKp + 64 && oDP == oDM + 8192, "B = [dR; dO], and B = [dM; dP]");
 }  // namespace ibtc
 
 // One bf16 element of shared memory by its 32-bit shared address (register + immediate addressing).
@@ -227,7 +231,8 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
   const volatile int2* s_next = reinterpret_cast<const volatile int2*>(tiles + oBar + 56);
   int2 cur = p.fast_list[blockIdx.x];
   request(cur);
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tiles + oBar + 48);
+  const uint32_t tmem = tc::uniform(*reinterpret_cast<volatile uint32_t*>(tiles + oBar + 48));
+  const int warp_u = (int)tc::uniform(warp);
   bool ok = true;
   uint32_t m_phase = 0, ld_phase = 0;
   // per-item scalars of this thread, fetched one item ahead: 2^G_last of its channel, the gate bias, A_log
@@ -263,8 +268,7 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
   }
   // The operand descriptors are functions of the tile base only; keeping the base opaque per item
   // stops the compiler from computing all sixty of them ahead of the loop and holding them in registers.
-  uint32_t dbase = base;
-  asm volatile("" : "+r"(dbase));
+  const uint32_t dbase = tc::uniform(base);
 
   // ---- 1. T <- diag(beta) T (row j scaled by beta_j: the beta of dE = beta dF moves onto T), then dR^T
   ok = tc::mbar_wait(barB, ld_phase) && ok;
@@ -283,7 +287,7 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
   }
   tc::fence_proxy_async();
   __syncthreads();
-  if (tid == 0) {
+  if (warp_u == 0 && tc::elect_one()) {
     tc::tc_fence_after();
     constexpr uint32_t idesc = tc::idesc_bf16(128, 64, true, true);
 #pragma unroll
@@ -321,17 +325,12 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
     for (int t = 0; t < 16; ++t) G[t] += pre;
     G_before = pre;
   }
-  // the state-coupled products that need nothing but landed tiles
+  // the state-coupled product that needs nothing but landed tiles
   ok = tc::mbar_wait(barC, ld_phase) && ok;
   ld_phase ^= 1;
-  if (tid == 0) {
+  if (warp_u == 0 && tc::elect_one()) {
     tc::tc_fence_after();
     constexpr uint32_t idesc = tc::idesc_bf16(128, 64, false, false);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      const uint32_t ko = (kk >> 2) * 16384 + (kk & 3) * 32;
-      tc::umma_bf16(tmem + cQs, tc::desc_kmajor(dbase + oS0 + ko), tc::desc_kmajor(dbase + oStk + 8192 + ko), idesc, kk > 0);
-    }
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
       const uint32_t ko = (kk >> 2) * 16384 + (kk & 3) * 32, ke = (kk >> 2) * 8192 + (kk & 3) * 32;
@@ -353,22 +352,24 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
   tc::fence_proxy_async();
   tc::tc_fence_before();
   __syncthreads();
-  if (tid == 0) {
-    tc::tc_fence_after();
+  if (tid == 32) {
     tc::tma_store_3d(&maps.dv, base + oStk, 0, h, tok0);
     tc::tma_store_3d(&maps.dv, base + oStk + 16384, 64, h, tok0);
     tc::bulk_commit();
+  }
+  if (warp_u == 0 && tc::elect_one()) {
+    tc::tc_fence_after();
     constexpr uint32_t idesc = tc::idesc_bf16(128, 64, false, false);
-    constexpr uint32_t idesc_neg = idesc | (1u << 13);  // A negated
+    constexpr uint32_t idesc2 = tc::idesc_bf16(128, 128, false, false);
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {  // [dR; dO] E^T
       const uint32_t ko = (kk >> 2) * 16384 + (kk & 3) * 32, ke = (kk >> 2) * 8192 + (kk & 3) * 32;
       tc::umma_bf16(tmem + cStk, tc::desc_kmajor(dbase + oStk + ko), tc::desc_kmajor(dbase + oE + ke), idesc, kk > 0);
     }
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {  // -S0 dR^T
+    for (int kk = 0; kk < 8; ++kk) {  // S0 [dR; dO]^T
       const uint32_t ko = (kk >> 2) * 16384 + (kk & 3) * 32;
-      tc::umma_bf16(tmem + cKs, tc::desc_kmajor(dbase + oS0 + ko), tc::desc_kmajor(dbase + oStk + ko), idesc_neg, kk > 0);
+      tc::umma_bf16(tmem + cKs, tc::desc_kmajor(dbase + oS0 + ko), tc::desc_kmajor(dbase + oStk + ko), idesc2, kk > 0);
     }
     tc::umma_commit(barM);
   }
@@ -376,12 +377,18 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
   // ---- 3b. while those run: the operands gated in place; sum_v S0 dS1 per channel
   {
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      const float e = ex2(G[t]), ei = __fdividef(1.f, e);
-      const uint32_t a0 = sa[t & 7] + 128 * t;
-      sts_bf16(a0 + oQ, lds_bf16(a0 + oQ) * e);
-      sts_bf16(a0 + oK, lds_bf16(a0 + oK) * e);
-      sts_bf16(a0 + oKt, lds_bf16(a0 + oKt) * ei);
+    for (int t = 0; t < 16; t += 2) {
+      const float2 e = f2(ex2(G[t]), ex2(G[t + 1])), ei = f2(__fdividef(1.f, e.x), __fdividef(1.f, e.y));
+      const uint32_t a0 = sa[t & 7] + 128 * t, a1 = sa[(t + 1) & 7] + 128 * (t + 1);
+      const float2 xq = mul2(f2(lds_bf16(a0 + oQ), lds_bf16(a1 + oQ)), e);
+      const float2 xk = mul2(f2(lds_bf16(a0 + oK), lds_bf16(a1 + oK)), e);
+      const float2 y = mul2(f2(lds_bf16(a0 + oKt), lds_bf16(a1 + oKt)), ei);
+      sts_bf16(a0 + oQ, xq.x);
+      sts_bf16(a1 + oQ, xq.y);
+      sts_bf16(a0 + oK, xk.x);
+      sts_bf16(a1 + oK, xk.y);
+      sts_bf16(a0 + oKt, y.x);
+      sts_bf16(a1 + oKt, y.y);
     }
     // channel c's row of both state tiles, values 32 sl .. 32 sl + 31 (four 16-byte pieces of one K block)
     const unsigned char* rs = tiles + oS0 + (sl >> 1) * 16384 + c * 128;
@@ -430,19 +437,20 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
   tc::fence_proxy_async();  // also covers the gated operands written in step 2
   tc::tc_fence_before();
   __syncthreads();
-  if (tid == 0) {
-    tc::tc_fence_after();
+  if (tid == 32) {
     // the raw k tile comes back into the (dead) entry-state tile for the preconditioner's backward
     tc::mbar_expect_tx(barK, 16384);
     tc::tma_load_3d(base + oS0, &maps.k, barK, 0, h, tok0);
     tc::tma_load_3d(base + oS0 + 8192, &maps.k, barK, 64, h, tok0);
-    constexpr uint32_t idesc_k = tc::idesc_bf16(128, 64, true, false);  // B = pair gradient as [i][j], K = j
+  }
+  if (warp_u == 0 && tc::elect_one()) {
+    tc::tc_fence_after();
+    constexpr uint32_t idesc_k = tc::idesc_bf16(128, 128, true, false);  // B = pair gradients as [i][j], K = j
     constexpr uint32_t idesc_m = tc::idesc_bf16(128, 64, true, true);   // B = pair gradient read as [j][i], K = i
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
-      const uint64_t ay = tc::desc_mnmajor(dbase + oKt + kk * 2048, 8192);
-      tc::umma_bf16(tmem + cR, ay, tc::desc_kmajor(dbase + oDP + kk * 32), idesc_k, kk > 0);    // Qp = Y^T dP^T
-      tc::umma_bf16(tmem + cStk, ay, tc::desc_kmajor(dbase + oDM + kk * 32), idesc_k, kk > 0);  // Kp = Y^T dM^T
+      tc::umma_bf16(tmem + cKp, tc::desc_mnmajor(dbase + oKt + kk * 2048, 8192), tc::desc_kmajor(dbase + oDM + kk * 32), idesc_k,
+                    kk > 0);  // [Kp; Qp] = Y^T [dM; dP]^T
     }
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
@@ -493,57 +501,81 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
     float* pkt = p.dkt + out0;
     float A = A_in, w = w_in;
     float dbv[8];
+    // Two tokens at a time on the packed fp32x2 instructions: of the 75 instructions a token took here, 30 less (684 -> 679 us
+    // for 8,192 items: the epilogue is half bound by the special-function unit)
+    float2 kds = f2(0.f, 0.f), dcs = f2(0.f, 0.f), cls = f2(0.f, 0.f);
+    const float2 gl2 = f2(gl, gl), sc2 = f2(p.scale, p.scale), eps2 = f2(p.eps, p.eps), nlnx2 = f2(-p.ln_x, -p.ln_x);
+    const float nlnx_l2e = -p.ln_x * kLog2e;
 #pragma unroll
     for (int qq = 0; qq < 4; ++qq) {  // four tokens at a time: all seven accumulator pieces of a token in one pass
       const uint32_t ta = tmem + lane_addr + j0 + 4 * qq;
       float aQ[4], bR[4], aK[4], bS[4], m[4], bP[4], aT[4];
       tc::tmem_ld4(ta + cQs, aQ);
-      tc::tmem_ld4(ta + cR, bR);
+      tc::tmem_ld4(ta + cQp, bR);
       tc::tmem_ld4(ta + cKs, aK);
-      tc::tmem_ld4(ta + cStk, bS);
+      tc::tmem_ld4(ta + cKp, bS);
       tc::tmem_ld4(ta + cKtM, m);
       tc::tmem_ld4(ta + cKtP, bP);
       tc::tmem_ld4(ta + cKts, aT);
       tc::tmem_ld_wait();
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 4; u += 2) {
         const int t = 4 * qq + u;
-        const uint32_t a0 = sa[t & 7] + 128 * t;
-        const float e = ex2(G[t]);
-        const float totq = p.scale * aQ[u] + bR[u];
-        const float xq = lds_bf16(a0 + oQ);
-        *pq = __float2bfloat16(e * totq);
+        const uint32_t a0 = sa[t & 7] + 128 * t, a1 = sa[(t + 1) & 7] + 128 * (t + 1);
+        const float2 e = f2(ex2(G[t]), ex2(G[t + 1]));
+        const float2 totq = fma2(sc2, f2(aQ[u], aQ[u + 1]), f2(bR[u], bR[u + 1]));
+        const float2 xq = f2(lds_bf16(a0 + oQ), lds_bf16(a1 + oQ));
+        const float2 dq = mul2(e, totq);
+        *pq = __float2bfloat16(dq.x);
         pq += gld;
-        const float totk = aK[u] + bS[u];
-        const float xk = lds_bf16(a0 + oK);
-        const float dkr = e * totk;
+        *pq = __float2bfloat16(dq.y);
+        pq += gld;
+        const float2 totk = add2(f2(-aK[u], -aK[u + 1]), f2(bS[u], bS[u + 1]));
+        const float2 xk = f2(lds_bf16(a0 + oK), lds_bf16(a1 + oK));
+        const float2 dkr = mul2(e, totk);
         // write-key gradient; the part of dbeta that flows through M (rows of KtM against Y)
-        const float bj = sBeta[j0 + t];
-        const float y = lds_bf16(a0 + oKt);
-        const float df = lds_bf16(a0 + oDF);
-        const float ev = lds_bf16(a0 + oE);
-        dbv[4 * (qq & 1) + u] = df * ev + y * m[u] * sBinv[j0 + t];
-        const float st = gl * bj * aT[u], pr = m[u] + bP[u];
-        const float dkt = __fdividef(st + pr, e);
-        const float kd = y * st;
-        dGv[t] = xq * totq + xk * totk - (y * pr + kd);
-        kdsum += kd;
+        const float2 y = f2(lds_bf16(a0 + oKt), lds_bf16(a1 + oKt));
+        const float2 df = f2(lds_bf16(a0 + oDF), lds_bf16(a1 + oDF));
+        const float2 ev = f2(lds_bf16(a0 + oE), lds_bf16(a1 + oE));
+        const float2 mm = f2(m[u], m[u + 1]);
+        const float2 db = fma2(df, ev, mul2(mul2(y, mm), *reinterpret_cast<const float2*>(sBinv + j0 + t)));
+        dbv[4 * (qq & 1) + u] = db.x;
+        dbv[4 * (qq & 1) + u + 1] = db.y;
+        const float2 st = mul2(mul2(gl2, *reinterpret_cast<const float2*>(sBeta + j0 + t)), f2(aT[u], aT[u + 1]));
+        const float2 pr = add2(mm, f2(bP[u], bP[u + 1]));
+        const float2 dkt = mul2(add2(st, pr), f2(__fdividef(1.f, e.x), __fdividef(1.f, e.y)));
+        const float2 kd = mul2(y, st);
+        const float2 yp = fma2(y, pr, kd);
+        const float2 dg = fma2(yp, f2(-1.f, -1.f), fma2(xq, totq, mul2(xk, totk)));
+        dGv[t] = dg.x;
+        dGv[t + 1] = dg.y;
+        kds = add2(kds, kd);
         // the preconditioner: A_t, the factor B(A_t) and its derivative (pkda_atk_bwd_kernel has the same math)
-        const float kc = lds_bf16(a0 + oS0);
-        const float pd = sPd[j0 + t];
-        A = pd * A + sBp[j0 + t] * kc * kc;
-        w *= pd;
-        const float dev = __logf(A + p.eps) - centre;
-        const float rden = __fdividef(1.f, 1.f + fabsf(dev));
-        const float Bf = __expf(-p.ln_x * dev * rden);
-        const float ddev = -p.ln_x * dkt * kc * Bf * rden * rden;
-        const float dA = __fdividef(ddev, A + p.eps);
-        *pkt = dA;
+        const float2 kc = f2(lds_bf16(a0 + oS0), lds_bf16(a1 + oS0));
+        const float2 pd = *reinterpret_cast<const float2*>(sPd + j0 + t);
+        const float2 in = mul2(mul2(*reinterpret_cast<const float2*>(sBp + j0 + t), kc), kc);
+        const float A0 = pd.x * A + in.x;
+        A = pd.y * A0 + in.y;
+        const float w0 = w * pd.x;
+        w = w0 * pd.y;
+        const float2 Ae = add2(f2(A0, A), eps2);
+        const float2 dev = f2(__logf(Ae.x) - centre, __logf(Ae.y) - centre);
+        const float2 rden = f2(__fdividef(1.f, 1.f + fabsf(dev.x)), __fdividef(1.f, 1.f + fabsf(dev.y)));
+        const float2 sq = mul2(mul2(dev, rden), f2(nlnx_l2e, nlnx_l2e));
+        const float2 Bf = f2(ex2(sq.x), ex2(sq.y));
+        const float2 ddev = mul2(mul2(mul2(nlnx2, mul2(dkt, kc)), Bf), mul2(rden, rden));
+        const float2 dA = mul2(ddev, f2(__fdividef(1.f, Ae.x), __fdividef(1.f, Ae.y)));
+        *pkt = dA.x;
         pkt += gld;
-        *pk = dkr + dkt * Bf;
+        *pkt = dA.y;
+        pkt += gld;
+        const float2 dk = fma2(dkt, Bf, dkr);
+        *pk = dk.x;
         pk += gld;
-        dcen -= ddev;
-        cloc += w * dA;
+        *pk = dk.y;
+        pk += gld;
+        dcs = add2(dcs, ddev);
+        cls = fma2(f2(w0, w), dA, cls);
       }
       if (qq & 1) {
         row_sums8(dbv, lane);
@@ -551,6 +583,9 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
           sDb[q4 * kChunk + j0 + 8 * (qq >> 1) + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = dbv[0];
       }
     }
+    kdsum = kds.x + kds.y;
+    cloc = cls.x + cls.y;
+    dcen = -(dcs.x + dcs.y);
     float tot = 0.f;
 #pragma unroll
     for (int t = 0; t < 16; ++t) tot += dGv[t];
@@ -620,8 +655,8 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
 #pragma unroll
     for (int w = 0; w < kThreads / 32; ++w) accc += sRed[16 + w];
     p.partC[chh] = accc;
-    tc::bulk_wait_read();  // the dv store has read the stack rows the next item's dR overwrites
   }
+  if (tid == 32) tc::bulk_wait_read();  // the dv store has read the stack rows the next item's dR overwrites
   __syncthreads();  // the exchange arrays and beta are rewritten by the next item
   }  // item loop
   if (__syncthreads_or(!ok) && tid == 0) atomicExch(p.status, 1);

@@ -299,7 +299,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tiles + oBar + 16);
+  const uint32_t tmem = tc::uniform(*reinterpret_cast<volatile uint32_t*>(tiles + oBar + 16));
+  const int warp_u = (int)tc::uniform(warp);
   bool ok = true;
   uint32_t ph = 0;  // bit 0: bar_mma, 1: bar_tma, 2: bar_in
 
@@ -377,8 +378,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   const bool full = valid == kChunk;
   // The operand descriptors depend on the tile base only; keeping the base opaque per item stops the
   // compiler from computing all of them ahead of the loop and holding them in registers.
-  uint32_t dbase = base;
-  asm volatile("" : "+r"(dbase));
+  const uint32_t dbase = tc::uniform(base);
 
   // ---- 0. V (and T when recomputing) by TMA; the strips of g, k and q are on their way into their operand slots
   auto request_v = [&]() {  // thread 0, when its stores from there are done
@@ -698,7 +698,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     for (int J = warp + 1 + (lane >> 3); J < 8; J += 4)
       *reinterpret_cast<uint4*>(tiles + oP + (r0 + (lane & 7)) * 128 + ((J ^ (lane & 7)) << 4)) = make_uint4(0, 0, 0, 0);
   } else if (!kRecompute) {
-    if (tid == 0) {
+    if (warp_u == 0 && tc::elect_one()) {
       tc::tc_fence_after();
       constexpr uint32_t idesc_pair = tc::idesc_bf16(128, 64, false, false);
 #pragma unroll
@@ -810,12 +810,12 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   if (nx.x >= 0) {
     if (tid == 32) request_g(nx);
   }
-  if (tid == 0) {
+  if (!kRecompute && full && tid == 0) {
+    tc::tma_store_3d(&tm_akk, base + oTm, 0, h, tok0);
+    tc::bulk_commit();
+  }
+  if (warp_u == 2 && tc::elect_one()) {  // (warp 0 stores T, warp 1 asks for the next gate)
     tc::tc_fence_after();
-    if (!kRecompute && full) {
-      tc::tma_store_3d(&tm_akk, base + oTm, 0, h, tok0);
-      tc::bulk_commit();
-    }
     constexpr uint32_t idesc = tc::idesc_bf16(128, 64, /*a_mn_major=*/true, /*b_mn_major=*/false);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)

@@ -54,12 +54,6 @@ struct ConvParams {
   float* part;  // [gridDim.y][channels][taps]
 };
 
-// Packed fp32x2 arithmetic (two channels per instruction).
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-
 // Four adjacent channels as two pairs.
 template <typename T> struct Vec4;
 template <> struct Vec4<bf16> {

@@ -81,7 +81,8 @@ pkda_scan_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_kg, const __grid_
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tiles + oBar + 48);
+  const uint32_t tmem = tc::uniform(*reinterpret_cast<volatile uint32_t*>(tiles + oBar + 48));
+  const int warp_u = (int)tc::uniform(warp);
   const uint32_t tS = tmem + ((uint32_t)(32 * q) << 16);       // this warp's lanes, dS columns
   const uint32_t tF = tS + 128;                                 // dF^T accumulator columns
 
@@ -187,7 +188,7 @@ pkda_scan_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_kg, const __grid_
       tc::tma_store_2d(&tm_dh, base + oD + (warp - 1) * 16384, 64 * (warp - 1), (int)(chh * kD));
       tc::bulk_commit();
     }
-    if (tid == 0) {
+    if (warp_u == 0 && tc::elect_one()) {
       tc::tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {  // d^T kg^T
@@ -265,7 +266,7 @@ pkda_scan_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_kg, const __grid_
       tc::tma_store_3d(&tm_df, base + oF + (warp - 3) * 8192, 64 * (warp - 3), h, tok0);
       tc::bulk_commit();
     }
-    if (tid == 0) {
+    if (warp_u == 0 && tc::elect_one()) {
       tc::tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {  // dS += W^T dE

@@ -139,7 +139,8 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tiles + oBar + 48);
+  const uint32_t tmem = tc::uniform(*reinterpret_cast<volatile uint32_t*>(tiles + oBar + 48));
+  const int warp_u = (int)tc::uniform(warp);
   bool ok = true;
 
   if (kOut && warp >= kThreads / 32) {
@@ -161,7 +162,7 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
     // P; it queues the second product when E stands; all four warps read the accumulator and stage o.
     // The issuing thread's own warp does nothing else while it waits (a lane that spins holds up the
     // other lanes of its warp), and nobody but that thread polls the scan's signals.
-    const bool issuer_warp = (e >> 5) == 1;
+    const bool issuer_warp = tc::uniform(e >> 5) == 1;
     const int sc = e < 32 ? e : e - 32;  // 0..95 among the threads that scale P
     float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = b0;  // beta of this thread's eight columns of P, one chunk ahead
     if (sq.nchunks > 0 && !issuer_warp) {
@@ -181,14 +182,15 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
           // the other buffer was last read by the products of chunk i - 1, which this thread saw complete
           if (i + 1 < sq.nchunks) fetch(i + 1);
           ok = tc::mbar_wait(bar_hready, i & 1) && ok;  // h of this chunk stands in its tile
-          if (ok) {
-            tc::tc_fence_after();  // (the accumulator is free: all four warps read it before the barrier after the read)
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok && tc::elect_one()) {
+          tc::tc_fence_after();  // (the accumulator is free: all four warps read it before the barrier after the read)
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-              tc::umma_bf16(tmem + 192, tc::desc_mnmajor(base + oH + kk * 2048, 16384),
-                            tc::desc_kmajor(qp + (kk >> 2) * 8192 + (kk & 3) * 32), idesc_o, kk > 0);
-            tc::umma_commit(bar_o1);
-          }
+          for (int kk = 0; kk < 8; ++kk)
+            tc::umma_bf16(tmem + 192, tc::desc_mnmajor(base + oH + kk * 2048, 16384),
+                          tc::desc_kmajor(qp + (kk >> 2) * 8192 + (kk & 3) * 32), idesc_o, kk > 0);
+          tc::umma_commit(bar_o1);
         }
         __syncwarp();
       } else {
@@ -210,17 +212,18 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
         tc::fence_proxy_async();
       }
       if (out_sync_or(!ok)) { ok = false; break; }
-      if (issuer) {
-        ok = tc::mbar_wait(bar_eready, i & 1) && ok;  // E of this chunk stands in its tile
-        if (ok) {
+      if (issuer_warp) {
+        if (issuer) ok = tc::mbar_wait(bar_eready, i & 1) && ok;  // E of this chunk stands in its tile
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok && tc::elect_one()) {
           tc::tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             tc::umma_bf16(tmem + 192, tc::desc_mnmajor(base + oE + kk * 2048, 8192),
                           tc::desc_kmajor(qp + 16384 + kk * 32), idesc_o, 1);
           tc::umma_commit(bar_o);
-          ok = tc::mbar_wait(bar_o, i & 1) && ok;
         }
+        if (issuer && ok) ok = tc::mbar_wait(bar_o, i & 1);
       }
       if (out_sync_or(!ok)) { ok = false; break; }
       tc::tc_fence_after();
@@ -352,7 +355,7 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
       tc::tma_store_2d(&tm_h, base + oH + (warp - 1) * 16384, 64 * (warp - 1), (int)(chh * kD));
       tc::bulk_commit();
     }
-    if (tid == 0) {
+    if (warp_u == 0 && tc::elect_one()) {
       tc::tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
@@ -424,7 +427,7 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
       tc::tma_store_3d(&tm_e, base + oE + (warp - 3) * 8192, 64 * (warp - 3), h, tok0);
       tc::bulk_commit();
     }
-    if (tid == 0) {
+    if (warp_u == 0 && tc::elect_one()) {
       tc::tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
