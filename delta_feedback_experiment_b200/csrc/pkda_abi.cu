@@ -292,7 +292,7 @@ int pkda_set_variant(const char* stage, int variant) {
 
 const char* pkda_stage_name(int stage) {
   static const char* names[] = {"chunk_offsets", "pack_beta", "atk_local", "atk_carry", "intra_fwd", "scan_fwd",
-                                "out_fwd", "scan_bwd", "intra_bwd", "atk_bwd_local", "atk_bwd_carry",
+                                "out_fwd", "scan_bwd", "intra_bwd", "atk_bwd_carry",
                                 "atk_bwd_final", "param_reduce", "recurrent", "qkv_conv_fwd", "qkv_conv_bwd",
                                 "qkv_conv_dw", "norm_gate_fwd", "norm_gate_bwd", "norm_gate_dw", "decode_step", "controls_fwd", "controls_bwd", "pack_control",
                                 "status_guard", "bwd_classify", "intra_bwd_rest"};

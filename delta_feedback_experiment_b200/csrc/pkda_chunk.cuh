@@ -348,8 +348,7 @@ struct IntraBwdParams {
   int use_tma;   // the five phase-A tiles of full chunks arrive by TMA (tensor maps valid)
   int out_tma;   // dq, dv, dk_read and dkt of full chunks leave by TMA from padded shared-memory tiles
   int* status;   // set to 1 if a bounded wait gives up
-  // The local part of the preconditioner's backward runs inside the tensor-memory kernel (the mma.sync
-  // kernel leaves it to pkda_atk_bwd_kernel<false>): with B the write-key factor kt = k B(A_t),
+  // The local part of the preconditioner's backward runs inside the chunk kernels: with B the write-key factor kt = k B(A_t),
   //   dkt buffer <- dA_local = d(loss)/dA_t through B alone,  dk_read buffer <- dk_read + dkt B,
   //   c_loc[chunk] = sum_r (prod_{j<=r} decay_j) dA_local_r,  partC[chunk] = d(loss)/d(centre).
   const float* g_atk;

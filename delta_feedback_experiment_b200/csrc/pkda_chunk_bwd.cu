@@ -237,6 +237,119 @@ static_assert(oBar % 8 == 0 && oA1 % 128 == 0 && oTm % 128 == 0 && oDE % 128 == 
               "TMA destinations and the mbarrier must be aligned");
 static_assert(oDR + kTileBytes <= oDP, "phase-A tiles must not reach the pair-gradient tiles");
 static_assert(oDE + kD * kLdD * 2 <= oDP, "dS1 tile must fit");
+// The preconditioner's part: what its row blocks exchange, in a region that is dead after the pairs.
+constexpr int kAtkBlocks = kThreads / 32, kAtkRows = kChunk / kAtkBlocks;  // one row block per warp
+constexpr int oAtkEx = oDP;    // f32: end[16][128] part[16][128] dec[16] centre[16]
+static_assert((2 * kAtkBlocks * kD + 2 * kAtkBlocks) * 4 <= 2 * kChunk * kLdC * 2,
+              "dead region");
+
+// ---- The local part of the preconditioner's backward, with the chunk's dkt and dk_read still in shared memory:
+//   dkt <- dA_local = d(loss)/dA_t through the write-key factor B alone,  dk_read <- dk_read + dkt B,
+//   the chunk's outgoing carry sum_r (prod_{j<=r} decay_j) dA_local_r and its share of the centre gradient.
+// Warp w owns rows 4 w .. 4 w + 3, lane l channels 4 l .. 4 l + 3, and the scan A_t = decay_t A_(t-1) + beta_t k_t^2 is
+// blocked: the row blocks exchange (decay product, end value).  Five special-function operations an element
+// (2,600 cycles of the unit per chunk), while the gradients' reverse sum runs on four of the warps.  Against a kernel of its own,
+// which read both gradients and k again and wrote the gradients a second time (225 MB in 37 us for 1,536 chunks): this kernel
+// 253 -> 281 us, the pass 838 -> 829 us.  (Plain row stores instead of TMA from the tiles: 284.)
+struct AtkIn {
+  uint2 k[kAtkRows];
+  float4 a0;      // the state in front of the chunk
+  float lg, beta; // of row lane % 4 of the warp's
+  float centre;
+};
+__device__ __forceinline__ void atk_request(AtkIn& a, const IntraBwdParams& p, size_t chh, int tok0, int valid, int h, int w,
+                                            int lane) {
+  const int r = kAtkRows * w + (lane & (kAtkRows - 1));
+  a.lg = a.beta = 0.f;  // rows past the end: decay 1, beta 0: the state passes through
+  if (r < valid) {
+    const size_t s = (size_t)(tok0 + r) * p.geo.heads + h;
+    a.lg = p.g_atk[s];
+    a.beta = __bfloat162float(p.beta_atk[s]);
+  }
+  a.centre = p.log_atk_scale[h];
+  a.a0 = *reinterpret_cast<const float4*>(p.a_start + chh * kD + 4 * lane);
+}
+// Before the barrier: the row block's end value from a zero start.
+__device__ __forceinline__ void atk_block_end(const AtkIn& in, int w, int lane, float* ex) {
+  const int c4 = 4 * lane;
+  const float pd_l = __expf(in.lg);
+  float A[4] = {0.f, 0.f, 0.f, 0.f}, dblk = 1.f;
+#pragma unroll
+  for (int i = 0; i < kAtkRows; ++i) {
+    const float2 x = unpack_bf16(in.k[i].x), y = unpack_bf16(in.k[i].y);
+    const float kc[4] = {x.x, x.y, y.x, y.y};
+    const float pd = __shfl_sync(0xffffffffu, pd_l, i), bp = __shfl_sync(0xffffffffu, in.beta, i);
+    dblk *= pd;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) A[e] = pd * A[e] + bp * kc[e] * kc[e];
+  }
+  *reinterpret_cast<float4*>(ex + w * kD + c4) = make_float4(A[0], A[1], A[2], A[3]);
+  if (lane == 0) ex[2 * kAtkBlocks * kD + w] = dblk;
+}
+// Behind it: the true states, the gradients.
+__device__ __forceinline__ void atk_local(const AtkIn& in, const IntraBwdParams& p, size_t row0, long gld, int valid, int w,
+                                          int lane, float* sOutKt, float* sOutK, float* ex, bool out_tma) {
+  const int r0 = kAtkRows * w, c4 = 4 * lane;
+  const float pd_l = __expf(in.lg);
+  float* const sDec = ex + 2 * kAtkBlocks * kD;
+  float A[4] = {in.a0.x, in.a0.y, in.a0.z, in.a0.w};
+#pragma unroll 4
+  for (int b = 0; b < w; ++b) {  // the state before this block's first row
+    const float d = sDec[b];
+    const float4 e4 = *reinterpret_cast<const float4*>(ex + b * kD + c4);
+    A[0] = d * A[0] + e4.x; A[1] = d * A[1] + e4.y; A[2] = d * A[2] + e4.z; A[3] = d * A[3] + e4.w;
+  }
+  float wt = 1.f, part[4] = {0.f, 0.f, 0.f, 0.f}, dc = 0.f;
+#pragma unroll
+  for (int i = 0; i < kAtkRows; ++i) {
+    const int r = r0 + i;
+    const bool ok = r < valid;
+    const float2 x = unpack_bf16(in.k[i].x), y = unpack_bf16(in.k[i].y);
+    const float kc[4] = {x.x, x.y, y.x, y.y};
+    const float pd = __shfl_sync(0xffffffffu, pd_l, i), bp = __shfl_sync(0xffffffffu, in.beta, i);
+    float4 dkt_i = *reinterpret_cast<float4*>(sOutKt + r * kLdG + c4), dkr_i = *reinterpret_cast<float4*>(sOutK + r * kLdG + c4);
+    float* dk_t = reinterpret_cast<float*>(&dkt_i);
+    float* dk_r = reinterpret_cast<float*>(&dkr_i);
+    wt *= pd;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float An = pd * A[e] + bp * kc[e] * kc[e];
+      const float dev = __logf(An + p.eps) - in.centre;
+      const float rden = __fdividef(1.f, 1.f + fabsf(dev));
+      const float Bf = __expf(-p.ln_x * dev * rden);
+      const float ddev = -p.ln_x * dk_t[e] * kc[e] * Bf * rden * rden;
+      dk_r[e] += dk_t[e] * Bf;
+      dk_t[e] = ok ? __fdividef(ddev, An + p.eps) : 0.f;
+      if (ok) dc -= ddev;
+      part[e] += wt * dk_t[e];
+      A[e] = An;
+    }
+    if (out_tma) {
+      *reinterpret_cast<float4*>(sOutKt + r * kLdG + c4) = dkt_i;
+      *reinterpret_cast<float4*>(sOutK + r * kLdG + c4) = dkr_i;
+    } else if (ok) {
+      *reinterpret_cast<float4*>(p.dkt + row0 + (size_t)r * gld + c4) = dkt_i;
+      *reinterpret_cast<float4*>(p.dk_read + row0 + (size_t)r * gld + c4) = dkr_i;
+    }
+  }
+  *reinterpret_cast<float4*>(ex + (kAtkBlocks + w) * kD + c4) = make_float4(part[0], part[1], part[2], part[3]);
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) dc += __shfl_xor_sync(0xffffffffu, dc, o);
+  if (lane == 0) sDec[kAtkBlocks + w] = dc;
+}
+// Behind a barrier: one thread per channel.
+__device__ __forceinline__ void atk_carry(const float* ex, const IntraBwdParams& p, size_t chh, int c) {
+  const float* const sDec = ex + 2 * kAtkBlocks * kD;
+  float acc = 0.f, wt = 1.f, dc = 0.f;
+#pragma unroll 4
+  for (int b = 0; b < kAtkBlocks; ++b) {
+    acc += wt * ex[(kAtkBlocks + b) * kD + c];
+    wt *= sDec[b];
+    dc += sDec[kAtkBlocks + b];
+  }
+  p.c_loc[chh * kD + c] = acc;
+  if (c == 0) p.partC[chh] = dc;
+}
 }  // namespace ib
 
 // One (chunk bx, head by) item; every thread of the CTA takes part.
@@ -716,6 +829,8 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
     if (!by_level || lvl == 1) break;
     lvl = lvl ? lvl >> 1 : 4;
   }
+  AtkIn atk;  // what the preconditioner's part below needs
+  atk_request(atk, p, chh, tok0, valid, h, warp, lane);
   // ungated diagonal of P
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
@@ -740,55 +855,35 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
     v += __shfl_xor_sync(0xffffffffu, v, 2);
     if (tq == 0) sRb[cq * kChunk + 16 * I + gq + 8 * half] = v;
   }
-  // outputs of this stage; dG goes through shared memory for the reverse cumulative sum.
-  // Full chunks send dq, dk_read and dkt through padded tiles in dead regions (q, k|kt and the
-  // decay tile) and TMA stores; the scattered fragment stores of the direct path cost more
-  // issue slots than the rest of this phase together.
+  // outputs of this stage, through padded tiles in dead regions; dG for the reverse cumulative sum, dkt and dk_read
+  // for the preconditioner's part.  Full chunks send dq, dk_read and dkt from there by TMA: scattered fragment
+  // stores cost more issue slots than the rest of this phase together.
   float* sdG = reinterpret_cast<float*>(smem + oStage);
-  if (out_tma) {
-    float* sOutKt = sG;  // the decay tile is dead after the level loop
+  float *sOutKt = sG, *sOutK = reinterpret_cast<float*>(smem + oA1);  // (the decay tile is dead after the pairs)
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+  for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = 16 * I + gq + 8 * half, c = 32 * cq + 8 * nt + 2 * tq;
-        *reinterpret_cast<float2*>(sOutKt + i * kLdG + c) = make_float2(dKt[0][nt][2 * half], dKt[0][nt][2 * half + 1]);
-        *reinterpret_cast<float2*>(sdG + i * kLdG + c) = make_float2(dG[0][nt][2 * half], dG[0][nt][2 * half + 1]);
-      }
-    tc::fence_proxy_async();
-  } else {
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = 16 * I + gq + 8 * half, c = 32 * cq + 8 * nt + 2 * tq;
-        if (i < valid) {
-          const size_t off = row0 + (size_t)i * gld + c;
-          *reinterpret_cast<uint32_t*>(p.dq + off) = pack_bf16(dQ[0][nt][2 * half], dQ[0][nt][2 * half + 1]);
-          *reinterpret_cast<float2*>(p.dk_read + off) = make_float2(dK[0][nt][2 * half], dK[0][nt][2 * half + 1]);
-          *reinterpret_cast<float2*>(p.dkt + off) = make_float2(dKt[0][nt][2 * half], dKt[0][nt][2 * half + 1]);
-        }
-        *reinterpret_cast<float2*>(sdG + i * kLdG + c) = make_float2(dG[0][nt][2 * half], dG[0][nt][2 * half + 1]);
-      }
-  }
-  __syncthreads();
-  if (out_tma) {
-    // every warp is past its reads of q and kt: their tiles take dq and dk_read
-    if (tid == 0) {
-      tc::tma_store_3d(&maps.dkt, smem_u32(sG), 0, h, tok0);
-      tc::bulk_commit();
+    for (int half = 0; half < 2; ++half) {
+      const int i = 16 * I + gq + 8 * half, c = 32 * cq + 8 * nt + 2 * tq;
+      *reinterpret_cast<float2*>(sOutKt + i * kLdG + c) = make_float2(dKt[0][nt][2 * half], dKt[0][nt][2 * half + 1]);
+      *reinterpret_cast<float2*>(sdG + i * kLdG + c) = make_float2(dG[0][nt][2 * half], dG[0][nt][2 * half + 1]);
     }
-    float* sOutK = reinterpret_cast<float*>(smem + oA1);
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+  for (int i = 0; i < kAtkRows; ++i)
+    atk.k[i] = *reinterpret_cast<const uint2*>(sK + (kAtkRows * warp + i) * kLdD + 4 * lane);
+  __syncthreads();
+  // every warp is past its reads of q, k and kt: their tiles take dq and dk_read
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = 16 * I + gq + 8 * half, c = 32 * cq + 8 * nt + 2 * tq;
-        *reinterpret_cast<uint32_t*>(sQ + i * kLdD + c) = pack_bf16(dQ[0][nt][2 * half], dQ[0][nt][2 * half + 1]);
-        *reinterpret_cast<float2*>(sOutK + i * kLdG + c) = make_float2(dK[0][nt][2 * half], dK[0][nt][2 * half + 1]);
-      }
-    tc::fence_proxy_async();
-  }
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int i = 16 * I + gq + 8 * half, c = 32 * cq + 8 * nt + 2 * tq;
+      const uint32_t dq = pack_bf16(dQ[0][nt][2 * half], dQ[0][nt][2 * half + 1]);
+      if (out_tma) *reinterpret_cast<uint32_t*>(sQ + i * kLdD + c) = dq;
+      else if (i < valid) *reinterpret_cast<uint32_t*>(p.dq + row0 + (size_t)i * gld + c) = dq;
+      *reinterpret_cast<float2*>(sOutK + i * kLdG + c) = make_float2(dK[0][nt][2 * half], dK[0][nt][2 * half + 1]);
+    }
+  tc::fence_proxy_async();
   // The raw gate of the tail phase is requested here, with the accumulators gone and the
   // reverse cumulative sum still to run: loaded where it is used, it cost the tail a full
   // memory round trip.
@@ -806,7 +901,13 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
     const float db = sDb[tid] + (b != 0.f ? s / b : 0.f);
     p.dbeta[(size_t)(tok0 + tid) * H + h] = __float2bfloat16(db);
   }
-  // reverse cumulative sum over the chunk (one channel per thread, in place) ...
+  atk_block_end(atk, warp, lane, reinterpret_cast<float*>(smem + oAtkEx));
+  __syncthreads();
+  if (out_tma && tid == 0) {
+    tc::tma_store_3d(&maps.dq, smem_u32(sQ), 0, h, tok0);
+    tc::bulk_commit();
+  }
+  // reverse cumulative sum over the chunk (one channel per thread, in place), beside the preconditioner's part ...
   if (tid < kD) {
     const int c = tid;
     float run = sCol[c] + sCol[kD + c] + sCol[2 * kD + c] + sCol[3 * kD + c] + sGcv[c] * sHdh[c];
@@ -816,10 +917,13 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
       sdG[r * kLdG + c] = run;
     }
   }
+  atk_local(atk, p, row0, gld, valid, warp, lane, sOutKt, sOutK,
+            reinterpret_cast<float*>(smem + oAtkEx), out_tma);
+  tc::fence_proxy_async();
   __syncthreads();
   if (out_tma && tid == 0) {
-    tc::tma_store_3d(&maps.dq, smem_u32(sQ), 0, h, tok0);
-    tc::tma_store_3d(&maps.dk_read, smem_u32(smem + oA1), 0, h, tok0);
+    tc::tma_store_3d(&maps.dkt, smem_u32(sOutKt), 0, h, tok0);
+    tc::tma_store_3d(&maps.dk_read, smem_u32(sOutK), 0, h, tok0);
     tc::bulk_commit();
   }
   // ... then the gate's own backward, elementwise over the tile with all threads:
@@ -874,6 +978,7 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
 #pragma unroll 8
     for (int g = 0; g < 32; ++g) acc += sPart[g * kLdG + tid];
     p.partB[chh * kD + tid] = acc;
+    atk_carry(reinterpret_cast<const float*>(smem + oAtkEx), p, chh, tid);
   }
   if (tid == 0) {
     float acc = 0.f;
@@ -912,20 +1017,13 @@ struct AtkBwdParams {
   const bf16* k;
   const float* g_atk;
   const bf16* beta_atk;
-  const float* log_atk_scale;
   const float* a_start;
-  float* dkt;      // in: d(loss)/d(kt); after the local pass: dA_local
-  float* dk_read;  // in: d(loss)/dk through the read path; after the local pass: + dkt B
+  const float* dkt;      // dA_local: d(loss)/dA_t through the write-key factor
+  const float* dk_read;  // d(loss)/dk without the part through A_t
   const float* lam_in;
-  float* c_loc;
   bf16* dk;
   float* dg_atk;
   bf16* dbeta_atk;
-  float* partC;
-  float ln_x, eps;
-  // local pass only: the (chunk * heads + head) items it works on and their number (NULL: every tile)
-  const int* tile_list;
-  const int* tile_count;
 };
 
 // One (chunk, head) per CTA, 256 threads, everything in registers.  Warp w owns
@@ -938,13 +1036,9 @@ struct AtkBwdParams {
 // memory, and each block continues from the carry it is owed -- every factor is a
 // product of decays <= 1, so nothing overflows.  The per-row channel sums are
 // transposed butterfly reductions (9 shuffles for 8 rows).
-//   kFinal = false (local pass): everything that needs the write-key factor B(A_t) -- it turns the
-//                   gradient buffers into dA_local (in the dkt buffer) and dk_read + dkt B, and leaves
-//                   the chunk's outgoing carry and its share of the centre gradient.  Runs on the
-//                   chunks the mma.sync chunk kernel handled; the tensor-memory kernel does the same
-//                   for its chunks itself.
-//   kFinal = true : incoming carry given; reverse scan of dA_local and all gradients.  No
-//                   transcendental per element: the states A_t are rebuilt with multiply-adds.
+// The chunk kernels leave dA_local, the lam-free part of dk and the outgoing carries; with the incoming carry given
+// this is the reverse scan of dA_local and all gradients.  No transcendental per element: the states A_t are
+// rebuilt with multiply-adds.
 namespace atkb {
 constexpr int kThreads = 256;
 constexpr int kRows = 8;  // rows per warp
@@ -954,20 +1048,15 @@ constexpr int kRows = 8;  // rows per warp
 // what it copied itself, so they need no barrier): per row k (8 B), dkt (16 B),
 // dk_read (16 B); per tile the chunk's entry state and incoming carry (16 B each).
 namespace atkb {
-template <bool kFinal> __host__ __device__ constexpr int slot_bytes() {
-  return kRows * (8 + 16 + 16) + 16 + (kFinal ? 16 : 0);
-}
-template <bool kFinal> __host__ __device__ constexpr int smem_bytes() { return kThreads * slot_bytes<kFinal>(); }
+constexpr int kSmem = kThreads * (kRows * (8 + 16 + 16) + 16 + 16);
 }  // namespace atkb
 
-template <bool kFinal>
 __global__ void __launch_bounds__(atkb::kThreads, 2)
 pkda_atk_bwd_kernel(const AtkBwdParams p, int n_tiles) {
   using namespace atkb;
   extern __shared__ __align__(16) unsigned char slots[];
   __shared__ __align__(16) float sEnd[8][kD];  // per row block: end value of its zero-start scan
   __shared__ float sDec[8];                    // per row block: product of its decays
-  __shared__ float sRed[8];
   const int H = p.geo.heads, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c4 = lane << 2, r0 = warp * kRows;
   const long gld = (long)H * kD;
@@ -982,22 +1071,14 @@ pkda_atk_bwd_kernel(const AtkBwdParams p, int n_tiles) {
   // The next tile's data is requested before the current tile is computed.
   int tok0_n = 0, valid_n = 0;
   bool live_n = false;
-  // The next tile's beta_atk and log-decay (lane i of a warp holds the values of the warp's row i) and centre,
+  // The next tile's beta_atk and log-decay (lane i of a warp holds the values of the warp's row i),
   // by plain loads that nothing consumes before the next iteration.
   uint32_t bpraw_n = 0;
-  float centre_n = 0.f, lg_n = 0.f;  // lg_n: the same for the row's log-decay
+  float lg_n = 0.f;  // lg_n: the same for the row's log-decay
   static_assert(kRows <= 32 && (kRows & (kRows - 1)) == 0, "one lane per row");
-  if (!kFinal && p.tile_list) n_tiles = *p.tile_count;
-  int tile_n = 0;  // the (chunk * heads + head) item behind the next position of the walk
-  auto request = [&](int pos) {
-    live_n = false;
-    int tile = 0;
-    if (pos < n_tiles) {
-      tile = (!kFinal && p.tile_list) ? p.tile_list[pos] : pos;
-      int n;
-      live_n = chunk_lookup_warp(p.geo, tile / H, n, tok0_n, valid_n);
-    }
-    tile_n = tile;
+  auto request = [&](int tile) {
+    int n;
+    live_n = tile < n_tiles && chunk_lookup_warp(p.geo, tile / H, n, tok0_n, valid_n);
     if (live_n) {
       const int hh = tile % H;
       const size_t col0 = ((size_t)tok0_n * H + hh) * kD + c4;
@@ -1020,46 +1101,34 @@ pkda_atk_bwd_kernel(const AtkBwdParams p, int n_tiles) {
           bpraw_n = *reinterpret_cast<const unsigned short*>(p.beta_atk + (size_t)(tok0_n + r) * H + hh);
           lg_n = p.g_atk[(size_t)(tok0_n + r) * H + hh];
         }
-        centre_n = p.log_atk_scale[hh];
       }
       cp_async16(sA0 + tid, p.a_start + (size_t)tile * kD + c4, true);
-      if (kFinal) cp_async16(sLin + tid, p.lam_in + (size_t)tile * kD + c4, true);
+      cp_async16(sLin + tid, p.lam_in + (size_t)tile * kD + c4, true);
     }
     cp_async_commit();
   };
   request(blockIdx.x);
-  for (int pos = blockIdx.x; pos < n_tiles; pos += gridDim.x) {
+  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
   const bool live = live_n;
-  const int tile = tile_n;
   const int tok0 = tok0_n, valid = valid_n, h = tile % H;
-  const size_t chh = (size_t)tile;
   const size_t col0 = ((size_t)tok0 * H + h) * kD + c4;
   cp_async_wait<0>();
   // ---- this tile's data: shared-memory slots -> registers
   uint2 kraw[kRows];
-  float4 dkt[kFinal ? kRows : 1], dkr[kFinal ? kRows : 1];  // the local pass takes these from its slots row by row
+  float4 dkt[kRows], dkr[kRows];
   float pd[kRows], bp[kRows];
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
     kraw[i] = sK[i * kThreads + tid];
-    if (kFinal) {
-      dkt[i] = sDkt[i * kThreads + tid];
-      dkr[i] = sDkr[i * kThreads + tid];
-    }
+    dkt[i] = sDkt[i * kThreads + tid];
+    dkr[i] = sDkr[i * kThreads + tid];
     pd[i] = __shfl_sync(0xffffffffu, lg_n, i);  // the log-decay for now
     bp[i] = __uint_as_float(__shfl_sync(0xffffffffu, bpraw_n, i) << 16);
   }
   const float4 a0 = sA0[tid];
-  float4 lin = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (kFinal) lin = sLin[tid];
-  const float centre = centre_n;
-  // final pass: the slots are free again, the next tile's copies fly during the computation; the local
-  // pass still reads its gradient rows from the slots and asks for the next tile after that
-  if (kFinal) request(pos + gridDim.x);
-  if (!live) {               // (uniform) index past the last real chunk of a packed batch
-    if (!kFinal) request(pos + gridDim.x);
-    continue;
-  }
+  const float4 lin = sLin[tid];
+  request(tile + gridDim.x);  // the slots are free again, the next tile's copies fly during the computation
+  if (!live) continue;        // (uniform) index past the last real chunk of a packed batch
   float dblk = 1.f;
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
@@ -1087,65 +1156,6 @@ pkda_atk_bwd_kernel(const AtkBwdParams p, int n_tiles) {
     A[0] = d * A[0] + e4.x; A[1] = d * A[1] + e4.y; A[2] = d * A[2] + e4.z; A[3] = d * A[3] + e4.w;
   }
   const float Ain[4] = {A[0], A[1], A[2], A[3]};
-  // ---- pass 2 (local pass only): true states; dA_local replaces dkt, dk_read takes the lam-free part
-  // of dk; the block's share of the outgoing carry = sum_r (prod_{j<=r} decay_j) dA_local_r
-  float dcacc = 0.f;
-  if (!kFinal) {
-    float w = 1.f, part[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int i = 0; i < kRows; ++i) {
-      const bool ok = r0 + i < valid;
-      const float2 x = unpack_bf16(kraw[i].x), y = unpack_bf16(kraw[i].y);
-      const float kc[4] = {x.x, x.y, y.x, y.y};
-      float4 dkt_i = sDkt[i * kThreads + tid], dkr_i = sDkr[i * kThreads + tid];
-      float* dk_t = reinterpret_cast<float*>(&dkt_i);
-      float* dk_r = reinterpret_cast<float*>(&dkr_i);
-      w *= pd[i];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float An = pd[i] * A[e] + bp[i] * kc[e] * kc[e];
-        const float dev = __logf(An + p.eps) - centre;
-        const float den = 1.f + fabsf(dev);
-        const float rden = __fdividef(1.f, den);
-        const float Bf = __expf(-p.ln_x * dev * rden);
-        const float ddev = -p.ln_x * dk_t[e] * kc[e] * Bf * rden * rden;
-        dk_r[e] += dk_t[e] * Bf;
-        dk_t[e] = ok ? __fdividef(ddev, An + p.eps) : 0.f;
-        if (ok) dcacc -= ddev;
-        part[e] += w * dk_t[e];
-        A[e] = An;
-      }
-      if (ok) {  // the gradient buffers now hold what the final pass reads
-        *reinterpret_cast<float4*>(p.dkt + col0 + (size_t)(r0 + i) * gld) = dkt_i;
-        *reinterpret_cast<float4*>(p.dk_read + col0 + (size_t)(r0 + i) * gld) = dkr_i;
-      }
-    }
-    request(pos + gridDim.x);  // the slots are free now
-    __syncthreads();  // every warp has read the forward end values
-    *reinterpret_cast<float4*>(&sEnd[warp][c4]) = make_float4(part[0], part[1], part[2], part[3]);
-    __syncthreads();
-    if (tid < kD) {
-      float acc = 0.f, w2 = 1.f;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        acc += w2 * sEnd[b][tid];
-        w2 *= sDec[b];
-      }
-      p.c_loc[chh * kD + tid] = acc;
-    }
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) dcacc += __shfl_xor_sync(0xffffffffu, dcacc, o);
-    if (lane == 0) sRed[warp] = dcacc;
-    __syncthreads();
-    if (tid == 0) {
-      float acc = 0.f;
-#pragma unroll
-      for (int w = 0; w < kThreads / 32; ++w) acc += sRed[w];
-      p.partC[chh] = acc;
-    }
-    __syncthreads();  // the exchange arrays are reused by the next tile
-    continue;
-  }
   // ---- reverse scan: block-local lam from a zero incoming value (into dkt), outgoing value exchanged
   {
     float l[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1174,7 +1184,7 @@ pkda_atk_bwd_kernel(const AtkBwdParams p, int n_tiles) {
   suf[kRows - 1] = 1.f;
 #pragma unroll
   for (int i = kRows - 2; i >= 0; --i) suf[i] = suf[i + 1] * pd[i + 1];
-  // ---- pass 3: outputs, walking the rows forward again for the state before each row
+  // ---- pass 2: outputs, walking the rows forward again for the state before each row
   float x1[kRows], x2[kRows];
   A[0] = Ain[0]; A[1] = Ain[1]; A[2] = Ain[2]; A[3] = Ain[3];
 #pragma unroll
@@ -1482,25 +1492,18 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
 
   AtkBwdParams ap;
   ap.geo = geo; ap.k = static_cast<const bf16*>(p.k); ap.g_atk = p.g_atk;
-  ap.beta_atk = static_cast<const bf16*>(p.beta_atk); ap.log_atk_scale = p.log_atk_scale;
-  ap.a_start = a->a_atk; ap.dkt = ws.dkt; ap.dk_read = ws.dk_read; ap.lam_in = ws.lam_in; ap.c_loc = ws.c_loc;
+  ap.beta_atk = static_cast<const bf16*>(p.beta_atk);
+  ap.a_start = a->a_atk; ap.dkt = ws.dkt; ap.dk_read = ws.dk_read; ap.lam_in = ws.lam_in;
   ap.dk = static_cast<bf16*>(a->dk); ap.dg_atk = a->dg_atk; ap.dbeta_atk = static_cast<bf16*>(a->dbeta_atk);
-  ap.partC = ws.partC; ap.ln_x = logf(p.squash_x); ap.eps = p.squash_eps;
-  // the tensor-memory chunk kernel has done the local pass of its own chunks
-  ap.tile_list = ip.slow_list; ap.tile_count = ip.slow_list ? ws.counts + 1 : nullptr;
-  begin_stage(kStageAtkBwdLocal, st);
   const int atk_tiles = geo.total_chunks * p.heads;
   const int atk_grid = atk_tiles < 2 * sms ? atk_tiles : 2 * sms;  // persistent: two CTAs per SM
-  if (!set_smem(pkda_atk_bwd_kernel<false>, atkb::smem_bytes<false>())) return PKDA_ERR_LAUNCH;
-  pkda_atk_bwd_kernel<false><<<atk_grid, atkb::kThreads, atkb::smem_bytes<false>(), st>>>(ap, atk_tiles);
-  PKDA_CHECK_LAUNCH();
   begin_stage(kStageAtkBwdCarry, st);
   pkda_atk_bwd_carry_kernel<<<dim3(p.n_seqs, p.heads), kD, 0, st>>>(geo, ws.c_loc, a->sa_atk, ws.lam_in,
                                                                    a->d_initial_A_state);
   PKDA_CHECK_LAUNCH();
   begin_stage(kStageAtkBwdFinal, st);
-  if (!set_smem(pkda_atk_bwd_kernel<true>, atkb::smem_bytes<true>())) return PKDA_ERR_LAUNCH;
-  pkda_atk_bwd_kernel<true><<<atk_grid, atkb::kThreads, atkb::smem_bytes<true>(), st>>>(ap, atk_tiles);
+  if (!set_smem(pkda_atk_bwd_kernel, atkb::kSmem)) return PKDA_ERR_LAUNCH;
+  pkda_atk_bwd_kernel<<<atk_grid, atkb::kThreads, atkb::kSmem, st>>>(ap, atk_tiles);
   PKDA_CHECK_LAUNCH();
   begin_stage(kStageParamReduce, st);
   const size_t guard_n = std::min<size_t>((size_t)p.total_tokens * p.heads * kD, 4096);

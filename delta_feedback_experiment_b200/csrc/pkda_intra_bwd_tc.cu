@@ -34,7 +34,7 @@
 // diagonal state A_t = decay_t A_(t-1) + gain_t k_t^2): it has dkt in registers, reloads the raw k
 // tile into the dead state tile and recomputes A_t per channel, so the gradient buffers leave as
 // dA_local (in the dkt buffer) and dk_read + dkt B, and the chunk-parallel reverse scan that follows
-// (pkda_atk_bwd_kernel<true>) needs no transcendental.
+// (pkda_atk_bwd_kernel) needs no transcendental.
 //
 // Every mbarrier wait is bounded; a CTA whose wait gives up sets the status word.
 #include "pkda_chunk.cuh"
@@ -550,7 +550,7 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
         dGv[t] = dg.x;
         dGv[t + 1] = dg.y;
         kds = add2(kds, kd);
-        // the preconditioner: A_t, the factor B(A_t) and its derivative (pkda_atk_bwd_kernel has the same math)
+        // the preconditioner: A_t, the factor B(A_t) and its derivative (atk_local of the mma.sync kernel has the same math)
         const float2 kc = f2(lds_bf16(a0 + oS0), lds_bf16(a1 + oS0));
         const float2 pd = *reinterpret_cast<const float2*>(sPd + j0 + t);
         const float2 in = mul2(mul2(*reinterpret_cast<const float2*>(sBp + j0 + t), kc), kc);

@@ -11,7 +11,7 @@ namespace pkda {
 // Kernel stages, for launch accounting and the optional per-stage timing.
 enum Stage {
   kStageOffsets = 0, kStagePackBeta, kStageAtkLocal, kStageAtkCarry, kStageIntraFwd, kStageScanFwd,
-  kStageOutFwd, kStageScanBwd, kStageIntraBwd, kStageAtkBwdLocal, kStageAtkBwdCarry, kStageAtkBwdFinal,
+  kStageOutFwd, kStageScanBwd, kStageIntraBwd, kStageAtkBwdCarry, kStageAtkBwdFinal,
   kStageParamReduce, kStageRecurrent, kStageConvFwd, kStageConvBwd, kStageConvDw, kStageNormGateFwd,
   kStageNormGateBwd, kStageNormGateDw, kStageDecodeStep, kStageControlsFwd, kStageControlsBwd,
   kStagePackControl, kStageStatusGuard, kStageBwdClassify, kStageIntraBwdRest, kStageCount
