@@ -311,7 +311,7 @@ struct IntraParams {
   float* gc;  // [chunks][H][D] exp of the chunk's total log-decay
   bf16 *w, *u, *kg, *qg;
   float scale, ln_x, eps;
-  int direct_cap;  // upper limit for the direct block size (64 = no limit, 1 = hierarchy only)
+  int direct_cap;  // below 64: every chunk by strips; below 8: by levels inside them
   int* status;     // device status word (tcgen05 kernel): set to 1 when a bounded wait gives up
   int* cursor;     // the CTAs draw their items with it (zeroed before every call)
   int by_strip;    // nonzero: every chunk is paired strip by strip, whatever it decays by

@@ -1007,6 +1007,7 @@ pkda_intra_bwd_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdMa
     if (item >= n_items) break;
     const int chh = p.slow_list[item];
     intra_bwd_item(p, maps, chh / H, chh % H);
+    tc::fence_proxy_async();  // the sums of ddt_bias lie where the next item's copies land
     __syncthreads();  // the next item reuses every shared-memory region (and s_item)
   }
 }
