@@ -877,7 +877,9 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 // ------------------------------------------------------------------ host side
 int launch_chain_init(float* a_chain, size_t items, int* zero, cudaStream_t st) {
   const size_t n = items * (kD / 4), most = 8 * (size_t)sm_count(), blocks = (n + 255) / 256;
+  begin_stage(kStageChainInit, st);
   pkda_chain_init_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, st>>>(reinterpret_cast<uint4*>(a_chain), n, zero);
+  end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 
