@@ -418,11 +418,18 @@ size_t chunk_fwd_workspace(const pkda_problem& p) { return carve_fwd(p, nullptr)
 bool forward_chain_possible(const pkda_problem& p) {
   if (p.cu_seqlens || stage_variant(kStageIntraFwd) != 0 || direct_block_cap() < 64) return false;
   // A hand-over from one chunk of a chain to the next takes about 0.6 us, an item 0.05 us of the chip: with a dozen
-  // (row, head) units side by side the hand-overs hide, and the two kernels in front of the intra stage, which it
-  // spares, make up for it down to 8 (16 units of 8,191 tokens 176 -> 164 us, 8 of 8,192 110 -> 94, 8 of 16,384 156 -> 147);
-  // of fewer units, short rows only.  The state is the same bit for bit either way.  (A packed batch goes sequence after
+  // (row, head) units side by side the hand-overs hide, and the chain spares two kernels in front of the intra stage.
+  // The fewer the units, the less there is to hide behind, and what a chain loses at one level it never makes up for, so the
+  // limit is one of length.  Whole forward, unchained -> chained, us (chunks that decay mildly; the strongly decaying ones, whose items
+  // take longer, lose less):
+  //   1 unit of 1,536 tokens 63.5 -> 59.5, 7 of 1,536 67.6 -> 65.5;        4 of 4,096 109 -> 119, 5 of 3,072 92 -> 98
+  //   8 units of 16,384 418 -> 412, 12 471 -> 462, 16 522 -> 496;          12 of 24,576 688 -> 696, 16 of 65,536 1,980 -> 2,074
+  //   24 units of 65,536 2,772 -> 2,650, 28 2,965 -> 2,805;                24 of 131,072 5,467 -> 5,623
+  //   32 units of 65,536 3,176 -> 2,996, of 131,072 6,325 -> 5,965
+  // The state is the same bit for bit either way.  (A packed batch goes sequence after
   // sequence, a chain per head side by side: 65,536 tokens of 32 heads 1,740 -> 1,731 us, of 12 heads 682 -> 768.)
-  return (long)p.n_seqs * p.heads >= 8 || p.seq_len <= 24 * kChunk;
+  const long units = (long)p.n_seqs * p.heads, chunks = ((long)p.seq_len + kChunk - 1) / kChunk;
+  return units >= 32 || chunks <= (units >= 24 ? 1024 : units >= 8 ? 256 : 24);
 }
 size_t chunk_fwd_status_offset(const pkda_problem& p) {
   return (size_t)(reinterpret_cast<unsigned char*>(carve_fwd(p, nullptr).status) - static_cast<unsigned char*>(nullptr));
