@@ -403,12 +403,10 @@ int run_prologue(const pkda_problem& p, int* chunk_offsets, float* beta_c, Geo* 
 // cursor: a zeroed int.
 // o / o_done: the forward's output tensor; *o_done says whether the state scan has already written it.
 // What the tensor-memory intra kernel needs to carry the preconditioner state across chunks itself
-// (dense batches): see IntraParams::chain.
+// (dense batches; NULL: it does not): see IntraParams::chain.
 struct ChainArgs {
   float *beta_c_w, *a_chain, *sa, *AT;
 };
-// True when the forward can run in chained mode (no preconditioner kernels in front of the intra stage).
-bool forward_chain_possible(const pkda_problem& p);
 int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_c, bf16* u_ws, bf16* Aqk,
                        bf16* Akk, bf16* kt, float* gc, const float* a_start, bf16* w, bf16* kg, bf16* v_new,
                        bf16* h, bf16* qg, float* ST, bool recompute, int* status, int* cursor,

@@ -415,7 +415,9 @@ static FwdWorkspace carve_fwd(const pkda_problem& p, void* base) {
 
 size_t chunk_fwd_workspace(const pkda_problem& p) { return carve_fwd(p, nullptr).bytes; }
 
-bool forward_chain_possible(const pkda_problem& p) {
+// True where the forward runs in chained mode (no preconditioner kernels in front of the intra stage).  Asked once a call:
+// it looks at the process-wide testing switches, and what runs in front of the intra stage and the stage itself must agree.
+static bool forward_chain_possible(const pkda_problem& p) {
   if (p.cu_seqlens || stage_variant(kStageIntraFwd) != 0 || direct_block_cap() < 64) return false;
   // A hand-over from one chunk of a chain to the next takes about 0.6 us, an item 0.05 us of the chip: with a dozen
   // (row, head) units side by side the hand-overs hide, and the chain spares two kernels in front of the intra stage.
@@ -488,7 +490,7 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   ip.chain = 0;
   ip.beta = static_cast<const bf16*>(p.beta); ip.A0 = p.initial_A_state;
   ip.beta_c_w = ip.a_chain = ip.sa = ip.AT = nullptr;
-  if (chain && !recompute && forward_chain_possible(p)) {
+  if (chain) {
     ip.chain = 1;
     ip.beta_c_w = chain->beta_c_w; ip.a_chain = chain->a_chain; ip.sa = chain->sa; ip.AT = chain->AT;
   }
