@@ -101,9 +101,7 @@ int check_problem(const pkda_problem& p) {
   if (!p.q || !p.k || !p.v || !p.g || !p.g_atk || !p.beta_atk || !p.beta || !p.A_log || !p.dt_bias ||
       !p.log_atk_scale)
     return PKDA_ERR_NULL;
-  const void* ptrs[] = {p.q, p.k, p.v, p.g, p.initial_state};
-  for (const void* x : ptrs)
-    if (x && (reinterpret_cast<uintptr_t>(x) & 15)) return PKDA_ERR_ALIGN;
+  if (!aligned({p.q, p.k, p.v, p.g, p.initial_state}, 16)) return PKDA_ERR_ALIGN;
   if (p.dtype != PKDA_BF16 && p.dtype != PKDA_F32) return PKDA_ERR_DTYPE;
   return PKDA_OK;
 }

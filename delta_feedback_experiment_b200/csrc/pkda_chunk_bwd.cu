@@ -1383,6 +1383,12 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
       !a->dbeta_atk || !a->dbeta || !a->dA_log || !a->ddt_bias || !a->dlog_atk_scale)
     return PKDA_ERR_NULL;
   if (!a->workspace || a->workspace_bytes < chunk_bwd_workspace(p)) return PKDA_ERR_WORKSPACE;
+  // What moves several values at a time or by TMA, as in the forward.  (The column scans touch the states' cotangents by scalars.)
+  if (!aligned({a->d_o, a->Aqk, a->Akk, a->k_precond, a->ac_atk, a->a_atk, a->w, a->kg, a->v_new, a->h, a->qg, a->dv, a->dg,
+                a->workspace, a->recompute ? p.dt_bias : nullptr}, 16) ||
+      !aligned({a->dk}, 8) || !aligned({a->dq}, 4))
+    return PKDA_ERR_ALIGN;
+  if (!scan_columns(p.n_seqs * p.heads) && !aligned({a->d_final_state, a->d_initial_state}, 16)) return PKDA_ERR_ALIGN;
   BwdWorkspace ws = carve_bwd(p, a->workspace);
   Geo geo;
   // On the default path the classifier of the intra stage runs first and packs beta on the way.

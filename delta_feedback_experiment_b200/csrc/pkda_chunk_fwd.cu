@@ -556,6 +556,12 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
       !a->kg || !a->v_new || !a->h || !a->qg)
     return PKDA_ERR_NULL;
   if (!a->workspace || a->workspace_bytes < chunk_fwd_workspace(p)) return PKDA_ERR_WORKSPACE;
+  // What moves sixteen or eight bytes at a time or by TMA.  (The column scans write o, h and v_new in eights and the
+  // states by scalars; a_atk, sa_atk and the preconditioner's states are scalars everywhere.)
+  if (!aligned({p.dt_bias, a->Aqk, a->Akk, a->ac_atk, a->w, a->kg, a->qg, a->workspace}, 16) || !aligned({a->k_precond}, 8))
+    return PKDA_ERR_ALIGN;
+  if (scan_columns(p.n_seqs * p.heads) ? !aligned({a->o, a->h, a->v_new}, 8) : !aligned({a->h, a->v_new, a->final_state}, 16))
+    return PKDA_ERR_ALIGN;
   FwdWorkspace ws = carve_fwd(p, a->workspace);
   Geo geo;
   rc = run_prologue(p, ws.chunk_offsets, nullptr, &geo, st);

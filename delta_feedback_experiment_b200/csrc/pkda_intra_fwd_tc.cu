@@ -98,10 +98,10 @@ __device__ __forceinline__ uint32_t ld_u16(const bf16* p) {
   return v;
 }
 // Before a chained launch: every word of the hand-over to kNotYet, the status word and the cursors to zero.
-__global__ void __launch_bounds__(256) pkda_chain_init_kernel(uint4* a_chain, size_t n, int* zero) {
+// (By single words: the caller's a_chain need not start on a 16-byte boundary.)
+__global__ void __launch_bounds__(256) pkda_chain_init_kernel(uint32_t* a_chain, size_t n, int* zero) {
   if (blockIdx.x == 0 && threadIdx.x < 8) zero[threadIdx.x] = 0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    a_chain[i] = make_uint4(kNotYet, kNotYet, kNotYet, kNotYet);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) a_chain[i] = kNotYet;
 }
 
 // ---- Pair products of a chunk that decays too much for one reference row.
@@ -876,9 +876,9 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 
 // ------------------------------------------------------------------ host side
 int launch_chain_init(float* a_chain, size_t items, int* zero, cudaStream_t st) {
-  const size_t n = items * (kD / 4), most = 8 * (size_t)sm_count(), blocks = (n + 255) / 256;
+  const size_t n = items * kD, most = 8 * (size_t)sm_count(), blocks = (n + 255) / 256;
   begin_stage(kStageChainInit, st);
-  pkda_chain_init_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, st>>>(reinterpret_cast<uint4*>(a_chain), n, zero);
+  pkda_chain_init_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, st>>>(reinterpret_cast<uint32_t*>(a_chain), n, zero);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

@@ -3,6 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
+#include <initializer_list>
+
 #include "../../include/pkda_b200.h"
 #include "pkda_common.cuh"
 
@@ -58,6 +61,14 @@ Geo make_geo(const pkda_problem& p, const int* chunk_offsets);
 inline int chunk_bound(const pkda_problem& p) {
   if (p.cu_seqlens) return p.total_tokens / kChunk + p.n_seqs;
   return p.n_seqs * ((p.seq_len + kChunk - 1) / kChunk);
+}
+
+// Whether every given address is a multiple of `bytes` (a NULL one is).  The kernels move several values at a time: an
+// entry point answers a misaligned buffer with PKDA_ERR_ALIGN before any launch.
+inline bool aligned(std::initializer_list<const void*> ptrs, uintptr_t bytes) {
+  for (const void* x : ptrs)
+    if (reinterpret_cast<uintptr_t>(x) % bytes) return false;
+  return true;
 }
 
 inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }

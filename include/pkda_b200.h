@@ -29,6 +29,10 @@
  *   states         S [N][H][D][D] (key-major), A [N][H][D]   fp32
  * "tokens" is the flat axis B*T (dense) or the packed total; N is B (dense) or
  * the number of packed sequences.
+ * Alignment: every activation-sized tensor, the states, dt_bias, ac_atk, a_atk and
+ * the workspaces start on 16-byte boundaries, the other per-token and per-head tensors on
+ * their element's.  Kernels move several values at a time; where one would, a misaligned
+ * buffer is answered with PKDA_ERR_ALIGN before any launch.
  */
 #ifndef PKDA_B200_H_
 #define PKDA_B200_H_

@@ -174,3 +174,45 @@ def test_exact_pair_refuses_misaligned_buffers_without_launch(lib):
     bwd.workspace = 260
     assert lib.pkda_recurrent_bwd(C.byref(bwd), None) == 6
     assert lib.pkda_last_launch_count() == 0
+
+
+def _chunk_args(args, size_query, units, pointers):
+    """Arguments of a dense call of `units` rows of 64 tokens, one head, every buffer on a 256-byte boundary."""
+    p = args.p
+    p.n_seqs, p.seq_len, p.total_tokens, p.heads, p.head_dim = units, 64, 64 * units, 1, 128
+    for f in ("q", "k", "v", "g", "g_atk", "beta_atk", "beta", "A_log", "dt_bias", "log_atk_scale"):
+        setattr(p, f, 256)
+    for f in pointers:
+        setattr(args, f, 256)
+    args.workspace, args.workspace_bytes = 256, size_query(C.byref(p))
+    return args
+
+
+FWD_POINTERS = ("o", "final_state", "final_A_state", "Aqk", "Akk", "k_precond", "ac_atk", "a_atk", "sa_atk", "w", "kg",
+                "v_new", "h", "qg")
+BWD_POINTERS = ("d_o", "d_final_state", "Aqk", "Akk", "k_precond", "ac_atk", "a_atk", "sa_atk", "w", "kg", "v_new", "h", "qg",
+                "dq", "dk", "dv", "dg", "dg_atk", "dbeta_atk", "dbeta", "dA_log", "ddt_bias", "dlog_atk_scale",
+                "d_initial_state", "d_initial_A_state")
+
+
+def test_chunked_pair_refuses_misaligned_buffers_without_launch(lib):
+    """Every buffer that a kernel of the chunked path moves several values at a time, or by TMA.  Few units take
+    the column scans, which touch the states by scalars, and many the tensor-memory scans, which do not.
+    (Only calls that are refused: these addresses must never reach a kernel.)"""
+    always = [("o", 4), ("Aqk", 8), ("Akk", 8), ("k_precond", 4), ("ac_atk", 4), ("ac_atk", 8), ("w", 8), ("kg", 8),
+              ("v_new", 4), ("h", 4), ("qg", 8), ("workspace", 8), ("p.dt_bias", 4)]
+    many = [("final_state", 4), ("v_new", 8), ("h", 8)]
+    for units, cases in ((2, always), (200, [c for c in always if c[0] != "o"] + many)):
+        for name, off in cases:
+            a = _chunk_args(_lib.ChunkFwdArgs(), lib.pkda_chunk_fwd_workspace_bytes, units, FWD_POINTERS)
+            setattr(a.p if name[:2] == "p." else a, name.removeprefix("p."), 256 + off)
+            assert lib.pkda_chunk_fwd(C.byref(a), None) == 6, (units, name, off)
+    always = [(n, 8) for n in ("d_o", "Aqk", "Akk", "k_precond", "ac_atk", "a_atk", "w", "kg", "v_new", "h", "qg", "dv", "dg",
+                               "workspace", "p.dt_bias")] + [("a_atk", 4), ("dk", 4), ("dq", 2)]
+    for units, cases in ((2, always), (200, [*always, ("d_final_state", 4), ("d_initial_state", 8)])):
+        for name, off in cases:
+            a = _chunk_args(_lib.ChunkBwdArgs(), lib.pkda_chunk_bwd_workspace_bytes, units, BWD_POINTERS)
+            a.recompute = 1
+            setattr(a.p if name[:2] == "p." else a, name.removeprefix("p."), 256 + off)
+            assert lib.pkda_chunk_bwd(C.byref(a), None) == 6, (units, name, off)
+    assert lib.pkda_last_launch_count() == 0

@@ -61,3 +61,17 @@ def test_static_scratch_rejects_oversized_problem():
     with pytest.raises(RuntimeError, match="static scratch"):
         ops.chunk_forward_static(*args, 128 ** -0.5, 1.5, 1e-6, q, _buffers(q, q))
     assert ops.static_scratch_bytes() == 16 << 20
+
+
+def test_scalar_buffers_need_no_more_than_their_element():
+    """The chained forward fills and passes on the preconditioner's chunk states word by word: they may start anywhere a
+    float may (the backward wants them on 16 bytes)."""
+    B, T, H = 8, 200, 2
+    d = make_inputs(B, T, H, 128, seed=504, dist="production", dtype=torch.bfloat16)
+    t = [d[n].cuda().contiguous() for n in INPUT_NAMES]
+    o_ref, _, _, saved_ref = ops.chunk_forward(*t, 128 ** -0.5, 1.5, 1e-6)
+    o, saved = torch.empty_like(o_ref), _buffers(t[0], t[2])
+    for i in (4, 5):  # a_atk, sa_atk
+        saved[i] = torch.empty(saved[i].numel() + 1, device="cuda")[1:].view(saved[i].shape)
+    ops.chunk_forward_static(*t, 128 ** -0.5, 1.5, 1e-6, o, saved)
+    assert torch.equal(o, o_ref) and torch.equal(saved[4], saved_ref[4]) and torch.equal(saved[5], saved_ref[5])
