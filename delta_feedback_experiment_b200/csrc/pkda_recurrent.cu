@@ -380,6 +380,7 @@ static int launch_rec_d(const RecParams& rp, bool save, cudaStream_t st) {
   const long units = (long)rp.geo.n_seqs * rp.geo.heads;
   const int few = units <= 2L * sm_count() ? 14 : 8;  // break-even in tokens, see that kernel
   if (rp.geo.seq_len > 0 && rp.geo.seq_len < few && units > sm_count()) {
+    if (!aligned({rp.ST}, 16)) return PKDA_ERR_ALIGN;  // (here, with four columns per lane and in the single step: states by float4)
     begin_stage(kStageRecurrent, st);
     pkda_recurrent_few_kernel<D, T><<<(unsigned)units, RecCfg<D>::kThreads, 0, st>>>(rp);
     end_stage(st);
@@ -388,7 +389,7 @@ static int launch_rec_d(const RecParams& rp, bool save, cudaStream_t st) {
   // Four columns per lane once the one-column warps number more than two per scheduler (4 per SM).
   constexpr bool kFour = D >= 64;
   const long warps = units * ScanLay<D, 1>::kWarps;
-  if (kFour && warps > 8L * sm_count()) return launch_rec<D, kFour ? 4 : 1, T, false>(rp, st);
+  if (kFour && warps > 8L * sm_count()) return aligned({rp.ST}, 16) ? launch_rec<D, kFour ? 4 : 1, T, false>(rp, st) : PKDA_ERR_ALIGN;
   return launch_rec<D, 1, T, false>(rp, st);
 }
 
@@ -451,8 +452,10 @@ int recurrent_fwd(const pkda_recurrent_args* a, void* saved, size_t saved_bytes,
   // One token per sequence on a cached state: the decode-step kernel (all loads of the step issued
   // up front), without its convolution and gate stages.
   if (!p.cu_seqlens && p.seq_len == 1 && p.initial_state && a->final_state &&
-      (p.dtype == PKDA_BF16 || p.dtype == PKDA_F32))
+      (p.dtype == PKDA_BF16 || p.dtype == PKDA_F32)) {
+    if (!aligned({a->final_state}, 16)) return PKDA_ERR_ALIGN;
     return decode_direct(p, a->o, a->final_state, a->final_A_state, st);
+  }
   return run_rec(p, a->o, a->final_state, a->final_A_state, nullptr, st);
 }
 

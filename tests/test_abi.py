@@ -216,3 +216,16 @@ def test_chunked_pair_refuses_misaligned_buffers_without_launch(lib):
             setattr(a.p if name[:2] == "p." else a, name.removeprefix("p."), 256 + off)
             assert lib.pkda_chunk_bwd(C.byref(a), None) == 6, (units, name, off)
     assert lib.pkda_last_launch_count() == 0
+
+
+@pytest.mark.parametrize("rows,T", [(2, 1), (200, 2), (2000, 40)])
+def test_token_by_token_forward_refuses_a_misaligned_final_state(lib, rows, T):
+    """The single step, the few-token kernel and the scan with four columns per lane write states by float4."""
+    a = _lib.RecurrentArgs()
+    p = a.p
+    p.n_seqs, p.seq_len, p.total_tokens, p.heads, p.head_dim = rows, T, rows * T, 1, 128
+    for f in ("q", "k", "v", "g", "g_atk", "beta_atk", "beta", "A_log", "dt_bias", "log_atk_scale", "initial_state"):
+        setattr(p, f, 256)
+    a.o, a.final_state = 256, 260
+    assert lib.pkda_recurrent_fwd(C.byref(a), None) == 6
+    assert lib.pkda_last_launch_count() == 0
