@@ -29,10 +29,15 @@ constexpr int kLdG = kD + 8;                  // smem row stride of a [64][128] 
 // others; chunks of the benchmark's gate distribution (about 75 +- 6 log2 units of decay per 64
 // tokens) then practically always form one block.
 constexpr float kDirectLimit = 112.f;
-// Where a strip decays by more than that, its rows are taken relative to its third row and its columns relative to the third
-// from the end, as long as 5 tokens decay by at most kDirectLimit and the 2 outer ones by at most this (log2 units).
+// Where a strip decays by more than that, each half of it (4 rows) is taken relative to its own first row and all columns
+// relative to the strip's fifth row, as long as 5 tokens decay by at most kDirectLimit, the 2 outer ones by at most this and the 3
+// behind the fifth row by twice this (log2 units): strip_decays.
 constexpr float kOuterLimit = 45.f;
-constexpr int kInnerRow = 2;
+constexpr int kHalfRow = 4;
+// {decay that kDirectLimit bounds, decay that kOuterLimit bounds} of a strip from the G of its rows.
+__device__ __forceinline__ float2 strip_decays(float g0, float g2, float g4, float g5, float g7) {
+  return make_float2(fmaxf(g0 - g5, g2 - g7), fmaxf(fmaxf(g0 - g2, g5 - g7), 0.5f * (g4 - g7)));
+}
 
 // 2^x by the hardware approximation (flushes denormal results to zero, which is
 // what the gating factors want: every argument here is <= 0).

@@ -440,15 +440,15 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   __syncthreads();
   if (tid < kD) {
     gate_cumsum(sG, tid);
-    // worst decays of a strip of 8 rows: all of it, all but its first or its last two tokens, these two alone
+    // worst decays of a strip of 8 rows: all of it, and what strip_decays says
     float worst[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int r = 0; r < kChunk; r += 8) {
       const float g0 = sG[r * kLdG + tid], g7 = sG[(r + 7) * kLdG + tid];
-      const float gx = sG[(r + kInnerRow) * kLdG + tid], gz = sG[(r + 7 - kInnerRow) * kLdG + tid];
+      const float2 d = strip_decays(g0, sG[(r + 2) * kLdG + tid], sG[(r + kHalfRow) * kLdG + tid], sG[(r + 5) * kLdG + tid], g7);
       worst[0] = fmaxf(worst[0], g0 - g7);
-      worst[1] = fmaxf(worst[1], fmaxf(g0 - gz, gx - g7));
-      worst[2] = fmaxf(worst[2], fmaxf(g0 - gx, gz - g7));
+      worst[1] = fmaxf(worst[1], d.x);
+      worst[2] = fmaxf(worst[2], d.y);
     }
 #pragma unroll
     for (int e = 0; e < 3; ++e) {  // (not negative, so their bit patterns have their order)
@@ -672,9 +672,11 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   float worst[3];
 #pragma unroll
   for (int e = 0; e < 3; ++e) worst[e] = fmaxf(fmaxf(sWorst[e], sWorst[3 + e]), fmaxf(sWorst[6 + e], sWorst[9 + e]));
-  const bool first_last = worst[0] <= kDirectLimit, inner = worst[1] <= kDirectLimit && worst[2] <= kOuterLimit;
-  const bool by_level = p.direct_cap < 8 || !(first_last || inner);
-  const int xo = first_last || by_level ? 0 : kInnerRow, zo = 7 - xo;  // reference rows of a strip
+  const bool first_last = worst[0] <= kDirectLimit, bounded = worst[1] <= kDirectLimit && worst[2] <= kOuterLimit;
+  const bool by_level = p.direct_cap < 8 || !(first_last || bounded);
+  auto pairs = [&](auto halves) {
+  constexpr bool kHalves = decltype(halves)::value;
+  constexpr int xo = kHalves ? kHalfRow : 0, zo = kHalves ? kHalfRow : 7;  // reference rows of a strip: x of the second half (of the first: 0), z
 #pragma unroll 1
   for (int lvl = 0;;) {
     // (a warp takes a row, four channels a lane: fp32 rows then move without bank conflicts)
@@ -682,7 +684,7 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
     for (int r = warp; r < kChunk; r += kThreads / 32) {
       const int c4 = lane << 2, own = lvl ? (r & ~(2 * lvl - 1)) + lvl : r & ~7;
       const float4 g = *reinterpret_cast<const float4*>(sG + r * kLdG + c4);
-      const float4 gx = *reinterpret_cast<const float4*>(sG + (lvl ? own : own + xo) * kLdG + c4);
+      const float4 gx = *reinterpret_cast<const float4*>(sG + (lvl ? own : own + (r & xo)) * kLdG + c4);
       const float4 gz = *reinterpret_cast<const float4*>(sG + (lvl ? own : own + zo) * kLdG + c4);
       float4 x = make_float4(ex2(g.x - gx.x), ex2(g.y - gx.y), ex2(g.z - gx.z), ex2(g.w - gx.w));
       float4 z = make_float4(ex2(gz.x - g.x), ex2(gz.y - g.y), ex2(gz.z - g.z), ex2(gz.w - g.w));
@@ -706,7 +708,7 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
       if (lvl) {
         if (Is == Js) d = make_float4(1.f, 1.f, 1.f, 1.f);
       } else if (!by_level || Js < Is) {
-        const float4 a = *reinterpret_cast<const float4*>(sG + (8 * Is + xo) * kLdG + 4 * lane);
+        const float4 a = *reinterpret_cast<const float4*>(sG + 8 * Is * kLdG + 4 * lane);
         const float4 b = *reinterpret_cast<const float4*>(sG + (8 * Js + zo) * kLdG + 4 * lane);
         d = make_float4(ex2(a.x - b.x), ex2(a.y - b.y), ex2(a.z - b.z), ex2(a.w - b.w));
       }
@@ -736,14 +738,36 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
         }
         const float* y = sY + (16 * K + 2 * tq) * kLdY + 32 * cq + gq;
         const float* d = sStrip + (tri + 2 * K) * kD + 32 * cq + gq;
+        // part 0: all rows; by halves 1: those of the first with their factors, 2: those of the second with theirs.  (The
+        // second half's columns of the strip itself have no rows in the first, and their factor no bound.)
+        auto take = [&](auto part) {
+          constexpr int kPart = decltype(part)::value;
+          const bool in = kPart == 0 || (gq < kHalfRow) == (kPart == 1);
+          const uint32_t ap[4] = {in ? a[0] : 0u, in ? a[1] : 0u, in ? a[2] : 0u, in ? a[3] : 0u};
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const float d0 = d[8 * nt], d1 = two ? d[kD + 8 * nt] : 0.f;
-          mma_bf16(t[0][nt], a, pack_bf16(y[8 * nt] * d0, y[kLdY + 8 * nt] * d0),
-                   pack_bf16(y[8 * kLdY + 8 * nt] * d1, y[9 * kLdY + 8 * nt] * d1));
+          for (int nt = 0; nt < 4; ++nt) {
+            float d0 = d[8 * nt], d1 = two ? d[kD + 8 * nt] : 0.f;
+            if (kPart == 1 && 2 * tq >= kHalfRow) {
+              if (2 * K == Is) d0 = 0.f;
+              if (2 * K + 1 == Is) d1 = 0.f;
+            }
+            if (kPart == 2) {
+              const float self = sStrip[(tri + Is) * kD + 32 * cq + gq + 8 * nt];
+              d0 = __fdividef(d0, self);
+              d1 = __fdividef(d1, self);
+            }
+            mma_bf16(t[0][nt], ap, pack_bf16(y[8 * nt] * d0, y[kLdY + 8 * nt] * d0),
+                     pack_bf16(y[8 * kLdY + 8 * nt] * d1, y[9 * kLdY + 8 * nt] * d1));
+          }
+        };
+        if (!kHalves) {
+          take(std::integral_constant<int, 0>{});
+        } else {
+          take(std::integral_constant<int, 1>{});
+          take(std::integral_constant<int, 2>{});
         }
       }
-      const int i = 8 * Is + gq, ref = lvl ? (i & ~(2 * lvl - 1)) + lvl : 8 * Is + xo;
+      const int i = 8 * Is + gq, ref = lvl ? (i & ~(2 * lvl - 1)) + lvl : 8 * Is + (gq & xo);
       if (!lvl || (i & lvl)) {
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
@@ -792,24 +816,39 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
             a[x] &= (level_pair_ok(i, j, lvl) ? 0x0000ffffu : 0u) | (level_pair_ok(i + 1, j, lvl) ? 0xffff0000u : 0u);
           }
         }
-        const uint32_t am[4] = {0u, 0u, a[2], a[3]};
+        auto take = [&](auto part) {
+          constexpr int kPart = decltype(part)::value;
+          const bool in = kPart == 0 || (2 * tq < kHalfRow) == (kPart == 1);
+          const uint32_t ap[4] = {in ? a[0] : 0u, in ? a[1] : 0u, in ? a[2] : 0u, in ? a[3] : 0u}, am[4] = {0u, 0u, ap[2], ap[3]};
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          float u[4] = {0.f, 0.f, 0.f, 0.f}, um[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_bf16(u, a, b[2 * x], b[2 * x + 1]);
-          mma_bf16(um, am, b[2 * x], b[2 * x + 1]);  // the part through M: its product with Y is dbeta's
+          for (int x = 0; x < 2; ++x) {
+            float u[4] = {0.f, 0.f, 0.f, 0.f}, um[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_bf16(u, ap, b[2 * x], b[2 * x + 1]);
+            mma_bf16(um, am, b[2 * x], b[2 * x + 1]);  // the part through M: its product with Y is dbeta's
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            float2 d = make_float2(0.f, 0.f);
-            if (!half || two) d = *reinterpret_cast<const float2*>(sStrip + (tri + half) * kD + c + 8 * x);
-            const float2 Y = unpack_bf16(pack_bf16(y[x][half].x * d.x, y[x][half].y * d.y));
-            const float u0 = u[2 * half], u1 = u[2 * half + 1];
-            w[x][2 * half] += d.x * u0;
-            w[x][2 * half + 1] += d.y * u1;
-            dG[0][2 * np + x][2 * half] -= Y.x * u0;
-            dG[0][2 * np + x][2 * half + 1] -= Y.y * u1;
-            rb[half] += Y.x * um[2 * half] + Y.y * um[2 * half + 1];
+            for (int half = 0; half < 2; ++half) {
+              float2 d = make_float2(0.f, 0.f);
+              if (!half || two) d = *reinterpret_cast<const float2*>(sStrip + (tri + half) * kD + c + 8 * x);
+              if (kPart == 1 && 2 * I + half == Is && gq >= kHalfRow) d = make_float2(0.f, 0.f);
+              if (kPart == 2) {
+                const float2 self = *reinterpret_cast<const float2*>(sStrip + Is * (Is + 3) / 2 * kD + c + 8 * x);
+                d = make_float2(__fdividef(d.x, self.x), __fdividef(d.y, self.y));
+              }
+              const float2 Y = unpack_bf16(pack_bf16(y[x][half].x * d.x, y[x][half].y * d.y));
+              const float u0 = u[2 * half], u1 = u[2 * half + 1];
+              w[x][2 * half] += d.x * u0;
+              w[x][2 * half + 1] += d.y * u1;
+              dG[0][2 * np + x][2 * half] -= Y.x * u0;
+              dG[0][2 * np + x][2 * half + 1] -= Y.y * u1;
+              rb[half] += Y.x * um[2 * half] + Y.y * um[2 * half + 1];
+            }
           }
+        };
+        if (!kHalves) {
+          take(std::integral_constant<int, 0>{});
+        } else {
+          take(std::integral_constant<int, 1>{});
+          take(std::integral_constant<int, 2>{});
         }
       }
 #pragma unroll
@@ -826,9 +865,12 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
       }
     }
     __syncthreads();
-    if (!by_level || lvl == 1) break;
+    if (kHalves || !by_level || lvl == 1) break;
     lvl = lvl ? lvl >> 1 : 4;
   }
+  };
+  if (first_last || by_level) pairs(std::false_type{});
+  else pairs(std::true_type{});
   AtkIn atk;  // what the preconditioner's part below needs
   atk_request(atk, p, chh, tok0, valid, h, warp, lane);
   // ungated diagonal of P

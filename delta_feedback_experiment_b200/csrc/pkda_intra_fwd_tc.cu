@@ -59,7 +59,7 @@ constexpr int oEnd = oL + 4096;             // f32 [8][128] per-strip end value 
 constexpr int oDec = oL + 8192;             // f32 [8] per-strip product of preconditioner decays
 constexpr int oSum = oDec + 32;             // f32 [8] per-strip sum of the preconditioner's log-decays
 constexpr int oA0 = oSum + 32;              // f32 [128] the chunk-entry preconditioner state (chained mode)
-constexpr int oZin = oL + 9216;             // f32 [8][128] G of the inner column reference of every strip
+constexpr int oZin = oL + 9216;             // f32 [8][128] G of the fifth row of every strip
 // between those and the products, the strip's own factors where its rows of P come later: strip w, 2 x f32 [128]
 constexpr int oD0 = oP, oD1 = oP + 512;     // + 1024 w
 // while the inverse runs: T in the (dead) write-key operand, its scratch in the (dead) q rows of block 0
@@ -113,9 +113,14 @@ __global__ void __launch_bounds__(256) pkda_chain_init_kernel(uint32_t* a_chain,
 // the first factor is in the A operand, staged once per strip; kt times the third is kept in fp32, and a warp
 // multiplies it with the second, one number per channel and strip pair, and rounds the product to the B operand.
 // x(I) is the strip's first row and z(J) its last, so every factor of two strips is <= 1; inside a strip the second one is
-// 2^(decay of 7 tokens), which kDirectLimit bounds.  Strips that decay by more take their third row and the third from the
-// end (kDirectLimit then bounds the decay of 5 tokens, kOuterLimit that of the outer two, whose factors are > 1: nothing inside a
-// strip is lost, and of two strips nothing above 2^(2 kOuterLimit - 126)).  Chunks beyond that go through pair_exact.  A strip pair costs 11 instructions per 16 channels and no exponential;
+// 2^(decay of 7 tokens), which kDirectLimit bounds.  Strips that decay by more go by halves: x is the first row of the row's
+// own half, z the strip's fifth row, and a strip pair takes one product per half (the other half's rows of the A operand are zero),
+// with the factors 2^(x - z) of either.  The factors of the rows behind z are > 1; strip_decays bounds them, so nothing
+// inside a strip is lost, and of two strips nothing above 2^(2 kOuterLimit - 126).  (One row in the middle as the reference of all
+// eight needs no second product, but then two of eight neighbours keep an operand as it is, not four, and neighbours are
+// what the gradient of such gates is made of: its error against 64 bits was 1.5 % larger on average.  The second product
+// costs 538 -> 546 us here and 1,386 -> 1,416 in the backward at 8 x 4,096 tokens of 16 heads, exp(A_log) from 1 to 16.)  Chunks beyond that go
+// through pair_exact.  A strip pair costs 11 instructions per 16 channels and no exponential;
 // gating both fragments from G by exponentials took 66, and with them the pairs were 10,000 of the 34,000 cycles of an
 // item alone on its SM instead of 4,500 (2,048 chunks: 182 us instead of 164).
 struct PairLane {
@@ -152,7 +157,8 @@ __device__ __forceinline__ void put_pair(unsigned char* tiles, const PairLane& L
   *reinterpret_cast<uint32_t*>(tiles + oP + i * 128 + ((J ^ L.g) << 4) + 4 * L.t) = pack_bf16(p0 * scale, p1 * scale);
 }
 // All pairs of strip I (the warp's), with the factors 2^(x(I) - z(I)) at oD0, 2^(x(I) - z(I - 1)) at oD1 and
-// 2^(z(J) - z(J - 1)) at oStep.
+// 2^(z(J) - z(J - 1)) at oStep; by halves x(I) is the first half's there, and the second half's is z(I).
+template <bool kHalves>
 __device__ __forceinline__ void pairs_of_strip(unsigned char* tiles, uint32_t base, int I, int lane, float scale) {
   using namespace intratc;
   const PairLane L(lane);
@@ -180,6 +186,8 @@ __device__ __forceinline__ void pairs_of_strip(unsigned char* tiles, uint32_t ba
     uint32_t an[4] = {0u, 0u, 0u, 0u};
     if (ks < 7) ldsm_x4(an, ra + ((ks + 1) >> 2) * L.s_blk + (L.a_x ^ (((ks + 1) & 3) << 5)));
     float2 f0 = ld_f2(d0 + to), f1 = ld_f2(d0 + to + 32);
+    const float2 c0 = make_float2(__fdividef(1.f, f0.x), __fdividef(1.f, f0.y));  // from the first half's factor to the second's
+    const float2 c1 = make_float2(__fdividef(1.f, f1.x), __fdividef(1.f, f1.y));
 #pragma unroll
     for (int d = 0; d < 8; ++d) {
       // in twos: a strip too many (before the chunk's first, or one that has vanished) is computed and dropped
@@ -192,7 +200,18 @@ __device__ __forceinline__ void pairs_of_strip(unsigned char* tiles, uint32_t ba
         f0.x *= s0.x; f0.y *= s0.y; f1.x *= s1.x; f1.y *= s1.y;
       }
       const float2 y0 = ld_f2(y + yo - d * 4096), y1 = ld_f2(y + (yo ^ 32) - d * 4096);
-      mma_bf16(acc[d], a, pack_bf16(y0.x * f0.x, y0.y * f0.y), pack_bf16(y1.x * f1.x, y1.y * f1.y));
+      uint32_t b0 = pack_bf16(y0.x * f0.x, y0.y * f0.y), b1 = pack_bf16(y1.x * f1.x, y1.y * f1.y);
+      if (!kHalves) {
+        mma_bf16(acc[d], a, b0, b1);
+      } else {
+        const bool lo = L.g < kHalfRow;
+        const uint32_t al[4] = {lo ? a[0] : 0u, lo ? a[1] : 0u, lo ? a[2] : 0u, lo ? a[3] : 0u};
+        const uint32_t ah[4] = {lo ? 0u : a[0], lo ? 0u : a[1], lo ? 0u : a[2], lo ? 0u : a[3]};
+        if (d == 0 && !lo) b0 = b1 = 0u;  // (columns of the second half have no rows in the first, and their factor no bound)
+        mma_bf16(acc[d], al, b0, b1);
+        if (d == 0) mma_bf16(acc[d], ah, pack_bf16(y0.x, y0.y), pack_bf16(y1.x, y1.y));
+        else mma_bf16(acc[d], ah, pack_bf16(y0.x * (f0.x * c0.x), y0.y * (f0.y * c0.y)), pack_bf16(y1.x * (f1.x * c1.x), y1.y * (f1.y * c1.y)));
+      }
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) a[e] = an[e];
@@ -518,7 +537,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   // totals of its four channels, the CTA all 128.)  If so, which reference rows do its strips take?
   const bool by_strip =
       __syncthreads_or(-fminf(fminf(Glast[0], Glast[1]), fminf(Glast[2], Glast[3])) > kDirectLimit) || p.by_strip;
-  int refs = 0;  // 0: first and last row, 1: kInnerRow from either end, 2: pair_exact
+  int refs = 0;  // 0: first and last row, 1: by halves, 2: pair_exact
   if (!kRecompute) {
     if (!by_strip) {
       if (tid == 0) request_v();
@@ -527,10 +546,11 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         all = fmaxf(all, G[0][e] - G[7][e]);
-        mid = fmaxf(mid, fmaxf(G[0][e] - G[7 - kInnerRow][e], G[kInnerRow][e] - G[7][e]));
-        outer = fmaxf(outer, fmaxf(G[0][e] - G[kInnerRow][e], G[7 - kInnerRow][e] - G[7][e]));
+        const float2 d = strip_decays(G[0][e], G[2][e], G[kHalfRow][e], G[5][e], G[7][e]);
+        mid = fmaxf(mid, d.x);
+        outer = fmaxf(outer, d.y);
       }
-      constexpr int kz = 7 - kInnerRow;
+      constexpr int kz = kHalfRow;
       *reinterpret_cast<float4*>(tiles + oZin + warp * 512 + (lane << 4)) = make_float4(G[kz][0], G[kz][1], G[kz][2], G[kz][3]);
       if (__syncthreads_or(all > kDirectLimit)) refs = 1 + (__syncthreads_or(mid > kDirectLimit || outer > kOuterLimit) != 0);
       if (p.direct_cap < 8) refs = 2;
@@ -576,8 +596,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        zr[c] = refs ? G[7 - kInnerRow][c] : G[7][c];
-        xr[c] = refs ? G[kInnerRow][c] : G[0][c];
+        zr[c] = refs ? G[kHalfRow][c] : G[7][c];
+        xr[c] = G[0][c];
       }
       unsigned char* at = tiles + warp * 1024 + (lane << 4);
       *reinterpret_cast<float4*>(at + oD0) = make_float4(ex2(xr[0] - zr[0]), ex2(xr[1] - zr[1]), ex2(xr[2] - zr[2]), ex2(xr[3] - zr[3]));
@@ -589,6 +609,10 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     uint2 k_next = ld_k(0), q_next = ld_q(0);
 #pragma unroll 1
     for (int i0 = 0; i0 < 8; i0 += 4) {
+    if (!kRecompute && refs == 1 && i0) {  // the second half's reference is its own first row
+#pragma unroll
+      for (int c = 0; c < 4; ++c) xr[c] = G[0][c];
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = i0 + i, off = slot_off(row);
@@ -682,8 +706,10 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   if (kRecompute && tid == 32) s_item[slot ^ 1] = describe(drawn);
   if (!kRecompute && by_strip) {
     if (tid == 32) s_item[slot ^ 1] = describe(drawn);
-    if (refs < 2) {
-      pairs_of_strip(tiles, base, warp, lane, p.scale);
+    if (refs == 0) {
+      pairs_of_strip<false>(tiles, base, warp, lane, p.scale);
+    } else if (refs == 1) {
+      pairs_of_strip<true>(tiles, base, warp, lane, p.scale);
     } else {
       pairs_of_strip_exact(tiles, base, warp, lane, p.scale);
       __syncwarp();  // (only this warp reads the k rows of its strip; they become Kd)

@@ -1,6 +1,6 @@
 """Chunks that decay too much for one reference row are paired strip by strip (8 rows), each strip relative to
-reference rows of its own.  Which rows those are follows the decay: the strip's first and last row, the third
-from either end, or a reference of its own for every level of pairs.  Each of the three, the lines between
+reference rows of its own.  Which rows those are follows the decay: the strip's first and last row, the first of
+either half and the fifth, or a reference of its own for every level of pairs.  Each of the three, the lines between
 them, ragged tails and a chunk of mixed heads are compared with the float64 oracle here, and the
 recompute pass of a lean backward with the forward it rebuilds."""
 
@@ -18,8 +18,8 @@ pytestmark = pytest.mark.gpu
 D = 128
 
 # Decay per token in log2 units (about; the raw gate spreads it by a seventh).  64 tokens: one reference row up to 112;
-# 7 tokens: first and last row up to 112; 5 tokens up to 112 and two up to 45: third row from either end.
-RATES = {"two strips meet": 2.0, "first and last row": 9.0, "line of the first": 13.5, "third row from either end": 15.5,
+# 7 tokens: first and last row up to 112; 5 tokens up to 112 and two up to 45: by halves.
+RATES = {"two strips meet": 2.0, "first and last row": 9.0, "line of the first": 13.5, "by halves": 15.5,
          "line of the second": 18.0, "own rows": 40.0, "everything vanishes": 300.0}
 
 
