@@ -72,8 +72,8 @@ STAGE_FLOPS = {
 # DRAM traffic per (token, head) of each kernel: dram__bytes_read.sum + dram__bytes_write.sum of one
 # ncu capture on the quarter-size workload (131,072 units), divided by its units; the traffic grows
 # in proportion to the units, so a launch of any size moves this many bytes per unit.
-STAGE_TRAFFIC_PER_UNIT = {"intra_fwd": 2188, "scan_fwd": 1245, "out_fwd": 1280, "scan_bwd": 1655,
-                          "intra_bwd": 4506}
+STAGE_TRAFFIC_PER_UNIT = {"intra_fwd": 2195, "scan_fwd": 1889, "out_fwd": 1280, "scan_bwd": 1649,
+                          "intra_bwd": 4484}
 # Bytes per (token, head) that each kernel must read and write by its own interface (its input and
 # output tensors, each touched once): the HBM view of the same kernels.
 STAGE_IO_BYTES = {

@@ -353,8 +353,9 @@ def set_direct_block_cap(cap: int) -> None:
 
 
 def set_variant(stage: str, legacy) -> None:
-    """Testing aid: pins the older mma.sync kernel of a stage (``"intra_fwd"``,
-    ``"scan_fwd"``, ``"out_fwd"``, ``"scan_bwd"``, ``"intra_bwd"``) or restores the default.
+    """Testing aid: pins the older mma.sync kernel of a stage (``"scan_fwd"``, ``"out_fwd"``,
+    ``"scan_bwd"``, ``"intra_bwd"``; ``"intra_fwd"``: the same kernel, every chunk strip by strip)
+    or restores the default.
     ``set_variant("out_fwd", 2)`` runs the stand-alone tcgen05 output kernel instead of
     letting the state scan produce the output."""
     check(load().pkda_set_variant(stage.encode(), int(legacy)), "pkda_set_variant")

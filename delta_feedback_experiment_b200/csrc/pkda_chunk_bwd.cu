@@ -11,8 +11,8 @@
 // log-decay gradient cancel exactly under the reverse cumulative sum.
 //
 // Pipeline:  [recompute forward stages]  scan_bwd (sequential over chunks)
-//   -> intra_bwd (per chunk) -> atk_bwd local / carry / final (preconditioner
-//   reverse scan, chunk-parallel) -> param_reduce.
+//   -> intra_bwd (per chunk; the preconditioner's reverse scan inside it too) -> atk_bwd
+//   carry / final (the same over chunks) -> param_reduce.
 #include <algorithm>
 
 #include "pkda_chunk.cuh"
@@ -400,7 +400,7 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   else if (tid >= kD && tid < 2 * kD) s_small = p.dt_bias[h * kD + tid - kD];
   GateRaw<kThreads> graw;  // the raw gate is needed next
   gate_load(graw, p.g + row0, gld, valid, tid);
-  // dS1 waits in the (not yet used) level-factor array until the dkg product, E in the (not yet
+  // dS1 waits where the strips' kt goes later until the dkg product, E in the (not yet
   // used) pair-gradient tiles until S0 has left the tile E belongs in
   bf16* sdSC = reinterpret_cast<bf16*>(smem + oFac);
   bf16* sEarly = reinterpret_cast<bf16*>(smem + oDP);
@@ -1039,7 +1039,7 @@ pkda_intra_bwd_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdMa
     intra_bwd_item(p, maps, blockIdx.x, blockIdx.y);
     return;
   }
-  // items differ in cost (the number of pairing levels follows the decay): CTAs draw them one at a time
+  // items differ in cost (how many strip pairs are left, and how they are taken, follows the decay): CTAs draw them one at a time
   __shared__ int s_item;
   const int n_items = p.fast_count[1], H = p.geo.heads;
   for (;;) {

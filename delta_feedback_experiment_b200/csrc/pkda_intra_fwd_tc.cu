@@ -1,6 +1,6 @@
 // Intra-chunk stage of the chunked forward on tcgen05 / tensor memory (D = 128, chunk 64).
 //
-// Persistent CTAs of 256 threads, two per SM (about 105 KB of shared memory and 256 tensor-memory
+// Persistent CTAs of 256 threads, two per SM (112 KB of shared memory and 256 tensor-memory
 // columns each), walk the (chunk, head) items.  What the stage computes is described at the top of
 // pkda_chunk_fwd.cu.  A chunk whose decay lets it be ONE direct block (pkda_chunk.cuh) has one set of gated
 // operands for all its pairs, k 2^G, q 2^G and kt 2^-G with G the cumulative log2-decay from the chunk
@@ -323,7 +323,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   bool ok = true;
   uint32_t ph = 0;  // bit 0: bar_mma, 1: bar_tma, 2: bar_in
 
-  // Items differ in cost (one that is paired by level takes longer), so
+  // Items differ in cost (one whose pairs go strip by strip takes longer), so
   // the CTAs draw them one at a time from a cursor instead of striding through them.  One thread draws the
   // next item and looks its chunk up while the current one waits for its products, and the item's rows are
   // asked into L2 from then on: drawn at the end of an item, the cursor, the lookup and the rows were four

@@ -254,7 +254,7 @@ int pkda_last_launch_count(void);
  * through several reference rows otherwise; b is chosen per
  * (chunk, head) from the data.  This caps b (a power of two in 1..64; 64 = no cap,
  * 1 = a reference for every level of pairs) so that tests can exercise every variant on
- * the same input.  (The forward knows b = 64, strips of 8 rows, and less than 8.)
+ * the same input.  (The kernels know b = 64, strips of 8 rows, and less than 8.)
  */
 int pkda_set_direct_block_cap(int cap);
 
