@@ -392,17 +392,21 @@ int launch_scan_fwd_tc(const Geo& geo, int total_tokens, int units, const bf16* 
 // tcgen05 / TMA reverse state scan of the backward (pkda_scan_bwd_tc.cu): one CTA per (sequence, head).
 int launch_scan_bwd_tc(const Geo& geo, int total_tokens, int units, const bf16* kg, const bf16* w, const bf16* qg,
                        const bf16* d_o, const bf16* Aqk, const float* beta_c, const float* gc, const float* dST,
-                       bf16* dh, bf16* dF, float* dS0, int* status, cudaStream_t st);
+                       bf16* dh, bf16* dF, float* dS0, int* status, bool beside, cudaStream_t st);
 
-// The same two scans with the value columns spread over four or eight SMs (pkda_scan_fwd.cu, pkda_scan_bwd.cu).
+// The same two scans with the value columns spread over `split` SMs (pkda_scan_fwd.cu, pkda_scan_bwd.cu).
 int launch_scan_fwd_cols(const Geo& geo, int total_tokens, int units, const bf16* w, const bf16* kg, const bf16* u,
                          const float* beta_c, const float* gc, const float* S0, bf16* h, bf16* v_new, float* ST,
-                         int* status, const bf16* qg, const bf16* Aqk, bf16* o, cudaStream_t st);
+                         int* status, const bf16* qg, const bf16* Aqk, bf16* o, int split, cudaStream_t st);
 int launch_scan_bwd_cols(const Geo& geo, int total_tokens, int units, const bf16* kg, const bf16* w, const bf16* qg,
                          const bf16* d_o, const bf16* Aqk, const float* beta_c, const float* gc, const float* dST,
-                         bf16* dh, bf16* dF, float* dS0, int* status, cudaStream_t st);
+                         bf16* dh, bf16* dF, float* dS0, int* status, int split, bool beside, cudaStream_t st);
 // CTAs per unit, 0 where the tensor-memory scans are taken: as many as still run in one wave (one per SM).
 int scan_columns(int units);
+// CTAs per unit of the two state scans of a lean backward, which need nothing of each other and run side by side while
+// both fit the chip; {0, 0} where they run one after the other.  (1: the tensor-memory scans.)
+struct ScanPair { int fwd, bwd; };
+ScanPair scan_pair(int units);
 
 // Host-side pieces defined in pkda_chunk_fwd.cu and reused by the backward.
 int check_chunk_problem(const pkda_problem& p);

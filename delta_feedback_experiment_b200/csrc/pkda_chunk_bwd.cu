@@ -1471,13 +1471,15 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
     // Columns over four or eight SMs for few units, else tcgen05 / TMEM / TMA, as in the forward; the older
     // mma.sync kernel runs only when it is pinned (pkda_set_variant).
     const bool scan_mma = stage_variant(kStageScanBwd) == 1;
+    // The recompute pass has just launched its scan, which leaves h and v_new; this one reads neither, so it runs beside it.
+    const ScanPair pair = a->recompute && stage_variant(kStageScanFwd) != 1 ? scan_pair(units) : ScanPair{0, 0};
     begin_stage(kStageScanBwd, st);
     if (!scan_mma && scan_columns(units))
-      rc = launch_scan_bwd_cols(geo, p.total_tokens, units, kg, w, qg, sp.d_o, Aqk, ws.beta_c, gc, a->d_final_state,
-                                ws.dh, ws.dF, a->d_initial_state, ws.status, st);
+      rc = launch_scan_bwd_cols(geo, p.total_tokens, units, kg, w, qg, sp.d_o, Aqk, ws.beta_c, gc, a->d_final_state, ws.dh,
+                                ws.dF, a->d_initial_state, ws.status, pair.bwd ? pair.bwd : scan_columns(units), pair.bwd != 0, st);
     else if (!scan_mma)
       rc = launch_scan_bwd_tc(geo, p.total_tokens, units, kg, w, qg, sp.d_o, Aqk, ws.beta_c, gc, a->d_final_state,
-                              ws.dh, ws.dF, a->d_initial_state, ws.status, st);
+                              ws.dh, ws.dF, a->d_initial_state, ws.status, pair.bwd != 0, st);
     else if (vb == 128) rc = launch_scan_bwd<128>(sp, units, st);
     else if (vb == 64) rc = launch_scan_bwd<64>(sp, units, st);
     else rc = launch_scan_bwd<32>(sp, units, st);

@@ -461,6 +461,19 @@ int scan_columns(int units) {
   return 8L * units <= sms ? 8 : 4L * units <= sms ? 4 : 0;
 }
 
+// A scan is a chain of chunk steps that keeps few SMs busy, so two side by side cost little more than the longer one.  Each
+// CTA takes an SM of its own (two do not fit its shared memory), so the rule is the most CTAs a unit with which both run in one wave, the
+// backward's, whose step is the longer, before the forward's.  Lean step (forward + backward, decays of the layer's initialisation), one
+// scan after the other -> side by side, us: 4,096 tokens of 8 units 467 -> 403, 12 547 -> 481, 16 643 -> 584, 24 828 -> 761,
+// 32 978 -> 940, 36 1,057 -> 1,028; 2,048 tokens of 48 units 803 -> 722, 64 950 -> 874; 1,024 of 72 551 -> 510.  From 75 units on
+// the tensor-memory scans fill more than half the chip each.
+ScanPair scan_pair(int units) {
+  static constexpr ScanPair kPairs[] = {{8, 8}, {4, 8}, {4, 4}, {2, 4}, {2, 2}, {1, 1}};
+  for (const ScanPair& s : kPairs)
+    if (units * (s.fwd + s.bwd) <= sm_count()) return s;
+  return {0, 0};
+}
+
 template <int VB, bool kRecompute>
 static int launch_scan_fwd(const ScanParams& sp, int units, cudaStream_t st) {
   if (!set_smem(pkda_scan_fwd_kernel<VB, kRecompute>, scan::L<VB>::kSmem)) return PKDA_ERR_LAUNCH;
@@ -516,7 +529,8 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   begin_stage(kStageScanFwd, st);
   if (status && !scan_mma && scan_columns(units)) {
     rc = launch_scan_fwd_cols(geo, p.total_tokens, units, w, kg, u_ws, beta_c, gc, p.initial_state, h, v_new,
-                              recompute ? nullptr : ST, status, qg, Aqk, fuse_out ? o : nullptr, st);
+                              recompute ? nullptr : ST, status, qg, Aqk, fuse_out ? o : nullptr,
+                            recompute && scan_pair(units).fwd ? scan_pair(units).fwd : scan_columns(units), st);
     if (o_done) *o_done = fuse_out;
   } else if (status && !scan_mma) {
     rc = launch_scan_fwd_tc(geo, p.total_tokens, units, w, kg, u_ws, beta_c, gc, p.initial_state, h, v_new, ST,

@@ -251,6 +251,12 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" :: "n"(N));
 }
 
+// Of two kernels that may run side by side (launch_beside): the first lets the second start once all its CTAs are
+// running, the second waits for the first to end, and for its memory to be visible, before it ends itself.  Both
+// do nothing where the launch does not ask for it.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Copies a [rows x cols] bf16 tile (cols a multiple of 8) from global memory
 // with row stride gld (elements) into shared memory with row stride sld; rows
 // >= valid_rows are zero filled.  All threads of the CTA take part.

@@ -47,6 +47,24 @@ inline bool ensure_dynamic_smem(K kernel, int bytes, int carveout = -1) {
 // SMs of the current device (148, the B200's, where there is none).
 int sm_count();
 
+// Launches `kernel`; beside = true: it may start as soon as every CTA of the launch before it on the stream has called
+// launch_dependents() or ended, and has to call wait_prerequisites() before it ends (pkda_common.cuh).
+template <typename... P, typename... A>
+inline int launch_beside(void (*kernel)(P...), bool beside, int grid, int threads, int smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = beside ? 1 : 0;
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, args...);
+  return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+}
+
 // Upper limit for the kernels' direct block size (64 unless lowered through
 // pkda_set_direct_block_cap, a testing aid).
 int direct_block_cap();

@@ -1,5 +1,5 @@
-// Reverse scan of the state cotangent dS for few units.  Eight or four CTAs per (sequence, head), 16 or 32
-// value columns each.  Per chunk (last first) and group of 16 columns (transposed, see pkda_scan.cuh):
+// Reverse scan of the state cotangent dS for few units.  Eight, four or (beside a
+// recompute pass's scan) two CTAs per (sequence, head), 16, 32 or 64 value columns each.  Per chunk (last first) and group of 16 columns (transposed, see pkda_scan.cuh):
 //   chain warp    d     = bf16(dS)                      registers, A operand as they stand
 //                 dF^T  = d^T kg^T + dO^T P             64 + 20 mma.sync
 //                 dE    = -beta * bf16(dF)              registers, A operand as they stand
@@ -30,7 +30,7 @@ template <int NW> struct ScanBwdLay {
   static constexpr int oP = oDo + scanw::kBlk, oBeta = oP + scanw::kBlk, oGc = oBeta + 256;
   static constexpr int kTx = oGc + 512;
   static constexpr int kStage = (kTx + 1023) / 1024 * 1024;
-  static constexpr int kStages = 3;
+  static constexpr int kStages = NW == 4 ? 2 : 3;
   static constexpr int kSlot = 4096 + 2048;           // d and dF fragments of one group
   static constexpr int oSlots = kStages * kStage;     // [NW][2]
   static constexpr int oBar = oSlots + NW * 2 * kSlot;
@@ -221,19 +221,20 @@ pkda_scan_bwd_cols_kernel(const __grid_constant__ CUtensorMap tm_kg, const __gri
     }
   }
   if (!ok && lane == 0) atomicExch(p.status, 1);
+  wait_prerequisites();  // (what follows on the stream also reads what a scan beside this one leaves)
 }
 
 template <int NW>
-static int launch(const CUtensorMap (&tm)[5], const ScanBwdColsParams& sp, int units, cudaStream_t st) {
+static int launch(const CUtensorMap (&tm)[5], const ScanBwdColsParams& sp, int units, bool beside, cudaStream_t st) {
   using Y = ScanBwdLay<NW>;
   if (!ensure_dynamic_smem(pkda_scan_bwd_cols_kernel<NW>, Y::kSmem)) return PKDA_ERR_LAUNCH;
-  pkda_scan_bwd_cols_kernel<NW><<<units * Y::kSplit, Y::kThreads, Y::kSmem, st>>>(tm[0], tm[1], tm[2], tm[3], tm[4], sp);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return launch_beside(pkda_scan_bwd_cols_kernel<NW>, beside, units * Y::kSplit, Y::kThreads, Y::kSmem, st, tm[0], tm[1], tm[2],
+                       tm[3], tm[4], sp);
 }
 
 int launch_scan_bwd_cols(const Geo& geo, int total_tokens, int units, const bf16* kg, const bf16* w, const bf16* qg,
                          const bf16* d_o, const bf16* Aqk, const float* beta_c, const float* gc, const float* dST,
-                         bf16* dh, bf16* dF, float* dS0, int* status, cudaStream_t st) {
+                         bf16* dh, bf16* dF, float* dS0, int* status, int split, bool beside, cudaStream_t st) {
   const uint64_t H = geo.heads, tok = total_tokens;
   CUtensorMap tm[5];
   if (!scanw::rows_map(&tm[0], kg, H, tok, 2) || !scanw::rows_map(&tm[1], w, H, tok, 2) ||
@@ -242,7 +243,9 @@ int launch_scan_bwd_cols(const Geo& geo, int total_tokens, int units, const bf16
     return PKDA_ERR_LAUNCH;
   ScanBwdColsParams sp;
   sp.geo = geo; sp.beta_c = beta_c; sp.gc = gc; sp.dST = dST; sp.dh = dh; sp.dF = dF; sp.dS0 = dS0; sp.status = status;
-  return scan_columns(units) == 8 ? launch<1>(tm, sp, units, st) : launch<2>(tm, sp, units, st);
+  return split == 8   ? launch<1>(tm, sp, units, beside, st)
+         : split == 4 ? launch<2>(tm, sp, units, beside, st)
+                      : launch<4>(tm, sp, units, beside, st);
 }
 
 }  // namespace pkda

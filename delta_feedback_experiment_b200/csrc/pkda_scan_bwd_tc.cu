@@ -298,11 +298,12 @@ pkda_scan_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_kg, const __grid_
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, kCols);
+  wait_prerequisites();  // (what follows on the stream also reads what a scan beside this one leaves)
 }
 
 int launch_scan_bwd_tc(const Geo& geo, int total_tokens, int units, const bf16* kg, const bf16* w, const bf16* qg,
                        const bf16* d_o, const bf16* Aqk, const float* beta_c, const float* gc, const float* dST,
-                       bf16* dh, bf16* dF, float* dS0, int* status, cudaStream_t st) {
+                       bf16* dh, bf16* dF, float* dS0, int* status, bool beside, cudaStream_t st) {
   const uint64_t H = geo.heads, chunks = geo.total_chunks, tok = total_tokens;
   CUtensorMap tm_kg, tm_w, tm_qg, tm_do, tm_p, tm_dh, tm_df;
   {
@@ -327,9 +328,8 @@ int launch_scan_bwd_tc(const Geo& geo, int total_tokens, int units, const bf16* 
   sp.geo = geo; sp.beta_c = beta_c; sp.gc = gc; sp.dST = dST; sp.dF = dF; sp.dS0 = dS0; sp.status = status;
   if (!ensure_dynamic_smem(pkda_scan_bwd_tc_kernel, scanbtc::kSmem))
     return PKDA_ERR_LAUNCH;
-  pkda_scan_bwd_tc_kernel<<<units, scanbtc::kThreads, scanbtc::kSmem, st>>>(tm_kg, tm_w, tm_qg, tm_do, tm_p, tm_dh,
-                                                                             tm_df, sp);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return launch_beside(pkda_scan_bwd_tc_kernel, beside, units, scanbtc::kThreads, scanbtc::kSmem, st, tm_kg, tm_w, tm_qg, tm_do,
+                       tm_p, tm_dh, tm_df, sp);
 }
 
 }  // namespace pkda

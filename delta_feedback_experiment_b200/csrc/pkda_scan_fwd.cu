@@ -1,5 +1,5 @@
-// Forward state scan for few units, with the output formed on the way.  Eight or four CTAs per (sequence,
-// head), 16 or 32 value columns each.  Per 64-token chunk and group of 16 columns (transposed, see pkda_scan.cuh):
+// Forward state scan for few units, with the output formed on the way.  Eight, four or (a recompute pass
+// beside the backward's scan) two CTAs per (sequence, head), 16, 32 or 64 value columns each.  Per 64-token chunk and group of 16 columns (transposed, see pkda_scan.cuh):
 //   chain warp    h    = bf16(S)                   registers, A operand as they stand
 //                 S   *= Gam_last (per k)
 //                 E^T  = U^T I - h^T W^T           64 + 8 mma.sync
@@ -75,6 +75,7 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       }
     tc::fence_barrier_init();
   }
+  if (!kOut) launch_dependents();  // (a recompute pass lets the backward's scan run beside it)
   __syncthreads();
   bool ok = true;
 
@@ -270,10 +271,10 @@ static int launch(const CUtensorMap (&tm)[5], const ScanFwdParams& sp, int units
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 
-// o == NULL: h, v_new and the final state only.
+// o == NULL: h, v_new and the final state only.  split: CTAs per unit, 8, 4 or (without o) 2.
 int launch_scan_fwd_cols(const Geo& geo, int total_tokens, int units, const bf16* w, const bf16* kg, const bf16* u,
                          const float* beta_c, const float* gc, const float* S0, bf16* h, bf16* v_new, float* ST,
-                         int* status, const bf16* qg, const bf16* Aqk, bf16* o, cudaStream_t st) {
+                         int* status, const bf16* qg, const bf16* Aqk, bf16* o, int split, cudaStream_t st) {
   const uint64_t H = geo.heads, tok = total_tokens;
   CUtensorMap tm[5];
   if (!scanw::rows_map(&tm[0], w, H, tok, 2) || !scanw::rows_map(&tm[1], kg, H, tok, 2) ||
@@ -287,9 +288,10 @@ int launch_scan_fwd_cols(const Geo& geo, int total_tokens, int units, const bf16
   ScanFwdParams sp;
   sp.geo = geo; sp.beta_c = beta_c; sp.gc = gc; sp.S0 = S0; sp.h = h; sp.v_new = v_new; sp.ST = ST; sp.o = o;
   sp.status = status;
-  const int split = scan_columns(units);
   if (o) return split == 8 ? launch<1, true>(tm, sp, units, st) : launch<2, true>(tm, sp, units, st);
-  return split == 8 ? launch<1, false>(tm, sp, units, st) : launch<2, false>(tm, sp, units, st);
+  return split == 8   ? launch<1, false>(tm, sp, units, st)
+         : split == 4 ? launch<2, false>(tm, sp, units, st)
+                      : launch<4, false>(tm, sp, units, st);
 }
 
 }  // namespace pkda

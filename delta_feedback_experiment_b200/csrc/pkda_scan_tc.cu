@@ -110,6 +110,7 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
 
   const size_t sbase = ((size_t)n * H + h) * kD * kD;
 
+  if (kRecompute) launch_dependents();  // (the backward's scan may run beside it)
   if (warp == 0) tc::tmem_alloc(tmem_slot, kCols);
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) tc::mbar_init(bar_full0 + 8 * s, 1);
