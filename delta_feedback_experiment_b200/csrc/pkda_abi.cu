@@ -42,6 +42,7 @@ bool dynamic_smem_once(const void* kernel, int bytes, int carveout) {
 int stage_variant(int stage) { return (stage >= 0 && stage < kStageCount) ? g_variant[stage] : 0; }
 
 __global__ void pkda_status_guard_kernel(const int* status, bf16* out0, bf16* out1, bf16* out2, size_t n) {
+  after_previous();
   if (*status == 0) return;
   const bf16 nan = __float2bfloat16(__int_as_float(0x7fc00000));
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -53,8 +54,8 @@ __global__ void pkda_status_guard_kernel(const int* status, bf16* out0, bf16* ou
 
 int launch_status_guard(const int* status, void* out0, void* out1, void* out2, size_t n, cudaStream_t st) {
   begin_stage(kStageStatusGuard, st);
-  pkda_status_guard_kernel<<<4, 256, 0, st>>>(status, static_cast<bf16*>(out0), static_cast<bf16*>(out1),
-                                              static_cast<bf16*>(out2), n);
+  launch_kernel(pkda_status_guard_kernel, 4, 256, 0, st, status, static_cast<bf16*>(out0), static_cast<bf16*>(out1),
+                static_cast<bf16*>(out2), n);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

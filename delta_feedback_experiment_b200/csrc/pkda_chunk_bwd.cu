@@ -51,6 +51,7 @@ template <int VB> struct L {
 template <int VB>
 __global__ void __launch_bounds__(scanb::threads<VB>())
 pkda_scan_bwd_kernel(const ScanBwdParams p) {
+  after_previous();
   using Lay = scanb::L<VB>;
   constexpr int ldv = Lay::ldv, NT = 4, kT = scanb::threads<VB>();
   extern __shared__ __align__(128) unsigned char smem[];
@@ -1035,6 +1036,8 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
 // grid (chunks, heads): one item per CTA; or, with a work list, a few persistent CTAs that walk it.
 __global__ void __launch_bounds__(ib::kThreads, 1)
 pkda_intra_bwd_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdMaps maps) {
+  if (!p.slow_list) wait_prerequisites();  // (with a work list it runs beside the tensor-memory kernel)
+  launch_dependents();
   if (!p.slow_list) {
     intra_bwd_item(p, maps, blockIdx.x, blockIdx.y);
     return;
@@ -1052,6 +1055,7 @@ pkda_intra_bwd_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdMa
     tc::fence_proxy_async();  // the sums of ddt_bias lie where the next item's copies land
     __syncthreads();  // the next item reuses every shared-memory region (and s_item)
   }
+  wait_prerequisites();
 }
 
 // ------------------------------------------------------------------ preconditioner backward
@@ -1096,6 +1100,7 @@ constexpr int kSmem = kThreads * (kRows * (8 + 16 + 16) + 16 + 16);
 
 __global__ void __launch_bounds__(atkb::kThreads, 2)
 pkda_atk_bwd_kernel(const AtkBwdParams p, int n_tiles) {
+  after_previous();
   using namespace atkb;
   extern __shared__ __align__(16) unsigned char slots[];
   __shared__ __align__(16) float sEnd[8][kD];  // per row block: end value of its zero-start scan
@@ -1271,6 +1276,7 @@ pkda_atk_bwd_kernel(const AtkBwdParams p, int n_tiles) {
 // Sequential carry over a sequence's chunks, last to first.
 __global__ void __launch_bounds__(kD)
 pkda_atk_bwd_carry_kernel(Geo geo, const float* c_loc, const float* sa, float* lam_in, float* dA0) {
+  after_previous();
   const int n = blockIdx.x, h = blockIdx.y, H = geo.heads, c = threadIdx.x;
   const SeqInfo sq = seq_info(geo, n);
   float lam = 0.f;
@@ -1302,16 +1308,7 @@ constexpr int kReduceSubs = 8;
 __global__ void __launch_bounds__(kD * kReduceSubs)
 pkda_param_reduce_kernel(Geo geo, const float* partA, const float* partB, const float* partC, float* dA_log,
                          float* ddt_bias, float* dcentre, const int* status, bf16* g0, bf16* g1, bf16* g2, size_t guard_n) {
-  // The backward's last kernel: if any kernel of the call gave up, the heads of dq, dk and dv become
-  // NaN, so that a caller who never reads the status word cannot take partial gradients for complete ones.
-  if (blockIdx.x == 0 && *status != 0) {
-    const bf16 nan = __float2bfloat16(__int_as_float(0x7fc00000));
-    for (size_t i = threadIdx.x; i < guard_n; i += blockDim.x) {
-      g0[i] = nan;
-      g1[i] = nan;
-      g2[i] = nan;
-    }
-  }
+  launch_dependents();  // (it runs beside the pass in front of it)
   __shared__ float sSub[kReduceSubs][kD];
   __shared__ float sR[2][4];
   const int h = blockIdx.x, H = geo.heads, tid = threadIdx.x, c = tid % kD, sub = tid / kD;
@@ -1345,6 +1342,17 @@ pkda_param_reduce_kernel(Geo geo, const float* partA, const float* partB, const 
   if (tid == 0) {
     dA_log[h] = sR[0][0] + sR[0][1] + sR[0][2] + sR[0][3];
     dcentre[h] = sR[1][0] + sR[1][1] + sR[1][2] + sR[1][3];
+  }
+  // The backward's last kernel: if any kernel of the call gave up, the heads of dq, dk and dv become
+  // NaN, so that a caller who never reads the status word cannot take partial gradients for complete ones.
+  wait_prerequisites();
+  if (blockIdx.x == 0 && *reinterpret_cast<const volatile int*>(status) != 0) {
+    const bf16 nan = __float2bfloat16(__int_as_float(0x7fc00000));
+    for (size_t i = tid; i < guard_n; i += blockDim.x) {
+      g0[i] = nan;
+      g1[i] = nan;
+      g2[i] = nan;
+    }
   }
 }
 
@@ -1411,7 +1419,7 @@ static bool set_smem(K kernel, int bytes) {
 template <int VB>
 static int launch_scan_bwd(const ScanBwdParams& sp, int units, cudaStream_t st) {
   if (!set_smem(pkda_scan_bwd_kernel<VB>, scanb::L<VB>::kSmem)) return PKDA_ERR_LAUNCH;
-  pkda_scan_bwd_kernel<VB><<<units * (kD / VB), scanb::threads<VB>(), scanb::L<VB>::kSmem, st>>>(sp);
+  launch_kernel(pkda_scan_bwd_kernel<VB>, units * (kD / VB), scanb::threads<VB>(), scanb::L<VB>::kSmem, st, sp);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 
@@ -1538,7 +1546,7 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   }
   if (!set_smem(pkda_intra_bwd_kernel, ib::kSmem)) return PKDA_ERR_LAUNCH;
   begin_stage(ip.slow_list ? kStageIntraBwdRest : kStageIntraBwd, st);
-  pkda_intra_bwd_kernel<<<gridc, ib::kThreads, ib::kSmem, st>>>(ip, maps);
+  launch_kernel(pkda_intra_bwd_kernel, gridc, ib::kThreads, ib::kSmem, st, ip, maps);
   PKDA_CHECK_LAUNCH();
 
   AtkBwdParams ap;
@@ -1549,18 +1557,18 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   const int atk_tiles = geo.total_chunks * p.heads;
   const int atk_grid = atk_tiles < 2 * sms ? atk_tiles : 2 * sms;  // persistent: two CTAs per SM
   begin_stage(kStageAtkBwdCarry, st);
-  pkda_atk_bwd_carry_kernel<<<dim3(p.n_seqs, p.heads), kD, 0, st>>>(geo, ws.c_loc, a->sa_atk, ws.lam_in,
-                                                                   a->d_initial_A_state);
+  launch_kernel(false, pkda_atk_bwd_carry_kernel, dim3(p.n_seqs, p.heads), kD, 0, st, geo, ws.c_loc, a->sa_atk, ws.lam_in,
+                a->d_initial_A_state);
   PKDA_CHECK_LAUNCH();
   begin_stage(kStageAtkBwdFinal, st);
   if (!set_smem(pkda_atk_bwd_kernel, atkb::kSmem)) return PKDA_ERR_LAUNCH;
-  pkda_atk_bwd_kernel<<<atk_grid, atkb::kThreads, atkb::kSmem, st>>>(ap, atk_tiles);
+  launch_kernel(pkda_atk_bwd_kernel, atk_grid, atkb::kThreads, atkb::kSmem, st, ap, atk_tiles);
   PKDA_CHECK_LAUNCH();
   begin_stage(kStageParamReduce, st);
   const size_t guard_n = std::min<size_t>((size_t)p.total_tokens * p.heads * kD, 4096);
-  pkda_param_reduce_kernel<<<p.heads, kD * kReduceSubs, 0, st>>>(
-      geo, ws.partA, ws.partB, ws.partC, a->dA_log, a->ddt_bias, a->dlog_atk_scale, ws.status,
-      static_cast<bf16*>(a->dq), static_cast<bf16*>(a->dk), static_cast<bf16*>(a->dv), guard_n);
+  launch_kernel(pkda_param_reduce_kernel, p.heads, kD * kReduceSubs, 0, st, geo, ws.partA, ws.partB, ws.partC, a->dA_log,
+                a->ddt_bias, a->dlog_atk_scale, ws.status, static_cast<bf16*>(a->dq), static_cast<bf16*>(a->dk),
+                static_cast<bf16*>(a->dv), guard_n);
   PKDA_CHECK_LAUNCH();
   return PKDA_OK;
 }

@@ -22,6 +22,7 @@ namespace pkda {
 
 // ------------------------------------------------------------------ small kernels
 __global__ void pkda_chunk_offsets_kernel(const int* cu, int n_seqs, int* offs) {
+  after_previous();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     int acc = 0;
     offs[0] = 0;
@@ -33,6 +34,7 @@ __global__ void pkda_chunk_offsets_kernel(const int* cu, int n_seqs, int* offs) 
 }
 
 __global__ void pkda_pack_beta_kernel(Geo geo, const bf16* beta, float* beta_c) {
+  after_previous();
   int n, tok0, valid;
   if (!chunk_lookup(geo, blockIdx.x, n, tok0, valid)) return;
   const int H = geo.heads;
@@ -52,6 +54,7 @@ __global__ void pkda_pack_beta_kernel(Geo geo, const bf16* beta, float* beta_c) 
 __global__ void __launch_bounds__(256)
 pkda_atk_local_kernel(Geo geo, const bf16* k, const float* g_atk, const bf16* beta_atk, const bf16* beta,
                       float* ac_local, float* sa, float* beta_c, int* zero) {
+  after_previous();
   __shared__ __align__(16) float sEnd[8][kD];
   __shared__ float sDec[8], sSum[8];
   if (blockIdx.x == 0 && threadIdx.x < 8) zero[threadIdx.x] = 0;  // status word and cursors of the kernels behind
@@ -132,6 +135,7 @@ pkda_atk_local_kernel(Geo geo, const bf16* k, const float* g_atk, const bf16* be
 __global__ void __launch_bounds__(kD)
 pkda_atk_carry_kernel(Geo geo, const float* ac_local, const float* sa, const float* A0,
                       float* a_start, float* AT) {
+  after_previous();
   const int n = blockIdx.x, h = blockIdx.y, H = geo.heads, c = threadIdx.x;
   const SeqInfo sq = seq_info(geo, n);
   float A = A0 ? A0[((size_t)n * H + h) * kD + c] : 0.f;
@@ -185,6 +189,7 @@ template <int VB> struct L {
 template <int VB, bool kRecompute>
 __global__ void __launch_bounds__(scan::threads<VB>())
 pkda_scan_fwd_kernel(const ScanParams p) {
+  after_previous();
   using Lay = scan::L<VB>;
   constexpr int ldv = Lay::ldv, NT = 4, kT = scan::threads<VB>();
   extern __shared__ __align__(128) unsigned char smem[];
@@ -335,6 +340,7 @@ constexpr int kSmem = oF + kTileBytes;
 
 __global__ void __launch_bounds__(outk::kThreads)
 pkda_out_fwd_kernel(const OutParams p) {
+  after_previous();
   using namespace outk;
   extern __shared__ __align__(128) unsigned char smem[];
   bf16* sQg = reinterpret_cast<bf16*>(smem + oQg);
@@ -477,7 +483,7 @@ ScanPair scan_pair(int units) {
 template <int VB, bool kRecompute>
 static int launch_scan_fwd(const ScanParams& sp, int units, cudaStream_t st) {
   if (!set_smem(pkda_scan_fwd_kernel<VB, kRecompute>, scan::L<VB>::kSmem)) return PKDA_ERR_LAUNCH;
-  pkda_scan_fwd_kernel<VB, kRecompute><<<units * (kD / VB), scan::threads<VB>(), scan::L<VB>::kSmem, st>>>(sp);
+  launch_kernel(pkda_scan_fwd_kernel<VB, kRecompute>, units * (kD / VB), scan::threads<VB>(), scan::L<VB>::kSmem, st, sp);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 
@@ -549,13 +555,13 @@ int run_prologue(const pkda_problem& p, int* chunk_offsets, float* beta_c, Geo* 
   // beta_c == nullptr: the caller fills the chunk-major beta itself (the forward does, in its first kernel)
   if (p.cu_seqlens) {
     begin_stage(kStageOffsets, st);
-    pkda_chunk_offsets_kernel<<<1, 32, 0, st>>>(p.cu_seqlens, p.n_seqs, chunk_offsets);
+    launch_kernel(pkda_chunk_offsets_kernel, 1, 32, 0, st, p.cu_seqlens, p.n_seqs, chunk_offsets);
     PKDA_CHECK_LAUNCH();
   }
   *geo = make_geo(p, chunk_offsets);
   if (beta_c) {
     begin_stage(kStagePackBeta, st);
-    pkda_pack_beta_kernel<<<geo->total_chunks, 256, 0, st>>>(*geo, static_cast<const bf16*>(p.beta), beta_c);
+    launch_kernel(pkda_pack_beta_kernel, geo->total_chunks, 256, 0, st, *geo, static_cast<const bf16*>(p.beta), beta_c);
     PKDA_CHECK_LAUNCH();
   }
   return PKDA_OK;
@@ -586,13 +592,13 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
   const bool chained = forward_chain_possible(p);
   if (!chained) {
     begin_stage(kStageAtkLocal, st);
-    pkda_atk_local_kernel<<<geo.total_chunks * p.heads, 256, 0, st>>>(geo, static_cast<const bf16*>(p.k), p.g_atk,
-                                                 static_cast<const bf16*>(p.beta_atk), static_cast<const bf16*>(p.beta),
-                                                 a->ac_atk, a->sa_atk, ws.beta_c, ws.status);
+    launch_kernel(pkda_atk_local_kernel, geo.total_chunks * p.heads, 256, 0, st, geo, static_cast<const bf16*>(p.k), p.g_atk,
+                  static_cast<const bf16*>(p.beta_atk), static_cast<const bf16*>(p.beta), a->ac_atk, a->sa_atk, ws.beta_c,
+                  ws.status);
     PKDA_CHECK_LAUNCH();
     begin_stage(kStageAtkCarry, st);
-    pkda_atk_carry_kernel<<<dim3(p.n_seqs, p.heads), kD, 0, st>>>(geo, a->ac_atk, a->sa_atk, p.initial_A_state,
-                                                                 a->a_atk, a->final_A_state);
+    launch_kernel(pkda_atk_carry_kernel, dim3(p.n_seqs, p.heads), kD, 0, st, geo, a->ac_atk, a->sa_atk, p.initial_A_state, a->a_atk,
+                  a->final_A_state);
     PKDA_CHECK_LAUNCH();
   }
 
@@ -627,7 +633,7 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
   op.beta_c = ws.beta_c; op.o = static_cast<bf16*>(a->o);
   if (!set_smem(pkda_out_fwd_kernel, outk::kSmem)) return PKDA_ERR_LAUNCH;
   begin_stage(kStageOutFwd, st);
-  pkda_out_fwd_kernel<<<dim3(geo.total_chunks, p.heads), outk::kThreads, outk::kSmem, st>>>(op);
+  launch_kernel(pkda_out_fwd_kernel, dim3(geo.total_chunks, p.heads), outk::kThreads, outk::kSmem, st, op);
   PKDA_CHECK_LAUNCH();
   return launch_status_guard(ws.status, a->o, nullptr, nullptr, guard_n, st);
 }

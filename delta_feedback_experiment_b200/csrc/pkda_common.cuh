@@ -251,11 +251,18 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" :: "n"(N));
 }
 
-// Of two kernels that may run side by side (launch_beside): the first lets the second start once all its CTAs are
-// running, the second waits for the first to end, and for its memory to be visible, before it ends itself.  Both
-// do nothing where the launch does not ask for it.
+// Every kernel is launched so that its CTAs may be set up while the launch in front of it on the stream still runs
+// (launch_kernel): once all CTAs of that launch have called launch_dependents() or have ended.  wait_prerequisites() then waits until
+// that launch has ended and its memory is visible; a kernel calls it before it touches memory, or, where it runs beside the one in
+// front of it because neither needs anything of the other, before it ends.  So when a launch has ended, all before it have.  Calling
+// launch_dependents() after wait_prerequisites() makes a kernel that runs beside find everything in front of both done.  A kernel
+// that allocates tensor memory does so before launch_dependents(): it must not wait for columns that one behind it holds.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() {
+  wait_prerequisites();
+  launch_dependents();
+}
 
 // Copies a [rows x cols] bf16 tile (cols a multiple of 8) from global memory
 // with row stride gld (elements) into shared memory with row stride sld; rows

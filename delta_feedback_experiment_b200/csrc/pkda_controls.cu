@@ -36,6 +36,7 @@ constexpr int kCtrlThreads = 256;
 template <typename T>
 __global__ void __launch_bounds__(kCtrlThreads)
 pkda_controls_fwd_kernel(const CtrlParams p) {
+  after_previous();
   const long long n = p.rows * p.heads;
   const T* packed = static_cast<const T*>(p.packed);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -59,6 +60,7 @@ __host__ __device__ inline int ctrl_rows(int heads) { return heads >= 512 ? 1 : 
 template <typename T>
 __global__ void __launch_bounds__(kCtrlThreads)
 pkda_controls_bwd_kernel(const CtrlParams p) {
+  after_previous();
   extern __shared__ float sAcc[];  // [2][H] sums of the CTA, then [2][rows][H] contributions
   const int H = p.heads, D = p.hidden, total = p.total, tid = threadIdx.x;
   const int R = ctrl_rows(H);
@@ -133,6 +135,7 @@ pkda_controls_bwd_kernel(const CtrlParams p) {
 // One CTA per sum: strided partial sums, then a tree (fixed order).
 __global__ void __launch_bounds__(128)
 pkda_controls_reduce_kernel(const float* part, float* dA_log, float* ddt_bias, int heads, int groups) {
+  after_previous();
   __shared__ float s[128];
   const int i = blockIdx.x, tid = threadIdx.x;
   float a = 0.f;
@@ -151,6 +154,7 @@ template <typename T>
 __global__ void __launch_bounds__(kCtrlThreads)
 pkda_pack_control_kernel(const T* g0, const T* g1, const T* g2, const T* g3, const T* g4, T* out, long long rows,
                          int s0, int s1, int s2, int s3, int s4) {
+  after_previous();
   const int total = s0 + s1 + s2 + s3 + s4;
   const long long n = rows * total;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -194,8 +198,8 @@ int controls_fwd(const pkda_controls_args* a, cudaStream_t st) {
   const long long blocks = (n + kCtrlThreads - 1) / kCtrlThreads, most = 16LL * sm_count();
   const int grid = (int)(blocks < most ? blocks : most);
   begin_stage(kStageControlsFwd, st);
-  if (a->dtype == PKDA_BF16) pkda_controls_fwd_kernel<bf16><<<grid, kCtrlThreads, 0, st>>>(p);
-  else pkda_controls_fwd_kernel<float><<<grid, kCtrlThreads, 0, st>>>(p);
+  if (a->dtype == PKDA_BF16) launch_kernel(pkda_controls_fwd_kernel<bf16>, grid, kCtrlThreads, 0, st, p);
+  else launch_kernel(pkda_controls_fwd_kernel<float>, grid, kCtrlThreads, 0, st, p);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
@@ -225,12 +229,12 @@ int controls_bwd(const pkda_controls_args* a, cudaStream_t st) {
                          reinterpret_cast<uintptr_t>(a->d_packed);
   p.pairs = !(a->heads & 1) && !(a->hidden & 1) && ptrs % (a->dtype == PKDA_BF16 ? 4 : 8) == 0;
   begin_stage(kStageControlsBwd, st);
-  if (a->dtype == PKDA_BF16) pkda_controls_bwd_kernel<bf16><<<grid, kCtrlThreads, smem, st>>>(p);
-  else pkda_controls_bwd_kernel<float><<<grid, kCtrlThreads, smem, st>>>(p);
+  if (a->dtype == PKDA_BF16) launch_kernel(pkda_controls_bwd_kernel<bf16>, grid, kCtrlThreads, smem, st, p);
+  else launch_kernel(pkda_controls_bwd_kernel<float>, grid, kCtrlThreads, smem, st, p);
   end_stage(st);
   begin_stage(kStageControlsBwd, st);
-  pkda_controls_reduce_kernel<<<2 * a->heads, 128, 0, st>>>(p.part, a->dA_log_precond, a->ddt_bias_precond,
-                                                                         a->heads, grid);
+  launch_kernel(pkda_controls_reduce_kernel, 2 * a->heads, 128, 0, st, p.part, a->dA_log_precond, a->ddt_bias_precond, a->heads,
+                grid);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
@@ -250,16 +254,15 @@ int pack_control_gradients(const pkda_pack_control_args* a, cudaStream_t st) {
   const int grid = (int)(blocks < most ? blocks : most);
   begin_stage(kStagePackControl, st);
   if (a->dtype == PKDA_BF16)
-    pkda_pack_control_kernel<bf16><<<grid, kCtrlThreads, 0, st>>>(
-        static_cast<const bf16*>(a->grads[0]), static_cast<const bf16*>(a->grads[1]), static_cast<const bf16*>(a->grads[2]),
-        static_cast<const bf16*>(a->grads[3]), static_cast<const bf16*>(a->grads[4]), static_cast<bf16*>(a->out), a->rows,
-        a->sizes[0], a->sizes[1], a->sizes[2], a->sizes[3], a->sizes[4]);
+    launch_kernel(pkda_pack_control_kernel<bf16>, grid, kCtrlThreads, 0, st, static_cast<const bf16*>(a->grads[0]),
+                  static_cast<const bf16*>(a->grads[1]), static_cast<const bf16*>(a->grads[2]), static_cast<const
+                  bf16*>(a->grads[3]), static_cast<const bf16*>(a->grads[4]), static_cast<bf16*>(a->out), a->rows, a->sizes[0],
+                  a->sizes[1], a->sizes[2], a->sizes[3], a->sizes[4]);
   else
-    pkda_pack_control_kernel<float><<<grid, kCtrlThreads, 0, st>>>(
-        static_cast<const float*>(a->grads[0]), static_cast<const float*>(a->grads[1]),
-        static_cast<const float*>(a->grads[2]), static_cast<const float*>(a->grads[3]),
-        static_cast<const float*>(a->grads[4]), static_cast<float*>(a->out), a->rows, a->sizes[0], a->sizes[1],
-        a->sizes[2], a->sizes[3], a->sizes[4]);
+    launch_kernel(pkda_pack_control_kernel<float>, grid, kCtrlThreads, 0, st, static_cast<const float*>(a->grads[0]),
+                  static_cast<const float*>(a->grads[1]), static_cast<const float*>(a->grads[2]), static_cast<const
+                  float*>(a->grads[3]), static_cast<const float*>(a->grads[4]), static_cast<float*>(a->out), a->rows, a->sizes[0],
+                  a->sizes[1], a->sizes[2], a->sizes[3], a->sizes[4]);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

@@ -41,6 +41,7 @@ template <typename T> __device__ __forceinline__ float round_to(float x) { retur
 template <int D, typename T>
 __global__ void __launch_bounds__(RecCfg<D>::kThreads, D == 128 ? 2 : 1)
 pkda_decode_step_kernel(const DecodeParams p) {
+  after_previous();
   using Cfg = RecCfg<D>;
   constexpr int VQ = Cfg::kVQ, KW = Cfg::kKW, R = Cfg::kR, kThreads = Cfg::kThreads;
   constexpr int kWarps = kThreads / 32;
@@ -220,7 +221,7 @@ pkda_decode_step_kernel(const DecodeParams p) {
 template <int D, typename T>
 static int launch_decode(const DecodeParams& dp, int stage, cudaStream_t st) {
   begin_stage(stage, st);
-  pkda_decode_step_kernel<D, T><<<dp.batch * dp.heads, RecCfg<D>::kThreads, 0, st>>>(dp);
+  launch_kernel(pkda_decode_step_kernel<D, T>, dp.batch * dp.heads, RecCfg<D>::kThreads, 0, st, dp);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

@@ -96,6 +96,7 @@ struct IntraBwdTcMaps {
 __global__ void __launch_bounds__(256)
 pkda_bwd_classify_kernel(Geo geo, const float* gc, int direct_cap, int2* fast_list, int* slow_list, int* counts,
                          const bf16* beta, float* beta_c) {
+  after_previous();
   __shared__ int sKind[64], sTok[64];
   const int H = geo.heads, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int items = geo.total_chunks * H;
@@ -145,6 +146,7 @@ pkda_bwd_classify_kernel(Geo geo, const float* gc, int direct_cap, int2* fast_li
 
 __global__ void __launch_bounds__(ibtc::kThreads, 1)
 pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdTcMaps maps) {
+  wait_prerequisites();
   using namespace ibtc;
   extern __shared__ unsigned char smem_raw[];
   const int n_items = *p.fast_count;
@@ -224,6 +226,7 @@ pkda_intra_bwd_tc_kernel(const IntraBwdParams p, const __grid_constant__ IntraBw
   if (warp == 1) tc::tmem_alloc(tmem_slot, kCols);
   tc::tc_fence_before();
   __syncthreads();
+  launch_dependents();
   tc::tc_fence_after();
   // The next item's list entry waits in shared memory from the top of an item on: loaded where it is
   // needed, it and the chunk lookup that the entry saves cost every item two to four dependent memory round
@@ -670,8 +673,8 @@ int launch_bwd_classify(const Geo& geo, const float* gc, int direct_cap, int2* f
                         const bf16* beta, float* beta_c, cudaStream_t st) {
   const int items = geo.total_chunks * geo.heads;
   begin_stage(kStageBwdClassify, st);
-  pkda_bwd_classify_kernel<<<(items + 63) / 64, 256, 0, st>>>(geo, gc, direct_cap, fast_list, slow_list, counts, beta,
-                                                             beta_c);
+  launch_kernel(pkda_bwd_classify_kernel, (items + 63) / 64, 256, 0, st, geo, gc, direct_cap, fast_list, slow_list, counts, beta,
+                beta_c);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
@@ -704,7 +707,7 @@ int launch_intra_bwd_tc(const IntraBwdParams& ip, cudaStream_t st) {
   const int items = ip.geo.total_chunks * ip.geo.heads;
   begin_stage(kStageIntraBwd, st);
   const int sms = sm_count();
-  pkda_intra_bwd_tc_kernel<<<items < sms ? items : sms, ibtc::kThreads, ibtc::kSmem, st>>>(ip, maps);
+  launch_kernel(false, pkda_intra_bwd_tc_kernel, items < sms ? items : sms, ibtc::kThreads, ibtc::kSmem, st, ip, maps);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

@@ -100,6 +100,7 @@ __device__ __forceinline__ uint32_t ld_u16(const bf16* p) {
 // Before a chained launch: every word of the hand-over to kNotYet, the status word and the cursors to zero.
 // (By single words: the caller's a_chain need not start on a 16-byte boundary.)
 __global__ void __launch_bounds__(256) pkda_chain_init_kernel(uint32_t* a_chain, size_t n, int* zero) {
+  after_previous();
   if (blockIdx.x == 0 && threadIdx.x < 8) zero[threadIdx.x] = 0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) a_chain[i] = kNotYet;
 }
@@ -272,6 +273,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
                          const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_g,
                          const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_q,
                          const IntraParams p) {
+  wait_prerequisites();
   using namespace intratc;
   extern __shared__ unsigned char smem_raw[];
   const int H = p.geo.heads;
@@ -317,6 +319,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   if (warp == 1) tc::tmem_alloc(tmem_slot, kCols);
   tc::tc_fence_before();
   __syncthreads();
+  launch_dependents();
   tc::tc_fence_after();
   const uint32_t tmem = tc::uniform(*reinterpret_cast<volatile uint32_t*>(tiles + oBar + 16));
   const int warp_u = (int)tc::uniform(warp);
@@ -904,7 +907,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 int launch_chain_init(float* a_chain, size_t items, int* zero, cudaStream_t st) {
   const size_t n = items * kD, most = 8 * (size_t)sm_count(), blocks = (n + 255) / 256;
   begin_stage(kStageChainInit, st);
-  pkda_chain_init_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, st>>>(reinterpret_cast<uint32_t*>(a_chain), n, zero);
+  launch_kernel(pkda_chain_init_kernel, (unsigned)(blocks < most ? blocks : most), 256, 0, st, reinterpret_cast<uint32_t*>(a_chain),
+                n, zero);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
@@ -933,13 +937,13 @@ int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) 
   if (recompute) {
     if (!ensure_dynamic_smem(pkda_intra_fwd_tc_kernel<true>, intratc::kSmem, 100))
       return PKDA_ERR_LAUNCH;
-    pkda_intra_fwd_tc_kernel<true><<<grid, intratc::kThreads, intratc::kSmem, st>>>(tm_v, tm_akk, tm_aqk, tm_w, tm_u, tm_g,
-                                                                                  tm_k, tm_q, ip);
+    launch_kernel(false, pkda_intra_fwd_tc_kernel<true>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_aqk, tm_w, tm_u,
+                  tm_g, tm_k, tm_q, ip);
   } else {
     if (!ensure_dynamic_smem(pkda_intra_fwd_tc_kernel<false>, intratc::kSmem, 100))
       return PKDA_ERR_LAUNCH;
-    pkda_intra_fwd_tc_kernel<false><<<grid, intratc::kThreads, intratc::kSmem, st>>>(tm_v, tm_akk, tm_aqk, tm_w, tm_u, tm_g,
-                                                                                  tm_k, tm_q, ip);
+    launch_kernel(false, pkda_intra_fwd_tc_kernel<false>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_aqk, tm_w, tm_u,
+                  tm_g, tm_k, tm_q, ip);
   }
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

@@ -47,22 +47,30 @@ inline bool ensure_dynamic_smem(K kernel, int bytes, int carveout = -1) {
 // SMs of the current device (148, the B200's, where there is none).
 int sm_count();
 
-// Launches `kernel`; beside = true: it may start as soon as every CTA of the launch before it on the stream has called
-// launch_dependents() or ended, and has to call wait_prerequisites() before it ends (pkda_common.cuh).
+// Launches `kernel` so that it is set up while the launch in front of it still runs.  Every kernel launched by this calls
+// wait_prerequisites() (pkda_common.cuh).
+// early = false: only behind the end of the launch in front.  The large kernels whose CTAs fill an SM's shared memory are better off
+// so (their CTAs would come to lie where room appears first): 1 x 8,191 tokens of 16 heads forward 313 -> 308 us, a lean step of
+// 2 x 4,096 tokens of 12 heads 785 -> 775.  Early: a decoding step of 8 units 6.1 -> 5.3 us, 4 x 48 tokens of 16 heads 26.6 -> 24.9,
+// the norm gate forward + backward at 8 x 4,096 tokens of 16 heads 197 -> 192.5.
 template <typename... P, typename... A>
-inline int launch_beside(void (*kernel)(P...), bool beside, int grid, int threads, int smem, cudaStream_t st, const A&... args) {
+inline int launch_kernel(bool early, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = beside ? 1 : 0;
+  cfg.numAttrs = early ? 1 : 0;
   const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, args...);
   return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+}
+template <typename... P, typename... A>
+inline int launch_kernel(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+  return launch_kernel(true, kernel, grid, threads, smem, st, args...);
 }
 
 // Upper limit for the kernels' direct block size (64 unless lowered through

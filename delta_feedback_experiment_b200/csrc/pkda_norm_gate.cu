@@ -93,6 +93,7 @@ __device__ __forceinline__ void copy_unit(T* slot, const T* g, bool ok) {
 template <typename T>
 __global__ void __launch_bounds__(ng::kThreads)
 pkda_norm_gate_fwd_kernel(const NormGateParams p) {
+  after_previous();
   using namespace ng;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* ring = reinterpret_cast<T*>(smem_raw);
@@ -152,6 +153,7 @@ pkda_norm_gate_fwd_kernel(const NormGateParams p) {
 template <typename T>
 __global__ void __launch_bounds__(ng::kThreads)
 pkda_norm_gate_bwd_kernel(const NormGateParams p) {
+  after_previous();
   using namespace ng;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* ring = reinterpret_cast<T*>(smem_raw);
@@ -253,6 +255,7 @@ pkda_norm_gate_bwd_kernel(const NormGateParams p) {
 // Sums the per-CTA partials: thread (sub, c) adds every kSub-th partial of channel c,
 // then the kSub sub-sums are added in order.
 __global__ void __launch_bounds__(1024) pkda_norm_gate_dw_kernel(const float* part, float* dw, int dim, int groups) {
+  after_previous();
   __shared__ float sSub[1024];
   const int c = threadIdx.x % dim, sub = threadIdx.x / dim, nsub = 1024 / dim;
   float a = 0.f;
@@ -307,13 +310,13 @@ int norm_gate_fwd(const pkda_norm_gate_args* a, cudaStream_t st) {
     if (!ng_allow_smem(pkda_norm_gate_fwd_kernel<bf16>, smem)) return PKDA_ERR_LAUNCH;
     const int grid = ng_grid(*a, pkda_norm_gate_fwd_kernel<bf16>, smem);
     begin_stage(kStageNormGateFwd, st);
-    pkda_norm_gate_fwd_kernel<bf16><<<grid, ng::kThreads, smem, st>>>(p);
+    launch_kernel(pkda_norm_gate_fwd_kernel<bf16>, grid, ng::kThreads, smem, st, p);
   } else {
     constexpr int smem = ng::fwd_smem<float>();
     if (!ng_allow_smem(pkda_norm_gate_fwd_kernel<float>, smem)) return PKDA_ERR_LAUNCH;
     const int grid = ng_grid(*a, pkda_norm_gate_fwd_kernel<float>, smem);
     begin_stage(kStageNormGateFwd, st);
-    pkda_norm_gate_fwd_kernel<float><<<grid, ng::kThreads, smem, st>>>(p);
+    launch_kernel(pkda_norm_gate_fwd_kernel<float>, grid, ng::kThreads, smem, st, p);
   }
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
@@ -343,17 +346,17 @@ int norm_gate_bwd(const pkda_norm_gate_args* a, cudaStream_t st) {
     if (!ng_allow_smem(pkda_norm_gate_bwd_kernel<bf16>, smem)) return PKDA_ERR_LAUNCH;
     grid = ng_grid(*a, pkda_norm_gate_bwd_kernel<bf16>, smem);
     begin_stage(kStageNormGateBwd, st);
-    pkda_norm_gate_bwd_kernel<bf16><<<grid, ng::kThreads, smem, st>>>(p);
+    launch_kernel(pkda_norm_gate_bwd_kernel<bf16>, grid, ng::kThreads, smem, st, p);
   } else {
     constexpr int smem = ng::bwd_smem<float>();
     if (!ng_allow_smem(pkda_norm_gate_bwd_kernel<float>, smem)) return PKDA_ERR_LAUNCH;
     grid = ng_grid(*a, pkda_norm_gate_bwd_kernel<float>, smem);
     begin_stage(kStageNormGateBwd, st);
-    pkda_norm_gate_bwd_kernel<float><<<grid, ng::kThreads, smem, st>>>(p);
+    launch_kernel(pkda_norm_gate_bwd_kernel<float>, grid, ng::kThreads, smem, st, p);
   }
   end_stage(st);
   begin_stage(kStageNormGateDw, st);
-  pkda_norm_gate_dw_kernel<<<1, 1024, 0, st>>>(p.part, a->dweight, a->dim, grid);
+  launch_kernel(pkda_norm_gate_dw_kernel, 1, 1024, 0, st, p.part, a->dweight, a->dim, grid);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(outtc::kThreads)
 pkda_out_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_qg,
                        const __grid_constant__ CUtensorMap tm_e, const __grid_constant__ CUtensorMap tm_p,
                        const __grid_constant__ CUtensorMap tm_o, const OutTcParams p) {
+  wait_prerequisites();
   using namespace outtc;
   extern __shared__ unsigned char smem_raw[];
   int n, tok0, valid;
@@ -222,8 +223,8 @@ int launch_out_fwd_tc(const Geo& geo, int total_tokens, const bf16* qg, const bf
   if (!ensure_dynamic_smem(pkda_out_fwd_tc_kernel, outtc::kSmem))
     return PKDA_ERR_LAUNCH;
   begin_stage(kStageOutFwd, st);
-  pkda_out_fwd_tc_kernel<<<dim3(geo.total_chunks, geo.heads), outtc::kThreads, outtc::kSmem, st>>>(tm_h, tm_qg, tm_e,
-                                                                                                   tm_p, tm_o, op);
+  launch_kernel(pkda_out_fwd_tc_kernel, dim3(geo.total_chunks, geo.heads), outtc::kThreads, outtc::kSmem, st, tm_h, tm_qg, tm_e,
+                tm_p, tm_o, op);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

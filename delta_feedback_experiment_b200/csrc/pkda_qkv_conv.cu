@@ -437,6 +437,7 @@ __device__ __forceinline__ void conv_bwd_walk(Feed<T> fx, Feed<T> fd, int row, i
 template <typename T, int kHeadLanes>
 __global__ void __launch_bounds__(conv::kThreads, sizeof(T) == 2 ? 3 : 2)
 pkda_qkv_conv_fwd_kernel(const ConvParams p) {
+  after_previous();
   using namespace conv;
   const int b = blockIdx.y / p.spans_per_row;
   const int lane = threadIdx.x % kLanes, grp = threadIdx.x / kLanes;
@@ -472,6 +473,7 @@ pkda_qkv_conv_fwd_kernel(const ConvParams p) {
 template <typename T, int kHeadLanes>
 __global__ void __launch_bounds__(conv::kThreads, sizeof(T) == 2 ? 2 : 1)
 pkda_qkv_conv_bwd_kernel(const ConvParams p) {
+  after_previous();
   using namespace conv;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* sPart = reinterpret_cast<float*>(smem_raw);  // [kGroups][kLanes][16]; entry 4 * channel + padded tap
@@ -537,6 +539,7 @@ pkda_qkv_conv_bwd_kernel(const ConvParams p) {
 }
 
 __global__ void pkda_qkv_conv_dw_kernel(const float* part, float* dw, int n, int groups) {
+  after_previous();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n) return;
   float a = 0.f;
@@ -580,7 +583,7 @@ template <typename T, int kHeadLanes>
 static int launch_conv_fwd(const ConvParams& p, dim3 grid, cudaStream_t st) {
   if (!ensure_dynamic_smem(pkda_qkv_conv_fwd_kernel<T, kHeadLanes>, conv::fwd_smem<T>())) return PKDA_ERR_LAUNCH;
   begin_stage(kStageConvFwd, st);
-  pkda_qkv_conv_fwd_kernel<T, kHeadLanes><<<grid, conv::kThreads, conv::fwd_smem<T>(), st>>>(p);
+  launch_kernel(pkda_qkv_conv_fwd_kernel<T, kHeadLanes>, grid, conv::kThreads, conv::fwd_smem<T>(), st, p);
   end_stage(st);
   return PKDA_OK;
 }
@@ -589,7 +592,7 @@ template <typename T, int kHeadLanes>
 static int launch_conv_bwd(const ConvParams& p, dim3 grid, cudaStream_t st) {
   if (!ensure_dynamic_smem(pkda_qkv_conv_bwd_kernel<T, kHeadLanes>, conv::bwd_smem<T>())) return PKDA_ERR_LAUNCH;
   begin_stage(kStageConvBwd, st);
-  pkda_qkv_conv_bwd_kernel<T, kHeadLanes><<<grid, conv::kThreads, conv::bwd_smem<T>(), st>>>(p);
+  launch_kernel(pkda_qkv_conv_bwd_kernel<T, kHeadLanes>, grid, conv::kThreads, conv::bwd_smem<T>(), st, p);
   end_stage(st);
   return PKDA_OK;
 }
@@ -642,7 +645,7 @@ int qkv_conv_bwd(const pkda_qkv_conv_args* a, cudaStream_t st) {
   if (a->dtype == PKDA_BF16) { PKDA_CONV_DISPATCH(launch_conv_bwd, bf16) } else { PKDA_CONV_DISPATCH(launch_conv_bwd, float) }
   if (rc != PKDA_OK) return rc;
   begin_stage(kStageConvDw, st);
-  pkda_qkv_conv_dw_kernel<<<(n + 255) / 256, 256, 0, st>>>(p.part, a->dweight, n, (int)grid.y);
+  launch_kernel(pkda_qkv_conv_dw_kernel, (n + 255) / 256, 256, 0, st, p.part, a->dweight, n, (int)grid.y);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

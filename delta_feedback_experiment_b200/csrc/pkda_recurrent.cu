@@ -37,6 +37,7 @@ struct RecParams {
 template <int D, int kCPL, typename T, bool kSave>
 __global__ void __launch_bounds__(ScanLay<D, kCPL>::kProd + 32 * ScanLay<D, kCPL>::kMaxConsumers)
 pkda_recurrent_kernel(const RecParams p) {
+  after_previous();
   using L = ScanLay<D, kCPL>;
   constexpr int TB = L::kTB, TPG = L::kTPG, RG = L::kRG, R = L::kR, VEC = L::kVecs * D;
   extern __shared__ __align__(16) float stage[];  // [2][TB][5][D]: exp(g) k, exp(g), beta kw, scale q, v
@@ -244,6 +245,7 @@ pkda_recurrent_kernel(const RecParams p) {
 template <int D, typename T>
 __global__ void __launch_bounds__(RecCfg<D>::kThreads, D == 128 ? 2 : 1)
 pkda_recurrent_few_kernel(const RecParams p) {
+  after_previous();
   using Cfg = RecCfg<D>;
   constexpr int VQ = Cfg::kVQ, KW = Cfg::kKW, R = Cfg::kR;
   const int tid = threadIdx.x;
@@ -362,12 +364,14 @@ static int launch_rec(RecParams rp, cudaStream_t st) {
   cfg.blockDim = dim3((unsigned)(32 * rp.nw + L::kProd));
   cfg.dynamicSmemBytes = L::kSmem;
   cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)rp.groups;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = rp.inplace_A ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)rp.groups;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = rp.inplace_A ? 2 : 1;
   begin_stage(kStageRecurrent, st);
   const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, rp);
   end_stage(st);
@@ -382,7 +386,7 @@ static int launch_rec_d(const RecParams& rp, bool save, cudaStream_t st) {
   if (rp.geo.seq_len > 0 && rp.geo.seq_len < few && units > sm_count()) {
     if (!aligned({rp.ST}, 16)) return PKDA_ERR_ALIGN;  // (here, with four columns per lane and in the single step: states by float4)
     begin_stage(kStageRecurrent, st);
-    pkda_recurrent_few_kernel<D, T><<<(unsigned)units, RecCfg<D>::kThreads, 0, st>>>(rp);
+    launch_kernel(pkda_recurrent_few_kernel<D, T>, (unsigned)units, RecCfg<D>::kThreads, 0, st, rp);
     end_stage(st);
     return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
   }

@@ -46,6 +46,7 @@ struct RecBwdParams {
 template <int D, typename T>
 __global__ void __launch_bounds__(ScanLay<D, 1>::kProd + 32 * ScanLay<D, 1>::kMaxConsumers)
 pkda_recurrent_dscan_kernel(const RecBwdParams p) {
+  after_previous();
   using L = ScanLay<D, 1>;
   constexpr int TB = L::kTB, TPG = L::kTPG, RG = L::kRG, R = L::kR, RUNS = L::kR / L::kU, VEC = L::kVecs * D;
   extern __shared__ __align__(16) float stage[];  // [2][TB][5][D]: scale q, w, -k, exp(g), do
@@ -215,6 +216,7 @@ __device__ __forceinline__ bool block_lookup(const Geo& g, long j, int& n, int& 
 template <int D, typename T>
 __global__ void __launch_bounds__(GradLay<D>::kThreads)
 pkda_recurrent_grad_kernel(const RecBwdParams p) {
+  after_previous();
   using L = GradLay<D>;
   constexpr int NS = L::kNS, NG = L::kNG, SUB = L::kSub, TPS = L::kTPS;
   extern __shared__ __align__(16) float sm[];
@@ -403,6 +405,7 @@ pkda_recurrent_grad_kernel(const RecBwdParams p) {
 // Replaces every block's outgoing lam by the one that enters it from behind.  One thread per channel.
 template <int D>
 __global__ void __launch_bounds__(D < 32 ? 32 : D) pkda_recurrent_carry_kernel(const RecBwdParams p) {
+  after_previous();
   constexpr int kAhead = 8;
   const int H = p.geo.heads, unit = blockIdx.x, n = unit / H, h = unit - n * H, c = threadIdx.x;
   const SeqInfo sq = seq_info(p.geo, n);
@@ -434,6 +437,7 @@ __global__ void __launch_bounds__(D < 32 ? 32 : D) pkda_recurrent_carry_kernel(c
 // One warp per token: dk, d beta_atk = <lam, k^2>, d g_atk = exp(gP) <lam, A before the token>.
 template <int D, typename T>
 __global__ void __launch_bounds__(256) pkda_recurrent_close_kernel(const RecBwdParams p) {
+  after_previous();
   const int H = p.geo.heads, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int n, t0;
   SeqInfo sq;
@@ -479,6 +483,7 @@ __global__ void __launch_bounds__(256) pkda_recurrent_close_kernel(const RecBwdP
 __global__ void __launch_bounds__(256)
 pkda_recurrent_bwd_reduce_kernel(int blocks, int H, int D, const float* partA, const float* partB, const float* partC,
                                  float* dA_log, float* ddt_bias, float* dcentre) {
+  after_previous();
   __shared__ float s[3][256];
   const int h = blockIdx.x, tid = threadIdx.x, c = tid % D, sl = tid / D, ns = 256 / D;
   float b = 0.f, a = 0.f, cc = 0.f;
@@ -544,17 +549,17 @@ static int launch_rec_bwd(RecBwdParams bp, size_t blocks, cudaStream_t st) {
       !ensure_dynamic_smem(pkda_recurrent_grad_kernel<D, T>, G::kFloats * 4))
     return PKDA_ERR_LAUNCH;
   begin_stage(kStageRecurrent, st);
-  pkda_recurrent_dscan_kernel<D, T><<<units * bp.groups, 32 * bp.nw + L::kProd, L::kSmem, st>>>(bp);
+  launch_kernel(pkda_recurrent_dscan_kernel<D, T>, units * bp.groups, 32 * bp.nw + L::kProd, L::kSmem, st, bp);
   end_stage(st);
   const dim3 grid((unsigned)blocks, (unsigned)H);
   begin_stage(kStageRecurrent, st);
-  pkda_recurrent_grad_kernel<D, T><<<grid, G::kThreads, G::kFloats * 4, st>>>(bp);
+  launch_kernel(pkda_recurrent_grad_kernel<D, T>, grid, G::kThreads, G::kFloats * 4, st, bp);
   end_stage(st);
   begin_stage(kStageRecurrent, st);
-  pkda_recurrent_carry_kernel<D><<<units, D < 32 ? 32 : D, 0, st>>>(bp);
+  launch_kernel(pkda_recurrent_carry_kernel<D>, units, D < 32 ? 32 : D, 0, st, bp);
   end_stage(st);
   begin_stage(kStageRecurrent, st);
-  pkda_recurrent_close_kernel<D, T><<<grid, 256, 0, st>>>(bp);
+  launch_kernel(pkda_recurrent_close_kernel<D, T>, grid, 256, 0, st, bp);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
@@ -606,8 +611,8 @@ int recurrent_bwd(const pkda_recurrent_bwd_args* a, const void* saved, size_t sa
                             : dispatch_rec_bwd<float>(p.head_dim, bp, blocks, st);
   if (rc != PKDA_OK) return rc;
   begin_stage(kStageParamReduce, st);
-  pkda_recurrent_bwd_reduce_kernel<<<p.heads, 256, 0, st>>>((int)blocks, p.heads, p.head_dim, ws.partA, ws.partB,
-                                                           ws.partC, a->dA_log, a->ddt_bias, a->dlog_atk_scale);
+  launch_kernel(pkda_recurrent_bwd_reduce_kernel, p.heads, 256, 0, st, (int)blocks, p.heads, p.head_dim, ws.partA, ws.partB,
+                ws.partC, a->dA_log, a->ddt_bias, a->dlog_atk_scale);
   end_stage(st);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }

@@ -20,6 +20,7 @@ struct ScanBwdColsParams {
   bf16 *dh, *dF;
   float* dS0;
   int* status;
+  int beside;  // the recompute pass's scan, launched in front of this one, may still run
 };
 
 // NW: column groups (of 16) per CTA.
@@ -43,6 +44,8 @@ __global__ void __launch_bounds__(ScanBwdLay<NW>::kThreads, 1)
 pkda_scan_bwd_cols_kernel(const __grid_constant__ CUtensorMap tm_kg, const __grid_constant__ CUtensorMap tm_w,
                           const __grid_constant__ CUtensorMap tm_qg, const __grid_constant__ CUtensorMap tm_do,
                           const __grid_constant__ CUtensorMap tm_p, const ScanBwdColsParams p) {
+  if (!p.beside) wait_prerequisites();
+  launch_dependents();
   using namespace scanw;
   using Y = ScanBwdLay<NW>;
   extern __shared__ unsigned char smem_raw[];
@@ -225,11 +228,11 @@ pkda_scan_bwd_cols_kernel(const __grid_constant__ CUtensorMap tm_kg, const __gri
 }
 
 template <int NW>
-static int launch(const CUtensorMap (&tm)[5], const ScanBwdColsParams& sp, int units, bool beside, cudaStream_t st) {
+static int launch(const CUtensorMap (&tm)[5], const ScanBwdColsParams& sp, int units, cudaStream_t st) {
   using Y = ScanBwdLay<NW>;
   if (!ensure_dynamic_smem(pkda_scan_bwd_cols_kernel<NW>, Y::kSmem)) return PKDA_ERR_LAUNCH;
-  return launch_beside(pkda_scan_bwd_cols_kernel<NW>, beside, units * Y::kSplit, Y::kThreads, Y::kSmem, st, tm[0], tm[1], tm[2],
-                       tm[3], tm[4], sp);
+  return launch_kernel(pkda_scan_bwd_cols_kernel<NW>, units * Y::kSplit, Y::kThreads, Y::kSmem, st, tm[0], tm[1], tm[2], tm[3],
+                       tm[4], sp);
 }
 
 int launch_scan_bwd_cols(const Geo& geo, int total_tokens, int units, const bf16* kg, const bf16* w, const bf16* qg,
@@ -243,9 +246,10 @@ int launch_scan_bwd_cols(const Geo& geo, int total_tokens, int units, const bf16
     return PKDA_ERR_LAUNCH;
   ScanBwdColsParams sp;
   sp.geo = geo; sp.beta_c = beta_c; sp.gc = gc; sp.dST = dST; sp.dh = dh; sp.dF = dF; sp.dS0 = dS0; sp.status = status;
-  return split == 8   ? launch<1>(tm, sp, units, beside, st)
-         : split == 4 ? launch<2>(tm, sp, units, beside, st)
-                      : launch<4>(tm, sp, units, beside, st);
+  sp.beside = beside;
+  return split == 8   ? launch<1>(tm, sp, units, st)
+         : split == 4 ? launch<2>(tm, sp, units, st)
+                      : launch<4>(tm, sp, units, st);
 }
 
 }  // namespace pkda

@@ -28,6 +28,7 @@ struct ScanBwdTcParams {
   bf16* dF;
   float* dS0;
   int* status;
+  int beside;  // the recompute pass's scan, launched in front of this one, may still run
 };
 
 namespace scanbtc {
@@ -58,6 +59,7 @@ pkda_scan_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_kg, const __grid_
                         const __grid_constant__ CUtensorMap tm_qg, const __grid_constant__ CUtensorMap tm_do,
                         const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_dh,
                         const __grid_constant__ CUtensorMap tm_df, const ScanBwdTcParams p) {
+  if (!p.beside) wait_prerequisites();
   using namespace scanbtc;
   extern __shared__ unsigned char smem_raw[];
   const int n = blockIdx.x / p.geo.heads, h = blockIdx.x - n * p.geo.heads, H = p.geo.heads;
@@ -80,6 +82,7 @@ pkda_scan_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_kg, const __grid_
   }
   tc::tc_fence_before();
   __syncthreads();
+  launch_dependents();
   tc::tc_fence_after();
   const uint32_t tmem = tc::uniform(*reinterpret_cast<volatile uint32_t*>(tiles + oBar + 48));
   const int warp_u = (int)tc::uniform(warp);
@@ -328,7 +331,8 @@ int launch_scan_bwd_tc(const Geo& geo, int total_tokens, int units, const bf16* 
   sp.geo = geo; sp.beta_c = beta_c; sp.gc = gc; sp.dST = dST; sp.dF = dF; sp.dS0 = dS0; sp.status = status;
   if (!ensure_dynamic_smem(pkda_scan_bwd_tc_kernel, scanbtc::kSmem))
     return PKDA_ERR_LAUNCH;
-  return launch_beside(pkda_scan_bwd_tc_kernel, beside, units, scanbtc::kThreads, scanbtc::kSmem, st, tm_kg, tm_w, tm_qg, tm_do,
+  sp.beside = beside;
+  return launch_kernel(pkda_scan_bwd_tc_kernel, units, scanbtc::kThreads, scanbtc::kSmem, st, tm_kg, tm_w, tm_qg, tm_do,
                        tm_p, tm_dh, tm_df, sp);
 }
 

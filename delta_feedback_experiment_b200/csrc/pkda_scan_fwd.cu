@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(ScanFwdLay<NW, kOut>::kThreads, 1)
 pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_kg,
                           const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_qg,
                           const __grid_constant__ CUtensorMap tm_p, const ScanFwdParams p) {
+  after_previous();
   using namespace scanw;
   using Y = ScanFwdLay<NW, kOut>;
   extern __shared__ unsigned char smem_raw[];
@@ -75,7 +76,6 @@ pkda_scan_fwd_cols_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       }
     tc::fence_barrier_init();
   }
-  if (!kOut) launch_dependents();  // (a recompute pass lets the backward's scan run beside it)
   __syncthreads();
   bool ok = true;
 
@@ -266,8 +266,8 @@ template <int NW, bool kOut>
 static int launch(const CUtensorMap (&tm)[5], const ScanFwdParams& sp, int units, cudaStream_t st) {
   using Y = ScanFwdLay<NW, kOut>;
   if (!ensure_dynamic_smem(pkda_scan_fwd_cols_kernel<NW, kOut>, Y::kSmem)) return PKDA_ERR_LAUNCH;
-  pkda_scan_fwd_cols_kernel<NW, kOut><<<units * Y::kSplit, Y::kThreads, Y::kSmem, st>>>(tm[0], tm[1], tm[2], tm[3],
-                                                                                       tm[4], sp);
+  launch_kernel(false, pkda_scan_fwd_cols_kernel<NW, kOut>, units * Y::kSplit, Y::kThreads, Y::kSmem, st, tm[0], tm[1], tm[2], tm[3],
+                tm[4], sp);
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 

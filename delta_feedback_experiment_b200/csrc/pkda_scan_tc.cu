@@ -95,6 +95,7 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
                         const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_h,
                         const __grid_constant__ CUtensorMap tm_e, const __grid_constant__ CUtensorMap tm_qg,
                         const __grid_constant__ CUtensorMap tm_p, const ScanTcParams p) {
+  wait_prerequisites();
   using namespace scantc;
   extern __shared__ unsigned char smem_raw[];
   const int n = blockIdx.x / p.geo.heads, h = blockIdx.x - n * p.geo.heads, H = p.geo.heads;
@@ -110,7 +111,6 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
 
   const size_t sbase = ((size_t)n * H + h) * kD * kD;
 
-  if (kRecompute) launch_dependents();  // (the backward's scan may run beside it)
   if (warp == 0) tc::tmem_alloc(tmem_slot, kCols);
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) tc::mbar_init(bar_full0 + 8 * s, 1);
@@ -139,6 +139,7 @@ pkda_scan_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
   tc::fence_proxy_async();
   tc::tc_fence_before();
   __syncthreads();
+  launch_dependents();
   tc::tc_fence_after();
   const uint32_t tmem = tc::uniform(*reinterpret_cast<volatile uint32_t*>(tiles + oBar + 48));
   const int warp_u = (int)tc::uniform(warp);
@@ -503,18 +504,18 @@ int launch_scan_fwd_tc(const Geo& geo, int total_tokens, int units, const bf16* 
   if (recompute) {
     if (!ensure_dynamic_smem(pkda_scan_fwd_tc_kernel<true, false>, scantc::kSmem))
       return PKDA_ERR_LAUNCH;
-    pkda_scan_fwd_tc_kernel<true, false><<<units, scantc::kThreads, scantc::kSmem, st>>>(tm_w, tm_kg, tm_u, tm_h, tm_e,
-                                                                                        tm_qg, tm_p, sp);
+    launch_kernel(false, pkda_scan_fwd_tc_kernel<true, false>, units, scantc::kThreads, scantc::kSmem, st, tm_w, tm_kg, tm_u, tm_h, tm_e,
+                  tm_qg, tm_p, sp);
   } else if (with_out) {
     if (!ensure_dynamic_smem(pkda_scan_fwd_tc_kernel<false, true>, scantc::kSmemOut))
       return PKDA_ERR_LAUNCH;
-    pkda_scan_fwd_tc_kernel<false, true><<<units, scantc::kThreads + scantc::kOutThreads, scantc::kSmemOut, st>>>(
-        tm_w, tm_kg, tm_u, tm_h, tm_e, tm_qg, tm_p, sp);
+    launch_kernel(false, pkda_scan_fwd_tc_kernel<false, true>, units, scantc::kThreads + scantc::kOutThreads, scantc::kSmemOut, st, tm_w,
+                  tm_kg, tm_u, tm_h, tm_e, tm_qg, tm_p, sp);
   } else {
     if (!ensure_dynamic_smem(pkda_scan_fwd_tc_kernel<false, false>, scantc::kSmem))
       return PKDA_ERR_LAUNCH;
-    pkda_scan_fwd_tc_kernel<false, false><<<units, scantc::kThreads, scantc::kSmem, st>>>(tm_w, tm_kg, tm_u, tm_h, tm_e,
-                                                                                         tm_qg, tm_p, sp);
+    launch_kernel(false, pkda_scan_fwd_tc_kernel<false, false>, units, scantc::kThreads, scantc::kSmem, st, tm_w, tm_kg, tm_u, tm_h, tm_e,
+                  tm_qg, tm_p, sp);
   }
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
