@@ -13,7 +13,9 @@
 // on S: producer warps make them for 8 tokens at a time, double buffered, while the consumer warps
 // run the chain; the sum for o is off the chain and is reduced for 8 tokens at once.
 // Measured: 4 x 16 units, 48 tokens, D = 128, bf16: 67 -> 27 us; 2 x 4 units, 512 tokens,
-// D = 64, fp32: 548 -> 86 us (90 when it leaves what the backward needs).
+// D = 64, fp32: 548 -> 86 us (90 when it leaves what the backward needs).  With the output of a token and the decay of the
+// state taken while the next token's sum goes through its shuffles (and four columns a lane reduced by three rounds of four shuffles instead
+// of five of one or two): 24.9 -> 23.9 us, and the pass of 512 tokens, forward and backward, 190.9 -> 188.1.
 #include "pkda_launch.h"
 #include "pkda_recurrent.cuh"
 
@@ -29,7 +31,8 @@ struct RecParams {
   void* o;
   float *ST, *AT;
   RecSaved save;     // kSave only
-  int nw, groups;    // consumer warps per CTA, CTAs per (sequence, head)
+  ScanWarps warps;   // consumer and producer warps of a CTA
+  int groups;        // CTAs per (sequence, head)
   int inplace_A;     // AT aliases A0: written only after every CTA of the unit has read it (a cluster)
   float scale, ln_x, eps;
 };
@@ -47,11 +50,12 @@ pkda_recurrent_kernel(const RecParams p) {
   const SeqInfo sq = seq_info(p.geo, n);
   const int nblk = (sq.len + TB - 1) / TB;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nthreads = 32 * p.nw + L::kProd;
+  const int nw = p.warps.nw, nthreads = 32 * nw + L::kProd;
 
-  if (warp >= p.nw) {
+  if (p.warps.idle(warp)) return;
+  if (warp >= nw) {
     // ------------------------------------------------ producers: row vectors of TB tokens at a time
-    const int ptid = threadIdx.x - 32 * p.nw;
+    const int ptid = 32 * p.warps.producer(warp) + lane;
     const int grp = ptid / L::kProdPerGroup, c = ptid - grp * L::kProdPerGroup;
     const bool act = c < D;
     const float ea = expf(p.A_log[h]), centre = p.log_atk_scale[h];
@@ -136,7 +140,7 @@ pkda_recurrent_kernel(const RecParams p) {
   // ---------------------------------------------------- consumers: the chain over tokens
   if (p.inplace_A) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
   const int rg = lane & (RG - 1);
-  const int col0 = (cg * p.nw + warp) * L::kCols + (lane / RG) * kCPL;
+  const int col0 = (cg * nw + warp) * L::kCols + (lane / RG) * kCPL;
   const size_t sbase = (size_t)unit * D * D + col0;
   float2 S[kCPL][R / 2];
   // element (row, column c) of the lane's part of the state
@@ -162,68 +166,99 @@ pkda_recurrent_kernel(const RecParams p) {
       else *dst = elem(i, 0);
     }
   };
-  T* o = static_cast<T*>(p.o);
   const size_t tstep = (size_t)H * D;
   const size_t tbase = ((size_t)sq.bos * H + h) * D + col0;
+  T* const o_row = static_cast<T*>(p.o) + tbase;
   for (int b = 0; b < nblk; ++b) {
     const int s = b & 1, t0 = b * TB;
     if (kSave && (t0 & (kCkpt - 1)) == 0)
       store_state(p.save.S + ((ckpt_base(p.geo, n, sq.bos) + t0 / kCkpt) * H + h) * (size_t)(D * D) + col0);
     bar_sync_n(1 + s, nthreads);
-    const float* st = stage + s * L::kStage;
+    const uint32_t st = smem_u32(stage + s * L::kStage);
     float oacc[L::kTO * kCPL], ekeep[L::kSums];  // [token][column]
-    float2 kx[R / 2];  // exp(g) k of the token
-    load_rows<L>(st, rg, kx);
-#pragma unroll
-    for (int t = 0; t < TB; ++t) {
-      const float* vec = st + t * VEC;
-      float e[kCPL];
+    // Two vectors of rows are held at a time.  x: exp(g) k, then exp(g) of a token; y: beta kw, then scale q.
+    float2 x[R / 2], y[R / 2];
+    load_rows<L>(st, rg, x);
+    auto out_sum = [&](int u) {  // the sum for o of token u (of the block)
 #pragma unroll
       for (int c = 0; c < kCPL; ++c) {
-        float2 a0 = __fmul2_rn(kx[0], S[c][0]), a1 = make_float2(0.f, 0.f);
+        float2 a0 = __fmul2_rn(y[0], S[c][0]);
+#pragma unroll
+        for (int i = 1; i < R / 2; ++i) a0 = __ffma2_rn(y[i], S[c][i], a0);
+        oacc[(u % L::kTO) * kCPL + c] = a0.x + a0.y;
+      }
+    };
+    auto out_round = [&](int u, int o) {  // a round over the lanes for the kTO tokens that end with u; behind the last they leave
+      if ((u + 1) % L::kTO) return;
+      rg_sum_round(oacc, rg, o, L::kTO * kCPL * o / RG);
+      if (o > 1) return;
+#pragma unroll
+      for (int i = 0; i < L::kSums; ++i) {
+        const int n = rg * L::kSums + i, to = t0 + u + 1 - L::kTO + n / kCPL;
+        if (to < sq.len) o_row[(size_t)to * tstep + n % kCPL] = from_f<T>(oacc[i]);
+      }
+    };
+#pragma unroll
+    for (int t = 0; t < TB; ++t) {
+      // e's sum over the lane's rows, then rounds of shuffles; behind each round's shuffles stands what does not depend on
+      // them: the output of the token before, the decay of the state, the loads.
+      const uint32_t vec = st + 4 * t * VEC;
+      float e[kCPL], r[kCPL], vt[kCPL];
+#pragma unroll
+      for (int c = 0; c < kCPL; ++c) {
+        float2 a0 = __fmul2_rn(x[0], S[c][0]), a1 = make_float2(0.f, 0.f);
 #pragma unroll
         for (int i = 1; i < R / 2; ++i) {
-          if (i & 1) a1 = __ffma2_rn(kx[i], S[c][i], a1);
-          else a0 = __ffma2_rn(kx[i], S[c][i], a0);
+          if (i & 1) a1 = __ffma2_rn(x[i], S[c][i], a1);
+          else a0 = __ffma2_rn(x[i], S[c][i], a0);
         }
         e[c] = (a0.x + a0.y) + (a1.x + a1.y);
       }
-      // every other row vector the token needs, and the next token's first one, is asked for before
-      // the shuffles below so that none of these loads sits on the chain
-      float2 al[R / 2], wk[R / 2], qs[R / 2];
-      load_rows<L>(vec + D, rg, al);
-      load_rows<L>(vec + 2 * D, rg, wk);
-      load_rows<L>(vec + 3 * D, rg, qs);
-      if (t + 1 < TB) load_rows<L>(vec + VEC, rg, kx);
-      float vt[kCPL];
-      if (kCPL == 4) *reinterpret_cast<float4*>(vt) = *reinterpret_cast<const float4*>(vec + 4 * D + col0);
-      else vt[0] = vec[4 * D + col0];
-      rg_sum<RG>(e, rg);
+      auto round = [&](int o) {
+#pragma unroll
+        for (int c = 0; c < kCPL; ++c) r[c] = xor_lane(e[c], o);
+      };
+      auto add = [&]() {
+#pragma unroll
+        for (int c = 0; c < kCPL; ++c) e[c] += r[c];
+      };
+      round(RG / 2);
+      load_rows<L>(vec + 4 * D, rg, x);
+      if (t > 0) out_sum(t - 1);
+      add();
+      round(RG / 4);
+      if (t > 0) out_round(t - 1, RG / 2);
+      load_rows<L>(vec + 8 * D, rg, y);
+#pragma unroll
+      for (int c = 0; c < kCPL; ++c)
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) S[c][i] = __fmul2_rn(x[i], S[c][i]);
+      add();
+      if (RG == 8) round(1);
+      if (t > 0) out_round(t - 1, RG / 4);
+      if (kCPL == 4) {
+        float2 v[2];
+        load_run<4>(vec + 16 * D + 4 * col0, v);
+        vt[0] = v[0].x; vt[1 % kCPL] = v[0].y; vt[2 % kCPL] = v[1].x; vt[3 % kCPL] = v[1].y;
+      } else {
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(vt[0]) : "r"(vec + 16 * D + 4 * col0));
+      }
+      if (t + 1 < TB) load_rows<L>(vec + 4 * VEC, rg, x);
+      if (RG == 8) add();
 #pragma unroll
       for (int c = 0; c < kCPL; ++c) e[c] = vt[c] - e[c];
       if (kSave && rg == t / L::kSums) ekeep[t % L::kSums] = e[0];
 #pragma unroll
       for (int c = 0; c < kCPL; ++c)
 #pragma unroll
-        for (int i = 0; i < R / 2; ++i)
-          S[c][i] = __ffma2_rn(wk[i], make_float2(e[c], e[c]), __fmul2_rn(al[i], S[c][i]));
-#pragma unroll
-      for (int c = 0; c < kCPL; ++c) {
-        float2 a0 = __fmul2_rn(qs[0], S[c][0]);
-#pragma unroll
-        for (int i = 1; i < R / 2; ++i) a0 = __ffma2_rn(qs[i], S[c][i], a0);
-        oacc[(t % L::kTO) * kCPL + c] = a0.x + a0.y;
-      }
-      if ((t + 1) % L::kTO == 0) {
-        rg_sum_transposed<RG, L::kTO * kCPL>(oacc, rg);
-#pragma unroll
-        for (int i = 0; i < L::kSums; ++i) {
-          const int x = rg * L::kSums + i, to = t0 + t + 1 - L::kTO + x / kCPL;
-          if (to < sq.len) o[tbase + (size_t)to * tstep + x % kCPL] = from_f<T>(oacc[i]);
-        }
-      }
+        for (int i = 0; i < R / 2; ++i) S[c][i] = __ffma2_rn(y[i], make_float2(e[c], e[c]), S[c][i]);
+      load_rows<L>(vec + 12 * D, rg, y);
+      if (RG == 8 && t > 0) out_round(t - 1, 1);
     }
+    out_sum(TB - 1);
     if (b + 2 < nblk) bar_arrive_n(3 + s, nthreads);
+#pragma unroll
+    for (int o = RG / 2; o >= 1; o >>= 1) out_round(TB - 1, o);
     if (kSave) {  // (one column per lane)
 #pragma unroll
       for (int i = 0; i < L::kSums; ++i) {
@@ -353,15 +388,16 @@ static int launch_rec(RecParams rp, cudaStream_t st) {
   using L = ScanLay<D, kCPL>;
   auto kernel = pkda_recurrent_kernel<D, kCPL, T, kSave>;
   const int units = rp.geo.n_seqs * rp.geo.heads;
-  rp.nw = scan_consumers(units, L::kWarps, L::kMaxConsumers, sm_count());
+  int nw = scan_consumers(units, L::kWarps, L::kMaxConsumers, sm_count());
   if (rp.inplace_A)  // the unit's CTAs form one cluster: at most eight of them
-    while (L::kWarps / rp.nw > 8) rp.nw *= 2;
-  rp.groups = L::kWarps / rp.nw;
+    while (L::kWarps / nw > 8) nw *= 2;
+  rp.groups = L::kWarps / nw;
   if (rp.groups == 1) rp.inplace_A = 0;
+  rp.warps = {nw, nw == 1 && !rp.inplace_A};  // (every thread takes part in the cluster's barrier)
   if (!ensure_dynamic_smem(kernel, L::kSmem)) return PKDA_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(units * rp.groups));
-  cfg.blockDim = dim3((unsigned)(32 * rp.nw + L::kProd));
+  cfg.blockDim = dim3((unsigned)rp.warps.threads(L::kProd));
   cfg.dynamicSmemBytes = L::kSmem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];

@@ -88,68 +88,61 @@ __device__ __forceinline__ void bar_arrive_n(int id, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// Sums over the kRG lanes of a column group, one per column; every lane gets all of them.  Four columns
-// trade halves first, so that the remaining steps run on one register.
-template <int kRG>
-__device__ __forceinline__ void rg_sum(float (&v)[1], int) {
-#pragma unroll
-  for (int o = kRG / 2; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+// Shared-memory loads and shuffles of the scans (volatile: the compiler keeps their order; the assembler may still move a load in
+// front of a shuffle).
+template <int kU>
+__device__ __forceinline__ void load_run(uint32_t s, float2* out) {
+  if (kU == 4)
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(out[0].x), "=f"(out[0].y), "=f"(out[1].x), "=f"(out[1].y) : "r"(s));
+  else
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(out[0].x), "=f"(out[0].y) : "r"(s));
 }
-template <int kRG>
-__device__ __forceinline__ void rg_sum(float (&v)[4], int rg) {
-  const bool hi = rg & (kRG / 2), hi2 = rg & (kRG / 4);
-  const float a = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], kRG / 2);
-  const float b = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], kRG / 2);
-  float x = (hi2 ? b : a) + __shfl_xor_sync(0xffffffffu, hi2 ? a : b, kRG / 4);
-#pragma unroll
-  for (int o = kRG / 8; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  const float y = __shfl_xor_sync(0xffffffffu, x, kRG / 4);
-  const float p = hi2 ? y : x, q = hi2 ? x : y;
-  const float r = __shfl_xor_sync(0xffffffffu, p, kRG / 2), t = __shfl_xor_sync(0xffffffffu, q, kRG / 2);
-  v[0] = hi ? r : p;
-  v[1] = hi ? t : q;
-  v[2] = hi ? p : r;
-  v[3] = hi ? q : t;
+__device__ __forceinline__ float xor_lane(float x, int o) {
+  float y;
+  asm volatile("shfl.sync.bfly.b32 %0, %1, %2, 0x1f, 0xffffffff;" : "=f"(y) : "f"(x), "r"(o));
+  return y;
 }
 
-// kN per-lane partial sums: afterwards lane rg holds the totals of entries rg * (kN / kRG) ... in
-// x[0 .. kN / kRG) (a transposing butterfly: about kN shuffles instead of kN * log2(kRG)).
+// The kR values of one row vector (shared address) that belong to the lane.
+template <typename L>
+__device__ __forceinline__ void load_rows(uint32_t vec, int rg, float2 (&x)[L::kR / 2]) {
+#pragma unroll
+  for (int b = 0; b < L::kR / L::kU; ++b) load_run<L::kU>(vec + 4 * L::row(b, rg), &x[b * (L::kU / 2)]);
+}
+
+// kN per-lane partial sums: after the rounds o = kRG / 2, kRG / 4, .. 1 (n = kN / 2, kN / 4, ..) lane rg holds the totals of entries
+// rg * (kN / kRG) ... in x[0 .. kN / kRG) (a transposing butterfly: about kN shuffles instead of kN * log2(kRG)).
+template <int kN>
+__device__ __forceinline__ void rg_sum_round(float (&x)[kN], int rg, int o, int n) {
+  const bool upper = rg & o;
+#pragma unroll
+  for (int i = 0; i < kN / 2; ++i) {
+    if (i < n) {
+      const float keep = upper ? x[i + n] : x[i];
+      const float send = upper ? x[i] : x[i + n];
+      x[i] = keep + xor_lane(send, o);
+    }
+  }
+}
 template <int kRG, int kN>
 __device__ __forceinline__ void rg_sum_transposed(float (&x)[kN], int rg) {
   int n = kN;
 #pragma unroll
-  for (int o = kRG / 2; o >= 1; o >>= 1) {
-    const bool upper = rg & o;
-    n >>= 1;
-#pragma unroll
-    for (int i = 0; i < kN / 2; ++i) {
-      if (i < n) {
-        const float keep = upper ? x[i + n] : x[i];
-        const float send = upper ? x[i] : x[i + n];
-        x[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-      }
-    }
-  }
+  for (int o = kRG / 2; o >= 1; o >>= 1) rg_sum_round(x, rg, o, n >>= 1);
 }
 
-// One run of kU consecutive fp32 values from shared memory, as pairs.
-template <int kU>
-__device__ __forceinline__ void load_run(const float* s, float2* out) {
-  if (kU == 4) {
-    const float4 x = *reinterpret_cast<const float4*>(s);
-    out[0] = make_float2(x.x, x.y);
-    out[1] = make_float2(x.z, x.w);
-  } else {
-    out[0] = *reinterpret_cast<const float2*>(s);
+// Where the warps of a scan CTA stand.  A warp's scheduler is its index modulo 4: a lone chain warp has one to itself, the producers'
+// warps lie on the other three (every fourth index stays empty).  With what stands between the shuffles of a token: 2 x 4 units,
+// 512 tokens, D = 64, fp32, a chain warp's token in the forward 335 -> 295 cycles.
+struct ScanWarps {
+  int nw, spread;  // chain warps; whether the producers are spread
+  __host__ __device__ int threads(int producers) const {
+    const int n = producers / 32;
+    return 32 * (spread ? 1 + n + (n - 1) / 3 : nw + n);
   }
-}
-
-// The kR values of one row vector that belong to the lane.
-template <typename L>
-__device__ __forceinline__ void load_rows(const float* vec, int rg, float2 (&x)[L::kR / 2]) {
-#pragma unroll
-  for (int b = 0; b < L::kR / L::kU; ++b) load_run<L::kU>(vec + L::row(b, rg), &x[b * (L::kU / 2)]);
-}
+  __device__ bool idle(int warp) const { return spread && warp > 0 && (warp & 3) == 0; }
+  __device__ int producer(int warp) const { return spread ? warp - 1 - (warp >> 2) : warp - nw; }
+};
 
 // Consumer warps per CTA: as few as possible while all CTAs run in one wave (a short chain wants
 // its own SM), at most kMaxConsumers (the producers of a CTA redo the same row vectors, so with more

@@ -37,7 +37,8 @@ struct RecBwdParams {
   float* dg_atk;
   float *partA, *partB, *partC;  // per (block, head): [blocks][H], [blocks][H][D], [blocks][H]
   float *dS0, *dA0;
-  int nw, groups;
+  ScanWarps warps;  // consumer and producer warps of a scan CTA
+  int groups;       // CTAs per (sequence, head)
   float scale, ln_x, eps;
 };
 
@@ -56,11 +57,12 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
   const SeqInfo sq = seq_info(p.geo, n);
   const int nblk = (sq.len + TB - 1) / TB;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nthreads = 32 * p.nw + L::kProd;
+  const int nw = p.warps.nw, nthreads = 32 * nw + L::kProd;
   const size_t tstep = (size_t)H * D;
 
-  if (warp >= p.nw) {
-    const int ptid = threadIdx.x - 32 * p.nw;
+  if (p.warps.idle(warp)) return;
+  if (warp >= nw) {
+    const int ptid = 32 * p.warps.producer(warp) + lane;
     const int grp = ptid / L::kProdPerGroup, c = ptid - grp * L::kProdPerGroup;
     const bool act = c < D;
     const size_t base = ((size_t)sq.bos * H + h) * D + (act ? c : 0);
@@ -108,7 +110,7 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
   }
 
   const int rg = lane & (RG - 1);
-  const int col0 = (cg * p.nw + warp) * L::kCols + lane / RG;
+  const int col0 = (cg * nw + warp) * L::kCols + lane / RG;
   const size_t sbase = (size_t)unit * D * D + col0;
   float2 S[R / 2];
 #pragma unroll
@@ -136,14 +138,16 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
     if (it == 0 || ((t0 + TB) & (kCkpt - 1)) == 0)
       store_state(p.dSck + ((ckpt_base(p.geo, n, sq.bos) + t0 / kCkpt) * H + h) * (size_t)(D * D) + col0);
     bar_sync_n(1 + s, nthreads);
-    const float* st = stage + s * L::kStage;
+    const uint32_t st = smem_u32(stage + s * L::kStage);
     float2 qs[R / 2], w[R / 2];
-    load_rows<L>(st + (TB - 1) * VEC, rg, qs);
-    load_rows<L>(st + (TB - 1) * VEC + D, rg, w);
+    float dot;
+    auto load_do = [&](int t) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(dot) : "r"(st + 4 * (t * VEC + 4 * D + col0))); };
+    load_do(TB - 1);
+    load_rows<L>(st + 4 * (TB - 1) * VEC, rg, qs);
+    load_rows<L>(st + 4 * ((TB - 1) * VEC + D), rg, w);
 #pragma unroll
     for (int t = TB - 1; t >= 0; --t) {
-      const float* vec = st + t * VEC;
-      const float dot = vec[4 * D + col0];
+      const uint32_t vec = st + 4 * t * VEC;
       float2 a0 = make_float2(0.f, 0.f), a1 = a0;
 #pragma unroll
       for (int i = 0; i < R / 2; ++i) {
@@ -151,19 +155,29 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
         if (i & 1) a1 = __ffma2_rn(w[i], S[i], a1);
         else a0 = __ffma2_rn(w[i], S[i], a0);
       }
-      float2 nk[R / 2], al[R / 2];  // asked for before the shuffles, like the next token's first two vectors
-      load_rows<L>(vec + 2 * D, rg, nk);
-      load_rows<L>(vec + 3 * D, rg, al);
+      // the token's other vectors and the next token's first ones are asked for between the rounds of shuffles
+      float2 nk[R / 2], al[R / 2];
+      float de = (a0.x + a0.y) + (a1.x + a1.y);
+      float r = xor_lane(de, RG / 2);
+      load_rows<L>(vec + 8 * D, rg, nk);
+      load_rows<L>(vec + 12 * D, rg, al);
+      de += r;
+      r = xor_lane(de, RG / 4);
       if (t > 0) {
-        load_rows<L>(vec - VEC, rg, qs);
-        load_rows<L>(vec - VEC + D, rg, w);
+        load_do(t - 1);
+        load_rows<L>(vec - 4 * VEC, rg, qs);
+        if (RG < 8) load_rows<L>(vec - 4 * VEC + 4 * D, rg, w);
       }
-      float de[1] = {(a0.x + a0.y) + (a1.x + a1.y)};
-      rg_sum<RG>(de, rg);
-      if (rg == t / L::kSums) keep[t % L::kSums] = de[0];
+      de += r;
+      if (RG == 8) {
+        r = xor_lane(de, 1);
+        if (t > 0) load_rows<L>(vec - 4 * VEC + 4 * D, rg, w);
+        de += r;
+      }
+      if (rg == t / L::kSums) keep[t % L::kSums] = de;
 #pragma unroll
       for (int i = 0; i < R / 2; ++i)
-        S[i] = __fmul2_rn(al[i], __ffma2_rn(nk[i], make_float2(de[0], de[0]), S[i]));
+        S[i] = __fmul2_rn(al[i], __ffma2_rn(nk[i], make_float2(de, de), S[i]));
     }
     if (it + 2 < nblk) bar_arrive_n(3 + s, nthreads);
 #pragma unroll
@@ -543,13 +557,14 @@ static int launch_rec_bwd(RecBwdParams bp, size_t blocks, cudaStream_t st) {
   using L = ScanLay<D, 1>;
   using G = GradLay<D>;
   const int units = bp.geo.n_seqs * bp.geo.heads, H = bp.geo.heads;
-  bp.nw = scan_consumers(units, L::kWarps, L::kMaxConsumers, sm_count());
-  bp.groups = L::kWarps / bp.nw;
+  const int nw = scan_consumers(units, L::kWarps, L::kMaxConsumers, sm_count());
+  bp.warps = {nw, nw == 1};
+  bp.groups = L::kWarps / nw;
   if (!ensure_dynamic_smem(pkda_recurrent_dscan_kernel<D, T>, L::kSmem) ||
       !ensure_dynamic_smem(pkda_recurrent_grad_kernel<D, T>, G::kFloats * 4))
     return PKDA_ERR_LAUNCH;
   begin_stage(kStageRecurrent, st);
-  launch_kernel(pkda_recurrent_dscan_kernel<D, T>, units * bp.groups, 32 * bp.nw + L::kProd, L::kSmem, st, bp);
+  launch_kernel(pkda_recurrent_dscan_kernel<D, T>, units * bp.groups, bp.warps.threads(L::kProd), L::kSmem, st, bp);
   end_stage(st);
   const dim3 grid((unsigned)blocks, (unsigned)H);
   begin_stage(kStageRecurrent, st);
@@ -604,7 +619,8 @@ int recurrent_bwd(const pkda_recurrent_bwd_args* a, const void* saved, size_t sa
   bp.dq = a->dq; bp.dk = a->dk; bp.dv = a->dv; bp.dg = a->dg; bp.dbeta_atk = a->dbeta_atk; bp.dbeta = a->dbeta;
   bp.dg_atk = a->dg_atk; bp.partA = ws.partA; bp.partB = ws.partB; bp.partC = ws.partC;
   bp.dS0 = a->d_initial_state; bp.dA0 = a->d_initial_A_state;
-  bp.nw = bp.groups = 0;
+  bp.warps = {0, 0};
+  bp.groups = 0;
   bp.scale = p.scale; bp.ln_x = logf(p.squash_x); bp.eps = p.squash_eps;
   const size_t blocks = ckpt_bound(p);
   rc = p.dtype == PKDA_BF16 ? dispatch_rec_bwd<bf16>(p.head_dim, bp, blocks, st)
