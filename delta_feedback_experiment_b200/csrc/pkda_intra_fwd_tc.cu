@@ -26,8 +26,10 @@
 //    and write L = tril(M, -1) diag(beta) in fp32 and scale tril(P) in bf16.
 //  * T = (I + L)^-1 stays on the CUDA cores and 3xTF32 mma.sync (pkda_chunk.cuh): it needs
 //    fp32-level accuracy and its products are at most 32 x 32.
-//  * W^T = Kd^T T^T and U^T = V^T T^T are two more accumulators (M = 128 channels, N = 64
-//    tokens, K = 64 tokens); V and the outputs of full chunks move by TMA.
+//  * W = T Kd and U = T V are two more accumulators (M = 64 tokens, N = 128 channels, K = 64
+//    tokens): a thread reads back channel pairs of two tokens, which it rounds and stores by stmatrix (with channels as rows a
+//    thread held one channel of 32 tokens, 64 two-byte stores: 414 -> 406 us at 8 x 4,096 tokens of 16 heads).  V and the
+//    outputs of full chunks move by TMA.
 //
 // Every mbarrier wait is bounded; a CTA whose wait gives up sets the status word.
 #include "pkda_chunk.cuh"
@@ -68,7 +70,7 @@ constexpr int oY2 = oA + 8192;              // f32 [1280]
 static_assert(oG + 32768 == oP && oBar % 8 == 0, "the decays fill what lies between the write keys and P");
 static_assert(oA0 + 512 <= oZin && oZin + 4096 <= oBeta && oT + 64 * kLdL * 4 <= oV && oY2 + 5120 <= oA + 16384, "aliases must fit");
 static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs per SM");
-constexpr uint32_t kCols = 256;             // pair accumulator 0..63, W^T 64..127, U^T 128..191
+constexpr uint32_t kCols = 256;             // pair accumulator 0..63; later W 0..127, U 128..255
 }  // namespace intratc
 
 __device__ __forceinline__ void unpack4(uint2 r, float (&f)[4]) {
@@ -835,7 +837,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     __syncthreads();
   }
 
-  // ---- 6. W^T = Kd^T T^T, U^T = V^T T^T
+  // ---- 6. W = T Kd, U = T V (64 rows: the tokens)
   if (nx.x >= 0) {
     if (tid == 32) request_g(nx);
   }
@@ -845,15 +847,14 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   }
   if (warp_u == 2 && tc::elect_one()) {  // (warp 0 stores T, warp 1 asks for the next gate)
     tc::tc_fence_after();
-    constexpr uint32_t idesc = tc::idesc_bf16(128, 64, /*a_mn_major=*/true, /*b_mn_major=*/false);
+    constexpr uint32_t idesc = tc::idesc_bf16(64, 128, /*a_mn_major=*/false, /*b_mn_major=*/true);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
-      tc::umma_bf16(tmem + 64, tc::desc_mnmajor(dbase + oA + kk * 2048, 16384), tc::desc_kmajor(dbase + oTm + kk * 32),
-                    idesc, kk > 0);
+      tc::umma_bf16(tmem, tc::desc_kmajor(dbase + oTm + kk * 32), tc::desc_mnmajor(dbase + oA + kk * 2048, 16384), idesc, kk > 0);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
-      tc::umma_bf16(tmem + 128, tc::desc_mnmajor(dbase + oV + kk * 2048, 8192), tc::desc_kmajor(dbase + oTm + kk * 32),
-                    idesc, kk > 0);
+      tc::umma_bf16(tmem + 128, tc::desc_kmajor(dbase + oTm + kk * 32), tc::desc_mnmajor(dbase + oV + kk * 2048, 8192), idesc,
+                    kk > 0);
     tc::umma_commit(bar_mma);
   }
   ok = tc::mbar_wait(bar_mma, ph & 1) && ok;
@@ -864,22 +865,26 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     request_scalars(nx);
   }
   {
-    const int ch = 32 * (warp & 3) + lane, t0 = 32 * (warp >> 2);  // accumulator row = channel; this warp's tokens
+    const int q = warp & 3, m = warp >> 2;  // this warp's 16 tokens; W or U
+    const int r = lane & 7, mat = lane >> 3;  // the row whose address this lane gives: row r of rows 8 (mat & 1) .., 8 columns (mat >> 1)
+    const uint32_t row = base + (m ? oX : oV) + (16 * q + 8 * (mat & 1) + r) * 128, rx = ((mat >> 1) ^ r) << 4;
 #pragma unroll 1
-    for (int m = 0; m < 2; ++m) {
+    for (int blk = 0; blk < 2; ++blk) {
       float acc[32];
-      tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 + 64 * m + t0, acc);
+      tc::tmem_ld_rows(tmem + ((uint32_t)(32 * q) << 16) + 128 * m + 64 * blk, acc);
       tc::tmem_ld_wait();
-      if (full) {  // transposed into a swizzled [token][channel] tile for the TMA store
-        unsigned char* out = tiles + (m ? oX : oV);
+      uint32_t x[16];
 #pragma unroll
-        for (int t = 0; t < 32; ++t)
-          *reinterpret_cast<bf16*>(out + sw128_offset(t0 + t, ch, 8192)) = __float2bfloat16(acc[t]);
+      for (int i = 0; i < 16; ++i) x[i] = pack_bf16(acc[2 * i], acc[2 * i + 1]);
+      if (full) {  // a swizzled [token][channel] tile for the TMA store
+#pragma unroll
+        for (int i = 0; i < 4; ++i) stsm_x4(row + blk * 8192 + (rx ^ (i << 5)), &x[4 * i]);
       } else {
-        bf16* dst = m ? p.u : p.w;
+        bf16* dst = (m ? p.u : p.w) + row0 + (size_t)(16 * q + (lane >> 2)) * gld + 64 * blk + 2 * (lane & 3);
 #pragma unroll
-        for (int t = 0; t < 32; ++t)
-          if (t0 + t < valid) dst[row0 + (size_t)(t0 + t) * gld + ch] = __float2bfloat16(acc[t]);
+        for (int i = 0; i < 16; ++i)
+          if (16 * q + (lane >> 2) + 8 * (i & 1) < valid)
+            *reinterpret_cast<uint32_t*>(dst + (size_t)(8 * (i & 1)) * gld + 8 * (i >> 1)) = x[i];
       }
     }
   }
