@@ -17,7 +17,7 @@
 //    the filter taps, which is what the sigmoid's tanh wants; silu' shares the forward's terms.
 // The backward recomputes the pre-activation instead of saving it.  The weight gradient is reduced in a
 // fixed order (registers -> across the CTA's token groups -> one partial per CTA -> a small second kernel).
-// At 8 x 4096 tokens of 16 heads x 128: forward 166 -> 133 us, backward 453 -> 298 us, against a version
+// At 8 x 4096 tokens of 16 heads x 128: forward 166 -> 133 us, backward 453 -> 292 us, against a version
 // with block-wide double-buffered tiles and per-token reductions (the traffic alone: 125 and 187 us).
 #include "pkda_common.cuh"
 #include "pkda_launch.h"
@@ -316,7 +316,7 @@ __device__ __forceinline__ void conv_fwd_walk(const T* col, int xs, Feed<T> feed
   }
 }
 
-// One warp's walk (backward): dx of `own` tokens from t0 and their part of the weight gradient.  dx of a
+// One warp's walk (backward): dx of `own` tokens from t0 and their rows' part of the weight gradient.  dx of a
 // token needs the pre-activation gradients of the three tokens after it, so the walk goes one step further
 // than its own tokens; those gradients stay in registers.  w holds half the taps: the doubled
 // pre-activation gradients make up for it in dx, and dwacc comes out doubled.
@@ -395,8 +395,8 @@ __device__ __forceinline__ void conv_bwd_walk(Feed<T> fx, Feed<T> fd, int row, i
         }
       }
     }
-    // The rows are read a second time for the weight gradient: kept in between, they would be the 28
-    // registers that the walk does not have.
+    // Four rows are read a second time for the weight gradient: kept in between, they would be registers that the
+    // walk does not have.  (Its three oldest rows kept unpacked for the next step instead: 291.6 -> 294.5 us.)
     asm volatile("" ::: "memory");
     if (kNorm) head_norms_back<kHeadLanes>(ss, sd, r, back, normed, eps, lane);
 #pragma unroll
@@ -404,30 +404,27 @@ __device__ __forceinline__ void conv_bwd_walk(Feed<T> fx, Feed<T> fd, int row, i
 #pragma unroll
       for (int pr = 0; pr < 2; ++pr)  // (r d - s r^3 <s, d>) silu'(y)
         dy[conv::kHalo + u][pr] = kNorm ? fma2(sc[u][pr], f2(back[u], back[u]), mul2(dc[u][pr], f2(r[u], r[u]))) : dc[u][pr];
-    if (t < own) {  // the walk's last step only looks ahead; tokens past the row's end have no gradient
-      float2 x[conv::kHalo + conv::kStep][2];
-#pragma unroll
-      for (int j = 0; j < conv::kHalo + conv::kStep; ++j)
-        Vec4<T>::unpack(Vec4<T>::fetch(j < conv::kHalo ? xp + j * conv::kWarpCh : xc + (j - conv::kHalo) * conv::kWarpCh), x[j]);
-#pragma unroll
-      for (int u = 0; u < conv::kStep; ++u)
-#pragma unroll
-        for (int pr = 0; pr < 2; ++pr)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dwacc[pr][j] = fma2(dy[conv::kHalo + u][pr], x[u + j][pr], dwacc[pr][j]);
-    }
+    // dx of the rows t - 3 .. t, and with the same four gradients of the pre-activation each row's part of the weight gradient.
+    // (A walk's weight gradient by the rows of x that it owns, not by their outputs, needs four rows a step instead of seven:
+    // 296.5 -> 291.6 us at 8 x 4,096 tokens of 16 heads.)
 #pragma unroll
     for (int u = 0; u < conv::kStep; ++u) {
-      float2 o[2];
+      const int e = t + u - conv::kHalo;
+      float2 o[2], x[2];
+      Vec4<T>::unpack(Vec4<T>::fetch(u < conv::kHalo ? xp + u * conv::kWarpCh : xc), x);
+      const bool mine = e >= 0 && e < own;  // (rows before the walk are the neighbour's, rows behind it too)
 #pragma unroll
       for (int pr = 0; pr < 2; ++pr) {
         float2 a = mul2(w[pr][3], dy[u][pr]);
         a = fma2(w[pr][2], dy[u + 1][pr], a);
         a = fma2(w[pr][1], dy[u + 2][pr], a);
         o[pr] = fma2(w[pr][0], dy[u + 3][pr], a);
+        if (mine) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dwacc[pr][j] = fma2(dy[u + 3 - j][pr], x[pr], dwacc[pr][j]);
+        }
       }
-      const int e = t + u - conv::kHalo;
-      if (active && e >= 0 && e < own) Vec4<T>::store(drow + u * xs, o);
+      if (active && mine) Vec4<T>::store(drow + u * xs, o);
     }
     drow += conv::kStep * xs;
     slot = (slot + 1) % conv::kRing;
