@@ -271,7 +271,7 @@ __device__ __forceinline__ void pairs_of_strip_exact(unsigned char* tiles, uint3
 template <bool kRecompute>
 __global__ void __launch_bounds__(intratc::kThreads, 2)
 pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_akk,
-                         const __grid_constant__ CUtensorMap tm_aqk, const __grid_constant__ CUtensorMap tm_w,
+                         const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_w,
                          const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_g,
                          const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_q,
                          const IntraParams p) {
@@ -289,7 +289,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   float* sL = reinterpret_cast<float*>(tiles + oL);
   float* sBeta = reinterpret_cast<float*>(tiles + oBeta);
   float* sDiag = reinterpret_cast<float*>(tiles + oDiag);
-  float* sTot = reinterpret_cast<float*>(tiles + oTot);
+  float* sTot = reinterpret_cast<float*>(tiles + (kRecompute ? oStep : oTot));  // (when recomputing, the write keys arrive in oL)
   float* sEnd = reinterpret_cast<float*>(tiles + oEnd);
   float* sDec = reinterpret_cast<float*>(tiles + oDec);
   float* sSum = reinterpret_cast<float*>(tiles + oSum);
@@ -350,7 +350,11 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   // With the scalars below, the hand-over in one word and the rows of pass 3 read ahead: 8 x 4,096 tokens of 16 heads
   // 466 -> 436 us; asked for at the top of an item, strips and scalars were 4,000 of its 30,000 cycles, and the stores 1,400.
   auto request_g = [&](const int4& it) {  // one thread; also arms the barrier for k and q
-    tc::mbar_expect_tx(bar_in, 6 * 8192);
+    tc::mbar_expect_tx(bar_in, (kRecompute ? 8 : 6) * 8192);
+    if (kRecompute) {
+      tc::tma_load_3d(base + oL, &tm_p, bar_in, 0, it.x % H, it.y);
+      tc::tma_load_3d(base + oL + 8192, &tm_p, bar_in, 64, it.x % H, it.y);
+    }
     tc::tma_load_3d(base + oY, &tm_g, bar_in, 0, it.x % H, it.y);
     tc::tma_load_3d(base + oY + 8192, &tm_g, bar_in, 64, it.x % H, it.y);
   };
@@ -415,13 +419,6 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     tc::bulk_wait_read();
     request_v();
   }  // (the forward asks for V once it knows whether the decays need its place first)
-  uint2 ktraw[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    ktraw[i] = make_uint2(0, 0);
-    if (kRecompute && r0 + i < valid)
-      ktraw[i] = *reinterpret_cast<const uint2*>(p.kt + row0 + (size_t)(r0 + i) * gld + c4);
-  }
   // (opaque, so that nothing is computed from them, and waits for them, where they were asked for)
   asm volatile("" : "+r"(n_beta), "+r"(n_bp), "+r"(n_chain), "+f"(n_pd), "+f"(n_alog), "+f"(n_centre), "+f"(n_bias.x), "+f"(n_bias.y),
                "+f"(n_bias.z), "+f"(n_bias.w));
@@ -433,6 +430,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   const float4 bias4 = n_bias;
   const float ea2 = __expf(n_alog) * kLog2e, centre = n_centre;
   uint32_t chain_a0 = n_chain;
+  int drawn = 0;
+  if (kRecompute && tid == 32) drawn = atomicAdd(p.cursor, 1);
   ok = tc::mbar_wait(bar_in, ph >> 2) && ok;
   ph ^= 4;
   if (!full) {  // rows past the sequence end read as zero, whatever lies there
@@ -542,8 +541,23 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   if (!kRecompute && tid == 0) tc::bulk_wait_read();  // the stores of the item before from the tiles that are written next
   // Does the chunk decay too much for one direct block?  (The same answer for all threads: every thread holds the
   // totals of its four channels, the CTA all 128.)  If so, which reference rows do its strips take?
+  if (kRecompute && tid == 32) s_item[slot ^ 1] = describe(drawn);
   const bool by_strip =
       __syncthreads_or(-fminf(fminf(Glast[0], Glast[1]), fminf(Glast[2], Glast[3])) > kDirectLimit) || p.by_strip;
+  // A recompute item is half as long and waits for memory first, so the next one is known here already: its scalars are asked for,
+  // its tiles into L2 (behind the products as in the forward, with the write keys by plain loads at the top of the item, the
+  // wait there was 6,000 of an item's 17,800 cycles; 8,192 items 296 -> 196 us, 1,536 strongly decaying ones 65 -> 47).
+  auto prefetch = [&](const int4& it) {  // the item's tiles of g, k, q and v into L2; when recomputing the write keys and T too
+    if (lane != 0 || it.x < 0) return;
+    const CUtensorMap* m = warp < 2 ? &tm_g : warp < 4 ? &tm_k : warp < 6 ? &tm_q : &tm_v;
+    tc::tma_prefetch_3d(m, 64 * (warp & 1), it.x % H, it.y);
+    if (kRecompute && warp < 2) tc::tma_prefetch_3d(&tm_p, 64 * warp, it.x % H, it.y);
+    if (kRecompute && warp == 2) tc::tma_prefetch_3d(&tm_akk, 0, it.x % H, it.y);
+  };
+  if (kRecompute) {
+    prefetch(s_item[slot ^ 1]);
+    if (s_item[slot ^ 1].x >= 0) request_scalars(s_item[slot ^ 1]);
+  }
   int refs = 0;  // 0: first and last row, 1: by halves, 2: pair_exact
   if (!kRecompute) {
     if (!by_strip) {
@@ -626,7 +640,8 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
       const uint2 kr = k_next, qr = q_next;
       k_next = ld_k((row + 1) & 7);
       q_next = ld_q((row + 1) & 7);
-      uint2 kt = ktraw[i];
+      uint2 kt = make_uint2(0, 0);
+      if (kRecompute) kt = *reinterpret_cast<const uint2*>(tiles + oL + blk * 8192 + half8 + off);
       if (!kRecompute) {
         const float pd = __shfl_sync(0xffffffffu, sc_pd, row), bp = __shfl_sync(0xffffffffu, sc_bp, row);
         float kc[4], f[4];
@@ -701,16 +716,13 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
     for (int i = 0; i < 4; ++i) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) G[i][c] = G[i + 4][c];
-      ktraw[i] = ktraw[i + 4];
     }
     }
   }
-  int drawn = 0;
-  if (tid == 32) drawn = atomicAdd(p.cursor, 1);  // (looked up while the pair products run)
+  if (!kRecompute && tid == 32) drawn = atomicAdd(p.cursor, 1);  // (looked up while the pair products run)
   tc::fence_proxy_async();
   tc::tc_fence_before();
   __syncthreads();  // (the strip exchange arrays are dead from here on: L takes their place)
-  if (kRecompute && tid == 32) s_item[slot ^ 1] = describe(drawn);
   if (!kRecompute && by_strip) {
     if (tid == 32) s_item[slot ^ 1] = describe(drawn);
     if (refs == 0) {
@@ -798,18 +810,13 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   __syncthreads();
   if (!kRecompute && by_strip && tid == 0) request_v();  // (the decays have been read)
   const int4 nx = s_item[slot ^ 1];
-  if (lane == 0) {  // the next item's tiles of g, k, q and v into L2
-    if (nx.x >= 0) {
-      const CUtensorMap* m = warp < 2 ? &tm_g : warp < 4 ? &tm_k : warp < 6 ? &tm_q : &tm_v;
-      tc::tma_prefetch_3d(m, 64 * (warp & 1), nx.x % H, nx.y);
-    }
-  }
+  if (!kRecompute) prefetch(nx);
 
   if (!kRecompute) {
     // ---- 5. scaled P -> Aqk;  T = (I + L)^-1 -> bf16 operand tile and Akk
     if (full) {
       if (tid == 0) {
-        tc::tma_store_3d(&tm_aqk, base + oP, 0, h, tok0);
+        tc::tma_store_3d(&tm_p, base + oP, 0, h, tok0);
         tc::bulk_commit();
       }
     } else {
@@ -864,7 +871,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
   tc::tc_fence_after();
   if (nx.x >= 0) {
     request_kq(nx);
-    request_scalars(nx);
+    if (!kRecompute) request_scalars(nx);
   }
   {
     const int q = warp & 3, m = warp >> 2;  // this warp's 16 tokens; W or U
@@ -922,19 +929,20 @@ int launch_chain_init(float* a_chain, size_t items, int* zero, cudaStream_t st) 
 
 int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) {
   const uint64_t H = ip.geo.heads, tok = ip.geo.total_tokens;
-  CUtensorMap tm_v, tm_akk, tm_aqk, tm_w, tm_u, tm_g, tm_k, tm_q;
+  CUtensorMap tm_v, tm_akk, tm_p, tm_w, tm_u, tm_g, tm_k, tm_q;  // tm_p: scaled P, which leaves; when recomputing the write keys, which arrive
   {
     const uint64_t dims[3] = {kD, H, tok}, str[2] = {kD * 2, H * kD * 2};
     const uint32_t box[3] = {64, 1, 64};
     if (!encode_bf16_map(&tm_v, ip.v, 3, dims, str, box) || !encode_bf16_map(&tm_w, ip.w, 3, dims, str, box) ||
         !encode_bf16_map(&tm_u, ip.u, 3, dims, str, box) || !encode_bf16_map(&tm_g, ip.g, 3, dims, str, box) ||
-        !encode_bf16_map(&tm_k, ip.k, 3, dims, str, box) || !encode_bf16_map(&tm_q, ip.q, 3, dims, str, box))
+        !encode_bf16_map(&tm_k, ip.k, 3, dims, str, box) || !encode_bf16_map(&tm_q, ip.q, 3, dims, str, box) ||
+        (recompute && !encode_bf16_map(&tm_p, ip.kt, 3, dims, str, box)))
       return PKDA_ERR_LAUNCH;
   }
   {
     const uint64_t dims[3] = {kChunk, H, tok}, str[2] = {kChunk * 2, H * kChunk * 2};
     const uint32_t box[3] = {64, 1, 64};
-    if (!encode_bf16_map(&tm_akk, ip.Akk, 3, dims, str, box) || !encode_bf16_map(&tm_aqk, ip.Aqk, 3, dims, str, box))
+    if (!encode_bf16_map(&tm_akk, ip.Akk, 3, dims, str, box) || (!recompute && !encode_bf16_map(&tm_p, ip.Aqk, 3, dims, str, box)))
       return PKDA_ERR_LAUNCH;
   }
   const int sms = sm_count();
@@ -944,12 +952,12 @@ int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) 
   if (recompute) {
     if (!ensure_dynamic_smem(pkda_intra_fwd_tc_kernel<true>, intratc::kSmem, 100))
       return PKDA_ERR_LAUNCH;
-    launch_kernel(false, pkda_intra_fwd_tc_kernel<true>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_aqk, tm_w, tm_u,
+    launch_kernel(false, pkda_intra_fwd_tc_kernel<true>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_p, tm_w, tm_u,
                   tm_g, tm_k, tm_q, ip);
   } else {
     if (!ensure_dynamic_smem(pkda_intra_fwd_tc_kernel<false>, intratc::kSmem, 100))
       return PKDA_ERR_LAUNCH;
-    launch_kernel(false, pkda_intra_fwd_tc_kernel<false>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_aqk, tm_w, tm_u,
+    launch_kernel(false, pkda_intra_fwd_tc_kernel<false>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_p, tm_w, tm_u,
                   tm_g, tm_k, tm_q, ip);
   }
   return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
