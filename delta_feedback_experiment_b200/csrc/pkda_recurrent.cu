@@ -169,16 +169,30 @@ pkda_recurrent_kernel(const RecParams p) {
   const size_t tstep = (size_t)H * D;
   const size_t tbase = ((size_t)sq.bos * H + h) * D + col0;
   T* const o_row = static_cast<T*>(p.o) + tbase;
+  // The vectors of a token, and its value (kTwoAhead).
+  struct Rows { float2 kx[R / 2], al[R / 2], wk[R / 2], qs[R / 2]; float v; };
+  Rows ahead[L::kTwoAhead ? 2 : 1];
+  auto load_token = [&](Rows& x, uint32_t vec) {
+    load_rows<L>(vec, rg, x.kx);
+    load_rows<L>(vec + 4 * D, rg, x.al);
+    load_rows<L>(vec + 8 * D, rg, x.wk);
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x.v) : "r"(vec + 16 * D + 4 * col0));
+    load_rows<L>(vec + 12 * D, rg, x.qs);
+  };
+  if (L::kTwoAhead && nblk > 0) {
+    bar_sync_n(1, nthreads);
+    load_token(ahead[0], smem_u32(stage));
+    load_token(ahead[L::kTwoAhead], smem_u32(stage) + 4 * VEC);
+  }
   for (int b = 0; b < nblk; ++b) {
     const int s = b & 1, t0 = b * TB;
     if (kSave && (t0 & (kCkpt - 1)) == 0)
       store_state(p.save.S + ((ckpt_base(p.geo, n, sq.bos) + t0 / kCkpt) * H + h) * (size_t)(D * D) + col0);
-    bar_sync_n(1 + s, nthreads);
+    if (!L::kTwoAhead) bar_sync_n(1 + s, nthreads);
     const uint32_t st = smem_u32(stage + s * L::kStage);
     float oacc[L::kTO * kCPL], ekeep[L::kSums];  // [token][column]
     // Two vectors of rows are held at a time.  x: exp(g) k, then exp(g) of a token; y: beta kw, then scale q.
     float2 x[R / 2], y[R / 2];
-    load_rows<L>(st, rg, x);
     auto out_sum = [&](int u) {  // the sum for o of token u (of the block)
 #pragma unroll
       for (int c = 0; c < kCPL; ++c) {
@@ -198,6 +212,36 @@ pkda_recurrent_kernel(const RecParams p) {
         if (to < sq.len) o_row[(size_t)to * tstep + n % kCPL] = from_f<T>(oacc[i]);
       }
     };
+    if constexpr (L::kTwoAhead) {
+      const uint32_t nx = smem_u32(stage + (s ^ 1) * L::kStage);
+#pragma unroll
+      for (int t = 0; t < TB; ++t) {
+        Rows& w = ahead[t & 1];
+        float2 a0 = __fmul2_rn(w.kx[0], S[0][0]), a1 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 1; i < R / 2; ++i) {
+          if (i & 1) a1 = __ffma2_rn(w.kx[i], S[0][i], a1);
+          else a0 = __ffma2_rn(w.kx[i], S[0][i], a0);
+        }
+        float e = (a0.x + a0.y) + (a1.x + a1.y);
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) S[0][i] = __fmul2_rn(w.al[i], S[0][i]);
+#pragma unroll
+        for (int o = RG / 2; o >= 1; o >>= 1) e += xor_lane(e, o);
+        e = w.v - e;
+        if (kSave && rg == t / L::kSums) ekeep[t % L::kSums] = e;
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) S[0][i] = __ffma2_rn(w.wk[i], make_float2(e, e), S[0][i]);
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) y[i] = w.qs[i];
+        out_sum(t);
+        if (t == TB - 2 && b + 1 < nblk) bar_sync_n(1 + (s ^ 1), nthreads);
+        if (t + 2 < TB) load_token(w, st + 4 * (t + 2) * VEC);
+        else if (b + 1 < nblk) load_token(w, nx + 4 * (t + 2 - TB) * VEC);
+      }
+      if (b + 2 < nblk) bar_arrive_n(3 + s, nthreads);
+    } else {
+    load_rows<L>(st, rg, x);
 #pragma unroll
     for (int t = 0; t < TB; ++t) {
       // e's sum over the lane's rows, then rounds of shuffles; behind each round's shuffles stands what does not depend on
@@ -257,6 +301,7 @@ pkda_recurrent_kernel(const RecParams p) {
     }
     out_sum(TB - 1);
     if (b + 2 < nblk) bar_arrive_n(3 + s, nthreads);
+    }
 #pragma unroll
     for (int o = RG / 2; o >= 1; o >>= 1) out_round(TB - 1, o);
     if (kSave) {  // (one column per lane)

@@ -39,6 +39,12 @@ template <int D, int kCPL_> struct ScanLay {
   static constexpr int kProdPerGroup = D < 32 ? 32 : D;
   static constexpr int kProd = kGroups * kProdPerGroup;
   static constexpr int kMaxConsumers = 8;             // consumer warps per CTA, at most
+  // Row vectors of two tokens in registers, those of a token asked for two tokens ahead: the loads of a token are 32 cycles of the
+  // warp's way to shared memory per vector at 64 rows, and shuffles queue behind them.  (With the other vectors of a token asked for
+  // while its sum is formed, a token of the state cotangent takes 223 cycles at 64 rows, 150 at 32, so 161 and 135; at 128 rows
+  // a lane has 16 rows and the registers are not there: 232 and 248.  2 x 512 tokens of 4 heads x 64, forward and backward: 188 -> 182 us;
+  // 2 x 824 of 8 x 32: 268 -> 238.)
+  static constexpr bool kTwoAhead = kCPL_ == 1 && kR <= 8;
   static constexpr int kVecs = 5;                     // row vectors per token
   static constexpr int kStage = kTB * kVecs * D;      // floats of one staged block
   static constexpr int kSmem = 2 * kStage * 4;

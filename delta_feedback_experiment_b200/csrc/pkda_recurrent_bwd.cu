@@ -132,13 +132,51 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
   };
   T* dv = static_cast<T*>(p.dv);
   const size_t tbase = ((size_t)sq.bos * H + h) * D + col0;
+  struct Rows { float2 qs[R / 2], w[R / 2], nk[R / 2], al[R / 2]; float dot; };  // the vectors of a token, and its dO (kTwoAhead)
+  Rows ahead[L::kTwoAhead ? 2 : 1];
+  auto load_token = [&](Rows& x, uint32_t vec) {
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x.dot) : "r"(vec + 16 * D + 4 * col0));
+    load_rows<L>(vec, rg, x.qs);
+    load_rows<L>(vec + 4 * D, rg, x.w);
+    load_rows<L>(vec + 8 * D, rg, x.nk);
+    load_rows<L>(vec + 12 * D, rg, x.al);
+  };
+  if (L::kTwoAhead && nblk > 0) {
+    bar_sync_n(1, nthreads);
+    load_token(ahead[L::kTwoAhead], smem_u32(stage) + 4 * (TB - 1) * VEC);
+    load_token(ahead[0], smem_u32(stage) + 4 * (TB - 2) * VEC);
+  }
   for (int it = 0; it < nblk; ++it) {
     const int s = it & 1, blk = nblk - 1 - it, t0 = blk * TB;
     float keep[L::kSums];
     if (it == 0 || ((t0 + TB) & (kCkpt - 1)) == 0)
       store_state(p.dSck + ((ckpt_base(p.geo, n, sq.bos) + t0 / kCkpt) * H + h) * (size_t)(D * D) + col0);
-    bar_sync_n(1 + s, nthreads);
+    if (!L::kTwoAhead) bar_sync_n(1 + s, nthreads);
     const uint32_t st = smem_u32(stage + s * L::kStage);
+    if constexpr (L::kTwoAhead) {
+      const uint32_t nx = smem_u32(stage + (s ^ 1) * L::kStage);
+#pragma unroll
+      for (int t = TB - 1; t >= 0; --t) {
+        Rows& x = ahead[t & 1];
+        float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) {
+          S[i] = __ffma2_rn(x.qs[i], make_float2(x.dot, x.dot), S[i]);
+          if (i & 1) a1 = __ffma2_rn(x.w[i], S[i], a1);
+          else a0 = __ffma2_rn(x.w[i], S[i], a0);
+        }
+        float de = (a0.x + a0.y) + (a1.x + a1.y);
+#pragma unroll
+        for (int o = RG / 2; o >= 1; o >>= 1) de += xor_lane(de, o);
+        if (rg == t / L::kSums) keep[t % L::kSums] = de;
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i)
+          S[i] = __fmul2_rn(x.al[i], __ffma2_rn(x.nk[i], make_float2(de, de), S[i]));
+        if (t == 1 && it + 1 < nblk) bar_sync_n(1 + (s ^ 1), nthreads);
+        if (t >= 2) load_token(x, st + 4 * (t - 2) * VEC);
+        else if (it + 1 < nblk) load_token(x, nx + 4 * (t - 2 + TB) * VEC);
+      }
+    } else {
     float2 qs[R / 2], w[R / 2];
     float dot;
     auto load_do = [&](int t) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(dot) : "r"(st + 4 * (t * VEC + 4 * D + col0))); };
@@ -178,6 +216,7 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
 #pragma unroll
       for (int i = 0; i < R / 2; ++i)
         S[i] = __fmul2_rn(al[i], __ffma2_rn(nk[i], make_float2(de, de), S[i]));
+    }
     }
     if (it + 2 < nblk) bar_arrive_n(3 + s, nthreads);
 #pragma unroll
