@@ -16,6 +16,8 @@
 // D = 64, fp32: 548 -> 86 us (90 when it leaves what the backward needs).  With the output of a token and the decay of the
 // state taken while the next token's sum goes through its shuffles (and four columns a lane reduced by three rounds of four shuffles instead
 // of five of one or two): 24.9 -> 23.9 us, and the pass of 512 tokens, forward and backward, 190.9 -> 188.1.
+#include <type_traits>
+
 #include "pkda_launch.h"
 #include "pkda_recurrent.cuh"
 
@@ -57,35 +59,50 @@ pkda_recurrent_kernel(const RecParams p) {
     // ------------------------------------------------ producers: row vectors of TB tokens at a time
     const int ptid = 32 * p.warps.producer(warp) + lane;
     const int grp = ptid / L::kProdPerGroup, c = ptid - grp * L::kProdPerGroup;
-    const bool act = c < D;
+    const bool act = D >= 32 || c < D;
     const float ea = expf(p.A_log[h]), centre = p.log_atk_scale[h];
     const float bias = act ? p.dt_bias[h * D + c] : 0.f;
     float A = (act && p.A0) ? p.A0[(size_t)unit * D + c] : 0.f;
     if (p.inplace_A) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
-    const size_t step = (size_t)H * D;
-    const size_t base = ((size_t)sq.bos * H + h) * D + (act ? c : 0);
-    const T *kp = static_cast<const T*>(p.k) + base, *qp = static_cast<const T*>(p.q) + base,
-            *gp = static_cast<const T*>(p.g) + base, *vp = static_cast<const T*>(p.v) + base;
+    // The producers set the pace of a scan that has its SM to itself, and the addresses and checks of a block's 16 loads were 1,000 of their
+    // 2,600 cycles: running pointers, 32-bit offsets, no checks in a whole block.  (The vectors that the backward needs are
+    // written by all CTAs of the unit in turn, a block each: by the first one alone, that one was late.)
+    const int step = H * D;
+    const size_t first = (size_t)sq.bos * H + h, base = first * D + (act ? c : 0), own = base + (size_t)(TPG * grp) * step;
+    const T *kp = static_cast<const T*>(p.k) + base, *qp = static_cast<const T*>(p.q) + own, *gp = static_cast<const T*>(p.g) + own,
+            *vp = static_cast<const T*>(p.v) + own;
+    const int kind = lane >> 3;  // of the lane's scalar: lane = 8 * kind + token
+    const float* pdp = p.g_atk + first + (size_t)(lane & 7) * H;
+    const T* bp = static_cast<const T*>(kind == 1 ? p.beta_atk : p.beta) + first + (size_t)(lane & 7) * H;
     typename Raw<T>::type kr[TB], qr[TPG], gr[TPG], vr[TPG], bt;
     float sc;
-    auto fetch = [&](int t0) {
+    auto fetch_block = [&](int left, auto whole) {  // left: tokens from the block's first one on
+      constexpr bool kWhole = decltype(whole)::value;
 #pragma unroll
-      for (int i = 0; i < TB; ++i) kr[i] = (act && t0 + i < sq.len) ? Raw<T>::load(kp + (size_t)(t0 + i) * step) : 0;
+      for (int i = 0; i < TB; ++i) kr[i] = act && (kWhole || i < left) ? Raw<T>::load(kp + i * step) : 0;
 #pragma unroll
       for (int i = 0; i < TPG; ++i) {
-        const int t = t0 + TPG * grp + i;
-        const bool ok = act && t < sq.len;
-        qr[i] = ok ? Raw<T>::load(qp + (size_t)t * step) : 0;
-        gr[i] = ok ? Raw<T>::load(gp + (size_t)t * step) : 0;
-        vr[i] = ok ? Raw<T>::load(vp + (size_t)t * step) : 0;
+        const bool ok = act && (kWhole || TPG * grp + i < left);
+        qr[i] = ok ? Raw<T>::load(qp + i * step) : 0;
+        gr[i] = ok ? Raw<T>::load(gp + i * step) : 0;
+        vr[i] = ok ? Raw<T>::load(vp + i * step) : 0;
       }
-      // the token's three scalars: lane = 8 * kind + token
-      const int t = t0 + (lane & 7), kind = lane >> 3;
-      const size_t sidx = (size_t)(sq.bos + t) * H + h;
+      const bool ok = kWhole || (lane & 7) < left;
       sc = 0.f;
       bt = 0;
-      if (t < sq.len && kind == 0) sc = p.g_atk[sidx];
-      if (t < sq.len && (kind == 1 || kind == 2)) bt = Raw<T>::load(static_cast<const T*>(kind == 1 ? p.beta_atk : p.beta) + sidx);
+      if (ok && kind == 0) sc = *pdp;
+      if (ok && kind != 0) bt = Raw<T>::load(bp);  // (the last eight lanes' are not used)
+    };
+    auto fetch = [&](int t0) {
+      const int left = sq.len - t0;
+      if (left >= TB) fetch_block(left, std::true_type{});
+      else fetch_block(left, std::false_type{});
+      kp += TB * step;
+      qp += TB * step;
+      gp += TB * step;
+      vp += TB * step;
+      pdp += TB * H;
+      bp += TB * H;
     };
     if (nblk > 0) fetch(0);
     for (int b = 0; b < nblk; ++b) {
@@ -122,7 +139,7 @@ pkda_recurrent_kernel(const RecParams p) {
           row[2 * D] = wk;
           row[3 * D] = qc[i] * p.scale;
           row[4 * D] = vc[i];
-          if (kSave && cg == 0 && ok) {
+          if (kSave && b % p.groups == cg && ok) {
             const size_t idx = base + (size_t)(t0 + tl) * step;
             p.save.al[idx] = al;
             p.save.w[idx] = wk;

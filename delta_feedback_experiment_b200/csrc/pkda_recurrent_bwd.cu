@@ -16,6 +16,8 @@
 // backwards over the tokens, and the terms that depend on it close the pass.
 // (One CTA per (sequence, head) that replayed and walked back every token with the whole state took
 // 1655 us for 2 x 4 units of 512 tokens at D = 64, fp32, behind a 551 us forward; these take 110 us, behind 90.)
+#include <type_traits>
+
 #include "pkda_launch.h"
 #include "pkda_recurrent.cuh"
 
@@ -64,25 +66,35 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
   if (warp >= nw) {
     const int ptid = 32 * p.warps.producer(warp) + lane;
     const int grp = ptid / L::kProdPerGroup, c = ptid - grp * L::kProdPerGroup;
-    const bool act = c < D;
-    const size_t base = ((size_t)sq.bos * H + h) * D + (act ? c : 0);
-    const T *kp = static_cast<const T*>(p.k) + base, *qp = static_cast<const T*>(p.q) + base,
-            *dop = static_cast<const T*>(p.d_o) + base;
-    const float *alp = p.s.al + base, *wp = p.s.w + base;
+    const bool act = D >= 32 || c < D;
+    // (running pointers, 32-bit offsets and no checks in a whole block, as in the forward)
+    const int step = H * D;
+    const size_t at = ((size_t)sq.bos * H + h) * D + (act ? c : 0) + (size_t)(nblk > 0 ? (nblk - 1) * TB + TPG * grp : 0) * step;
+    const T *kp = static_cast<const T*>(p.k) + at, *qp = static_cast<const T*>(p.q) + at, *dop = static_cast<const T*>(p.d_o) + at;
+    const float *alp = p.s.al + at, *wp = p.s.w + at;
     typename Raw<T>::type qr[TPG], kr[TPG], dr[TPG];
     float wr[TPG], ar[TPG];
-    auto fetch = [&](int t0) {
+    auto fetch_block = [&](int left, auto whole) {  // left: tokens from the block's first one on
+      constexpr bool kWhole = decltype(whole)::value;
 #pragma unroll
       for (int i = 0; i < TPG; ++i) {
-        const int t = t0 + TPG * grp + i;
-        const bool ok = act && t < sq.len;
-        const size_t at = (size_t)t * tstep;
-        qr[i] = ok ? Raw<T>::load(qp + at) : 0;
-        wr[i] = ok ? wp[at] : 0.f;
-        kr[i] = ok ? Raw<T>::load(kp + at) : 0;
-        dr[i] = ok ? Raw<T>::load(dop + at) : 0;
-        ar[i] = ok ? alp[at] : 1.f;  // a token past the end leaves dS as it is
+        const bool ok = act && (kWhole || TPG * grp + i < left);
+        qr[i] = ok ? Raw<T>::load(qp + i * step) : 0;
+        wr[i] = ok ? wp[i * step] : 0.f;
+        kr[i] = ok ? Raw<T>::load(kp + i * step) : 0;
+        dr[i] = ok ? Raw<T>::load(dop + i * step) : 0;
+        ar[i] = ok ? alp[i * step] : 1.f;  // a token past the end leaves dS as it is
       }
+    };
+    auto fetch = [&](int t0) {
+      const int left = sq.len - t0;
+      if (left >= TB) fetch_block(left, std::true_type{});
+      else fetch_block(left, std::false_type{});
+      kp -= TB * step;
+      qp -= TB * step;
+      dop -= TB * step;
+      alp -= TB * step;
+      wp -= TB * step;
     };
     if (nblk > 0) fetch((nblk - 1) * TB);
     for (int it = 0; it < nblk; ++it) {
