@@ -283,6 +283,9 @@ __global__ void __launch_bounds__(GradLay<D>::kThreads)
 pkda_recurrent_grad_kernel(const RecBwdParams p) {
   after_previous();
   using L = GradLay<D>;
+  // The next column group's state and the chain rule's inputs are asked for ahead where the registers are there (up to 64 rows:
+  // 32 checkpoint blocks of 4 heads x 64 33.6 -> 29 us; with the loads of the closing pass together and the last sums beside it, 161 -> 156 us a pass).
+  constexpr bool kAhead = D <= 64;
   constexpr int NS = L::kNS, NG = L::kNG, SUB = L::kSub, TPS = L::kTPS;
   extern __shared__ __align__(16) float sm[];
   float4* s_row = reinterpret_cast<float4*>(sm);  // [32][D]: exp(g), w, k, scale q
@@ -309,7 +312,8 @@ pkda_recurrent_grad_kernel(const RecBwdParams p) {
   const int nt = min(kCkpt, sq.len - t0);
   const size_t tstep = (size_t)H * D;
   const size_t tbase = ((size_t)(sq.bos + t0) * H + h) * D;
-  for (int i = tid; i < kCkpt * D; i += L::kThreads) {
+#pragma unroll 4
+  for (int i = tid; i < kCkpt * D; i += L::kThreads) {  // (28 loads in flight)
     const int t = i / D, c = i - t * D;
     const bool ok = t < nt;
     const size_t idx = tbase + (size_t)t * tstep + c;
@@ -329,13 +333,28 @@ pkda_recurrent_grad_kernel(const RecBwdParams p) {
 
   const float ea = expf(p.A_log[h]), centre = p.log_atk_scale[h], bias = p.dt_bias[h * D + r];
   float accA = 0.f, accB = 0.f, accC = 0.f;
+  float4 S4n = kAhead ? *reinterpret_cast<const float4*>(S0) : make_float4(0.f, 0.f, 0.f, 0.f);
   for (int sb = (nt - 1) / SUB; sb >= 0; --sb) {
+    // what the chain rule below needs of memory
+    float An_n[TPS], bw_n[TPS], g_n[TPS];
+    auto chain_inputs = [&](int i) {
+      const int t = min(SUB * sb + TPS * sub + i, nt - 1);
+      const size_t sidx = (size_t)(sq.bos + t0 + t) * H + h;
+      An_n[i] = p.s.A[sidx * D + r];
+      bw_n[i] = to_f(static_cast<const T*>(p.beta)[sidx]);
+      g_n[i] = to_f(static_cast<const T*>(p.g)[sidx * D + r]);
+    };
+    if (kAhead) {
+#pragma unroll
+      for (int i = 0; i < TPS; ++i) chain_inputs(i);
+    }
     float acc[4 * SUB];  // [token][dqs, dw, dk_read, dg]
 #pragma unroll
     for (int i = 0; i < 4 * SUB; ++i) acc[i] = 0.f;
 #pragma unroll 1
     for (int cg = 0; cg < NG; ++cg) {
-      const float4 S4 = *reinterpret_cast<const float4*>(S0 + cg * L::kGC);
+      const float4 S4 = kAhead ? S4n : *reinterpret_cast<const float4*>(S0 + cg * L::kGC);
+      if (kAhead) S4n = *reinterpret_cast<const float4*>(S0 + (cg + 1 < NG ? cg + 1 : 0) * L::kGC);
       float2 S[2] = {make_float2(S4.x, S4.y), make_float2(S4.z, S4.w)};
       const float* ec = s_e + cg * L::kGC + 4 * sub;
       const float* dec = s_de + cg * L::kGC + 4 * sub;
@@ -398,10 +417,11 @@ pkda_recurrent_grad_kernel(const RecBwdParams p) {
       const bool ok = t < nt;
       float x_db = 0.f;
       if (ok) {
-        const size_t sidx = (size_t)(sq.bos + t0 + t) * H + h, idx = sidx * D + r;
+        const size_t idx = ((size_t)(sq.bos + t0 + t) * H + h) * D + r;
         const float kc = s_row[t * D + r].z;
-        const float An = p.s.A[idx], bw = to_f(static_cast<const T*>(p.beta)[sidx]);
-        const float rawz = to_f(static_cast<const T*>(p.g)[idx]) + bias;
+        if (!kAhead) chain_inputs(i);
+        const float An = An_n[i], bw = bw_n[i];
+        const float rawz = g_n[i] + bias;
         const float dev = logf(An + p.eps) - centre, den = 1.f + fabsf(dev);
         const float Bf = expf(-p.ln_x * dev / den);
         const float dw = acc[4 * i + 1], dgl = acc[4 * i + 3];
@@ -517,20 +537,50 @@ __global__ void __launch_bounds__(256) pkda_recurrent_close_kernel(const RecBwdP
     const float y = __shfl_down_sync(0xffffffffu, suffix, o);
     if (lane + o < 32) suffix *= y;
   }
-  for (int tl = warp; tl < nt; tl += 8) {
-    const int t = t0 + tl;
-    const float fade = __shfl_sync(0xffffffffu, suffix, tl);
+  // a warp's four tokens: every load of all four is issued before the first is used
+  constexpr int N = (D + 31) / 32;
+  typename Raw<T>::type kr[4][N], br[4];
+  float lm[4][N], ap[4][N], dp[4][N], cr[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) cr[j] = lane + 32 * j < D ? p.carry[slot * D + lane + 32 * j] : 0.f;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int tl = warp + 8 * u, t = t0 + tl;
+    br[u] = 0;
     const size_t sidx = (size_t)(sq.bos + t) * H + h;
-    const float bp = to_f(static_cast<const T*>(p.beta_atk)[sidx]);
+    if (tl < nt) br[u] = Raw<T>::load(static_cast<const T*>(p.beta_atk) + sidx);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const int c = lane + 32 * j;
+      const size_t idx = sidx * D + c;
+      kr[u][j] = 0;
+      lm[u][j] = ap[u][j] = dp[u][j] = 0.f;
+      if (tl < nt && c < D) {
+        kr[u][j] = Raw<T>::load(static_cast<const T*>(p.k) + idx);
+        lm[u][j] = p.lam[idx];
+        dp[u][j] = p.dkp[idx];
+        if (t > 0) ap[u][j] = p.s.A[idx - (size_t)H * D];
+        else if (p.A0) ap[u][j] = p.A0[((size_t)n * H + h) * D + c];
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int tl = warp + 8 * u;
+    if (tl >= nt) break;
+    const float fade = __shfl_sync(0xffffffffu, suffix, tl);
+    const size_t sidx = (size_t)(sq.bos + t0 + tl) * H + h;
+    const float bp = Raw<T>::value(br[u]);
     float sb = 0.f, sg = 0.f;
 #pragma unroll
-    for (int c = lane; c < D; c += 32) {
-      const size_t idx = sidx * D + c;
-      const float kc = to_f(static_cast<const T*>(p.k)[idx]), lam = p.lam[idx] + fade * p.carry[slot * D + c];
-      const float Ap = t > 0 ? p.s.A[idx - (size_t)H * D] : (p.A0 ? p.A0[((size_t)n * H + h) * D + c] : 0.f);
-      static_cast<T*>(p.dk)[idx] = from_f<T>(p.dkp[idx] + 2.f * lam * bp * kc);
-      sb += lam * kc * kc;
-      sg += lam * Ap;
+    for (int j = 0; j < N; ++j) {
+      const int c = lane + 32 * j;
+      if (c < D) {
+        const float kc = Raw<T>::value(kr[u][j]), lam = lm[u][j] + fade * cr[j];
+        static_cast<T*>(p.dk)[sidx * D + c] = from_f<T>(dp[u][j] + 2.f * lam * bp * kc);
+        sb += lam * kc * kc;
+        sg += lam * ap[u][j];
+      }
     }
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
@@ -548,7 +598,7 @@ __global__ void __launch_bounds__(256) pkda_recurrent_close_kernel(const RecBwdP
 __global__ void __launch_bounds__(256)
 pkda_recurrent_bwd_reduce_kernel(int blocks, int H, int D, const float* partA, const float* partB, const float* partC,
                                  float* dA_log, float* ddt_bias, float* dcentre) {
-  after_previous();
+  launch_dependents();  // (it needs nothing of the pass in front of it and runs beside it)
   __shared__ float s[3][256];
   const int h = blockIdx.x, tid = threadIdx.x, c = tid % D, sl = tid / D, ns = 256 / D;
   float b = 0.f, a = 0.f, cc = 0.f;
@@ -566,6 +616,7 @@ pkda_recurrent_bwd_reduce_kernel(int blocks, int H, int D, const float* partA, c
     __syncthreads();
   }
   if (tid == 0) { dA_log[h] = s[1][0]; dcentre[h] = s[2][0]; }
+  wait_prerequisites();
 }
 
 struct RecBwdWorkspace {
