@@ -210,6 +210,7 @@ pkda_scan_bwd_kernel(const ScanBwdParams p) {
 // the shared-memory tile never reaches the neighbouring head.
 struct IntraBwdMaps {
   CUtensorMap d_o, dF, h, dh, Akk, E;
+  CUtensorMap q, k, kt, g;
   CUtensorMap dq, dv, dk_read, dkt;
 };
 
@@ -228,11 +229,14 @@ constexpr int oDM = oDP + kChunk * kLdC * 2;
 constexpr int oFac = oDM + kChunk * kLdC * 2; // f32 [64][kLdY]: kt 2^(z - G)
 constexpr int kLdY = kD + 4;                  // = 4 (mod 32): rows 2 t and channels g of a fragment lie in different banks
 constexpr int oSmall = oFac + kChunk * kLdG * 4;
-// small: beta[64] db[64] hdh[128] gcv[128] col[4][128] rb[4][64] red[16] bias[128] worst[4][3] diag[64] there[36]
-constexpr int kSmallFloats = 64 + 64 + 128 + 128 + 512 + 256 + 16 + 128 + 12 + 64 + 36;
-constexpr int oBar = oSmall + kSmallFloats * 4;  // one mbarrier
-constexpr int kSmem = oBar + 16;
-constexpr uint32_t kTmaBytes = (3 * kChunk + 2 * kD) * kLdD * 2 + kChunk * kLdC * 2;  // dO, dF, E, S0, dS1 and Tm tiles
+// small: beta[64] db[64] hdh[128] gcv[128] col[4][128] rb[4][64] red[16] bias[2][128] worst[4][3] diag[64] there[36]
+constexpr int kSmallFloats = 64 + 64 + 128 + 128 + 512 + 256 + 16 + 256 + 12 + 64 + 36;
+constexpr int oBar = oSmall + kSmallFloats * 4;  // three mbarriers: the tiles of phase A, those of phase B, what comes ahead
+constexpr int oRaw = (oBar + 32 + 127) / 128 * 128;  // bf16 [64][136]: the raw gate of a full chunk, asked for while the item before ends
+constexpr int kSmem = oRaw + kTileBytes;
+static_assert(kSmem <= 232448, "shared memory of one SM");
+// A copy takes its issuing thread some 500 cycles, so every one has a warp of its own (the first lane arrives with its bytes).
+constexpr int kCopiesA = 6, kCopiesB = 3, kCopiesAhead = 2;
 static_assert(2 * kChunk * kLdC * 2 >= kTileBytes && oDP % 128 == 0, "E waits in the pair-gradient tiles");
 static_assert(oBar % 8 == 0 && oA1 % 128 == 0 && oTm % 128 == 0 && oDE % 128 == 0 && oFac % 128 == 0,
               "TMA destinations and the mbarrier must be aligned");
@@ -353,8 +357,45 @@ __device__ __forceinline__ void atk_carry(const float* ex, const IntraBwdParams&
 }
 }  // namespace ib
 
-// One (chunk bx, head by) item; every thread of the CTA takes part.
-__device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const IntraBwdMaps& maps, int bx, int by) {
+// Chunk, head, first token and valid tokens of an item (chunk * heads + head); chunk -1 for none.
+__device__ __forceinline__ int4 describe_item(const Geo& geo, int item) {
+  int n, tok0, valid;
+  const int chunk = item / geo.heads;
+  if (item < 0 || !chunk_lookup(geo, chunk, n, tok0, valid)) return make_int4(-1, 0, 0, 0);
+  return make_int4(chunk, item - chunk * geo.heads, tok0, valid);
+}
+// What a full chunk needs first, asked for while the item before it ends: the raw gate, beta, Gam_last and the gate's bias.  All of it
+// lands in shared memory: in registers, the tail of the item before waited for it.  phase: the barrier's for that chunk.  With the
+// next item drawn on the way and a warp for every copy, the first 8,000 of an item's 47,000 cycles are 5,000 (1,408 items 289 -> 280 us,
+// 256 92 -> 86, 7,168 1,300 -> 1,276).
+__device__ __forceinline__ void intra_bwd_ahead(const IntraBwdParams& p, const IntraBwdMaps& maps, int4 it, uint32_t phase) {
+  using namespace ib;
+  extern __shared__ __align__(128) unsigned char smem[];
+  if (it.x < 0 || !p.use_tma || it.w != kChunk) return;
+  const int tid = threadIdx.x, h = it.y;
+  const uint32_t bar = smem_u32(smem + oBar) + 16;
+  float* sBeta = reinterpret_cast<float*>(smem + oSmall);
+  if (tid == kThreads - 64) {
+    tc::mbar_expect_tx(bar, kTileBytes);
+    tc::tma_load_2d(smem_u32(smem + oRaw), &maps.g, bar, h * kD, it.z);
+  }
+  if (tid == kThreads - 96) {
+    const size_t chh = (size_t)it.x * p.geo.heads + h;
+    tc::mbar_expect_tx(bar, (kChunk + kD) * 4);
+    tc::bulk_load(smem_u32(sBeta), p.beta_c + chh * kChunk, kChunk * 4, bar);
+    tc::bulk_load(smem_u32(sBeta + 256), p.gc + chh * kD, kD * 4, bar);
+  }
+  if (tid >= kD && tid < 2 * kD)  // (dt_bias may start at any float)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(sBeta + 64 + 64 + 128 + 128 + 512 + 256 + 16 + phase * kD + tid - kD)),
+                 "l"(p.dt_bias + h * kD + tid - kD));
+  cp_async_commit();
+}
+
+// The item in s_next (chunk, head, first token, valid tokens); every thread of the CTA takes part.  With a work list one thread draws
+// the CTA's next item near the end, in steps that nothing waits for, and leaves it in s_next (chunk -1: none).  (Drawn early, the last turn
+// is less even: 290 -> 302 us for 1,408 items.)  A word behind the barriers holds their phase, which changes with every full chunk; in a
+// register it cost spills and the whole gain.
+__device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const IntraBwdMaps& maps, int4* s_next) {
   using namespace ib;
   extern __shared__ __align__(128) unsigned char smem[];
   bf16* sdO = reinterpret_cast<bf16*>(smem + oA0);
@@ -376,14 +417,12 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   float* sCol = sGcv + 128;  // [4][128]
   float* sRb = sCol + 512;   // [4][64]
   float* sRed = sRb + 256;   // [16]
-  float* sBias = sRed + 16;  // [128]
-  float* sWorst = sBias + 128;    // [4][3]
+  float* sWorst = sRed + 16 + 256;    // [4][3]
   float* sDiag = sWorst + 12;     // [64] diagonal of dP
   int* sThere = reinterpret_cast<int*>(sDiag + 64);  // [36]
 
-  int n, tok0, valid;
-  if (!chunk_lookup(p.geo, bx, n, tok0, valid)) return;
-  const int h = by, H = p.geo.heads;
+  volatile uint32_t* const s_phase = reinterpret_cast<volatile uint32_t*>(smem + oBar + 24);
+  const int bx = s_next->x, h = s_next->y, tok0 = s_next->z, valid = s_next->w, H = p.geo.heads;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gq = lane >> 2, tq = lane & 3;
   const int I = warp & 3, cq = warp >> 2;
@@ -394,34 +433,42 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   const long cld = (long)H * kChunk;
 
   // ================= phase A: state-coupled terms =================
-  // The per-row scalars the first barrier waits for are requested before everything else.
+  const bool by_tma = p.use_tma && valid == kChunk;
+  const bool drawer = p.slow_list && tid == kThreads - 32;
+  // (a ragged chunk takes the half of the bias that the full chunk behind it does not)
+  auto bias = [&]() { return sRed + 16 + (by_tma ? *s_phase : *s_phase ^ 1) * kD; };  // [128]
+  GateRaw<kThreads> graw;
   float s_small = 0.f;
-  if (tid < kChunk) s_small = p.beta_c[chh * kChunk + tid];
-  else if (tid >= 2 * kD && tid < 3 * kD) s_small = p.gc[chh * kD + tid - 2 * kD];
-  else if (tid >= kD && tid < 2 * kD) s_small = p.dt_bias[h * kD + tid - kD];
-  GateRaw<kThreads> graw;  // the raw gate is needed next
-  gate_load(graw, p.g + row0, gld, valid, tid);
+  if (!by_tma) {
+    if (tid < kChunk) s_small = p.beta_c[chh * kChunk + tid];
+    else if (tid >= 2 * kD && tid < 3 * kD) s_small = p.gc[chh * kD + tid - 2 * kD];
+    else if (tid >= kD && tid < 2 * kD) s_small = p.dt_bias[h * kD + tid - kD];
+    gate_load(graw, p.g + row0, gld, valid, tid);
+  }
   // dS1 waits where the strips' kt goes later until the dkg product, E in the (not yet
   // used) pair-gradient tiles until S0 has left the tile E belongs in
   bf16* sdSC = reinterpret_cast<bf16*>(smem + oFac);
   bf16* sEarly = reinterpret_cast<bf16*>(smem + oDP);
-  // Full chunks: one thread starts five TMA tile copies and everybody goes on to the
+  // Full chunks: six warps start a TMA tile copy each and everybody goes on to the
   // gate computation while they land.  Ragged chunks (rows past the sequence end must
   // read as zero) take 16-byte cp.async copies.
-  const bool by_tma = p.use_tma && valid == kChunk;
   const bool out_tma = by_tma && p.out_tma;  // gradients of full chunks leave by TMA from padded tiles
-  const uint32_t bar = smem_u32(smem + oBar);
+  const uint32_t bar = smem_u32(smem + oBar), bar_b = bar + 8;
+  auto copy = [&](uint32_t b, const void* dst, const CUtensorMap* map, int bytes, int c0, int c1) {
+    tc::mbar_expect_tx(b, bytes);
+    tc::tma_load_2d(smem_u32(dst), map, b, c0, c1);
+  };
   if (by_tma) {
-    if (tid == 0) {
-      tc::mbar_init(bar, 1);
-      tc::fence_barrier_init();
-      tc::mbar_expect_tx(bar, kTmaBytes);
-      tc::tma_load_2d(smem_u32(sdO), &maps.d_o, bar, h * kD, tok0);
-      tc::tma_load_2d(smem_u32(sS0), &maps.h, bar, 0, (int)(chh * kD));
-      tc::tma_load_2d(smem_u32(sTm), &maps.Akk, bar, h * kChunk, tok0);
-      tc::tma_load_2d(smem_u32(sdE), &maps.dF, bar, h * kD, tok0);  // raw dF; scaled by beta below
-      tc::tma_load_2d(smem_u32(sdSC), &maps.dh, bar, 0, (int)(chh * kD));
-      tc::tma_load_2d(smem_u32(sEarly), &maps.E, bar, h * kD, tok0);
+    if (lane == 0) {
+      switch (warp) {
+        case 0: copy(bar, sdO, &maps.d_o, kTileBytes, h * kD, tok0); break;
+        case 1: copy(bar, sS0, &maps.h, 2 * kTileBytes, 0, (int)(chh * kD)); break;
+        case 2: copy(bar, sTm, &maps.Akk, kChunk * kLdC * 2, h * kChunk, tok0); break;
+        case 3: copy(bar, sdE, &maps.dF, kTileBytes, h * kD, tok0); break;  // raw dF; scaled by beta below
+        case 4: copy(bar, sdSC, &maps.dh, 2 * kTileBytes, 0, (int)(chh * kD)); break;
+        case 5: copy(bar, sEarly, &maps.E, kTileBytes, h * kD, tok0); break;
+        default: break;
+      }
     }
   } else {
     tile_load_async(sdO, kLdD, p.d_o + row0, gld, kChunk, kD, valid, kThreads);
@@ -431,13 +478,18 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
     tile_load_async(sdSC, kLdD, p.dh + chh * kD * kD, kD, kD, kD, kD, kThreads);
     tile_load_async(sEarly, kLdD, p.v_new + row0, gld, kChunk, kD, valid, kThreads);
     cp_async_commit();
+    if (tid < kChunk) sBeta[tid] = s_small;
+    else if (tid >= 2 * kD && tid < 3 * kD) sGcv[tid - 2 * kD] = s_small;
+    else if (tid >= kD && tid < 2 * kD) bias()[tid - kD] = s_small;
   }
-  if (tid < kChunk) sBeta[tid] = s_small;
-  else if (tid >= 2 * kD && tid < 3 * kD) sGcv[tid - 2 * kD] = s_small;
-  else if (tid >= kD && tid < 2 * kD) sBias[tid - kD] = s_small;
+  if (by_tma) {
+    cp_async_wait<0>();
+    if (!tc::mbar_wait(bar_b + 8, *s_phase) && tid == 0) atomicExch(p.status, 1);
+    gate_load(graw, reinterpret_cast<const bf16*>(smem + oRaw), kLdD, kChunk, tid);
+  }
   __syncthreads();
   // log2-domain cumulative log-decay, exactly as the forward computes it
-  gate_apply(graw, sG, valid, sBias, __expf(p.A_log[h]) * kLog2e, tid);
+  gate_apply(graw, sG, valid, bias(), __expf(p.A_log[h]) * kLog2e, tid);
   __syncthreads();
   if (tid < kD) {
     gate_cumsum(sG, tid);
@@ -458,7 +510,7 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
     }
   }
   if (by_tma) {
-    if (!tc::mbar_wait(bar, 0) && tid == 0) atomicExch(p.status, 1);  // gave up: flag it, results are void
+    if (!tc::mbar_wait(bar, *s_phase) && tid == 0) atomicExch(p.status, 1);  // gave up: flag it, results are void
   } else {
     cp_async_wait<0>();
   }
@@ -535,7 +587,7 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
     }
   if (out_tma) tc::fence_proxy_async();
   __syncthreads();
-  if (out_tma && tid == 0) {  // dv is the dR tile as it stands
+  if (out_tma && tid == kThreads - 32) {  // dv is the dR tile as it stands
     tc::tma_store_3d(&maps.dv, smem_u32(sdR), 0, h, tok0);
     tc::bulk_commit();
   }
@@ -598,14 +650,23 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
         *reinterpret_cast<uint32_t*>(sdP + i * kLdC + j) = pack_bf16(j < i ? p0 : 0.f, j + 1 < i ? p1 : 0.f);
       }
   }
-  if (out_tma && tid == 0) tc::bulk_wait_read();  // the dv store has read the dR tile
+  if (out_tma && tid == kThreads - 32) tc::bulk_wait_read();  // the dv store has read the dR tile
+  tc::fence_proxy_async();
   __syncthreads();  // dO, dR, E no longer needed
   // dkg = F dS1^T  ->  dkt_a = exp(G_last - G) * dkg
   // q, k and kt tiles of the pair-product phase land while the dkg product runs
-  tile_load_async(reinterpret_cast<bf16*>(smem + oA0), kLdD, p.q + row0, gld, kChunk, kD, valid, kThreads);
-  tile_load_async(reinterpret_cast<bf16*>(smem + oA1), kLdD, p.k + row0, gld, kChunk, kD, valid, kThreads);
-  tile_load_async(reinterpret_cast<bf16*>(smem + oA1 + kTileBytes), kLdD, p.kt + row0, gld, kChunk, kD, valid, kThreads);
-  cp_async_commit();
+  if (by_tma) {
+    if (lane == 0) {
+      if (warp == 0) copy(bar_b, smem + oA0, &maps.q, kTileBytes, h * kD, tok0);
+      if (warp == 1) copy(bar_b, smem + oA1, &maps.k, kTileBytes, h * kD, tok0);
+      if (warp == 2) copy(bar_b, smem + oA1 + kTileBytes, &maps.kt, kTileBytes, h * kD, tok0);
+    }
+  } else {
+    tile_load_async(reinterpret_cast<bf16*>(smem + oA0), kLdD, p.q + row0, gld, kChunk, kD, valid, kThreads);
+    tile_load_async(reinterpret_cast<bf16*>(smem + oA1), kLdD, p.k + row0, gld, kChunk, kD, valid, kThreads);
+    tile_load_async(reinterpret_cast<bf16*>(smem + oA1 + kTileBytes), kLdD, p.kt + row0, gld, kChunk, kD, valid, kThreads);
+    cp_async_commit();
+  }
   zero_acc(t);
   warp_gemm<1, 4, false, false>(t, sF, kLdD, 16 * I, sdSC, kLdD, 32 * cq, 0, kD);
 #pragma unroll
@@ -627,8 +688,12 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   bf16* sKt = reinterpret_cast<bf16*>(smem + oA1 + kTileBytes);
   bf16* sXq = reinterpret_cast<bf16*>(smem + oStage);
   bf16* sXk = sXq + kChunk * kLdD;
-  cp_async_wait<0>();
-  __syncthreads();
+  if (by_tma) {
+    if (!tc::mbar_wait(bar_b, *s_phase) && tid == 0) atomicExch(p.status, 1);
+  } else {
+    cp_async_wait<0>();
+    __syncthreads();
+  }
   {
     // dG starts from the state-coupled parts; column sums of kt * dkt_a feed the
     // chunk's last row (d/dG_last of exp(G_last - G_j)).
@@ -872,6 +937,8 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   };
   if (first_last || by_level) pairs(std::false_type{});
   else pairs(std::true_type{});
+  int next = 0;  // the drawer's: position in the list, then the item
+  if (drawer) next = atomicAdd(p.fast_count + 2, 1);
   AtkIn atk;  // what the preconditioner's part below needs
   atk_request(atk, p, chh, tok0, valid, h, warp, lane);
   // ungated diagonal of P
@@ -915,6 +982,8 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   for (int i = 0; i < kAtkRows; ++i)
     atk.k[i] = *reinterpret_cast<const uint2*>(sK + (kAtkRows * warp + i) * kLdD + 4 * lane);
   __syncthreads();
+  if (drawer) next = next < p.fast_count[1] ? p.slow_list[next] : -1;
+  if (by_tma && tid == 0) *s_phase ^= 1;
   // every warp is past its reads of q, k and kt: their tiles take dq and dk_read
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt)
@@ -946,7 +1015,7 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   }
   atk_block_end(atk, warp, lane, reinterpret_cast<float*>(smem + oAtkEx));
   __syncthreads();
-  if (out_tma && tid == 0) {
+  if (out_tma && tid == kThreads - 32) {
     tc::tma_store_3d(&maps.dq, smem_u32(sQ), 0, h, tok0);
     tc::bulk_commit();
   }
@@ -962,16 +1031,19 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   }
   atk_local(atk, p, row0, gld, valid, warp, lane, sOutKt, sOutK,
             reinterpret_cast<float*>(smem + oAtkEx), out_tma);
+  if (drawer) *s_next = describe_item(p.geo, next);
   tc::fence_proxy_async();
   __syncthreads();
-  if (out_tma && tid == 0) {
-    tc::tma_store_3d(&maps.dkt, smem_u32(sOutKt), 0, h, tok0);
-    tc::tma_store_3d(&maps.dk_read, smem_u32(sOutK), 0, h, tok0);
+  if (p.slow_list) intra_bwd_ahead(p, maps, *s_next, *s_phase);
+  if (out_tma && (tid == kThreads - 32 || tid == kThreads - 64)) {
+    if (tid == kThreads - 32) tc::tma_store_3d(&maps.dkt, smem_u32(sOutKt), 0, h, tok0);
+    else tc::tma_store_3d(&maps.dk_read, smem_u32(sOutK), 0, h, tok0);
     tc::bulk_commit();
   }
   // ... then the gate's own backward, elementwise over the tile with all threads:
   //   g = -exp(A_log) softplus(raw + bias);  draw = dg * (-exp(A_log)) sigmoid(raw + bias)
   // Per-thread partial sums (dA_log: scalar; ddt_bias: per channel) are reduced in a fixed order.
+  const float* sBias = sRed + 16 + (*s_phase ^ 1) * kD;
   float* sPart = sY;  // [32][kLdG] per-(row group, channel) partials of ddt_bias (y is dead)
   {
     const float ea = __expf(p.A_log[h]);
@@ -1028,9 +1100,8 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
 #pragma unroll
     for (int w = 0; w < kThreads / 32; ++w) acc += sRed[w];
     p.partA[chh] = acc;
-    if (out_tma) tc::bulk_wait_read();  // the tiles stay in place until the stores have read them
-    if (by_tma) tc::mbar_inval(bar);    // a CTA that walks a work list sets the barrier up anew per item
   }
+  if (out_tma && (tid == kThreads - 32 || tid == kThreads - 64)) tc::bulk_wait_read();  // the tiles stay in place until the stores have read them
 }
 
 // grid (chunks, heads): one item per CTA; or, with a work list, a few persistent CTAs that walk it.
@@ -1038,27 +1109,34 @@ __global__ void __launch_bounds__(ib::kThreads, 1)
 pkda_intra_bwd_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdMaps maps) {
   if (!p.slow_list) wait_prerequisites();  // (with a work list it runs beside the tensor-memory kernel)
   launch_dependents();
-  if (!p.slow_list) {
-    intra_bwd_item(p, maps, blockIdx.x, blockIdx.y);
-    return;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ int4 s_next;  // the item: chunk, head, first token, valid tokens
+  // with a work list items differ in cost (how many strip pairs are left, and how they are taken, follows the decay): CTAs draw them one
+  // at a time
+  if (threadIdx.x == 0) {
+    tc::mbar_init(smem_u32(smem + ib::oBar), ib::kCopiesA);
+    tc::mbar_init(smem_u32(smem + ib::oBar) + 8, ib::kCopiesB);
+    tc::mbar_init(smem_u32(smem + ib::oBar) + 16, ib::kCopiesAhead);
+    *reinterpret_cast<uint32_t*>(smem + ib::oBar + 24) = 0;
+    tc::fence_barrier_init();
+    int item = blockIdx.x * p.geo.heads + blockIdx.y;
+    if (p.slow_list) {
+      const int at = atomicAdd(p.fast_count + 2, 1);
+      item = at < p.fast_count[1] ? p.slow_list[at] : -1;
+    }
+    s_next = describe_item(p.geo, item);
   }
-  // items differ in cost (how many strip pairs are left, and how they are taken, follows the decay): CTAs draw them one at a time
-  __shared__ int s_item;
-  const int n_items = p.fast_count[1], H = p.geo.heads;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(p.fast_count + 2, 1);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= n_items) break;
-    const int chh = p.slow_list[item];
-    intra_bwd_item(p, maps, chh / H, chh % H);
+  __syncthreads();
+  intra_bwd_ahead(p, maps, s_next, 0);
+  while (s_next.x >= 0) {
+    intra_bwd_item(p, maps, &s_next);
+    if (!p.slow_list) break;
     tc::fence_proxy_async();  // the sums of ddt_bias lie where the next item's copies land
-    __syncthreads();  // the next item reuses every shared-memory region (and s_item)
+    __syncthreads();  // the next item reuses every shared-memory region
   }
   wait_prerequisites();
 }
 
-// ------------------------------------------------------------------ preconditioner backward
 struct AtkBwdParams {
   Geo geo;
   const bf16* k;
@@ -1520,6 +1598,10 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
     ip.use_tma = tok >= kChunk && encode_bf16_map(&maps.d_o, ip.d_o, 2, act_dims, act_str, act_box, false) &&
                  encode_bf16_map(&maps.dF, ip.dF, 2, act_dims, act_str, act_box, false) &&
                  encode_bf16_map(&maps.E, ip.v_new, 2, act_dims, act_str, act_box, false) &&
+                 encode_bf16_map(&maps.q, ip.q, 2, act_dims, act_str, act_box, false) &&
+                 encode_bf16_map(&maps.k, ip.k, 2, act_dims, act_str, act_box, false) &&
+                 encode_bf16_map(&maps.kt, ip.kt, 2, act_dims, act_str, act_box, false) &&
+                 encode_bf16_map(&maps.g, ip.g, 2, act_dims, act_str, act_box, false) &&
                  encode_bf16_map(&maps.h, ip.h, 2, st_dims, st_str, st_box, false) &&
                  encode_bf16_map(&maps.dh, ip.dh, 2, st_dims, st_str, st_box, false) &&
                  encode_bf16_map(&maps.Akk, ip.Akk, 2, pr_dims, pr_str, pr_box, false);
