@@ -21,15 +21,34 @@
 namespace pkda {
 
 // ------------------------------------------------------------------ small kernels
-__global__ void pkda_chunk_offsets_kernel(const int* cu, int n_seqs, int* offs) {
+// First chunk of every packed sequence: a prefix sum over the sequences' chunk counts, 1,024 of them a turn.  (One thread that walks
+// them waits for memory on the way: 4,000 sequences 222 -> 10 us, 44 6 -> 3.)
+__global__ void __launch_bounds__(1024) pkda_chunk_offsets_kernel(const int* cu, int n_seqs, int* offs) {
   after_previous();
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    int acc = 0;
-    offs[0] = 0;
-    for (int n = 0; n < n_seqs; ++n) {
-      acc += (cu[n + 1] - cu[n] + kChunk - 1) / kChunk;
-      offs[n + 1] = acc;
+  __shared__ int s_sum[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int acc = 0;  // chunks of the turns before
+  if (tid == 0) offs[0] = 0;
+  for (int n0 = 0; n0 < n_seqs; n0 += 1024) {
+    const int n = n0 + tid;
+    int x = n < n_seqs ? (cu[n + 1] - cu[n] + kChunk - 1) / kChunk : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
+    if (lane == 31) s_sum[warp] = x;
+    __syncthreads();
+    int before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) {
+      const int y = s_sum[w];
+      before += w < warp ? y : 0;
+      all += y;
+    }
+    if (n < n_seqs) offs[n + 1] = acc + before + x;
+    acc += all;
+    __syncthreads();  // (the sums are rewritten by the next turn)
   }
 }
 
@@ -555,7 +574,7 @@ int run_prologue(const pkda_problem& p, int* chunk_offsets, float* beta_c, Geo* 
   // beta_c == nullptr: the caller fills the chunk-major beta itself (the forward does, in its first kernel)
   if (p.cu_seqlens) {
     begin_stage(kStageOffsets, st);
-    launch_kernel(pkda_chunk_offsets_kernel, 1, 32, 0, st, p.cu_seqlens, p.n_seqs, chunk_offsets);
+    launch_kernel(pkda_chunk_offsets_kernel, 1, 1024, 0, st, p.cu_seqlens, p.n_seqs, chunk_offsets);
     PKDA_CHECK_LAUNCH();
   }
   *geo = make_geo(p, chunk_offsets);
