@@ -357,11 +357,12 @@ __device__ __forceinline__ void atk_carry(const float* ex, const IntraBwdParams&
 }
 }  // namespace ib
 
-// Chunk, head, first token and valid tokens of an item (chunk * heads + head); chunk -1 for none.
+// Chunk, head, first token and valid tokens of an item (chunk * heads + head); chunk -1 for none.  Packed: all lanes of a warp
+// together.
 __device__ __forceinline__ int4 describe_item(const Geo& geo, int item) {
   int n, tok0, valid;
   const int chunk = item / geo.heads;
-  if (item < 0 || !chunk_lookup(geo, chunk, n, tok0, valid)) return make_int4(-1, 0, 0, 0);
+  if (item < 0 || !chunk_lookup_warp(geo, chunk, n, tok0, valid)) return make_int4(-1, 0, 0, 0);
   return make_int4(chunk, item - chunk * geo.heads, tok0, valid);
 }
 // What a full chunk needs first, asked for while the item before it ends: the raw gate, beta, Gam_last and the gate's bias.  All of it
@@ -1031,7 +1032,12 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
   }
   atk_local(atk, p, row0, gld, valid, warp, lane, sOutKt, sOutK,
             reinterpret_cast<float*>(smem + oAtkEx), out_tma);
-  if (drawer) *s_next = describe_item(p.geo, next);
+  if (p.slow_list && !p.geo.cu_seqlens) {
+    if (drawer) *s_next = describe_item(p.geo, next);
+  } else if (p.slow_list && warp == kThreads / 32 - 1) {  // packed: the drawer's warp looks the sequence up together
+    const int4 d = describe_item(p.geo, __shfl_sync(0xffffffffu, next, 0));
+    if (drawer) *s_next = d;
+  }
   tc::fence_proxy_async();
   __syncthreads();
   if (p.slow_list) intra_bwd_ahead(p, maps, *s_next, *s_phase);
@@ -1119,12 +1125,18 @@ pkda_intra_bwd_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdMa
     tc::mbar_init(smem_u32(smem + ib::oBar) + 16, ib::kCopiesAhead);
     *reinterpret_cast<uint32_t*>(smem + ib::oBar + 24) = 0;
     tc::fence_barrier_init();
+  }
+  if (threadIdx.x < 32) {
     int item = blockIdx.x * p.geo.heads + blockIdx.y;
     if (p.slow_list) {
-      const int at = atomicAdd(p.fast_count + 2, 1);
-      item = at < p.fast_count[1] ? p.slow_list[at] : -1;
+      if (threadIdx.x == 0) {
+        const int at = atomicAdd(p.fast_count + 2, 1);
+        item = at < p.fast_count[1] ? p.slow_list[at] : -1;
+      }
+      item = __shfl_sync(0xffffffffu, item, 0);
     }
-    s_next = describe_item(p.geo, item);
+    const int4 d = describe_item(p.geo, item);
+    if (threadIdx.x == 0) s_next = d;
   }
   __syncthreads();
   intra_bwd_ahead(p, maps, s_next, 0);
