@@ -15,7 +15,8 @@
 // digits that S - w e^T loses under strong decay).  The preconditioner's cotangent, a diagonal scan
 // backwards over the tokens, and the terms that depend on it close the pass.
 // (One CTA per (sequence, head) that replayed and walked back every token with the whole state took
-// 1655 us for 2 x 4 units of 512 tokens at D = 64, fp32, behind a 551 us forward; these take 110 us, behind 90.)
+// 1655 us for 2 x 4 units of 512 tokens at D = 64, fp32, behind a 551 us forward; these took 110 us, behind 90;
+// with what pkda_recurrent.cu says of the scans and the loads below asked for ahead, all of it takes 156.)
 #include <type_traits>
 
 #include "pkda_launch.h"
