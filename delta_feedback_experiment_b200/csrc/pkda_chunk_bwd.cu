@@ -1495,12 +1495,6 @@ size_t chunk_bwd_status_offset(const pkda_problem& p) {
   return (size_t)(reinterpret_cast<unsigned char*>(carve_bwd(p, nullptr).status) - static_cast<unsigned char*>(nullptr));
 }
 
-#define PKDA_CHECK_LAUNCH()                                        \
-  do {                                                             \
-    end_stage(st);                                                 \
-    if (cudaGetLastError() != cudaSuccess) return PKDA_ERR_LAUNCH; \
-  } while (0)
-
 template <typename K>
 static bool set_smem(K kernel, int bytes) {
   return ensure_dynamic_smem(kernel, bytes);
@@ -1509,8 +1503,7 @@ static bool set_smem(K kernel, int bytes) {
 template <int VB>
 static int launch_scan_bwd(const ScanBwdParams& sp, int units, cudaStream_t st) {
   if (!set_smem(pkda_scan_bwd_kernel<VB>, scanb::L<VB>::kSmem)) return PKDA_ERR_LAUNCH;
-  launch_kernel(pkda_scan_bwd_kernel<VB>, units * (kD / VB), scanb::threads<VB>(), scanb::L<VB>::kSmem, st, sp);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return launch_kernel(pkda_scan_bwd_kernel<VB>, units * (kD / VB), scanb::threads<VB>(), scanb::L<VB>::kSmem, st, sp);
 }
 
 int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
@@ -1640,8 +1633,9 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   }
   if (!set_smem(pkda_intra_bwd_kernel, ib::kSmem)) return PKDA_ERR_LAUNCH;
   begin_stage(ip.slow_list ? kStageIntraBwdRest : kStageIntraBwd, st);
-  launch_kernel(pkda_intra_bwd_kernel, gridc, ib::kThreads, ib::kSmem, st, ip, maps);
-  PKDA_CHECK_LAUNCH();
+  rc = launch_kernel(pkda_intra_bwd_kernel, gridc, ib::kThreads, ib::kSmem, st, ip, maps);
+  end_stage(st);
+  if (rc != PKDA_OK) return rc;
 
   AtkBwdParams ap;
   ap.geo = geo; ap.k = static_cast<const bf16*>(p.k); ap.g_atk = p.g_atk;
@@ -1651,19 +1645,22 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   const int atk_tiles = geo.total_chunks * p.heads;
   const int atk_grid = atk_tiles < 2 * sms ? atk_tiles : 2 * sms;  // persistent: two CTAs per SM
   begin_stage(kStageAtkBwdCarry, st);
-  launch_kernel(false, pkda_atk_bwd_carry_kernel, dim3(p.n_seqs, p.heads), kD, 0, st, geo, ws.c_loc, a->sa_atk, ws.lam_in,
+  rc = launch_kernel(false, pkda_atk_bwd_carry_kernel, dim3(p.n_seqs, p.heads), kD, 0, st, geo, ws.c_loc, a->sa_atk, ws.lam_in,
                 a->d_initial_A_state);
-  PKDA_CHECK_LAUNCH();
+  end_stage(st);
+  if (rc != PKDA_OK) return rc;
   begin_stage(kStageAtkBwdFinal, st);
   if (!set_smem(pkda_atk_bwd_kernel, atkb::kSmem)) return PKDA_ERR_LAUNCH;
-  launch_kernel(pkda_atk_bwd_kernel, atk_grid, atkb::kThreads, atkb::kSmem, st, ap, atk_tiles);
-  PKDA_CHECK_LAUNCH();
+  rc = launch_kernel(pkda_atk_bwd_kernel, atk_grid, atkb::kThreads, atkb::kSmem, st, ap, atk_tiles);
+  end_stage(st);
+  if (rc != PKDA_OK) return rc;
   begin_stage(kStageParamReduce, st);
   const size_t guard_n = std::min<size_t>((size_t)p.total_tokens * p.heads * kD, 4096);
-  launch_kernel(pkda_param_reduce_kernel, p.heads, kD * kReduceSubs, 0, st, geo, ws.partA, ws.partB, ws.partC, a->dA_log,
+  rc = launch_kernel(pkda_param_reduce_kernel, p.heads, kD * kReduceSubs, 0, st, geo, ws.partA, ws.partB, ws.partC, a->dA_log,
                 a->ddt_bias, a->dlog_atk_scale, ws.status, static_cast<bf16*>(a->dq), static_cast<bf16*>(a->dk),
                 static_cast<bf16*>(a->dv), guard_n);
-  PKDA_CHECK_LAUNCH();
+  end_stage(st);
+  if (rc != PKDA_OK) return rc;
   return PKDA_OK;
 }
 

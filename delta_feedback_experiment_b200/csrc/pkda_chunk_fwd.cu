@@ -467,12 +467,6 @@ static bool set_smem(K kernel, int bytes) {
   return ensure_dynamic_smem(kernel, bytes);
 }
 
-#define PKDA_CHECK_LAUNCH()                                        \
-  do {                                                             \
-    end_stage(st);                                                 \
-    if (cudaGetLastError() != cudaSuccess) return PKDA_ERR_LAUNCH; \
-  } while (0)
-
 int check_chunk_problem(const pkda_problem& p) {
   int rc = check_problem(p);
   if (rc != PKDA_OK) return rc;
@@ -502,8 +496,7 @@ ScanPair scan_pair(int units) {
 template <int VB, bool kRecompute>
 static int launch_scan_fwd(const ScanParams& sp, int units, cudaStream_t st) {
   if (!set_smem(pkda_scan_fwd_kernel<VB, kRecompute>, scan::L<VB>::kSmem)) return PKDA_ERR_LAUNCH;
-  launch_kernel(pkda_scan_fwd_kernel<VB, kRecompute>, units * (kD / VB), scan::threads<VB>(), scan::L<VB>::kSmem, st, sp);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return launch_kernel(pkda_scan_fwd_kernel<VB, kRecompute>, units * (kD / VB), scan::threads<VB>(), scan::L<VB>::kSmem, st, sp);
 }
 
 // Shared by the forward and by the backward's recompute mode.
@@ -571,19 +564,21 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
 }
 
 int run_prologue(const pkda_problem& p, int* chunk_offsets, float* beta_c, Geo* geo, cudaStream_t st) {
+  int rc = PKDA_OK;
   // beta_c == nullptr: the caller fills the chunk-major beta itself (the forward does, in its first kernel)
   if (p.cu_seqlens) {
     begin_stage(kStageOffsets, st);
-    launch_kernel(pkda_chunk_offsets_kernel, 1, 1024, 0, st, p.cu_seqlens, p.n_seqs, chunk_offsets);
-    PKDA_CHECK_LAUNCH();
+    rc = launch_kernel(pkda_chunk_offsets_kernel, 1, 1024, 0, st, p.cu_seqlens, p.n_seqs, chunk_offsets);
+    end_stage(st);
+    if (rc != PKDA_OK) return rc;
   }
   *geo = make_geo(p, chunk_offsets);
   if (beta_c) {
     begin_stage(kStagePackBeta, st);
-    launch_kernel(pkda_pack_beta_kernel, geo->total_chunks, 256, 0, st, *geo, static_cast<const bf16*>(p.beta), beta_c);
-    PKDA_CHECK_LAUNCH();
+    rc = launch_kernel(pkda_pack_beta_kernel, geo->total_chunks, 256, 0, st, *geo, static_cast<const bf16*>(p.beta), beta_c);
+    end_stage(st);
   }
-  return PKDA_OK;
+  return rc;
 }
 
 int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
@@ -611,14 +606,16 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
   const bool chained = forward_chain_possible(p);
   if (!chained) {
     begin_stage(kStageAtkLocal, st);
-    launch_kernel(pkda_atk_local_kernel, geo.total_chunks * p.heads, 256, 0, st, geo, static_cast<const bf16*>(p.k), p.g_atk,
+    rc = launch_kernel(pkda_atk_local_kernel, geo.total_chunks * p.heads, 256, 0, st, geo, static_cast<const bf16*>(p.k), p.g_atk,
                   static_cast<const bf16*>(p.beta_atk), static_cast<const bf16*>(p.beta), a->ac_atk, a->sa_atk, ws.beta_c,
                   ws.status);
-    PKDA_CHECK_LAUNCH();
+    end_stage(st);
+    if (rc != PKDA_OK) return rc;
     begin_stage(kStageAtkCarry, st);
-    launch_kernel(pkda_atk_carry_kernel, dim3(p.n_seqs, p.heads), kD, 0, st, geo, a->ac_atk, a->sa_atk, p.initial_A_state, a->a_atk,
+    rc = launch_kernel(pkda_atk_carry_kernel, dim3(p.n_seqs, p.heads), kD, 0, st, geo, a->ac_atk, a->sa_atk, p.initial_A_state, a->a_atk,
                   a->final_A_state);
-    PKDA_CHECK_LAUNCH();
+    end_stage(st);
+    if (rc != PKDA_OK) return rc;
   }
 
   // (The local scan also zeroes the status word and the cursor when it runs.)
@@ -652,8 +649,9 @@ int chunk_fwd(const pkda_chunk_fwd_args* a, cudaStream_t st) {
   op.beta_c = ws.beta_c; op.o = static_cast<bf16*>(a->o);
   if (!set_smem(pkda_out_fwd_kernel, outk::kSmem)) return PKDA_ERR_LAUNCH;
   begin_stage(kStageOutFwd, st);
-  launch_kernel(pkda_out_fwd_kernel, dim3(geo.total_chunks, p.heads), outk::kThreads, outk::kSmem, st, op);
-  PKDA_CHECK_LAUNCH();
+  rc = launch_kernel(pkda_out_fwd_kernel, dim3(geo.total_chunks, p.heads), outk::kThreads, outk::kSmem, st, op);
+  end_stage(st);
+  if (rc != PKDA_OK) return rc;
   return launch_status_guard(ws.status, a->o, nullptr, nullptr, guard_n, st);
 }
 

@@ -198,10 +198,10 @@ int controls_fwd(const pkda_controls_args* a, cudaStream_t st) {
   const long long blocks = (n + kCtrlThreads - 1) / kCtrlThreads, most = 16LL * sm_count();
   const int grid = (int)(blocks < most ? blocks : most);
   begin_stage(kStageControlsFwd, st);
-  if (a->dtype == PKDA_BF16) launch_kernel(pkda_controls_fwd_kernel<bf16>, grid, kCtrlThreads, 0, st, p);
-  else launch_kernel(pkda_controls_fwd_kernel<float>, grid, kCtrlThreads, 0, st, p);
+  const int rc = a->dtype == PKDA_BF16 ? launch_kernel(pkda_controls_fwd_kernel<bf16>, grid, kCtrlThreads, 0, st, p)
+                                       : launch_kernel(pkda_controls_fwd_kernel<float>, grid, kCtrlThreads, 0, st, p);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 size_t controls_bwd_workspace(const pkda_controls_args& a) {
@@ -229,14 +229,15 @@ int controls_bwd(const pkda_controls_args* a, cudaStream_t st) {
                          reinterpret_cast<uintptr_t>(a->d_packed);
   p.pairs = !(a->heads & 1) && !(a->hidden & 1) && ptrs % (a->dtype == PKDA_BF16 ? 4 : 8) == 0;
   begin_stage(kStageControlsBwd, st);
-  if (a->dtype == PKDA_BF16) launch_kernel(pkda_controls_bwd_kernel<bf16>, grid, kCtrlThreads, smem, st, p);
-  else launch_kernel(pkda_controls_bwd_kernel<float>, grid, kCtrlThreads, smem, st, p);
+  int rc = a->dtype == PKDA_BF16 ? launch_kernel(pkda_controls_bwd_kernel<bf16>, grid, kCtrlThreads, smem, st, p)
+                                 : launch_kernel(pkda_controls_bwd_kernel<float>, grid, kCtrlThreads, smem, st, p);
   end_stage(st);
+  if (rc != PKDA_OK) return rc;
   begin_stage(kStageControlsBwd, st);
-  launch_kernel(pkda_controls_reduce_kernel, 2 * a->heads, 128, 0, st, p.part, a->dA_log_precond, a->ddt_bias_precond, a->heads,
+  rc = launch_kernel(pkda_controls_reduce_kernel, 2 * a->heads, 128, 0, st, p.part, a->dA_log_precond, a->ddt_bias_precond, a->heads,
                 grid);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 int pack_control_gradients(const pkda_pack_control_args* a, cudaStream_t st) {
@@ -253,18 +254,19 @@ int pack_control_gradients(const pkda_pack_control_args* a, cudaStream_t st) {
   const long long blocks = (n + kCtrlThreads - 1) / kCtrlThreads, most = 32LL * sm_count();
   const int grid = (int)(blocks < most ? blocks : most);
   begin_stage(kStagePackControl, st);
+  int rc;
   if (a->dtype == PKDA_BF16)
-    launch_kernel(pkda_pack_control_kernel<bf16>, grid, kCtrlThreads, 0, st, static_cast<const bf16*>(a->grads[0]),
+    rc = launch_kernel(pkda_pack_control_kernel<bf16>, grid, kCtrlThreads, 0, st, static_cast<const bf16*>(a->grads[0]),
                   static_cast<const bf16*>(a->grads[1]), static_cast<const bf16*>(a->grads[2]), static_cast<const
                   bf16*>(a->grads[3]), static_cast<const bf16*>(a->grads[4]), static_cast<bf16*>(a->out), a->rows, a->sizes[0],
                   a->sizes[1], a->sizes[2], a->sizes[3], a->sizes[4]);
   else
-    launch_kernel(pkda_pack_control_kernel<float>, grid, kCtrlThreads, 0, st, static_cast<const float*>(a->grads[0]),
+    rc = launch_kernel(pkda_pack_control_kernel<float>, grid, kCtrlThreads, 0, st, static_cast<const float*>(a->grads[0]),
                   static_cast<const float*>(a->grads[1]), static_cast<const float*>(a->grads[2]), static_cast<const
                   float*>(a->grads[3]), static_cast<const float*>(a->grads[4]), static_cast<float*>(a->out), a->rows, a->sizes[0],
                   a->sizes[1], a->sizes[2], a->sizes[3], a->sizes[4]);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 }  // namespace pkda

@@ -221,9 +221,9 @@ pkda_decode_step_kernel(const DecodeParams p) {
 template <int D, typename T>
 static int launch_decode(const DecodeParams& dp, int stage, cudaStream_t st) {
   begin_stage(stage, st);
-  launch_kernel(pkda_decode_step_kernel<D, T>, dp.batch * dp.heads, RecCfg<D>::kThreads, 0, st, dp);
+  const int rc = launch_kernel(pkda_decode_step_kernel<D, T>, dp.batch * dp.heads, RecCfg<D>::kThreads, 0, st, dp);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 template <typename T>

@@ -673,10 +673,10 @@ int launch_bwd_classify(const Geo& geo, const float* gc, int direct_cap, int2* f
                         const bf16* beta, float* beta_c, cudaStream_t st) {
   const int items = geo.total_chunks * geo.heads;
   begin_stage(kStageBwdClassify, st);
-  launch_kernel(pkda_bwd_classify_kernel, (items + 63) / 64, 256, 0, st, geo, gc, direct_cap, fast_list, slow_list, counts, beta,
+  const int rc = launch_kernel(pkda_bwd_classify_kernel, (items + 63) / 64, 256, 0, st, geo, gc, direct_cap, fast_list, slow_list, counts, beta,
                 beta_c);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 int launch_intra_bwd_tc(const IntraBwdParams& ip, cudaStream_t st) {
@@ -707,9 +707,9 @@ int launch_intra_bwd_tc(const IntraBwdParams& ip, cudaStream_t st) {
   const int items = ip.geo.total_chunks * ip.geo.heads;
   begin_stage(kStageIntraBwd, st);
   const int sms = sm_count();
-  launch_kernel(false, pkda_intra_bwd_tc_kernel, items < sms ? items : sms, ibtc::kThreads, ibtc::kSmem, st, ip, maps);
+  const int rc = launch_kernel(false, pkda_intra_bwd_tc_kernel, items < sms ? items : sms, ibtc::kThreads, ibtc::kSmem, st, ip, maps);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 }  // namespace pkda

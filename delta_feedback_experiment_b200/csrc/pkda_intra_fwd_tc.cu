@@ -921,10 +921,10 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 int launch_chain_init(float* a_chain, size_t items, int* zero, cudaStream_t st) {
   const size_t n = items * kD, most = 8 * (size_t)sm_count(), blocks = (n + 255) / 256;
   begin_stage(kStageChainInit, st);
-  launch_kernel(pkda_chain_init_kernel, (unsigned)(blocks < most ? blocks : most), 256, 0, st, reinterpret_cast<uint32_t*>(a_chain),
+  const int rc = launch_kernel(pkda_chain_init_kernel, (unsigned)(blocks < most ? blocks : most), 256, 0, st, reinterpret_cast<uint32_t*>(a_chain),
                 n, zero);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) {
@@ -952,15 +952,14 @@ int launch_intra_fwd_tc(const IntraParams& ip, bool recompute, cudaStream_t st) 
   if (recompute) {
     if (!ensure_dynamic_smem(pkda_intra_fwd_tc_kernel<true>, intratc::kSmem, 100))
       return PKDA_ERR_LAUNCH;
-    launch_kernel(false, pkda_intra_fwd_tc_kernel<true>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_p, tm_w, tm_u,
+    return launch_kernel(false, pkda_intra_fwd_tc_kernel<true>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_p, tm_w, tm_u,
                   tm_g, tm_k, tm_q, ip);
   } else {
     if (!ensure_dynamic_smem(pkda_intra_fwd_tc_kernel<false>, intratc::kSmem, 100))
       return PKDA_ERR_LAUNCH;
-    launch_kernel(false, pkda_intra_fwd_tc_kernel<false>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_p, tm_w, tm_u,
+    return launch_kernel(false, pkda_intra_fwd_tc_kernel<false>, grid, intratc::kThreads, intratc::kSmem, st, tm_v, tm_akk, tm_p, tm_w, tm_u,
                   tm_g, tm_k, tm_q, ip);
   }
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 
 }  // namespace pkda

@@ -47,14 +47,22 @@ inline bool ensure_dynamic_smem(K kernel, int bytes, int carveout = -1) {
 // SMs of the current device (148, the B200's, where there is none).
 int sm_count();
 
+inline int launch_code(cudaError_t err) {
+  const cudaError_t pending = cudaGetLastError();  // (holds err, and is cleared)
+  return err == cudaSuccess && pending == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+}
+
 // Launches `kernel` so that it is set up while the launch in front of it still runs.  Every kernel launched by this calls
 // wait_prerequisites() (pkda_common.cuh).
 // early = false: only behind the end of the launch in front.  The large kernels whose CTAs fill an SM's shared memory are better off
 // so (their CTAs would come to lie where room appears first): 1 x 8,191 tokens of 16 heads forward 313 -> 308 us, a lean step of
 // 2 x 4,096 tokens of 12 heads 785 -> 775.  Early: a decoding step of 8 units 6.1 -> 5.3 us, 4 x 48 tokens of 16 heads 26.6 -> 24.9,
 // the norm gate forward + backward at 8 x 4,096 tokens of 16 heads 197 -> 192.5.
+// The code has to be passed on: what a launch is refused for is asked for here and nowhere else, and an error that was pending
+// before is taken with it.
 template <typename... P, typename... A>
-inline int launch_kernel(bool early, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+[[nodiscard]] inline int launch_kernel(bool early, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st,
+                                       const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)threads);
@@ -65,11 +73,10 @@ inline int launch_kernel(bool early, void (*kernel)(P...), dim3 grid, int thread
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = early ? 1 : 0;
-  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, args...);
-  return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return launch_code(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 template <typename... P, typename... A>
-inline int launch_kernel(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+[[nodiscard]] inline int launch_kernel(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
   return launch_kernel(true, kernel, grid, threads, smem, st, args...);
 }
 

@@ -307,7 +307,8 @@ static bool ng_aligned(const void* x) { return (reinterpret_cast<uintptr_t>(x) &
 
 int norm_gate_fwd(const pkda_norm_gate_args* a, cudaStream_t st) {
   NormGateParams p;
-  if (int rc = ng_check(*a, p)) return rc;
+  int rc = ng_check(*a, p);
+  if (rc != PKDA_OK) return rc;
   if (a->rows == 0) return PKDA_OK;
   if (!a->x || !a->gate || !a->weight || !a->y || !a->rstd) return PKDA_ERR_NULL;
   if (!ng_aligned(a->x) || !ng_aligned(a->gate) || !ng_aligned(a->y)) return PKDA_ERR_ALIGN;
@@ -316,16 +317,16 @@ int norm_gate_fwd(const pkda_norm_gate_args* a, cudaStream_t st) {
     if (!ng_allow_smem(pkda_norm_gate_fwd_kernel<bf16>, smem)) return PKDA_ERR_LAUNCH;
     const int grid = ng_grid(*a, pkda_norm_gate_fwd_kernel<bf16>, smem);
     begin_stage(kStageNormGateFwd, st);
-    launch_kernel(pkda_norm_gate_fwd_kernel<bf16>, grid, ng::kThreads, smem, st, p);
+    rc = launch_kernel(pkda_norm_gate_fwd_kernel<bf16>, grid, ng::kThreads, smem, st, p);
   } else {
     constexpr int smem = ng::fwd_smem<float>();
     if (!ng_allow_smem(pkda_norm_gate_fwd_kernel<float>, smem)) return PKDA_ERR_LAUNCH;
     const int grid = ng_grid(*a, pkda_norm_gate_fwd_kernel<float>, smem);
     begin_stage(kStageNormGateFwd, st);
-    launch_kernel(pkda_norm_gate_fwd_kernel<float>, grid, ng::kThreads, smem, st, p);
+    rc = launch_kernel(pkda_norm_gate_fwd_kernel<float>, grid, ng::kThreads, smem, st, p);
   }
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 size_t norm_gate_bwd_workspace(const pkda_norm_gate_args& a) {
@@ -336,7 +337,8 @@ size_t norm_gate_bwd_workspace(const pkda_norm_gate_args& a) {
 
 int norm_gate_bwd(const pkda_norm_gate_args* a, cudaStream_t st) {
   NormGateParams p;
-  if (int rc = ng_check(*a, p)) return rc;
+  int rc = ng_check(*a, p);
+  if (rc != PKDA_OK) return rc;
   if (!a->dweight) return PKDA_ERR_NULL;
   if (a->rows == 0)
     return cudaMemsetAsync(a->dweight, 0, (size_t)a->dim * sizeof(float), st) == cudaSuccess ? PKDA_OK
@@ -352,19 +354,20 @@ int norm_gate_bwd(const pkda_norm_gate_args* a, cudaStream_t st) {
     if (!ng_allow_smem(pkda_norm_gate_bwd_kernel<bf16>, smem)) return PKDA_ERR_LAUNCH;
     grid = ng_grid(*a, pkda_norm_gate_bwd_kernel<bf16>, smem);
     begin_stage(kStageNormGateBwd, st);
-    launch_kernel(pkda_norm_gate_bwd_kernel<bf16>, grid, ng::kThreads, smem, st, p);
+    rc = launch_kernel(pkda_norm_gate_bwd_kernel<bf16>, grid, ng::kThreads, smem, st, p);
   } else {
     constexpr int smem = ng::bwd_smem<float>();
     if (!ng_allow_smem(pkda_norm_gate_bwd_kernel<float>, smem)) return PKDA_ERR_LAUNCH;
     grid = ng_grid(*a, pkda_norm_gate_bwd_kernel<float>, smem);
     begin_stage(kStageNormGateBwd, st);
-    launch_kernel(pkda_norm_gate_bwd_kernel<float>, grid, ng::kThreads, smem, st, p);
+    rc = launch_kernel(pkda_norm_gate_bwd_kernel<float>, grid, ng::kThreads, smem, st, p);
   }
   end_stage(st);
+  if (rc != PKDA_OK) return rc;
   begin_stage(kStageNormGateDw, st);
-  launch_kernel(pkda_norm_gate_dw_kernel, a->dim / 8, 1024, 0, st, p.part, a->dweight, a->dim, grid);
+  rc = launch_kernel(pkda_norm_gate_dw_kernel, a->dim / 8, 1024, 0, st, p.part, a->dweight, a->dim, grid);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 }  // namespace pkda

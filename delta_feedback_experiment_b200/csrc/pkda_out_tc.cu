@@ -223,10 +223,10 @@ int launch_out_fwd_tc(const Geo& geo, int total_tokens, const bf16* qg, const bf
   if (!ensure_dynamic_smem(pkda_out_fwd_tc_kernel, outtc::kSmem))
     return PKDA_ERR_LAUNCH;
   begin_stage(kStageOutFwd, st);
-  launch_kernel(pkda_out_fwd_tc_kernel, dim3(geo.total_chunks, geo.heads), outtc::kThreads, outtc::kSmem, st, tm_h, tm_qg, tm_e,
+  const int rc = launch_kernel(pkda_out_fwd_tc_kernel, dim3(geo.total_chunks, geo.heads), outtc::kThreads, outtc::kSmem, st, tm_h, tm_qg, tm_e,
                 tm_p, tm_o, op);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 }  // namespace pkda

@@ -591,18 +591,18 @@ template <typename T, int kHeadLanes>
 static int launch_conv_fwd(const ConvParams& p, dim3 grid, cudaStream_t st) {
   if (!ensure_dynamic_smem(pkda_qkv_conv_fwd_kernel<T, kHeadLanes>, conv::fwd_smem<T>())) return PKDA_ERR_LAUNCH;
   begin_stage(kStageConvFwd, st);
-  launch_kernel(pkda_qkv_conv_fwd_kernel<T, kHeadLanes>, grid, conv::kThreads, conv::fwd_smem<T>(), st, p);
+  const int rc = launch_kernel(pkda_qkv_conv_fwd_kernel<T, kHeadLanes>, grid, conv::kThreads, conv::fwd_smem<T>(), st, p);
   end_stage(st);
-  return PKDA_OK;
+  return rc;
 }
 
 template <typename T, int kHeadLanes>
 static int launch_conv_bwd(const ConvParams& p, dim3 grid, cudaStream_t st) {
   if (!ensure_dynamic_smem(pkda_qkv_conv_bwd_kernel<T, kHeadLanes>, conv::bwd_smem<T>())) return PKDA_ERR_LAUNCH;
   begin_stage(kStageConvBwd, st);
-  launch_kernel(pkda_qkv_conv_bwd_kernel<T, kHeadLanes>, grid, conv::kThreads, conv::bwd_smem<T>(), st, p);
+  const int rc = launch_kernel(pkda_qkv_conv_bwd_kernel<T, kHeadLanes>, grid, conv::kThreads, conv::bwd_smem<T>(), st, p);
   end_stage(st);
-  return PKDA_OK;
+  return rc;
 }
 
 // Picks the instantiation for the activation type and the lanes per head.
@@ -624,8 +624,7 @@ int qkv_conv_fwd(const pkda_qkv_conv_args* a, cudaStream_t st) {
   const dim3 grid = conv_grid(p);
   int rc = PKDA_OK;
   if (a->dtype == PKDA_BF16) { PKDA_CONV_DISPATCH(launch_conv_fwd, bf16) } else { PKDA_CONV_DISPATCH(launch_conv_fwd, float) }
-  if (rc != PKDA_OK) return rc;
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 size_t qkv_conv_bwd_workspace(const pkda_qkv_conv_args& a) {
@@ -653,9 +652,9 @@ int qkv_conv_bwd(const pkda_qkv_conv_args* a, cudaStream_t st) {
   if (a->dtype == PKDA_BF16) { PKDA_CONV_DISPATCH(launch_conv_bwd, bf16) } else { PKDA_CONV_DISPATCH(launch_conv_bwd, float) }
   if (rc != PKDA_OK) return rc;
   begin_stage(kStageConvDw, st);
-  launch_kernel(pkda_qkv_conv_dw_kernel, (n + 31) / 32, 256, 0, st, p.part, a->dweight, n, (int)grid.y);
+  rc = launch_kernel(pkda_qkv_conv_dw_kernel, (n + 31) / 32, 256, 0, st, p.part, a->dweight, n, (int)grid.y);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 }  // namespace pkda

@@ -472,9 +472,9 @@ static int launch_rec(RecParams rp, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = rp.inplace_A ? 2 : 1;
   begin_stage(kStageRecurrent, st);
-  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, rp);
+  const int rc = launch_code(cudaLaunchKernelEx(&cfg, kernel, rp));
   end_stage(st);
-  return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 template <int D, typename T>
@@ -485,9 +485,9 @@ static int launch_rec_d(const RecParams& rp, bool save, cudaStream_t st) {
   if (rp.geo.seq_len > 0 && rp.geo.seq_len < few && units > sm_count()) {
     if (!aligned({rp.ST}, 16)) return PKDA_ERR_ALIGN;  // (here, with four columns per lane and in the single step: states by float4)
     begin_stage(kStageRecurrent, st);
-    launch_kernel(pkda_recurrent_few_kernel<D, T>, (unsigned)units, RecCfg<D>::kThreads, 0, st, rp);
+    const int rc = launch_kernel(pkda_recurrent_few_kernel<D, T>, (unsigned)units, RecCfg<D>::kThreads, 0, st, rp);
     end_stage(st);
-    return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+    return rc;
   }
   // Four columns per lane once the one-column warps number more than two per scheduler (4 per SM).
   constexpr bool kFour = D >= 64;

@@ -667,19 +667,22 @@ static int launch_rec_bwd(RecBwdParams bp, size_t blocks, cudaStream_t st) {
       !ensure_dynamic_smem(pkda_recurrent_grad_kernel<D, T>, G::kFloats * 4))
     return PKDA_ERR_LAUNCH;
   begin_stage(kStageRecurrent, st);
-  launch_kernel(pkda_recurrent_dscan_kernel<D, T>, units * bp.groups, bp.warps.threads(L::kProd), L::kSmem, st, bp);
+  int rc = launch_kernel(pkda_recurrent_dscan_kernel<D, T>, units * bp.groups, bp.warps.threads(L::kProd), L::kSmem, st, bp);
   end_stage(st);
+  if (rc != PKDA_OK) return rc;
   const dim3 grid((unsigned)blocks, (unsigned)H);
   begin_stage(kStageRecurrent, st);
-  launch_kernel(pkda_recurrent_grad_kernel<D, T>, grid, G::kThreads, G::kFloats * 4, st, bp);
+  rc = launch_kernel(pkda_recurrent_grad_kernel<D, T>, grid, G::kThreads, G::kFloats * 4, st, bp);
   end_stage(st);
+  if (rc != PKDA_OK) return rc;
   begin_stage(kStageRecurrent, st);
-  launch_kernel(pkda_recurrent_carry_kernel<D>, units, D < 32 ? 32 : D, 0, st, bp);
+  rc = launch_kernel(pkda_recurrent_carry_kernel<D>, units, D < 32 ? 32 : D, 0, st, bp);
   end_stage(st);
+  if (rc != PKDA_OK) return rc;
   begin_stage(kStageRecurrent, st);
-  launch_kernel(pkda_recurrent_close_kernel<D, T>, grid, 256, 0, st, bp);
+  rc = launch_kernel(pkda_recurrent_close_kernel<D, T>, grid, 256, 0, st, bp);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 template <typename T>
@@ -730,10 +733,10 @@ int recurrent_bwd(const pkda_recurrent_bwd_args* a, const void* saved, size_t sa
                             : dispatch_rec_bwd<float>(p.head_dim, bp, blocks, st);
   if (rc != PKDA_OK) return rc;
   begin_stage(kStageParamReduce, st);
-  launch_kernel(pkda_recurrent_bwd_reduce_kernel, p.heads, 256, 0, st, (int)blocks, p.heads, p.head_dim, ws.partA, ws.partB,
-                ws.partC, a->dA_log, a->ddt_bias, a->dlog_atk_scale);
+  rc = launch_kernel(pkda_recurrent_bwd_reduce_kernel, p.heads, 256, 0, st, (int)blocks, p.heads, p.head_dim, ws.partA, ws.partB,
+                     ws.partC, a->dA_log, a->ddt_bias, a->dlog_atk_scale);
   end_stage(st);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
+  return rc;
 }
 
 }  // namespace pkda

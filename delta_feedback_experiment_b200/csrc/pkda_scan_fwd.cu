@@ -266,9 +266,8 @@ template <int NW, bool kOut>
 static int launch(const CUtensorMap (&tm)[5], const ScanFwdParams& sp, int units, cudaStream_t st) {
   using Y = ScanFwdLay<NW, kOut>;
   if (!ensure_dynamic_smem(pkda_scan_fwd_cols_kernel<NW, kOut>, Y::kSmem)) return PKDA_ERR_LAUNCH;
-  launch_kernel(false, pkda_scan_fwd_cols_kernel<NW, kOut>, units * Y::kSplit, Y::kThreads, Y::kSmem, st, tm[0], tm[1], tm[2], tm[3],
+  return launch_kernel(false, pkda_scan_fwd_cols_kernel<NW, kOut>, units * Y::kSplit, Y::kThreads, Y::kSmem, st, tm[0], tm[1], tm[2], tm[3],
                 tm[4], sp);
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 
 // o == NULL: h, v_new and the final state only.  split: CTAs per unit, 8, 4 or (without o) 2.

@@ -504,20 +504,19 @@ int launch_scan_fwd_tc(const Geo& geo, int total_tokens, int units, const bf16* 
   if (recompute) {
     if (!ensure_dynamic_smem(pkda_scan_fwd_tc_kernel<true, false>, scantc::kSmem))
       return PKDA_ERR_LAUNCH;
-    launch_kernel(false, pkda_scan_fwd_tc_kernel<true, false>, units, scantc::kThreads, scantc::kSmem, st, tm_w, tm_kg, tm_u, tm_h, tm_e,
+    return launch_kernel(false, pkda_scan_fwd_tc_kernel<true, false>, units, scantc::kThreads, scantc::kSmem, st, tm_w, tm_kg, tm_u, tm_h, tm_e,
                   tm_qg, tm_p, sp);
   } else if (with_out) {
     if (!ensure_dynamic_smem(pkda_scan_fwd_tc_kernel<false, true>, scantc::kSmemOut))
       return PKDA_ERR_LAUNCH;
-    launch_kernel(false, pkda_scan_fwd_tc_kernel<false, true>, units, scantc::kThreads + scantc::kOutThreads, scantc::kSmemOut, st, tm_w,
+    return launch_kernel(false, pkda_scan_fwd_tc_kernel<false, true>, units, scantc::kThreads + scantc::kOutThreads, scantc::kSmemOut, st, tm_w,
                   tm_kg, tm_u, tm_h, tm_e, tm_qg, tm_p, sp);
   } else {
     if (!ensure_dynamic_smem(pkda_scan_fwd_tc_kernel<false, false>, scantc::kSmem))
       return PKDA_ERR_LAUNCH;
-    launch_kernel(false, pkda_scan_fwd_tc_kernel<false, false>, units, scantc::kThreads, scantc::kSmem, st, tm_w, tm_kg, tm_u, tm_h, tm_e,
+    return launch_kernel(false, pkda_scan_fwd_tc_kernel<false, false>, units, scantc::kThreads, scantc::kSmem, st, tm_w, tm_kg, tm_u, tm_h, tm_e,
                   tm_qg, tm_p, sp);
   }
-  return cudaGetLastError() == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 
 }  // namespace pkda
