@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(256) pkda_recurrent_close_kernel(const RecBwdP
 __global__ void __launch_bounds__(256)
 pkda_recurrent_bwd_reduce_kernel(int blocks, int H, int D, const float* partA, const float* partB, const float* partC,
                                  float* dA_log, float* ddt_bias, float* dcentre) {
-  launch_dependents();  // (it needs nothing of the pass in front of it and runs beside it)
+  launch_dependents();  // (it needs nothing of the pass in front of it and runs beside it; what it reads, see launch_rec_bwd)
   __shared__ float s[3][256];
   const int h = blockIdx.x, tid = threadIdx.x, c = tid % D, sl = tid / D, ns = 256 / D;
   float b = 0.f, a = 0.f, cc = 0.f;
@@ -676,7 +676,9 @@ static int launch_rec_bwd(RecBwdParams bp, size_t blocks, cudaStream_t st) {
   end_stage(st);
   if (rc != PKDA_OK) return rc;
   begin_stage(kStageRecurrent, st);
-  rc = launch_kernel(pkda_recurrent_carry_kernel<D>, units, D < 32 ? 32 : D, 0, st, bp);
+  // (An ordinary launch: the reduction that runs beside the closing pass reads the partial sums without a wait of its own, so the
+  // pass that leaves them has to have ended in front of a launch in between.)
+  rc = launch_kernel(false, pkda_recurrent_carry_kernel<D>, units, D < 32 ? 32 : D, 0, st, bp);
   end_stage(st);
   if (rc != PKDA_OK) return rc;
   begin_stage(kStageRecurrent, st);

@@ -1,0 +1,94 @@
+"""A kernel that runs beside the one in front of it reads what earlier kernels left before it has waited for anything.
+Only an ordinary (not programmatic) launch between the two makes that complete and visible, so every such reader has one
+behind its last writer.  Shown on the captured launches: a programmatic launch is a programmatic edge of the graph."""
+
+import pytest
+import torch
+
+from delta_feedback_experiment_b200 import chunk_precond_kda
+from delta_feedback_experiment_b200.synthetic import INPUT_NAMES, make_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+def captured_launches(fn):
+    """``(kernel name, starts early, grid.x)`` of everything that ``fn`` launches, in stream order; copies and fills have no name."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1:]
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    nodes = ok(driver.cuGraphGetNodes(raw, ok(driver.cuGraphGetNodes(raw, 0))[1]))[0]
+    n_edges = ok(driver.cuGraphGetEdges_v2(raw, 0))[3]
+    src, dst, data = ok(driver.cuGraphGetEdges_v2(raw, n_edges))[:3]
+    follows, early = {int(a): int(b) for a, b in zip(src, dst)}, {}
+    for b, e in zip(dst, data):
+        early[int(b)] = e.type == int(driver.CUgraphDependencyType.CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC)
+    by_id = {int(x): x for x in nodes}
+    at = next(i for i in by_id if i not in early)
+    launches = []
+    while at is not None:
+        name, grid = "", 0
+        if ok(driver.cuGraphNodeGetType(by_id[at]))[0] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ok(driver.cuGraphKernelNodeGetParams(by_id[at]))[0]
+            raw_name = driver.cuFuncGetName(params.func) if int(params.func) else driver.cuKernelGetName(params.kern)
+            name, grid = ok(raw_name)[0].decode(), params.gridDimX
+        launches.append((name, early.get(at, False), grid))
+        at = follows.get(at)
+    assert len(launches) == len(by_id)  # one stream, one chain
+    return launches
+
+
+def _exact(d):
+    x = {n: d[n].detach().requires_grad_(True) for n in INPUT_NAMES}
+    o, _, _ = chunk_precond_kda(**x)
+    return torch.autograd.grad(o, list(x.values()), d["do"])
+
+
+def _lean(d):
+    x = {n: d[n].detach().requires_grad_(True) for n in INPUT_NAMES}
+    o, _, _ = chunk_precond_kda(**x, disable_recompute=False)
+    return torch.autograd.grad(o, list(x.values()), d["do"])
+
+
+def _inputs(step, seed=1):
+    if step is _exact:
+        d = make_inputs(2, 200, 4, 64, seed=seed, dist="unit", dtype=torch.float32)
+    else:
+        d = make_inputs(2, 200, 4, 128, seed=seed, dist="production", dtype=torch.bfloat16)
+    return {n: t.cuda() for n, t in d.items() if torch.is_tensor(t)}
+
+
+@pytest.mark.parametrize("step,writer,reader", [(_exact, "pkda_recurrent_grad_kernel", "pkda_recurrent_bwd_reduce_kernel"),
+                                                (_lean, "pkda_intra_fwd_tc_kernel", "pkda_scan_bwd"),
+                                                (_lean, "pkda_scan_bwd", "pkda_intra_bwd_kernel"),
+                                                (_lean, "pkda_intra_bwd_kernel", "pkda_param_reduce_kernel")])
+def test_an_ordinary_launch_stands_between_writer_and_reader(step, writer, reader):
+    d = _inputs(step)
+    step(d)
+    torch.cuda.synchronize()
+    launches = captured_launches(lambda: step(d))
+    names = [name for name, _, _ in launches]
+    r = next(i for i, name in enumerate(names) if reader in name)
+    w = max(i for i, name in enumerate(names[:r]) if writer in name)
+    assert launches[r][1]
+    assert any(not early for _, early, _ in launches[w + 1:r]), names[w:r + 1]
+
+
+def test_exact_backwards_of_changing_inputs_in_a_row():
+    """The partial sums lie where those of the call before lay: no gradient of a parameter may take any of them."""
+    inputs = [_inputs(_exact, seed) for seed in (1, 2)]
+    want = []
+    for d in inputs:
+        want.append(_exact(d))
+        torch.cuda.synchronize()
+    for _ in range(20):
+        got = [_exact(d) for d in inputs]
+        for g, w in zip(got, want):
+            for name, a, b in zip(INPUT_NAMES, g, w):
+                assert torch.equal(a, b), name
