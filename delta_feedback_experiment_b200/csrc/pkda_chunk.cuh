@@ -415,12 +415,14 @@ int run_prologue(const pkda_problem& p, int* chunk_offsets, float* beta_c, Geo* 
 // o / o_done: the forward's output tensor; *o_done says whether the state scan has already written it.
 // What the tensor-memory intra kernel needs to carry the preconditioner state across chunks itself
 // (dense batches; NULL: it does not): see IntraParams::chain.
+// scan_split: CTAs per unit of a recompute pass's scan beside which the backward's runs (ScanPair::fwd), 0 where it runs alone.
 struct ChainArgs {
   float *beta_c_w, *a_chain, *sa, *AT;
 };
 int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_c, bf16* u_ws, bf16* Aqk,
                        bf16* Akk, bf16* kt, float* gc, const float* a_start, bf16* w, bf16* kg, bf16* v_new,
                        bf16* h, bf16* qg, float* ST, bool recompute, int* status, int* cursor,
-                       cudaStream_t st, bf16* o = nullptr, bool* o_done = nullptr, const ChainArgs* chain = nullptr);
+                       cudaStream_t st, bf16* o = nullptr, bool* o_done = nullptr, const ChainArgs* chain = nullptr,
+                       int scan_split = 0);
 
 }  // namespace pkda

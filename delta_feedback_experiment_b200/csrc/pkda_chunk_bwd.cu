@@ -1544,11 +1544,16 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
                              static_cast<const bf16*>(p.beta), ws.beta_c, st);
     if (rc != PKDA_OK) return rc;
   }
+  const int units = p.n_seqs * p.heads;
+  // The older mma.sync scans run only when they are pinned (pkda_set_variant).
+  const bool scan_mma = stage_variant(kStageScanBwd) == 1;
+  // The recompute pass ends with its scan, which leaves h and v_new; the reverse scan reads neither, so the two run side by side.
+  const ScanPair pair = a->recompute && !scan_mma && stage_variant(kStageScanFwd) != 1 ? scan_pair(units) : ScanPair{0, 0};
   if (a->recompute) {
     // The recompute kernels only read the products, write keys and decay totals.
     rc = run_forward_stages(p, geo, ws.beta_c, ws.u, const_cast<bf16*>(Aqk), const_cast<bf16*>(Akk),
                             const_cast<bf16*>(kt), const_cast<float*>(gc), a->a_atk, w, kg, v_new, h, qg,
-                            nullptr, true, ws.status, ws.fwd_cursor, st);
+                            nullptr, true, ws.status, ws.fwd_cursor, st, nullptr, nullptr, nullptr, pair.fwd);
     if (rc != PKDA_OK) return rc;
   }
 
@@ -1557,13 +1562,9 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   sp.beta_c = ws.beta_c; sp.gc = gc; sp.dST = a->d_final_state; sp.dh = ws.dh; sp.dF = ws.dF;
   sp.dS0 = a->d_initial_state;
   {
-    const int units = p.n_seqs * p.heads;
     const int vb = units >= 120 ? 128 : (units >= 60 ? 64 : 32);  // value columns per CTA of the mma.sync kernel
-    // Columns over four or eight SMs for few units, else tcgen05 / TMEM / TMA, as in the forward; the older
-    // mma.sync kernel runs only when it is pinned (pkda_set_variant).
-    const bool scan_mma = stage_variant(kStageScanBwd) == 1;
-    // The recompute pass has just launched its scan, which leaves h and v_new; this one reads neither, so it runs beside it.
-    const ScanPair pair = a->recompute && stage_variant(kStageScanFwd) != 1 ? scan_pair(units) : ScanPair{0, 0};
+    // Columns over eight, four or (beside the recompute pass's scan) two SMs for few units, else tcgen05 / TMEM / TMA, as
+    // in the forward.
     begin_stage(kStageScanBwd, st);
     if (!scan_mma && scan_columns(units))
       rc = launch_scan_bwd_cols(geo, p.total_tokens, units, kg, w, qg, sp.d_o, Aqk, ws.beta_c, gc, a->d_final_state, ws.dh,

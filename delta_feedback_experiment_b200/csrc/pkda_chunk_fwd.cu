@@ -504,7 +504,7 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
                        bf16* Aqk, bf16* Akk, bf16* kt, float* gc, const float* a_start,
                        bf16* w, bf16* kg, bf16* v_new, bf16* h, bf16* qg, float* ST,
                        bool recompute, int* status, int* cursor, cudaStream_t st, bf16* o,
-                       bool* o_done, const ChainArgs* chain) {
+                       bool* o_done, const ChainArgs* chain, int scan_split) {
   IntraParams ip;
   ip.geo = geo;
   ip.q = static_cast<const bf16*>(p.q); ip.k = static_cast<const bf16*>(p.k);
@@ -533,8 +533,9 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   ScanParams sp;
   sp.geo = geo; sp.w = w; sp.u = u_ws; sp.kg = kg; sp.beta_c = beta_c; sp.gc = gc;
   sp.S0 = p.initial_state; sp.h = h; sp.v_new = v_new; sp.ST = ST;
-  // Few units (scan_columns: while four or eight CTAs per unit run in one wave): the value columns of a unit
-  // spread over that many SMs, with the state in mma.sync accumulators.  More units: tcgen05 / TMEM / TMA,
+  // Few units (scan_columns: while four or eight CTAs per unit run in one wave; scan_split of them, two at least, where the
+  // backward's scan runs beside this one): the value columns of a unit spread over that many SMs, with the state in
+  // mma.sync accumulators.  More units: tcgen05 / TMEM / TMA,
   // one CTA per (sequence, head).  The older mma.sync kernel, which slices the value columns when there are
   // fewer units than SMs, runs only when it is pinned (pkda_set_variant).  Same bits from the first two.
   const int units = p.n_seqs * p.heads;
@@ -548,7 +549,7 @@ int run_forward_stages(const pkda_problem& p, const Geo& geo, const float* beta_
   if (status && !scan_mma && scan_columns(units)) {
     rc = launch_scan_fwd_cols(geo, p.total_tokens, units, w, kg, u_ws, beta_c, gc, p.initial_state, h, v_new,
                               recompute ? nullptr : ST, status, qg, Aqk, fuse_out ? o : nullptr,
-                            recompute && scan_pair(units).fwd ? scan_pair(units).fwd : scan_columns(units), st);
+                              scan_split ? scan_split : scan_columns(units), st);
     if (o_done) *o_done = fuse_out;
   } else if (status && !scan_mma) {
     rc = launch_scan_fwd_tc(geo, p.total_tokens, units, w, kg, u_ws, beta_c, gc, p.initial_state, h, v_new, ST,

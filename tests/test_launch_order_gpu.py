@@ -5,7 +5,7 @@ behind its last writer.  Shown on the captured launches: a programmatic launch i
 import pytest
 import torch
 
-from delta_feedback_experiment_b200 import chunk_precond_kda
+from delta_feedback_experiment_b200 import _lib, chunk_precond_kda
 from delta_feedback_experiment_b200.synthetic import INPUT_NAMES, make_inputs
 
 pytestmark = pytest.mark.gpu
@@ -56,11 +56,11 @@ def _lean(d):
     return torch.autograd.grad(o, list(x.values()), d["do"])
 
 
-def _inputs(step, seed=1):
+def _inputs(step, seed=1, H=4):
     if step is _exact:
-        d = make_inputs(2, 200, 4, 64, seed=seed, dist="unit", dtype=torch.float32)
+        d = make_inputs(2, 200, H, 64, seed=seed, dist="unit", dtype=torch.float32)
     else:
-        d = make_inputs(2, 200, 4, 128, seed=seed, dist="production", dtype=torch.bfloat16)
+        d = make_inputs(2, 200, H, 128, seed=seed, dist="production", dtype=torch.bfloat16)
     return {n: t.cuda() for n, t in d.items() if torch.is_tensor(t)}
 
 
@@ -92,3 +92,21 @@ def test_exact_backwards_of_changing_inputs_in_a_row():
         for g, w in zip(got, want):
             for name, a, b in zip(INPUT_NAMES, g, w):
                 assert torch.equal(a, b), name
+
+
+@pytest.mark.parametrize("pinned", [(), ("scan_fwd",), ("scan_bwd",)])
+def test_a_scan_with_nothing_beside_it_takes_all_its_columns(pinned):
+    """16 units: four CTAs each for the recompute pass's scan where the reverse scan runs beside it, else eight (the pinned
+    mma.sync scan: four of 32 value columns)."""
+    d = _inputs(_lean, H=8)
+    for stage in pinned:
+        _lib.set_variant(stage, True)
+    try:
+        _lean(d)
+        torch.cuda.synchronize()
+        launches = captured_launches(lambda: _lean(d))
+    finally:
+        for stage in pinned:
+            _lib.set_variant(stage, False)
+    scans = [(early, grid) for name, early, grid in launches if "scan_fwd" in name]
+    assert [grid for _, grid in scans] == {(): [128, 64], ("scan_fwd",): [64, 64], ("scan_bwd",): [128, 128]}[pinned]
