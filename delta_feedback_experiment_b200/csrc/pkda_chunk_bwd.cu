@@ -1547,8 +1547,11 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   const int units = p.n_seqs * p.heads;
   // The older mma.sync scans run only when they are pinned (pkda_set_variant).
   const bool scan_mma = stage_variant(kStageScanBwd) == 1;
-  // The recompute pass ends with its scan, which leaves h and v_new; the reverse scan reads neither, so the two run side by side.
-  const ScanPair pair = a->recompute && !scan_mma && stage_variant(kStageScanFwd) != 1 ? scan_pair(units) : ScanPair{0, 0};
+  // The recompute pass ends with its scan, which leaves h and v_new; the reverse scan reads neither, so the two run side by side,
+  // unless the caller lets the state's gradient take the place of the state, which the first one still reads.
+  const uintptr_t S0 = reinterpret_cast<uintptr_t>(p.initial_state), dS0 = reinterpret_cast<uintptr_t>(a->d_initial_state);
+  const bool in_place = S0 && dS0 && (S0 < dS0 ? dS0 - S0 : S0 - dS0) < (size_t)units * kD * kD * sizeof(float);
+  const ScanPair pair = a->recompute && !in_place && !scan_mma && stage_variant(kStageScanFwd) != 1 ? scan_pair(units) : ScanPair{0, 0};
   if (a->recompute) {
     // The recompute kernels only read the products, write keys and decay totals.
     rc = run_forward_stages(p, geo, ws.beta_c, ws.u, const_cast<bf16*>(Aqk), const_cast<bf16*>(Akk),

@@ -228,7 +228,7 @@ typedef struct pkda_chunk_bwd_args {
   void* dq; void* dk; void* dv; void* dg;
   float* dg_atk; void* dbeta_atk; void* dbeta;
   float* dA_log; float* ddt_bias; float* dlog_atk_scale;
-  float* d_initial_state;    /* [N][H][D][D] or NULL */
+  float* d_initial_state;    /* [N][H][D][D] or NULL; may overlap p.initial_state (which a lean call then scans alone) */
   float* d_initial_A_state;  /* [N][H][D] or NULL */
   void* workspace; size_t workspace_bytes;
 } pkda_chunk_bwd_args;
