@@ -2,6 +2,8 @@
 Only an ordinary (not programmatic) launch between the two makes that complete and visible, so every such reader has one
 behind its last writer.  Shown on the captured launches: a programmatic launch is a programmatic edge of the graph."""
 
+from typing import NamedTuple
+
 import pytest
 import torch
 
@@ -11,8 +13,15 @@ from delta_feedback_experiment_b200.synthetic import INPUT_NAMES, make_inputs
 pytestmark = pytest.mark.gpu
 
 
+class Launch(NamedTuple):
+    name: str     # of the kernel, mangled; copies and fills have none
+    early: bool   # a programmatic launch
+    grid: int     # CTAs along x
+    threads: int  # of a CTA
+
+
 def captured_launches(fn):
-    """``(kernel name, starts early, grid.x)`` of everything that ``fn`` launches, in stream order; copies and fills have no name."""
+    """Everything that ``fn`` launches, in stream order."""
     from cuda.bindings import driver
 
     def ok(result):
@@ -33,12 +42,12 @@ def captured_launches(fn):
     at = next(i for i in by_id if i not in early)
     launches = []
     while at is not None:
-        name, grid = "", 0
+        name, grid, threads = "", 0, 0
         if ok(driver.cuGraphNodeGetType(by_id[at]))[0] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
             params = ok(driver.cuGraphKernelNodeGetParams(by_id[at]))[0]
             raw_name = driver.cuFuncGetName(params.func) if int(params.func) else driver.cuKernelGetName(params.kern)
-            name, grid = ok(raw_name)[0].decode(), params.gridDimX
-        launches.append((name, early.get(at, False), grid))
+            name, grid, threads = ok(raw_name)[0].decode(), params.gridDimX, params.blockDimX
+        launches.append(Launch(name, early.get(at, False), grid, threads))
         at = follows.get(at)
     assert len(launches) == len(by_id)  # one stream, one chain
     return launches
@@ -73,11 +82,11 @@ def test_an_ordinary_launch_stands_between_writer_and_reader(step, writer, reade
     step(d)
     torch.cuda.synchronize()
     launches = captured_launches(lambda: step(d))
-    names = [name for name, _, _ in launches]
+    names = [x.name for x in launches]
     r = next(i for i, name in enumerate(names) if reader in name)
     w = max(i for i, name in enumerate(names[:r]) if writer in name)
-    assert launches[r][1]
-    assert any(not early for _, early, _ in launches[w + 1:r]), names[w:r + 1]
+    assert launches[r].early
+    assert any(not x.early for x in launches[w + 1:r]), names[w:r + 1]
 
 
 def test_exact_backwards_of_changing_inputs_in_a_row():
@@ -108,5 +117,12 @@ def test_a_scan_with_nothing_beside_it_takes_all_its_columns(pinned):
     finally:
         for stage in pinned:
             _lib.set_variant(stage, False)
-    scans = [(early, grid) for name, early, grid in launches if "scan_fwd" in name]
-    assert [grid for _, grid in scans] == {(): [128, 64], ("scan_fwd",): [64, 64], ("scan_bwd",): [128, 128]}[pinned]
+    assert [x.grid for x in launches if "scan_fwd" in x.name] == {(): [128, 64], ("scan_fwd",): [64, 64], ("scan_bwd",): [128, 128]}[pinned]
+
+
+def test_the_exact_reverse_scan_is_placed_when_the_forward_has_ended():
+    """Its CTAs are a long chain each and fill their SM: they must not be laid beside one another while others stay idle."""
+    d = _inputs(_exact)
+    _exact(d)
+    torch.cuda.synchronize()
+    assert [x.early for x in captured_launches(lambda: _exact(d)) if "dscan" in x.name] == [False]

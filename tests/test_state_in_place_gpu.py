@@ -78,6 +78,6 @@ def test_scans_of_overlapping_states_run_alone():
         a, _, keep = _call(d, dS, torch.zeros(2 * n, device="cuda"), shift)
         _backward(a)
         torch.cuda.synchronize()
-        scans = [g for name, _, g in captured_launches(lambda: _backward(a)) if "pkda_scan_" in name]
+        scans = [x.grid for x in captured_launches(lambda: _backward(a)) if "pkda_scan_" in x.name]
         assert scans == [grid, grid], shift
         del keep
