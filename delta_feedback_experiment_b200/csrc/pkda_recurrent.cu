@@ -40,7 +40,7 @@ struct RecParams {
   float scale, ln_x, eps;
 };
 
-template <int D, int kCPL, typename T, bool kSave>
+template <int D, int kCPL, typename T, bool kSave, bool kTwoAhead>
 __global__ void __launch_bounds__(ScanLay<D, kCPL>::kProd + 32 * ScanLay<D, kCPL>::kMaxConsumers)
 pkda_recurrent_kernel(const RecParams p) {
   after_previous();
@@ -189,7 +189,7 @@ pkda_recurrent_kernel(const RecParams p) {
   T* const o_row = static_cast<T*>(p.o) + tbase;
   // The vectors of a token, and its value (kTwoAhead).
   struct Rows { float2 kx[R / 2], al[R / 2], wk[R / 2], qs[R / 2]; float v; };
-  Rows ahead[L::kTwoAhead ? 2 : 1];
+  Rows ahead[kTwoAhead ? 2 : 1];
   auto load_token = [&](Rows& x, uint32_t vec) {
     load_rows<L>(vec, rg, x.kx);
     load_rows<L>(vec + 4 * D, rg, x.al);
@@ -197,16 +197,16 @@ pkda_recurrent_kernel(const RecParams p) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x.v) : "r"(vec + 16 * D + 4 * col0));
     load_rows<L>(vec + 12 * D, rg, x.qs);
   };
-  if (L::kTwoAhead && nblk > 0) {
+  if (kTwoAhead && nblk > 0) {
     bar_sync_n(1, nthreads);
     load_token(ahead[0], smem_u32(stage));
-    load_token(ahead[L::kTwoAhead], smem_u32(stage) + 4 * VEC);
+    load_token(ahead[kTwoAhead], smem_u32(stage) + 4 * VEC);
   }
   for (int b = 0; b < nblk; ++b) {
     const int s = b & 1, t0 = b * TB;
     if (kSave && (t0 & (kCkpt - 1)) == 0)
       store_state(p.save.S + ((ckpt_base(p.geo, n, sq.bos) + t0 / kCkpt) * H + h) * (size_t)(D * D) + col0);
-    if (!L::kTwoAhead) bar_sync_n(1 + s, nthreads);
+    if (!kTwoAhead) bar_sync_n(1 + s, nthreads);
     const uint32_t st = smem_u32(stage + s * L::kStage);
     float oacc[L::kTO * kCPL], ekeep[L::kSums];  // [token][column]
     // Two vectors of rows are held at a time.  x: exp(g) k, then exp(g) of a token; y: beta kw, then scale q.
@@ -230,7 +230,7 @@ pkda_recurrent_kernel(const RecParams p) {
         if (to < sq.len) o_row[(size_t)to * tstep + n % kCPL] = from_f<T>(oacc[i]);
       }
     };
-    if constexpr (L::kTwoAhead) {
+    if constexpr (kTwoAhead) {
       const uint32_t nx = smem_u32(stage + (s ^ 1) * L::kStage);
 #pragma unroll
       for (int t = 0; t < TB; ++t) {
@@ -449,13 +449,14 @@ pkda_recurrent_few_kernel(const RecParams p) {
 template <int D, int kCPL, typename T, bool kSave>
 static int launch_rec(RecParams rp, cudaStream_t st) {
   using L = ScanLay<D, kCPL>;
-  auto kernel = pkda_recurrent_kernel<D, kCPL, T, kSave>;
   const int units = rp.geo.n_seqs * rp.geo.heads;
   int nw = scan_consumers(units, L::kWarps, L::kMaxConsumers, sm_count());
   if (rp.inplace_A)  // the unit's CTAs form one cluster: at most eight of them
     while (L::kWarps / nw > 8) nw *= 2;
   rp.groups = L::kWarps / nw;
   if (rp.groups == 1) rp.inplace_A = 0;
+  constexpr int kMost = kCPL == 1 ? two_ahead_forward<D>() : 0;
+  auto kernel = nw <= kMost ? pkda_recurrent_kernel<D, kCPL, T, kSave, (kMost > 0)> : pkda_recurrent_kernel<D, kCPL, T, kSave, false>;
   rp.warps = {nw, nw == 1 && !rp.inplace_A};  // (every thread takes part in the cluster's barrier)
   if (!ensure_dynamic_smem(kernel, L::kSmem)) return PKDA_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};

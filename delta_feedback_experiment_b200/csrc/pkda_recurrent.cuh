@@ -39,12 +39,6 @@ template <int D, int kCPL_> struct ScanLay {
   static constexpr int kProdPerGroup = D < 32 ? 32 : D;
   static constexpr int kProd = kGroups * kProdPerGroup;
   static constexpr int kMaxConsumers = 8;             // consumer warps per CTA, at most
-  // Row vectors of two tokens in registers, those of a token asked for two tokens ahead: the loads of a token are 32 cycles of the
-  // warp's way to shared memory per vector at 64 rows, and shuffles queue behind them.  (With the other vectors of a token asked for
-  // while its sum is formed, a token of the state cotangent takes 223 cycles at 64 rows, 150 at 32, so 161 and 135; at 128 rows
-  // a lane has 16 rows and the registers are not there: 232 and 248.  2 x 512 tokens of 4 heads x 64, forward and backward: 188 -> 182 us;
-  // 2 x 824 of 8 x 32: 268 -> 238.)
-  static constexpr bool kTwoAhead = kCPL_ == 1 && kR <= 8;
   static constexpr int kVecs = 5;                     // row vectors per token
   static constexpr int kStage = kTB * kVecs * D;      // floats of one staged block
   static constexpr int kSmem = 2 * kStage * 4;
@@ -136,6 +130,18 @@ __device__ __forceinline__ void rg_sum_transposed(float (&x)[kN], int rg) {
 #pragma unroll
   for (int o = kRG / 2; o >= 1; o >>= 1) rg_sum_round(x, rg, o, n >>= 1);
 }
+
+// A scan may hold the row vectors of two tokens in registers and ask for a token's two tokens ahead: the loads of a token are 32
+// cycles of the warp's way to shared memory per vector at 64 rows, and shuffles queue behind them.  It pays only where a chain warp
+// has (nearly) a scheduler to itself, and the registers cost an SM its second CTA.  The most chain warps of a CTA with which it is
+// done (0: never); 512 tokens, us, one token ahead -> two:
+//   forward, 64 rows: 1 warp (8 units) 69 -> 64, leaving what the backward needs 74 -> 68; 2 (16 units) 72 -> 76; 8 (40 units)
+//   110 -> 119; beyond 148 units, leaving it, 345 -> 374.  32 rows: 1 warp 57 -> 55; 4 (40 units) 57 -> 61; 150 units 125 -> 162.
+//   state cotangent, 64 rows: 1, 2, 4 warps 71 -> 57, 76 -> 62, 82 -> 77; 8 106 -> 112, beyond 148 units 291 -> 333.  32 rows: up to
+//   2 warps no difference, 4 53 -> 56, 8 66 -> 75.
+// (8 and 16 rows: 3 to 10 % slower everywhere.  At 128 rows a lane has 16 of them and the registers are not there.)
+template <int D> constexpr int two_ahead_forward() { return D == 32 || D == 64 ? 1 : 0; }
+template <int D> constexpr int two_ahead_reverse() { return D == 64 ? 4 : 0; }
 
 // Where the warps of a scan CTA stand.  A warp's scheduler is its index modulo 4: a lone chain warp has one to itself, the producers'
 // warps lie on the other three (every fourth index stays empty).  With what stands between the shuffles of a token: 2 x 4 units,

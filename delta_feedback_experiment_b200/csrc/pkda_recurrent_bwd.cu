@@ -47,7 +47,7 @@ struct RecBwdParams {
 
 // ---------------------------------------------------------------- state cotangent, last token first
 // The mirror image of the forward scan: same column slices, same producer / consumer split.
-template <int D, typename T>
+template <int D, typename T, bool kTwoAhead>
 __global__ void __launch_bounds__(ScanLay<D, 1>::kProd + 32 * ScanLay<D, 1>::kMaxConsumers)
 pkda_recurrent_dscan_kernel(const RecBwdParams p) {
   after_previous();
@@ -146,7 +146,7 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
   T* dv = static_cast<T*>(p.dv);
   const size_t tbase = ((size_t)sq.bos * H + h) * D + col0;
   struct Rows { float2 qs[R / 2], w[R / 2], nk[R / 2], al[R / 2]; float dot; };  // the vectors of a token, and its dO (kTwoAhead)
-  Rows ahead[L::kTwoAhead ? 2 : 1];
+  Rows ahead[kTwoAhead ? 2 : 1];
   auto load_token = [&](Rows& x, uint32_t vec) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x.dot) : "r"(vec + 16 * D + 4 * col0));
     load_rows<L>(vec, rg, x.qs);
@@ -154,9 +154,9 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
     load_rows<L>(vec + 8 * D, rg, x.nk);
     load_rows<L>(vec + 12 * D, rg, x.al);
   };
-  if (L::kTwoAhead && nblk > 0) {
+  if (kTwoAhead && nblk > 0) {
     bar_sync_n(1, nthreads);
-    load_token(ahead[L::kTwoAhead], smem_u32(stage) + 4 * (TB - 1) * VEC);
+    load_token(ahead[kTwoAhead], smem_u32(stage) + 4 * (TB - 1) * VEC);
     load_token(ahead[0], smem_u32(stage) + 4 * (TB - 2) * VEC);
   }
   for (int it = 0; it < nblk; ++it) {
@@ -164,9 +164,9 @@ pkda_recurrent_dscan_kernel(const RecBwdParams p) {
     float keep[L::kSums];
     if (it == 0 || ((t0 + TB) & (kCkpt - 1)) == 0)
       store_state(p.dSck + ((ckpt_base(p.geo, n, sq.bos) + t0 / kCkpt) * H + h) * (size_t)(D * D) + col0);
-    if (!L::kTwoAhead) bar_sync_n(1 + s, nthreads);
+    if (!kTwoAhead) bar_sync_n(1 + s, nthreads);
     const uint32_t st = smem_u32(stage + s * L::kStage);
-    if constexpr (L::kTwoAhead) {
+    if constexpr (kTwoAhead) {
       const uint32_t nx = smem_u32(stage + (s ^ 1) * L::kStage);
 #pragma unroll
       for (int t = TB - 1; t >= 0; --t) {
@@ -663,13 +663,16 @@ static int launch_rec_bwd(RecBwdParams bp, size_t blocks, cudaStream_t st) {
   const int nw = scan_consumers(units, L::kWarps, L::kMaxConsumers, sm_count());
   bp.warps = {nw, nw == 1};
   bp.groups = L::kWarps / nw;
-  if (!ensure_dynamic_smem(pkda_recurrent_dscan_kernel<D, T>, L::kSmem) ||
+  constexpr int kMost = two_ahead_reverse<D>();
+  auto dscan = nw <= kMost ? pkda_recurrent_dscan_kernel<D, T, (kMost > 0)> : pkda_recurrent_dscan_kernel<D, T, false>;
+  if (!ensure_dynamic_smem(dscan, L::kSmem) ||
       !ensure_dynamic_smem(pkda_recurrent_grad_kernel<D, T>, G::kFloats * 4))
     return PKDA_ERR_LAUNCH;
   begin_stage(kStageRecurrent, st);
-  // (An ordinary launch: set up while the forward's scan still runs, its CTAs come to lie two on an SM beside idle ones.  512 tokens of
-  // 40 units at 64 rows, one token ahead: 188 us against 106; 76 units at 32 rows: 108 against 66.)
-  int rc = launch_kernel(false, pkda_recurrent_dscan_kernel<D, T>, units * bp.groups, bp.warps.threads(L::kProd), L::kSmem, st, bp);
+  // Set up while the forward's scan still runs, its CTAs come to lie two on an SM beside idle ones (512 tokens of 40 units at 64 rows,
+  // one token ahead: 188 us against 106; 76 units at 32 rows: 108 against 66), unless two do not fit: two tokens ahead they do not,
+  // by their registers (exact step of 2 x 512 tokens of 4 heads x 64: 158 us early, 160 behind the forward).
+  int rc = launch_kernel(nw <= kMost, dscan, units * bp.groups, bp.warps.threads(L::kProd), L::kSmem, st, bp);
   end_stage(st);
   if (rc != PKDA_OK) return rc;
   const dim3 grid((unsigned)blocks, (unsigned)H);

@@ -120,9 +120,10 @@ def test_a_scan_with_nothing_beside_it_takes_all_its_columns(pinned):
     assert [x.grid for x in launches if "scan_fwd" in x.name] == {(): [128, 64], ("scan_fwd",): [64, 64], ("scan_bwd",): [128, 128]}[pinned]
 
 
-def test_the_exact_reverse_scan_is_placed_when_the_forward_has_ended():
-    """Its CTAs are a long chain each and fill their SM: they must not be laid beside one another while others stay idle."""
-    d = _inputs(_exact)
+@pytest.mark.parametrize("H,D,early", [(20, 32, False), (4, 64, True), (20, 64, False)])
+def test_the_exact_reverse_scan_is_placed_when_the_forward_has_ended(H, D, early):
+    """Its CTAs are a long chain each: where two fit an SM they must not be laid beside one another while others stay idle."""
+    d = {n: t.cuda() for n, t in make_inputs(2, 200, H, D, seed=1, dist="unit", dtype=torch.float32).items() if torch.is_tensor(t)}
     _exact(d)
     torch.cuda.synchronize()
-    assert [x.early for x in captured_launches(lambda: _exact(d)) if "dscan" in x.name] == [False]
+    assert [x.early for x in captured_launches(lambda: _exact(d)) if "dscan" in x.name] == [early]
