@@ -457,7 +457,7 @@ static int launch_rec(RecParams rp, cudaStream_t st) {
   if (rp.groups == 1) rp.inplace_A = 0;
   constexpr int kMost = kCPL == 1 ? two_ahead_forward<D>() : 0;
   auto kernel = nw <= kMost ? pkda_recurrent_kernel<D, kCPL, T, kSave, (kMost > 0)> : pkda_recurrent_kernel<D, kCPL, T, kSave, false>;
-  rp.warps = {nw, nw == 1 && !rp.inplace_A};  // (every thread takes part in the cluster's barrier)
+  rp.warps = {nw, spread_producers(nw, units * rp.groups, sm_count()) && !rp.inplace_A};  // (every thread takes part in the cluster's barrier)
   if (!ensure_dynamic_smem(kernel, L::kSmem)) return PKDA_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(units * rp.groups));

@@ -156,6 +156,10 @@ struct ScanWarps {
   __device__ int producer(int warp) const { return spread ? warp - 1 - (warp >> 2) : warp - nw; }
 };
 
+// Only where the CTA has its SM to itself: the empty indexes of several CTAs crowd the other schedulers.  (One chain warp a CTA and more
+// CTAs than SMs is 8 rows: 512 tokens of 300 units, leaving what the backward needs, spread 120 us, one after another 95.)
+inline bool spread_producers(int nw, int ctas, int sms) { return nw == 1 && ctas <= sms; }
+
 // Consumer warps per CTA: as few as possible while all CTAs run in one wave (a short chain wants
 // its own SM), at most kMaxConsumers (the producers of a CTA redo the same row vectors, so with more
 // units than SMs wide CTAs waste less).

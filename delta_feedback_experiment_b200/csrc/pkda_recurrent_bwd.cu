@@ -661,8 +661,8 @@ static int launch_rec_bwd(RecBwdParams bp, size_t blocks, cudaStream_t st) {
   using G = GradLay<D>;
   const int units = bp.geo.n_seqs * bp.geo.heads, H = bp.geo.heads;
   const int nw = scan_consumers(units, L::kWarps, L::kMaxConsumers, sm_count());
-  bp.warps = {nw, nw == 1};
   bp.groups = L::kWarps / nw;
+  bp.warps = {nw, spread_producers(nw, units * bp.groups, sm_count())};
   constexpr int kMost = two_ahead_reverse<D>();
   auto dscan = nw <= kMost ? pkda_recurrent_dscan_kernel<D, T, (kMost > 0)> : pkda_recurrent_dscan_kernel<D, T, false>;
   if (!ensure_dynamic_smem(dscan, L::kSmem) ||

@@ -38,3 +38,16 @@ def test_form_and_bits(D, units, forward, reverse):
     one = lambda pattern: [m.group(1) == "1" for m in (re.search(pattern, x.name) for x in launches) if m]
     assert one(r"recurrent_kernelI.*Lb1ELb([01])EEE") == [forward]
     assert one(r"dscan_kernelI.*Lb([01])EEE") == [reverse]
+
+
+@pytest.mark.parametrize("units,threads", [(148, 192), (149, 160)])
+def test_producers_are_spread_only_on_an_sm_of_their_own(units, threads):
+    """8 rows: one chain warp and four producers' warps a CTA, and an empty one where the producers keep off the chain's scheduler."""
+    d = make_inputs(units, 67, 1, 8, seed=units, dist="unit", dtype=torch.float32)
+    d = {n: t.cuda() for n, t in d.items() if torch.is_tensor(t)}
+    d["dS"] = torch.randn(units, 1, 8, 8, device="cuda") * 0.1
+    for a, b in zip(_step(d), _step(d, 1)):
+        assert torch.equal(a[:1], b)
+    torch.cuda.synchronize()
+    launches = captured_launches(lambda: _step(d))
+    assert [x.threads for x in launches if "recurrent_kernel" in x.name or "dscan_kernel" in x.name] == [threads, threads]
