@@ -54,8 +54,8 @@ __global__ void pkda_status_guard_kernel(const int* status, bf16* out0, bf16* ou
 
 int launch_status_guard(const int* status, void* out0, void* out1, void* out2, size_t n, cudaStream_t st) {
   begin_stage(kStageStatusGuard, st);
-  const int rc = launch_kernel(pkda_status_guard_kernel, 4, 256, 0, st, status, static_cast<bf16*>(out0), static_cast<bf16*>(out1),
-                static_cast<bf16*>(out2), n);
+  const int rc = launch_kernel(pkda_status_guard_kernel, 4, 256, 0, st, status, static_cast<bf16*>(out0),
+                               static_cast<bf16*>(out1), static_cast<bf16*>(out2), n);
   end_stage(st);
   return rc;
 }

@@ -1113,7 +1113,9 @@ __device__ __forceinline__ void intra_bwd_item(const IntraBwdParams& p, const In
 // grid (chunks, heads): one item per CTA; or, with a work list, a few persistent CTAs that walk it.
 __global__ void __launch_bounds__(ib::kThreads, 1)
 pkda_intra_bwd_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdMaps maps) {
-  if (!p.slow_list) wait_prerequisites();  // (with a work list it runs beside the tensor-memory kernel)
+  // With a work list it runs beside the tensor-memory kernel, an ordinary launch behind the classifier and the scans whose results both
+  // read: no launch may come between the two.
+  if (!p.slow_list) wait_prerequisites();
   launch_dependents();
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int4 s_next;  // the item: chunk, head, first token, valid tokens
@@ -1149,6 +1151,7 @@ pkda_intra_bwd_kernel(const IntraBwdParams p, const __grid_constant__ IntraBwdMa
   wait_prerequisites();
 }
 
+// ------------------------------------------------------------------ preconditioner backward
 struct AtkBwdParams {
   Geo geo;
   const bf16* k;
@@ -1398,7 +1401,9 @@ constexpr int kReduceSubs = 8;
 __global__ void __launch_bounds__(kD * kReduceSubs)
 pkda_param_reduce_kernel(Geo geo, const float* partA, const float* partB, const float* partC, float* dA_log,
                          float* ddt_bias, float* dcentre, const int* status, bf16* g0, bf16* g1, bf16* g2, size_t guard_n) {
-  launch_dependents();  // (it runs beside the pass in front of it)
+  // It runs beside the pass in front of it, and the carry in front of that is an ordinary launch behind the kernels that leave the
+  // partial sums: no launch may come between those two.
+  launch_dependents();
   __shared__ float sSub[kReduceSubs][kD];
   __shared__ float sR[2][4];
   const int h = blockIdx.x, H = geo.heads, tid = threadIdx.x, c = tid % kD, sub = tid / kD;
@@ -1547,8 +1552,8 @@ int chunk_bwd(const pkda_chunk_bwd_args* a, cudaStream_t st) {
   const int units = p.n_seqs * p.heads;
   // The older mma.sync scans run only when they are pinned (pkda_set_variant).
   const bool scan_mma = stage_variant(kStageScanBwd) == 1;
-  // The recompute pass ends with its scan, which leaves h and v_new; the reverse scan reads neither, so the two run side by side,
-  // unless the caller lets the state's gradient take the place of the state, which the first one still reads.
+  // The recompute pass ends with its scan, an ordinary launch, which leaves h and v_new; the reverse scan, the very next launch, reads
+  // neither, so the two run side by side, unless the caller lets the state's gradient take the place of the state, which the first one still reads.
   const uintptr_t S0 = reinterpret_cast<uintptr_t>(p.initial_state), dS0 = reinterpret_cast<uintptr_t>(a->d_initial_state);
   const bool in_place = S0 && dS0 && (S0 < dS0 ? dS0 - S0 : S0 - dS0) < (size_t)units * kD * kD * sizeof(float);
   const ScanPair pair = a->recompute && !in_place && !scan_mma && stage_variant(kStageScanFwd) != 1 ? scan_pair(units) : ScanPair{0, 0};

@@ -480,12 +480,11 @@ int scan_columns(int units) {
   return 8L * units <= sms ? 8 : 4L * units <= sms ? 4 : 0;
 }
 
-// A scan is a chain of chunk steps that keeps few SMs busy, so two side by side cost little more than the longer one.  Each
-// CTA takes an SM of its own (two do not fit its shared memory), so the rule is the most CTAs a unit with which both run in one wave, the
-// backward's, whose step is the longer, before the forward's.  Lean step (forward + backward, decays of the layer's initialisation), one
-// scan after the other -> side by side, us: 4,096 tokens of 8 units 467 -> 403, 12 547 -> 481, 16 643 -> 584, 24 828 -> 761,
-// 32 978 -> 940, 36 1,057 -> 1,028; 2,048 tokens of 48 units 803 -> 722, 64 950 -> 874; 1,024 of 72 551 -> 510.  From 75 units on
-// the tensor-memory scans fill more than half the chip each.
+// A scan is a chain of chunk steps that keeps few SMs busy, so two side by side cost little more than the longer one.  Each CTA
+// takes an SM of its own (two do not fit its shared memory), so the rule is the most CTAs a unit with which both run in one wave,
+// the backward's, whose step is the longer, before the forward's.  Lean step, one scan after the other -> side by side, us: 4,096
+// tokens of 8 units 467 -> 403, 16 643 -> 584, 24 828 -> 761, 36 1,057 -> 1,028; 2,048 tokens of 64 units 950 -> 874; 1,024 of 72
+// 551 -> 510.  From 75 units on the tensor-memory scans fill more than half the chip each.
 ScanPair scan_pair(int units) {
   static constexpr ScanPair kPairs[] = {{8, 8}, {4, 8}, {4, 4}, {2, 4}, {2, 2}, {1, 1}};
   for (const ScanPair& s : kPairs)

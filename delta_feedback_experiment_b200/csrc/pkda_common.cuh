@@ -255,12 +255,14 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" :: "n"(N));
 }
 
-// Every kernel is launched so that its CTAs may be set up while the launch in front of it on the stream still runs
-// (launch_kernel): once all CTAs of that launch have called launch_dependents() or have ended.  wait_prerequisites() then waits until
-// that launch has ended and its memory is visible; a kernel calls it before it touches memory, or, where it runs beside the one in
-// front of it because neither needs anything of the other, before it ends.  So when a launch has ended, all before it have.  Calling
-// launch_dependents() after wait_prerequisites() makes a kernel that runs beside find everything in front of both done.  A kernel
-// that allocates tensor memory does so before launch_dependents(): it must not wait for columns that one behind it holds.
+// The CTAs of an early launch (launch_kernel; the others are ordinary launches) may be set up while the launch in front of it on the
+// stream still runs: once all CTAs of that launch have called launch_dependents() or have ended.  wait_prerequisites() then waits until
+// that launch has ended and its memory is visible; launch_dependents() by itself orders nothing.  Every kernel calls the wait before it
+// touches memory, or, where it runs beside the one in front of it because neither needs anything of the other, before it ends.  So when
+// a launch has ended, all before it have.  A kernel that runs beside reads what earlier launches left without a wait of its own: between
+// its last writer and it there has to be an ordinary launch, which starts when everything before it has ended, and the launches from
+// there on call launch_dependents() behind their wait.  (Nothing may be inserted into such a pair that does not keep this.)  A
+// kernel that allocates tensor memory does so before launch_dependents(): it must not wait for columns that one behind it holds.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void after_previous() {

@@ -41,15 +41,16 @@ namespace pkda {
 namespace intratc {
 constexpr int kThreads = 256;
 constexpr int kLdL = 68;                    // row stride of L and T: float4 rows, and conflict-free MMA fragments
-constexpr int oA = 0;                       // 2 blocks [128 rows][64 ch]: rows 0..63 k 2^G (= Kd, the MN-major A of
-                                            // W^T), rows 64..127 q 2^G (together the K-major A of the pair products)
+constexpr int oA = 0;                       // 2 blocks [128 rows][64 ch]: rows 0..63 k 2^G (= Kd, the MN-major B of
+                                            // W = T Kd), rows 64..127 q 2^G (together the K-major A of the pair products)
 constexpr int oY = oA + 32768;              // 2 blocks [64 rows][64 ch]: kt 2^-G (K-major B); + 1 KB so that T fits
-constexpr int oV = oY + 16384 + 1024;       // 2 blocks [64 tok][64 ch]: V (MN-major A of U^T)
-constexpr int oTm = oV + 16384;             // [64 i][64 j] bf16 T (K-major B)
+constexpr int oV = oY + 16384 + 1024;       // 2 blocks [64 tok][64 ch]: V (MN-major B of U = T V)
+constexpr int oTm = oV + 16384;             // [64 i][64 j] bf16 T (K-major A)
 constexpr int oX = oTm + 8192;              // the last quarter of oG; with oP the place U leaves from (W: from oV)
 constexpr int oG = oV;                      // f32 [64][128], while a chunk is paired by strips: kt 2^(z - G), or G; V, T and 8 KB more
 constexpr int oP = oX + 8192;               // [64 i][64 j] bf16 scale * P
-constexpr int oL = oP + 8192;               // f32 [64][68] L; before the products: the scan exchange arrays
+constexpr int oL = oP + 8192;               // f32 [64][68] L; before the products: the scan exchange arrays; when recomputing the
+                                            // write keys, 2 blocks [64 tok][64 ch] by TMA
 constexpr int oBeta = oL + 64 * kLdL * 4;   // f32 [64]
 constexpr int oDiag = oBeta + 256;          // f32 [64] q_i . kt_i
 constexpr int oStep = oDiag + 256;          // f32 [8][128] factors between the strips (pairs_of_strip)
@@ -68,6 +69,7 @@ constexpr int oD0 = oP, oD1 = oP + 512;     // + 1024 w
 constexpr int oT = oY;                      // f32 [64][68]
 constexpr int oY2 = oA + 8192;              // f32 [1280]
 static_assert(oG + 32768 == oP && oBar % 8 == 0, "the decays fill what lies between the write keys and P");
+static_assert(oL % 1024 == 0 && oL + 16384 <= oBeta, "the write keys arrive in swizzled blocks");
 static_assert(oA0 + 512 <= oZin && oZin + 4096 <= oBeta && oT + 64 * kLdL * 4 <= oV && oY2 + 5120 <= oA + 16384, "aliases must fit");
 static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs per SM");
 constexpr uint32_t kCols = 256;             // pair accumulator 0..63; later W 0..127, U 128..255
@@ -580,7 +582,7 @@ pkda_intra_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_
 
   // ---- 3. one pass over the strip: preconditioner states of its rows -> write keys kt = k * B(A_t)
   // (to global memory), kg = kt * decay to the chunk end, the diagonal q_i . kt_i, and the gated operands
-  // in place: Kd = k 2^G (rows 0..63 of the stacked operand, later the operand of W^T), q 2^G (rows
+  // in place: Kd = k 2^G (rows 0..63 of the stacked operand, later an operand of W), q 2^G (rows
   // 64..127), kt 2^-G (into the slots g has left); qg goes to global memory.  The decay to the chunk
   // end is 2^G_last times the 2^-G the operand needs anyway.  Nothing of the strip is needed afterwards.
   // A chunk that is paired by strips leaves its operands as pairs_of_strip or pair_exact reads them.

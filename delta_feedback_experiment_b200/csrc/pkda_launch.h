@@ -52,12 +52,10 @@ inline int launch_code(cudaError_t err) {
   return err == cudaSuccess && pending == cudaSuccess ? PKDA_OK : PKDA_ERR_LAUNCH;
 }
 
-// Launches `kernel` so that it is set up while the launch in front of it still runs.  Every kernel launched by this calls
-// wait_prerequisites() (pkda_common.cuh).
-// early = false: only behind the end of the launch in front.  The large kernels whose CTAs fill an SM's shared memory are better off
-// so (their CTAs would come to lie where room appears first): 1 x 8,191 tokens of 16 heads forward 313 -> 308 us, a lean step of
-// 2 x 4,096 tokens of 12 heads 785 -> 775.  Early: a decoding step of 8 units 6.1 -> 5.3 us, 4 x 48 tokens of 16 heads 26.6 -> 24.9,
-// the norm gate forward + backward at 8 x 4,096 tokens of 16 heads 197 -> 192.5.
+// early: `kernel` is set up while the launch in front of it still runs, and calls wait_prerequisites() (pkda_common.cuh).  Steps of 8
+// units that follow one another 6.1 -> 5.3 us, 4 x 48 tokens of 16 heads 26.6 -> 24.9.
+// Otherwise it starts when that launch has ended: where a kernel behind relies on it, and where CTAs would come to lie where room
+// appears first (those that fill an SM's shared memory: 1 x 8,191 tokens of 16 heads forward 313 -> 308 us).
 // The code has to be passed on: what a launch is refused for is asked for here and nowhere else, and an error that was pending
 // before is taken with it.
 template <typename... P, typename... A>

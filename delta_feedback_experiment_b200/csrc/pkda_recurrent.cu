@@ -12,11 +12,9 @@
 // with one CTA holding the whole state the step crossed three block barriers and two shared-memory reductions.  The row vectors (exp(g), k, beta kw, q) do not depend
 // on S: producer warps make them for 8 tokens at a time, double buffered, while the consumer warps
 // run the chain; the sum for o is off the chain and is reduced for 8 tokens at once.
-// Measured: 4 x 16 units, 48 tokens, D = 128, bf16: 67 -> 27 us; 2 x 4 units, 512 tokens,
-// D = 64, fp32: 548 -> 86 us (90 when it leaves what the backward needs).  Since then, the calls of 48 and (forward and backward) of
-// 512 tokens, us: the output of a token and the decay of the state taken while the next token's sum goes through its shuffles, four columns
-// a lane reduced by three rounds of four shuffles instead of five of one or two, 24.9 -> 23.9 and 190.9 -> 188.1; vectors two tokens ahead
-// (kTwoAhead) 188 -> 182; cheaper producers 23.8 -> 21.7 and 182 -> 161.
+// The output of a token and the decay of the state are taken while the next token's sum goes through its shuffles.
+// Measured, against one CTA with the whole state: 4 x 16 units, 48 tokens, D = 128, bf16: 67 -> 21.7 us; 2 x 4 units, 512
+// tokens, D = 64, fp32: 548 -> 64 us (72 when it leaves what the backward needs).
 #include <type_traits>
 
 #include "pkda_launch.h"

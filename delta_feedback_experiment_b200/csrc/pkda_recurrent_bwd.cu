@@ -15,8 +15,7 @@
 // digits that S - w e^T loses under strong decay).  The preconditioner's cotangent, a diagonal scan
 // backwards over the tokens, and the terms that depend on it close the pass.
 // (One CTA per (sequence, head) that replayed and walked back every token with the whole state took
-// 1655 us for 2 x 4 units of 512 tokens at D = 64, fp32, behind a 551 us forward; these took 110 us, behind 90;
-// with what pkda_recurrent.cu says of the scans and the loads below asked for ahead, all of it takes 156.)
+// 1655 us for 2 x 4 units of 512 tokens at D = 64, fp32, behind a 551 us forward; these take 88 us, behind 72.)
 #include <type_traits>
 
 #include "pkda_launch.h"
@@ -285,7 +284,7 @@ pkda_recurrent_grad_kernel(const RecBwdParams p) {
   after_previous();
   using L = GradLay<D>;
   // The next column group's state and the chain rule's inputs are asked for ahead where the registers are there (up to 64 rows:
-  // 32 checkpoint blocks of 4 heads x 64 33.6 -> 29 us; with the loads of the closing pass together and the last sums beside it, 161 -> 156 us a pass).
+  // 32 checkpoint blocks of 4 heads x 64 33.6 -> 29 us).
   constexpr bool kAhead = D <= 64;
   constexpr int NS = L::kNS, NG = L::kNG, SUB = L::kSub, TPS = L::kTPS;
   extern __shared__ __align__(16) float sm[];

@@ -1,5 +1,5 @@
-// Reverse scan of the state cotangent dS for few units.  Eight, four or (beside a
-// recompute pass's scan) two CTAs per (sequence, head), 16, 32 or 64 value columns each.  Per chunk (last first) and group of 16 columns (transposed, see pkda_scan.cuh):
+// Reverse scan of the state cotangent dS for few units.  Eight, four or (beside a recompute pass's scan) two CTAs per
+// (sequence, head), 16, 32 or 64 value columns each.  Per chunk (last first) and group of 16 columns (transposed, see pkda_scan.cuh):
 //   chain warp    d     = bf16(dS)                      registers, A operand as they stand
 //                 dF^T  = d^T kg^T + dO^T P             64 + 20 mma.sync
 //                 dE    = -beta * bf16(dF)              registers, A operand as they stand

@@ -1,5 +1,6 @@
-// Forward state scan for few units, with the output formed on the way.  Eight, four or (a recompute pass
-// beside the backward's scan) two CTAs per (sequence, head), 16, 32 or 64 value columns each.  Per 64-token chunk and group of 16 columns (transposed, see pkda_scan.cuh):
+// Forward state scan for few units, with the output formed on the way.  Eight, four or (a recompute pass beside the
+// backward's scan) two CTAs per (sequence, head), 16, 32 or 64 value columns each.  Per 64-token chunk and group of 16 columns
+// (transposed, see pkda_scan.cuh):
 //   chain warp    h    = bf16(S)                   registers, A operand as they stand
 //                 S   *= Gam_last (per k)
 //                 E^T  = U^T I - h^T W^T           64 + 8 mma.sync
